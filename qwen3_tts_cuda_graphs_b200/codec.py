@@ -387,6 +387,7 @@ class CodecDecoder:
         o = Op()
         o.m_begin = max(0, min(int(m_begin), M - 1))
         o.kind, o.flags = K_GEMM, flags | (F_OUT_F32 if out_f32 else 0)
+        o.reserved = 1      # weights: nothing in the list writes them
         o.M, o.N, o.K, o.taps, o.cin = M, N, taps * cin, taps, cin
         o.a_rows, o.lda = A.shape[0], A.shape[1]
         o.col_mod = col_mod or N

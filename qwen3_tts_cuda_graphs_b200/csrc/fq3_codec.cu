@@ -25,6 +25,12 @@ std::atomic<int64_t> g_launches{0};
 thread_local int64_t t_launches = 0;
 inline void count_launches(int64_t n) { g_launches += n; t_launches += n; }
 
+// Programmatic dependent launch: a kernel that the host launches with launch_after lets the next launch begin as soon as all its blocks run, and waits
+// itself for the end of everything in front of it before it touches memory.  Without the launch attribute both return at once.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_begin() { grid_dep_launch(); grid_dep_wait(); }
+
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
@@ -379,13 +385,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 // Split-K (splits > 1, short-and-wide problems that would leave most SMs idle): blockIdx.z takes a contiguous range of
 // k-blocks and stores its raw fp32 tile into the workspace [split][M][Nw]; fq3c_splitk_reduce_kernel adds the splits in
 // order and applies the fused epilogue.
-// TMA = true: the operand tiles arrive by cp.async.bulk.tensor — one elected thread asks for the A box (128 rows x 64
-// columns at row m0 + tap offset: rows outside the tensor, i.e. the causal padding, come back as zeros) and the B box (BN x 64) of a
-// k-block and both count their bytes on the stage's `full` mbarrier; SWIZZLE_128B writes exactly the layout described above.  Used
-// whenever a k-block cannot straddle two taps (one tap, or c_in a multiple of 64); the cp.async loaders stay for the rest.
-template <int MINB, bool TMA>  // MINB: CTAs per SM the register budget is planned for: 2 with three stages, 1 with six
-__global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3c_op o, const int BN, const int splits, const int Nw, const int NST,
-                                                                        const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+// This kernel is left for operands that a tensor map does not take (c_in = 8 modulo 16 over several taps); everything else runs on
+// fq3c_gemm_persist_kernel (fq3_gemm.cuh).
+template <int MINB>  // CTAs per SM the register budget is planned for: 2 with three stages, 1 with six
+__global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3c_op o, const int BN, const int splits, const int Nw, const int NST) {
   extern __shared__ unsigned char tsmem_raw[];
   const uint32_t raw = smem_u32(tsmem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // swizzle atoms are 1024-byte aligned
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3
 
   if (tid == 0) {
     for (int s = 0; s < NST; ++s) {
-      mbar_init(full + 8u * s, TMA ? 1 : TLOADERS);
+      mbar_init(full + 8u * s, TLOADERS);
       mbar_init(empty + 8u * s, 1);
     }
     mbar_init(done, 1);
@@ -427,7 +430,7 @@ __global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3
       for (int kt = 0; kt < KT; ++kt) {
         const int st = kt % NST;
         mbar_wait(full + 8u * st, (uint32_t)((kt / NST) & 1));
-        if (!TMA) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async (generic proxy) writes -> tensor core (async proxy) reads
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async (generic proxy) writes -> tensor core (async proxy) reads
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a0 = a_smem + (uint32_t)st * T_A_BYTES, b0 = b_smem + (uint32_t)st * T_B_BYTES;
 #pragma unroll
@@ -451,28 +454,6 @@ __global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3
     // warps 0-3: A rows r0 + 16 i (i < 8), chunk c; warps 4-7: B rows likewise.  Eight lanes cover one 128-byte line of a row.
     const int lt = tid & 127, c = lt & 7, r0 = lt >> 3;
     const bool is_a = warp < 4;
-    if (TMA) {
-      if (tid == 0) {
-        const uint32_t tx = (uint32_t)(T_A_BYTES + BN * TK * 2);
-        for (int kt = 0; kt < KT; ++kt) {
-          const int st = kt % NST;
-          if (kt >= NST) mbar_wait(empty + 8u * st, (uint32_t)(((kt / NST) - 1) & 1));
-          const int k0 = (kt_begin + kt) * TK;
-          const int tap = k0 / o.cin, ci = k0 - tap * o.cin;
-          const int toff = (tap < 8) ? o.tap_off[tap] : 0;
-          const uint32_t fb = full + 8u * st;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(tx) : "memory");
-          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                           a_smem + (uint32_t)st * T_A_BYTES),
-                       "l"(&tmA), "r"(ci), "r"(m0 + toff), "r"(fb)
-                       : "memory");
-          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                           b_smem + (uint32_t)st * T_B_BYTES),
-                       "l"(&tmB), "r"(k0), "r"(n0), "r"(fb)
-                       : "memory");
-        }
-      }
-    } else
     for (int kt = 0; kt < KT; ++kt) {
       const int st = kt % NST;
       if (kt >= NST) {  // one lane per warp polls: 256 spinning threads would swamp the shared-memory pipe the copies need
@@ -578,6 +559,7 @@ __global__ void __launch_bounds__(256) fq3c_splitk_reduce_kernel(const fq3c_op o
 }
 
 __global__ void fq3c_rvq_kernel(const fq3c_op o) {
+  grid_dep_begin();
   const long long* codes = reinterpret_cast<const long long*>(o.A);
   const bf16* cb = reinterpret_cast<const bf16*>(o.B);
   const int Q = o.i1, nsem = o.i0, dim = o.i2, cbsize = o.K;
@@ -608,6 +590,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 __global__ void fq3c_rmsnorm_kernel(const fq3c_op o) {
+  grid_dep_begin();
   __shared__ float red[32];
   const bf16* x = reinterpret_cast<const bf16*>(o.A) + (size_t)blockIdx.x * o.lda;
   bf16* y = reinterpret_cast<bf16*>(o.C) + (size_t)blockIdx.x * o.ldc;
@@ -634,6 +617,7 @@ __device__ __forceinline__ void row_rmsnorm(const fq3c_op& o, int row, float* re
     y[c] = __float2bfloat16_rn(bf16r(bf16r(__bfloat162float(x[c]) * rs) * w[c]));
 }
 __global__ void __launch_bounds__(256) fq3c_rownorm_kernel(const fq3c_op o) {
+  grid_dep_begin();
   __shared__ float red[32];
   row_rmsnorm(o, o.m_begin + blockIdx.x, red);
 }
@@ -658,6 +642,7 @@ __global__ void __launch_bounds__(256) fq3c_splitk_reduce_norm_kernel(const fq3c
 }
 
 __global__ void fq3c_layernorm_kernel(const fq3c_op o) {
+  grid_dep_begin();
   __shared__ float red[32];
   const bf16* x = reinterpret_cast<const bf16*>(o.A) + (size_t)blockIdx.x * o.lda;
   bf16* y = reinterpret_cast<bf16*>(o.C) + (size_t)blockIdx.x * o.ldc;
@@ -675,6 +660,7 @@ __global__ void fq3c_layernorm_kernel(const fq3c_op o) {
 
 // RoPE in place on q and k inside the fused qkv buffer (HF rotate_half convention, bf16 rounding per product).
 __global__ void fq3c_rope_kernel(const fq3c_op o) {
+  grid_dep_begin();
   const int t = blockIdx.x, nheads = o.i0, d = o.i1, col0 = o.i2, half = d / 2;
   const int pos = t + (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0);
   bf16* row = reinterpret_cast<bf16*>(const_cast<void*>(o.A)) + (size_t)t * o.lda + col0;
@@ -791,6 +777,7 @@ __device__ __forceinline__ void attn_warp_generic(const fq3c_op& o, int t_out, i
   }
 }
 __global__ void fq3c_attn_kernel(const fq3c_op o) {
+  grid_dep_begin();
   const int nh = o.i0, T = o.M;
   const int wpb = blockDim.x >> 5;
   const int gw = blockIdx.x * wpb + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -814,6 +801,7 @@ __global__ void fq3c_attn_kernel(const fq3c_op o) {
 // another order, which the prefill tests bound against the oracle and the chunked prefill.  M = 240 (ICL prompt): 78 -> ~12 us per layer.
 constexpr int APF_WARPS = 8;
 __global__ void __launch_bounds__(APF_WARPS * 32) fq3c_attn_prefill_kernel(const fq3c_op o, const int tpad) {
+  grid_dep_begin();
   extern __shared__ unsigned char apf_smem[];
   const int nh = o.i0, nkv = o.i1, T = o.M, win = o.K;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -917,6 +905,7 @@ __global__ void __launch_bounds__(APF_WARPS * 32) fq3c_attn_prefill_kernel(const
 //   k / v heads: the finished row is also written to the static KV cache C (K) / C2 (V), laid out [kv_head][ldc][128].
 // Same arithmetic as head_norm_rope / the KV append of the decode kernel (fq3_kernel.cuh), so decode steps can attend to it.
 __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
+  grid_dep_begin();
   const int nq = o.i0, nkv = o.i1, pos0 = o.i2, nheads = nq + 2 * nkv;
   const int wpb = blockDim.x >> 5;
   const int gw = blockIdx.x * wpb + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -956,6 +945,7 @@ __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
 }
 
 __global__ void fq3c_dwconv_kernel(const fq3c_op o) {
+  grid_dep_begin();
   const size_t n = (size_t)o.M * o.N;
   const bf16* x = reinterpret_cast<const bf16*>(o.A);
   const float* w = reinterpret_cast<const float*>(o.B);
@@ -1021,6 +1011,7 @@ __global__ void fq3c_snake_kernel(const fq3c_op o) {
 }
 
 #include "fq3_seq.cuh"
+#include "fq3_gemm.cuh"
 
 int fail(const std::string& m) { g_err = m; return -1; }
 
@@ -1051,6 +1042,91 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, u
   const cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One launch; `after`: it may begin before the launches in front of it on the stream have ended (its kernel waits for them itself, with
+// griddepcontrol.wait).  cluster: CTAs per cluster.
+template <typename... P, typename... A>
+void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool after, int cluster, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (after) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; ++n; }
+  if (cluster > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; ++n; }
+  cfg.attrs = at; cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// ---- the tcgen05 GEMM: what a launch looks like ------------------------------------------------------------------------------
+constexpr int GP_SMS = 148;
+constexpr int GP_SMEM_MAX = 227 * 1024, GP_SMEM_HALF = 112 * 1024;
+// Whether the epilogue may move whole 32-byte sectors (16 columns of bf16, 8 of f32).
+bool gemm_vec16(const fq3c_op& o) {
+  auto off = [](const void* p, int a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
+  if (o.N % 16 || o.col_mod % 16) return false;
+  if (((o.flags & FQ3C_BIAS) && off(o.bias, 16)) || ((o.flags & FQ3C_SCALE) && off(o.scale, 16))) return false;
+  const bool f32 = (o.flags & FQ3C_OUT_F32) != 0;
+  if (o.flags & FQ3C_SWIGLU) return o.ldc % 8 == 0 && !off(o.C, 32);
+  if (o.ldc % (f32 && !(o.flags & FQ3C_SNAKE2) ? 8 : 16) || off(o.C, 32)) return false;
+  if ((o.flags & FQ3C_RESID) && (o.ldr % 16 || off(o.res, 32))) return false;
+  if ((o.flags & FQ3C_SNAKE2) && (off(o.C2, 32) || off(o.p0, 16) || off(o.p1, 16))) return false;
+  return true;
+}
+struct GemmLaunch { GemmPlan g; bool half; unsigned grid; size_t smem; };
+GemmLaunch gemm_plan(const fq3c_op& o) {
+  GemmLaunch L{};
+  GemmPlan& g = L.g;
+  const int rows = o.M - o.m_begin;
+  g.mt = (rows + TM - 1) / TM;
+  g.a_rows = g.mt == 1 ? (rows + 7) / 8 * 8 : TM;
+  g.kpt = o.taps == 1 ? (o.K + TK - 1) / TK : (o.cin + TK - 1) / TK;
+  g.kb = o.taps == 1 ? g.kpt : g.kpt * o.taps;
+  const int last = (o.taps == 1 ? o.K : o.cin) - (g.kpt - 1) * TK;
+  g.tail = (last + 15) / 16;
+  // Split over K when the tiles would cover less than half of the SMs and the reduction is long (the transformer's o / down projections at 8-240
+  // rows: 16-48 tiles of 32-48 k-blocks): up to eight CTAs per tile, a cluster.  The count must not depend on m_begin: a tail-only decode has to add
+  // the same partial sums in the same order.
+  const int KT = (o.K + TK - 1) / TK;
+  g.splits = 1;
+  if (o.ws && o.M <= 4 * TM && KT >= 8) {
+    const int bn = o.N >= 64 ? 64 : 32;
+    const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
+    const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));
+    if (sp > 1) { g.splits = sp; g.bn = bn; }
+  }
+  long kl = 0, ep = 0;
+  if (g.splits == 1) {
+    // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  Measured: a k-block (four MMAs) takes 427 cycles at 32
+    // columns, 458 at 128, 480 at 224, 512 at 256, or its operand bytes at about 60 a cycle; the epilogue about 20 a column, four times that with sines.
+    long best = -1;
+    const int per_col = (o.flags & FQ3C_SNAKE2) ? 80 : 20;
+    for (int cand = 256; cand >= 16; cand -= 16) {
+      const int nt = (o.N + cand - 1) / cand;
+      const int bn = std::min(256, ((o.N + nt - 1) / nt + 15) / 16 * 16);
+      if (bn != cand && cand != 16) continue;
+      const long tiles = (long)nt * g.mt, waves = (tiles + GP_SMS - 1) / GP_SMS;
+      const long k = (long)g.kb * std::max(420 + bn / 3, (g.a_rows + bn) * 128 / 60), e = (long)bn * per_col;
+      const long cost = waves * std::max(k, e) + std::min(k, e);
+      if (best < 0 || cost < best) { best = cost; g.bn = bn; kl = k; ep = e; }
+    }
+  }
+  g.nt = (o.N + g.bn - 1) / g.bn;
+  g.acc_cols = 32;
+  while (g.acc_cols < g.bn) g.acc_cols *= 2;
+  g.early_b = o.reserved & 1;
+  g.vec16 = gemm_vec16(o) ? 1 : 0;
+  const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = g.splits > 1 ? (g.kb + g.splits - 1) / g.splits : g.kb;
+  // Two CTAs per SM: tiles of one wave keep to half of an SM, so that the next launch's CTAs fit beside them and ask for their weights early; tiles
+  // bound by their epilogue get twice the epilogue warps.
+  L.half = g.acc_cols <= 128 && ((sb * 4 + 2048 <= GP_SMEM_HALF && tiles * g.splits <= 2 * GP_SMS) || (sb * 3 + 2048 <= GP_SMEM_HALF && g.splits == 1 && ep > kl));
+  // The MMA reads 128 rows of A also where the box has fewer: the last stage's are inside the allocation.  A partial tile (at least four k-blocks
+  // per split, 4 x 128 bytes a row against 4 x (bn + 4)) fits in the stages.
+  const int room = (L.half ? GP_SMEM_HALF : GP_SMEM_MAX) - 1024, fit = std::min((room - GP_BAR_BYTES) / sb, (room - T_A_BYTES) / sb + 1);
+  g.stages = std::max(2, std::min(std::min(fit, 16), g.splits > 1 ? n_kb : 16));
+  L.smem = (size_t)std::max(g.stages * sb + GP_BAR_BYTES, (g.stages - 1) * sb + T_A_BYTES) + 1024;
+  L.grid = g.splits > 1 ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, L.half ? 2 * GP_SMS : GP_SMS);
+  return L;
 }
 
 // ---- sequence-model ops: launch logic ---------------------------------------------------------------------------------------
@@ -1602,10 +1678,10 @@ static bool device_attrs_ready() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   if (done[dev]) return true;
-  if (cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, T_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(3)) != cudaSuccess ||
-      cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, T_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(3)) != cudaSuccess ||
+  if (cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, T_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(3)) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_HALF) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, APF_WARPS * (128 + 2048) * 4) != cudaSuccess)
     return false;
   done[dev] = true;
@@ -1639,9 +1715,15 @@ int fq3c_run(const fq3c_op* ops, int n_ops, void* stream) {
 }
 static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, SideStream*& open) {
   cudaStream_t s = main_stream;
+  // FQ3C_PDL=0: every launch waits for the end of the one in front.  Otherwise a kernel that waits for itself may begin early, as long as the launch in
+  // front of it on its stream belongs to this list (what ran before the list is complete when its first launch begins).
+  static const bool pdl = [] { const char* e = getenv("FQ3C_PDL"); return e == nullptr || atoi(e) != 0; }();
+  bool chained = false;
   for (int i = 0; i < n_ops; ++i) {
     const fq3c_op& o = ops[i];
     if (o.M <= 0) continue;
+    const bool after = pdl && chained;
+    chained = o.kind != FQ3C_BRANCH;
     switch (o.kind) {
       case FQ3C_BRANCH: {
         if (o.i0 == 0) {
@@ -1690,6 +1772,20 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         if (use_tc5 && !device_attrs_ready()) return fail("cannot reserve shared memory for the tcgen05 GEMM / prefill attention");
         static int tc5_min_k = -1;
         if (tc5_min_k < 0) { const char* e3 = getenv("FQ3C_TC5_MINK"); tc5_min_k = e3 ? atoi(e3) : TK; }  // one k-block is enough: the vectorised epilogue beats the mma.sync kernel even at K = 96
+        if (use_tc5 && o.N >= 16 && o.K >= tc5_min_k && (o.taps == 1 || o.cin % 16 == 0)) {
+          const GemmLaunch L = gemm_plan(o);
+          CUtensorMap tmA, tmB;
+          if (make_map(&tmA, o.A, (uint64_t)o.cin, (uint64_t)o.a_rows, (uint64_t)o.lda, (uint32_t)L.g.a_rows) &&
+              make_map(&tmB, o.B, (uint64_t)o.K, (uint64_t)o.N, (uint64_t)o.K, (uint32_t)L.g.bn)) {
+            if (L.half) launch_after(fq3c_gemm_persist_kernel<2>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
+            else launch_after(fq3c_gemm_persist_kernel<1>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
+            if (o.norm_out) {
+              launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, pdl, 1, o);
+              count_launches(1);
+            }
+            break;
+          }
+        }
         if (use_tc5 && o.N >= 16 && o.K >= tc5_min_k) {
           // Tile width: a multiple of 16 columns (a legal UMMA N at M = 128), chosen so that the grid covers the SMs.
           // Tall operands (M >= 128) keep BN >= 64 (every column tile re-reads the A rows); short ones (the transformer at
@@ -1728,22 +1824,9 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           static int two_ctas = -1;
           if (two_ctas < 0) { const char* e2 = getenv("FQ3C_TWO_CTAS"); two_ctas = (e2 == nullptr || atoi(e2) != 0) ? 1 : 0; }
           const long n_ctas = (long)grid.x * grid.y * grid.z;
-          // operand tiles by TMA tensor loads where a 64-column k-block stays inside one tap (FQ3C_TMA=0: cp.async loaders everywhere)
-          static int use_tma = -1;
-          if (use_tma < 0) { const char* e4 = getenv("FQ3C_TMA"); use_tma = (e4 == nullptr || atoi(e4) != 0) ? 1 : 0; }
-          CUtensorMap tmA, tmB;
-          memset(&tmA, 0, sizeof tmA); memset(&tmB, 0, sizeof tmB);
-          const bool tma = use_tma && (o.taps == 1 || o.cin % TK == 0) &&
-                           make_map(&tmA, o.A, (uint64_t)o.cin, (uint64_t)o.a_rows, (uint64_t)o.lda, TM) &&
-                           make_map(&tmB, o.B, (uint64_t)o.K, (uint64_t)o.N, (uint64_t)o.K, (uint32_t)bn);
           const bool two = two_ctas && n_ctas >= 2 * 148 && KT <= 24;
-          if (tma) {
-            if (two) fq3c_gemm_tc5_kernel<2, true><<<grid, TTHREADS, t_smem(3), s>>>(o, bn, splits, Nw, 3, tmA, tmB);
-            else fq3c_gemm_tc5_kernel<1, true><<<grid, TTHREADS, T_SMEM, s>>>(o, bn, splits, Nw, TSTAGES, tmA, tmB);
-          } else {
-            if (two) fq3c_gemm_tc5_kernel<2, false><<<grid, TTHREADS, t_smem(3), s>>>(o, bn, splits, Nw, 3, tmA, tmB);
-            else fq3c_gemm_tc5_kernel<1, false><<<grid, TTHREADS, T_SMEM, s>>>(o, bn, splits, Nw, TSTAGES, tmA, tmB);
-          }
+          if (two) fq3c_gemm_tc5_kernel<2><<<grid, TTHREADS, t_smem(3), s>>>(o, bn, splits, Nw, 3);
+          else fq3c_gemm_tc5_kernel<1><<<grid, TTHREADS, T_SMEM, s>>>(o, bn, splits, Nw, TSTAGES);
           if (splits > 1) {
             if (o.norm_out) {
               fq3c_splitk_reduce_norm_kernel<<<(unsigned)(o.M - o.m_begin), 256, 0, s>>>(o, splits, Nw);
@@ -1766,10 +1849,10 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         }
         break;
       }
-      case FQ3C_RVQ: fq3c_rvq_kernel<<<o.M, 128, 0, s>>>(o); break;
-      case FQ3C_RMSNORM: fq3c_rmsnorm_kernel<<<o.M, 256, 0, s>>>(o); break;
-      case FQ3C_LAYERNORM: fq3c_layernorm_kernel<<<o.M, 256, 0, s>>>(o); break;
-      case FQ3C_ROPE: fq3c_rope_kernel<<<o.M, 256, 0, s>>>(o); break;
+      case FQ3C_RVQ: launch_after(fq3c_rvq_kernel, o.M, 128, 0, s, after, 1, o); break;
+      case FQ3C_RMSNORM: launch_after(fq3c_rmsnorm_kernel, o.M, 256, 0, s, after, 1, o); break;
+      case FQ3C_LAYERNORM: launch_after(fq3c_layernorm_kernel, o.M, 256, 0, s, after, 1, o); break;
+      case FQ3C_ROPE: launch_after(fq3c_rope_kernel, o.M, 256, 0, s, after, 1, o); break;
       case FQ3C_ATTN: {
         if (o.i2 > 128) return fail("attn: head_dim > 128");
         static int use_apf = -1;
@@ -1780,22 +1863,22 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           const size_t smem = (size_t)APF_WARPS * 128 * 4 + (size_t)APF_WARPS * tpad * 4;
           if (!device_attrs_ready()) return fail("cannot reserve shared memory for the prefill attention");
           const int warps = o.M * o.i0;
-          fq3c_attn_prefill_kernel<<<(warps + APF_WARPS - 1) / APF_WARPS, APF_WARPS * 32, smem, s>>>(o, tpad);
+          launch_after(fq3c_attn_prefill_kernel, (warps + APF_WARPS - 1) / APF_WARPS, APF_WARPS * 32, smem, s, after, 1, o, tpad);
           break;
         }
         const int warps = o.M * o.i0;
-        fq3c_attn_kernel<<<(warps + 7) / 8, 256, 0, s>>>(o);
+        launch_after(fq3c_attn_kernel, (warps + 7) / 8, 256, 0, s, after, 1, o);
         break;
       }
       case FQ3C_DWCONV: {
         const size_t n = (size_t)o.M * o.N;
-        fq3c_dwconv_kernel<<<(unsigned)std::min<size_t>(2048, (n + 255) / 256), 256, 0, s>>>(o);
+        launch_after(fq3c_dwconv_kernel, (unsigned)std::min<size_t>(2048, (n + 255) / 256), 256, 0, s, after, 1, o);
         break;
       }
       case FQ3C_QKNORM_ROPE_KV: {
         if (o.lda % 4 || !o.C || !o.C2 || !o.p0 || !o.p1 || !o.B || !o.bias) return fail("qknorm_rope_kv: missing operand");
         const int warps = o.M * (o.i0 + 2 * o.i1);
-        fq3c_qknorm_rope_kv_kernel<<<(warps + 7) / 8, 256, 0, s>>>(o);
+        launch_after(fq3c_qknorm_rope_kv_kernel, (warps + 7) / 8, 256, 0, s, after, 1, o);
         break;
       }
       case FQ3C_SNAKE: {

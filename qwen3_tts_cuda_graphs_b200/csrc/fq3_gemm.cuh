@@ -1,0 +1,423 @@
+// fq3_gemm.cuh — the tcgen05 GEMM of the op lists: persistent, warp-specialised, operand tiles by TMA.
+//
+// Included by fq3_codec.cu behind its epilogues.  C = epi(A . B^T), A [rows, K] activations (rows shifted per tap for the implicit
+// convolutions), B [N, K] weights, both bf16, accumulators f32 in tensor memory.
+#pragma once
+
+// What the host decides about a launch.
+struct GemmPlan {
+  int bn;        // columns of a tile (multiple of 16)
+  int stages;    // operand stages in shared memory
+  int a_rows;    // rows of the A box: 128, or what a single row tile needs (multiple of 8; the accumulator rows behind it are never read)
+  int mt, nt;    // row and column tiles
+  int splits;    // CTAs that share a tile's k-blocks: a cluster, its partial tiles meet in shared memory
+  int kpt, kb;   // k-blocks per tap, in all
+  int tail;      // MMAs (16 columns each) of a tap's last k-block
+  int acc_cols;  // tensor-memory columns of one accumulator (power of two); two of them unless splits > 1
+  int early_b;   // B is not written by the launches in front: its first stages are asked for before they have ended
+  int vec16;     // the epilogue may move 16 columns of a row at a time
+};
+constexpr int GP_EPI_WARPS = 8, GP_MMA_WARP = 8, GP_TMA_WARP = 9, GP_THREADS = 320;
+constexpr int GP_BAR_BYTES = 512;   // barriers, tensor-memory address, error word
+__host__ __device__ constexpr int gp_a_bytes(int a_rows) { return (a_rows * TK * 2 + 1023) & ~1023; }
+__host__ __device__ constexpr int gp_stage_bytes(int a_rows, int bn) { return gp_a_bytes(a_rows) + bn * TK * 2; }
+__host__ __device__ constexpr int gp_part_pitch(int bn) { return bn + 4; }   // floats per row of a partial tile: 16-byte rows, 4 banks apart
+
+// A bounded wait of a whole warp.  When the limit (about a second) runs out it sets the error word and `dead`, and this and all later waits of the block
+// return at once: the loops around them keep their counts, so that the compiler sees control flow that is the same for the whole warp (descriptors
+// in uniform registers), and end on whatever is there.
+__device__ __forceinline__ void gp_wait(const uint32_t bar, const uint32_t parity, volatile int* dead) {
+  int i = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if (++i > 256) {      // (a try suspends the thread for a while by itself)
+      if (__any_sync(0xffffffffu, *dead != 0)) return;
+      __nanosleep(i > 8192 ? 1000 : 20);
+      if (i > (1 << 20)) {
+        *dead = 1;
+        seq_wait_error = 1;
+        return;
+      }
+    }
+  }
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void mbar_expect(const uint32_t bar, const uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(const uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void umma_bf16(const uint32_t d, const uint64_t da, const uint64_t db, const uint32_t idesc, const uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// arrives on the barrier when the MMAs issued so far are done (implies tcgen05.fence::before_thread_sync)
+__device__ __forceinline__ void umma_commit(const uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_2d(const uint32_t dst, const CUtensorMap* map, const int x, const int y, const uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(const uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+        "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 32 bytes of a row in one instruction (a whole sector): the rows of a warp are apart, so every store or load of a lane is a sector of its own
+__device__ __forceinline__ void st32(void* p, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+__device__ __forceinline__ void ld32(const void* p, uint32_t (&w)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t bf_pair(const float a, const float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// both rounded to bf16
+__device__ __forceinline__ void round2(float& a, float& b) {
+  const uint32_t w = bf_pair(a, b);
+  a = __uint_as_float(w << 16);
+  b = __uint_as_float(w & 0xffff0000u);
+}
+__device__ __forceinline__ void round16(float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) round2(v[j], v[j + 1]);
+}
+__device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = bf_pair(v[2 * j], v[2 * j + 1]);
+}
+
+// Epilogue of 16 consecutive columns of one row: the arithmetic and order of epilogue_pair, every access a whole 32-byte sector.  The host
+// has checked sizes, pitches and addresses (gemm_vec16).  r: the residual's 16 entries, asked for before the accumulator was read.
+__device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8]) {
+  if (row >= o.M || col >= o.N) return;
+  float v[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc[j]);
+  const int c0 = o.col_mod == o.N ? col : col % o.col_mod;
+  if (o.flags & FQ3C_BIAS) {
+    const float4* b = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.bias) + c0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 q = __ldg(b + j);
+      v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+    }
+  }
+  if (o.flags & FQ3C_RELU2) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
+  }
+  const bool round = !(o.flags & FQ3C_NOROUND);
+  if (round) round16(v);
+  if (o.flags & FQ3C_SWIGLU) {
+    float y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) y[j] = round ? bf16r(bf16r(silu_f(v[2 * j])) * v[2 * j + 1]) : glu_f(o.flags, v[2 * j], v[2 * j + 1]);
+    const size_t at = (size_t)row * o.ldc + (col >> 1);
+    if (!round && (o.flags & FQ3C_OUT_F32)) {
+      uint32_t w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(y[j]);
+      st32(reinterpret_cast<float*>(o.C) + at, w);
+    } else {
+      *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(o.C) + at) = make_uint4(bf_pair(y[0], y[1]), bf_pair(y[2], y[3]), bf_pair(y[4], y[5]), bf_pair(y[6], y[7]));
+    }
+    return;
+  }
+  if (o.flags & FQ3C_GELU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = gelu_f(v[j]);
+    if (round) round16(v);
+  }
+  if (o.flags & FQ3C_SILU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = silu_f(v[j]);
+    round16(v);
+  }
+  if (o.flags & FQ3C_SCALE) {
+    const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.scale) + c0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 q = __ldg(s + j);
+      v[4 * j] *= q.x; v[4 * j + 1] *= q.y; v[4 * j + 2] *= q.z; v[4 * j + 3] *= q.w;
+    }
+    round16(v);
+  }
+  if (o.flags & FQ3C_RESID) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[2 * j] += __uint_as_float(r[j] << 16);
+      v[2 * j + 1] += __uint_as_float(r[j] & 0xffff0000u);
+    }
+    round16(v);
+  }
+  if (o.flags & FQ3C_CLAMP) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = fminf(fmaxf(v[j], -1.f), 1.f);
+  }
+  const size_t at = (size_t)row * o.ldc + col;
+  uint32_t w[8];
+  if (o.flags & FQ3C_OUT_F32) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(v[8 * h + j]);
+      st32(reinterpret_cast<float*>(o.C) + at + 8 * h, w);
+    }
+  } else {
+    pack16(v, w);
+    st32(reinterpret_cast<bf16*>(o.C) + at, w);
+  }
+  if (o.flags & FQ3C_SNAKE2) {
+    const float4* ea = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.p0) + c0);
+    const float4* ib = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.p1) + c0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 a = __ldg(ea + j), b = __ldg(ib + j);
+      const float s0 = sinf(v[4 * j] * a.x), s1 = sinf(v[4 * j + 1] * a.y), s2 = sinf(v[4 * j + 2] * a.z), s3 = sinf(v[4 * j + 3] * a.w);
+      v[4 * j] += b.x * s0 * s0; v[4 * j + 1] += b.y * s1 * s1; v[4 * j + 2] += b.z * s2 * s2; v[4 * j + 3] += b.w * s3 * s3;
+    }
+    pack16(v, w);
+    st32(reinterpret_cast<bf16*>(o.C2) + at, w);
+  }
+}
+__device__ __forceinline__ void gp_epilogue(const fq3c_op& o, const GemmPlan& g, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8]) {
+  if (g.vec16) {
+    epilogue_row16(o, row, col, acc, r);
+    return;
+  }
+  float h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = __uint_as_float(acc[j]);
+  epilogue_row8(o, row, col, h);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = __uint_as_float(acc[8 + j]);
+  epilogue_row8(o, row, col + 8, h);
+}
+
+// One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  Warp 9 asks for the operand
+// boxes up to `stages` k-blocks ahead, across tiles; warp 8 issues the MMAs of tile n + 1 into the second accumulator while warps 0-7 take tile n
+// through the epilogue.  With splits > 1 a cluster of CTAs shares one tile: each takes a run of k-blocks, leaves its f32 partial tile in its
+// shared memory, and each then adds the partial tiles of a part of the rows in split order.
+// The launch may begin before the ones in front of it have ended (programmatic dependent launch): nothing but B (early_b) is touched before
+// grid_dep_wait.
+template <int MINB>
+__global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ GemmPlan g,
+                                                                              const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+  extern __shared__ unsigned char gp_raw[];
+  const uint32_t raw = smem_u32(gp_raw), base = (raw + 1023u) & ~1023u;
+  unsigned char* gbase = gp_raw + (base - raw);
+  const int sb = gp_stage_bytes(g.a_rows, g.bn), ab = gp_a_bytes(g.a_rows);
+  const uint32_t bars = base + g.stages * sb;
+  const uint32_t full = bars, empty = bars + 8u * g.stages, acc_full = bars + 16u * g.stages, acc_empty = acc_full + 16;
+  uint32_t* words = reinterpret_cast<uint32_t*>(gbase + g.stages * sb + 16 * g.stages + 32);   // tensor-memory address | dead | k-blocks asked for
+  volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int tiles = g.mt * g.nt, z = g.splits > 1 ? (int)(blockIdx.x % g.splits) : 0;
+  const int t0 = g.splits > 1 ? (int)(blockIdx.x / g.splits) : (int)blockIdx.x, dt = g.splits > 1 ? tiles : (int)gridDim.x;
+  const int kb0 = (int)(((long)z * g.kb) / g.splits), kb1 = (int)(((long)(z + 1) * g.kb) / g.splits);
+  const int bufs = g.splits > 1 ? 1 : 2;
+  const uint32_t cols = (uint32_t)(g.acc_cols * bufs);
+
+  if (tid == 0) {
+    for (int s = 0; s < g.stages; ++s) { mbar_init(full + 8u * s, 1); mbar_init(empty + 8u * s, 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, GP_EPI_WARPS); }
+    words[1] = 0;
+    words[2] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == GP_MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(words)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp == GP_TMA_WARP && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, words[0], 0);
+  grid_dep_launch();
+
+  // The two issuing warps run their loops whole, with one elected lane at the copies and MMAs: in code of a single lane every descriptor goes through
+  // per-lane registers (a k-block took 700-800 cycles to issue that way, whatever its size).
+  if (warp == GP_TMA_WARP) {
+    const bool leader = elect_one();
+    const uint32_t tx = (uint32_t)(g.a_rows * TK * 2 + g.bn * TK * 2);
+    int it = 0, early = 0, st = 0;
+    uint32_t ph = 0;      // parity of the stage's current use
+    if (g.early_b && t0 < tiles) {   // the first tile's weights
+      early = min(g.stages, kb1 - kb0);
+      const int n0 = (t0 / g.mt) * g.bn;
+      int tap = kb0 / g.kpt, c = kb0 - tap * g.kpt;
+      for (int i = 0; i < early; ++i) {
+        if (leader) {
+          mbar_expect(full + 8u * i, tx);
+          tma_2d(base + i * sb + ab, &tmB, tap * o.cin + c * TK, n0, full + 8u * i);
+        }
+        if (++c == g.kpt) { c = 0; ++tap; }
+      }
+    }
+    grid_dep_wait();
+    for (int t = t0; t < tiles; t += dt) {
+      const int n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
+      int tap = kb0 / g.kpt, c = kb0 - tap * g.kpt;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        if (it >= g.stages) gp_wait(empty + 8u * st, ph ^ 1u, dead);
+        const uint32_t fb = full + 8u * st, a_dst = base + st * sb;
+        if (leader) {
+          if (it >= early) {
+            mbar_expect(fb, tx);
+            tma_2d(a_dst + ab, &tmB, tap * o.cin + c * TK, n0, fb);
+          }
+          tma_2d(a_dst, &tmA, c * TK, m0 + o.tap_off[tap], fb);
+        }
+        if (++c == g.kpt) { c = 0; ++tap; }
+        if (++st == g.stages) { st = 0; ph ^= 1u; }
+      }
+    }
+    if (leader) words[2] = (uint32_t)max(it, early);
+  } else if (warp == GP_MMA_WARP) {
+    grid_dep_wait();
+    const bool leader = elect_one();
+    // instruction descriptor: D = F32, A = B = BF16, both K-major, N = bn, M = 128
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bn >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+    int st = 0, n = 0;
+    uint32_t ph = 0;
+    for (int t = t0; t < tiles; t += dt, ++n) {
+      const int buf = n & 1;
+      const uint32_t d = tmem + (uint32_t)(buf * g.acc_cols);
+      if (n >= 2) gp_wait(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      int left = g.kpt - kb0 % g.kpt;      // k-blocks to the end of the tap
+      for (int kb = kb0; kb < kb1; ++kb) {
+        gp_wait(full + 8u * st, ph, dead);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t da = umma_desc_sw128(base + st * sb), db = umma_desc_sw128(base + st * sb + ab);
+        const int mmas = --left == 0 ? g.tail : TK / 16;
+        if (left == 0) left = g.kpt;
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < TK / 16; ++kk)
+            if (kk < mmas) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);      // 16 columns = 32 bytes further
+          umma_commit(empty + 8u * st);
+        }
+        if (++st == g.stages) { st = 0; ph ^= 1u; }
+      }
+      if (leader) umma_commit(acc_full + 8u * buf);
+    }
+  } else {
+    grid_dep_wait();
+    // warp w reads tensor-memory lanes 32 (w & 3) .. +31 (= rows of the tile); warps 0-3 take the first half of the 16-column pieces, 4-7 the rest
+    const int pieces = g.bn / 16, half = (pieces + 1) / 2, p0 = (warp >> 2) * half, p1 = min(pieces, p0 + half);
+    const int r_in = (warp & 3) * 32 + lane;
+    const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && g.splits == 1;
+    int n = 0;
+    for (int t = t0; t < tiles; t += dt, ++n) {
+      const int buf = bufs == 1 ? 0 : n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
+      const int row = m0 + r_in;
+      const bool rows = m0 + (warp & 3) * 32 < o.M;      // (warp-uniform)
+      uint32_t rx[8], ry[8];
+      // the residual's next two pieces, on their way while the accumulator is waited for or worked on
+      auto ask = [&](const int p) {
+        if (resid && row < o.M) {
+          const bf16* src = reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16;
+          if (n0 + p * 16 < o.N) ld32(src, rx);
+          if (p + 1 < p1 && n0 + p * 16 + 16 < o.N) ld32(src + 16, ry);
+        }
+      };
+      if (rows && p0 < p1) ask(p0);
+      gp_wait(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t ta = tmem + (uint32_t)(buf * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
+      if (rows)
+        for (int p = p0; p < p1; p += 2) {
+          uint32_t x[16], y[16];
+          const bool two = p + 1 < p1;
+          tmem_ld16(ta + p * 16, x);
+          if (two) tmem_ld16(ta + p * 16 + 16, y);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (p + 2 >= p1) {      // this warp's last read of the accumulator
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
+          }
+          if (g.splits > 1) {
+            float* part = reinterpret_cast<float*>(gbase) + (size_t)r_in * gp_part_pitch(g.bn);
+            if (row < o.M) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                *reinterpret_cast<uint4*>(part + p * 16 + 4 * j) = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+                if (two) *reinterpret_cast<uint4*>(part + p * 16 + 16 + 4 * j) = make_uint4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+              }
+            }
+            continue;
+          }
+          gp_epilogue(o, g, row, n0 + p * 16, x, rx);
+          if (two) gp_epilogue(o, g, row, n0 + p * 16 + 16, y, ry);
+          if (p + 2 < p1) ask(p + 2);
+        }
+      if ((!rows || p0 >= p1) && lane == 0) mbar_arrive(acc_empty + 8u * buf);
+    }
+  }
+  __syncwarp();
+  if (g.splits > 1) {
+    // every CTA of the cluster comes here, also after a wait that ran out
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int n0 = (t0 / g.mt) * g.bn, m0 = o.m_begin + (t0 % g.mt) * TM;
+    const int pieces = g.bn / 8, items = min(TM, o.M - m0) * pieces;
+    const int i0 = (int)((long)items * z / g.splits), i1 = (int)((long)items * (z + 1) / g.splits);
+    for (int i = i0 + tid; i < i1; i += GP_THREADS) {
+      const int r = i / pieces, p = i - r * pieces;
+      const uint32_t mine = base + (uint32_t)((r * gp_part_pitch(g.bn) + p * 8) * 4);
+      float4 q[8][2];      // every split's part is on its way before the first is added
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < g.splits) {
+          uint32_t far;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(mine), "r"(s));
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q[s][j].x), "=f"(q[s][j].y), "=f"(q[s][j].z), "=f"(q[s][j].w) : "r"(far + 16u * j) : "memory");
+        }
+      float a[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < g.splits) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) { a[4 * j] += q[s][j].x; a[4 * j + 1] += q[s][j].y; a[4 * j + 2] += q[s][j].z; a[4 * j + 3] += q[s][j].w; }
+        }
+      epilogue_row8(o, m0 + r, n0 + p * 8, a);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // the others have read this CTA's partial tile
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*dead && tid == 0) {      // copies still on their way land before the shared memory is given back
+    for (int i = max(0, (int)words[2] - g.stages); i < (int)words[2]; ++i) mbar_wait_bounded(full + 8u * (i % g.stages), (uint32_t)((i / g.stages) & 1));
+  }
+  __syncthreads();
+  if (warp == GP_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}

@@ -73,6 +73,7 @@ class DensePrefill:
         def gemm(A, W, N, K, out, flags=0, res=None):
             o = Op()
             o.kind, o.flags = K_GEMM, flags
+            o.reserved = 1      # weights: nothing in the list writes them
             o.M, o.N, o.K, o.taps, o.cin = cap, N, K, 1, K
             o.a_rows, o.lda, o.col_mod = cap, A.shape[1], N
             o.ldc = out.shape[1]

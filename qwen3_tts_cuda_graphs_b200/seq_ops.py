@@ -178,7 +178,8 @@ class StepBuilder:
             flags |= F_NOROUND      # f32 results and the activation's argument stay unrounded; with a few rows the flag also picks the weight-streaming product
         if glu:
             flags |= F_SWIGLU | (F_GELU_TANH if glu_gelu else 0)
-        kw = dict(M=M, N=N, K=K, taps=1, cin=K, a_rows=x.shape[0], lda=x.shape[1], ldc=out.shape[1], col_mod=N, A=x, B=w, C=out, flags=flags)
+        # reserved = 1: w is written by no op of the list
+        kw = dict(M=M, N=N, K=K, taps=1, cin=K, a_rows=x.shape[0], lda=x.shape[1], ldc=out.shape[1], col_mod=N, A=x, B=w, C=out, flags=flags, reserved=1)
         if bias is not None:
             kw["bias"] = bias
         o = self._op(K_GEMM, **kw)
