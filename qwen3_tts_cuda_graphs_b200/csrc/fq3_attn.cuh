@@ -1,0 +1,386 @@
+// fq3_attn.cuh — softmax attention of many queries on tcgen05: heads of 128, keys and values bf16.
+//
+// Included by fq3_codec.cu behind fq3_gemm.cuh.  Serves the talker's prompt (FQ3C_ATTN with flags bit 0: queries, keys and values in the projected
+// rows) and prompt portions of the sequence models (FQ3C_CACHE_ATTN over a bf16 cache).
+#pragma once
+
+struct AttnArgs {
+  const void* q;            // PROMPT: bf16 rows, else f32 rows; head h at column h * 128
+  const bf16 *k, *v;        // row j of key / value head g at j * ld + g * 128
+  long ldq, ldk, ldv;
+  int H, G, M;
+  const int* p0;            // position of query 0 (device), or null: 0
+  float scale, cap, mult;   // mult != 0 multiplies the output
+  int window, keep, chunk;  // 0: none
+  const float *r12, *sink, *gate;
+  int gate_ld, entry, out_f32;
+  void* out;
+  long ldo;
+};
+enum { AT_PROMPT, AT_PLAIN, AT_CAP, AT_DIST };   // AT_PROMPT: scores rounded to bf16 before and behind the scale; AT_DIST: cap and distance penalty, both optional
+constexpr int AT_KEYS = 128, AT_THREADS = 640, AT_LOADERS = 96;
+constexpr int AT_TILE = 128 * 128 * 2;           // a query, key or value tile: two halves of 64 columns, 128-byte lines, 128-byte swizzle
+constexpr int AT_SMEM = 6 * AT_TILE + 1024 + 256 + 2 * 2 * 256 * 4;   // tiles, alignment, barriers, the half rows' maxima (two tiles in turn)
+constexpr float AT_SLACK = 8.f;                  // a row's reference score moves when its maximum is further above it than this
+
+__device__ __forceinline__ void tmem_ld32(const uint32_t a, float* f) {
+  uint32_t v[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+      "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+        "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+        "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(a)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(const uint32_t a, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+      "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[128 x 128] (+)= A (tensor memory, bf16 pairs) . B (shared memory)
+__device__ __forceinline__ void umma_bf16_ta(const uint32_t d, const uint32_t a, const uint64_t db, const uint32_t idesc, const uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ float ex2f(const float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// A CTA takes two groups of 128 rows of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
+// staged tile.  Warps 0-7 and 8-15: two threads per row of group 0 and 1, 64 keys of a tile each; warps 16-18 stage key and value tiles of 128 positions (two
+// stages); warp 19 issues the MMAs.  Per group and tile: S = Q K^T into tensor memory; the row's threads scale, cap and mask its 128 scores, agree on the
+// maximum, take e^(score - reference) and write every weight as a bf16 pair hi + lo (16 mantissa bits) over S; O += hi V + lo V with the weights read from
+// tensor memory.  While one group's threads work, the tensor pipe has the other group's products.  The reference is the first tile's maximum and
+// moves only when a later one is more than 8 above it: then the row's output is rescaled in tensor memory.  Tiles outside every row's window, chunk
+// and kept positions are not fetched.
+// Bound by the tensor pipe (about 115 cycles per 128 x 128 x 16 MMA: 24 of them a tile) and, with a cap, by the special-function unit (three a score).
+template <int MODE>
+__global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __grid_constant__ AttnArgs a) {
+  extern __shared__ unsigned char at_raw[];
+  const uint32_t raw = smem_u32(at_raw), base = (raw + 1023u) & ~1023u;
+  unsigned char* gbase = at_raw + (base - raw);
+  const uint32_t q_s = base, k_s = base + 2 * AT_TILE, v_s = base + 4 * AT_TILE, bars = base + 6 * AT_TILE;
+  const uint32_t q_full = bars, k_full = bars + 16, k_empty = bars + 32, v_full = bars + 48, v_empty = bars + 64, s_full = bars + 80, p_full = bars + 96, o_done = bars + 112;
+  uint32_t* words = reinterpret_cast<uint32_t*>(gbase + 6 * AT_TILE + 128);
+  volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(q_full + 8u * i, 8);
+      mbar_init(k_full + 8u * i, AT_LOADERS); mbar_init(k_empty + 8u * i, 1);
+      mbar_init(v_full + 8u * i, AT_LOADERS); mbar_init(v_empty + 8u * i, 1);
+      mbar_init(s_full + 8u * i, 1); mbar_init(p_full + 8u * i, 8); mbar_init(o_done + 8u * i, 1);
+    }
+    words[1] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 19) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(words)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, words[0], 0);   // S0 | S1 | O0 | O1, 128 columns each
+  grid_dep_launch();
+  grid_dep_wait();
+
+  const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
+  const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * QB;   // the last queries (most keys) start first
+  const int P = a.p0 ? *a.p0 : 0;
+  int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    nq[g] = max(0, min(QB, a.M - m0 - g * QB));
+    first[g] = P + m0 + g * QB;
+    last[g] = first[g] + nq[g] - 1;
+    tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
+    int lo = a.window > 0 ? max(0, first[g] - a.window + 1) : 0;
+    if (a.chunk > 0) lo = max(lo, first[g] - first[g] % a.chunk);
+    tlo[g] = lo / AT_KEYS;
+  }
+  const int tkeep = a.window > 0 && a.chunk <= 0 ? (a.keep + AT_KEYS - 1) / AT_KEYS : 0;
+  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + 2 * QB) - 1;
+  auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
+
+  if (warp == 19) {
+    const bool leader = elect_one();
+    const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);   // F32 += BF16 x BF16, both K-major
+    const uint32_t idesc_o = idesc_s | (1u << 16);                                                        // B (values: rows = keys) MN-major
+    bool pend[2] = {false, false}, begun[2] = {false, false};
+    int prev = 0;
+    gp_wait(q_full, 0, dead);
+    if (nq[1] > 0) gp_wait(q_full + 8, 0, dead);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // O[g] += P[g] V of the tile in stage st
+    auto values = [&](const int g, const int st) {
+      const uint32_t pa = tmem + g * 128, d = tmem + 256 + g * 128;
+      // MN-major, 128-byte swizzle: 64 columns further is a half tile further, eight keys further 1024 bytes
+      const uint64_t vd = (uint64_t)(((v_s + st * AT_TILE) & 0x3ffffu) >> 4) | ((uint64_t)(AT_TILE / 2 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+      if (leader) {
+#pragma unroll
+        for (int part = 0; part < 2; ++part)
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_bf16_ta(d, pa + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, (begun[g] || part || kk) ? 1u : 0u);
+        if (prev == tiles[g] - 1) umma_commit(o_done + 8u * g);
+      }
+      begun[g] = true;
+    };
+    int n = 0, np[2] = {0, 0};
+    for (int t = 0; t <= ntiles; ++t) {
+      const bool more = t < ntiles;
+      const bool n0 = more && need(0, t), n1 = more && need(1, t);
+      if (more && !n0 && !n1) continue;
+      const int st = n & 1;
+      if (more) {
+        gp_wait(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      if (pend[0] || pend[1]) {
+        gp_wait(v_full + 8u * (st ^ 1), (uint32_t)(((n - 1) >> 1) & 1), dead);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (pend[g]) {
+          gp_wait(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          values(g, st ^ 1);
+          pend[g] = false;
+        }
+        if (g ? n1 : n0) {
+          if (leader) {
+            const uint64_t qd = umma_desc_sw128(q_s + g * AT_TILE), kd = umma_desc_sw128(k_s + st * AT_TILE);
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+              const uint32_t off = (kk >> 2) * (AT_TILE / 2 >> 4) + (kk & 3) * 2;
+              umma_bf16(tmem + g * 128, qd + off, kd + off, idesc_s, kk ? 1u : 0u);
+            }
+            umma_commit(s_full + 8u * g);
+          }
+          pend[g] = true;
+        }
+      }
+      if (leader) {
+        if (n > 0) umma_commit(v_empty + 8u * (st ^ 1));
+        if (more) umma_commit(k_empty + 8u * st);
+      }
+      prev = t;
+      ++n;
+    }
+  } else if (warp >= 16) {
+    // ---- key and value tiles ----
+    const int lt = tid - 512;
+    const bf16 *kc = a.k + (size_t)kvh * 128, *vc = a.v + (size_t)kvh * 128;
+    auto stage = [&](const bf16* src, const long ld, const uint32_t dst, const int j0, const uint32_t bar) {
+      for (int i = lt; i < 128 * 16; i += AT_LOADERS) {      // 16 lanes read a row
+        const int r = i >> 4, c = i & 15, j = j0 + r;
+        const bool ok = j <= jend;
+        const uint32_t at = dst + (uint32_t)((c >> 3) * (AT_TILE / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src + (size_t)(ok ? j : 0) * ld + c * 8), "r"(ok ? 16 : 0) : "memory");
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");   // when this thread's copies have landed
+    };
+    int n = 0;
+    for (int t = 0; t < ntiles; ++t) {
+      if (!need(0, t) && !need(1, t)) continue;
+      const int st = n & 1;
+      const uint32_t ph = (uint32_t)(((n >> 1) - 1) & 1);
+      if (n >= 2) gp_wait(k_empty + 8u * st, ph, dead);
+      stage(kc, a.ldk, k_s + st * AT_TILE, t * AT_KEYS, k_full + 8u * st);
+      if (n >= 2) gp_wait(v_empty + 8u * st, ph, dead);
+      stage(vc, a.ldv, v_s + st * AT_TILE, t * AT_KEYS, v_full + 8u * st);
+      ++n;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    // ---- two threads per row ----
+    const int g = warp >> 3, half = (warp >> 2) & 1, wq = warp & 3;
+    const int nqg = g ? nq[1] : nq[0], firstg = g ? first[1] : first[0], tilesg = g ? tiles[1] : tiles[0];
+    if (nqg > 0) {
+      {   // the group's queries: a warp per row, rounded to bf16 once
+        unsigned char* qt = gbase + g * AT_TILE;
+#pragma unroll 8
+        for (int i = 0; i < 16; ++i) {
+          const int r = (half * 4 + wq) * 16 + i, qi = r / HG, hh = r - qi * HG;
+          uint2 w = make_uint2(0u, 0u);
+          if (qi < nqg) {
+            const size_t at = (size_t)(m0 + g * QB + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4;
+            if (MODE == AT_PROMPT) w = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(a.q) + at);
+            else {
+              const float4 f = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.q) + at);
+              w = make_uint2(bf_pair(f.x, f.y), bf_pair(f.z, f.w));
+            }
+          }
+          const int c = lane >> 1;
+          *reinterpret_cast<uint2*>(qt + (c >> 3) * (AT_TILE / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4) + (lane & 1) * 8) = w;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(q_full + 8u * g);
+      }
+      const int r = wq * 32 + lane, qi = r / HG, head = kvh * HG + (r - qi * HG), pos = firstg + qi;
+      const bool live = qi < nqg;
+      const int wfirst = firstg + (wq * 32) / HG, wlast = firstg + min(nqg - 1, (wq * 32 + 31) / HG);
+      const bool wfull = (wq * 32 + 31) / HG < nqg;
+      const int lo = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 ? pos - pos % a.chunk : 0);
+      const int keep = a.window > 0 && a.chunk <= 0 ? a.keep : 0;
+      constexpr float L2E = 1.4426950408889634f;
+      const float icap = a.cap > 0.f ? 1.f / a.cap : 0.f;
+      float r1 = 0.f, r2 = 0.f;
+      if (MODE == AT_DIST && a.r12) { r1 = a.r12[head]; r2 = a.r12[a.H + head]; }
+      const uint32_t lanes = (uint32_t)(wq * 32) << 16, s_t = tmem + lanes + g * 128 + half * 64, o_t = tmem + lanes + 256 + g * 128 + half * 64;
+      // where this thread and the row's other one leave a number for each other, two tiles in turn; the two warps meet at a barrier of their own
+      float* mine = reinterpret_cast<float*>(gbase + 6 * AT_TILE + 256) + g * 256 + half * 128 + r;
+      const float* other = reinterpret_cast<float*>(gbase + 6 * AT_TILE + 256) + g * 256 + (half ^ 1) * 128 + r;
+      const int pair_bar = 1 + g * 4 + wq;
+      auto meet = [&](const float v, const int turn) {
+        mine[turn * 512] = v;
+        asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+        return other[turn * 512];
+      };
+      // the score of entry i of the tile in front of the mask, from the raw product
+      auto score2 = [&](float& x, float& y, const int key) {
+        if (MODE == AT_PROMPT) {
+          round2(x, y);
+          x *= a.scale; y *= a.scale;
+          round2(x, y);
+        } else {
+          x *= a.scale; y *= a.scale;
+          if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) { x = a.cap * fast_tanh(x * icap); y = a.cap * fast_tanh(y * icap); }
+          if (MODE == AT_DIST && a.r12) {
+            x -= r1 * __logf(fmaf(r2, fmaxf((float)(pos - key), 0.f), 1.f));
+            y -= r1 * __logf(fmaf(r2, fmaxf((float)(pos - key - 1), 0.f), 1.f));
+          }
+        }
+      };
+      float ref = -INFINITY, sum = 0.f;
+      int c = 0;
+      for (int t = 0; t < tilesg; ++t) {
+        if (!need(g, t)) continue;
+        gp_wait(s_full + 8u * g, (uint32_t)(c & 1), dead);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int j0 = t * AT_KEYS, k0 = j0 + half * 64;
+        // tiles that every row of the warp sees whole need no per-score test
+        const bool whole = wfull && j0 + AT_KEYS - 1 <= wfirst && (a.window <= 0 || wlast - j0 < a.window) && (a.chunk <= 0 || j0 >= wlast - wlast % a.chunk);
+        const int hi_k = live ? pos - k0 : -1, lo_k = lo - k0, kp_k = keep - k0;
+        float mx = -INFINITY;
+        float s[2][32];
+        tmem_ld32(s_t, s[0]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h == 0) tmem_ld32(s_t + 32, s[1]);      // on its way while the first half is worked on
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i);
+          if (!whole) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int k = h * 32 + i;
+              if (!(k <= hi_k && (k >= lo_k || k < kp_k))) s[h][i] = -INFINITY;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[h][i]);
+          if (h == 0) tmem_ld_wait();
+        }
+        mx = fmaxf(mx, meet(mx, c & 1));
+        if (c == 0) ref = mx;
+        else if (__any_sync(0xffffffffu, mx > ref + AT_SLACK)) {      // (from -inf too: nothing summed yet)
+          const bool up = mx > ref + AT_SLACK;
+          const float al = up ? (ref == -INFINITY ? 0.f : expf(ref - mx)) : 1.f;
+          if (up) ref = mx;
+          sum *= al;
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {      // the product in front has ended: this tile's scores were issued behind it
+            uint32_t x[16];
+            tmem_ld16(o_t + i * 16, x);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = __float_as_uint(__uint_as_float(x[j]) * al);
+            tmem_st16(o_t + i * 16, x);
+          }
+        }
+        const float u = ref == -INFINITY ? 0.f : -ref * L2E;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t hi[16], lw[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float p = ex2f(fmaf(s[h][2 * j], L2E, u)), q = ex2f(fmaf(s[h][2 * j + 1], L2E, u));
+            sum += p + q;
+            hi[j] = bf_pair(p, q);
+            lw[j] = bf_pair(p - __uint_as_float(hi[j] << 16), q - __uint_as_float(hi[j] & 0xffff0000u));
+          }
+          tmem_st16(s_t + h * 32, hi);
+          tmem_st16(s_t + h * 32 + 16, lw);
+        }
+        tmem_st_wait();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + 8u * g);
+        ++c;
+      }
+      gp_wait(o_done + 8u * g, 0, dead);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float f = 1.f, den = sum + meet(sum, c & 1);
+      if (MODE != AT_PROMPT && a.sink && live) {
+        const float sk = a.sink[head], mm = fmaxf(ref, sk);
+        f = ref == -INFINITY ? 0.f : expf(ref - mm);
+        den = den * f + expf(sk - mm);
+      }
+      const int m = pos - P;
+      float sc = f / den;
+      if (MODE != AT_PROMPT && live) {
+        if (a.gate && !a.entry) sc *= sigmoid_f(a.gate[(size_t)m * a.gate_ld + head]);
+        if (a.mult != 0.f) sc *= a.mult;
+      }
+      const float* ge = MODE != AT_PROMPT && a.entry ? a.gate + (size_t)m * a.gate_ld + (size_t)head * 128 + half * 64 : nullptr;
+      const size_t at = (size_t)m * a.ldo + (size_t)head * 128 + half * 64;
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) {
+        uint32_t x[16], w[8];
+        tmem_ld16(o_t + i * 16, x);
+        tmem_ld_wait();
+        if (live) {
+          float v[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]) * sc;
+          if (ge) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] *= sigmoid_f(ge[i * 16 + j]);
+          }
+          if (a.out_f32) {
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + at + i * 16);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          } else {
+            pack16(v, w);
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(a.out) + at + i * 16);
+            dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 19) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}

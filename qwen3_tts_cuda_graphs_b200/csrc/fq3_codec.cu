@@ -1012,6 +1012,7 @@ __global__ void fq3c_snake_kernel(const fq3c_op o) {
 
 #include "fq3_seq.cuh"
 #include "fq3_gemm.cuh"
+#include "fq3_attn.cuh"
 
 int fail(const std::string& m) { g_err = m; return -1; }
 
@@ -1127,6 +1128,33 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   L.smem = (size_t)std::max(g.stages * sb + GP_BAR_BYTES, (g.stages - 1) * sb + T_A_BYTES) + 1024;
   L.grid = g.splits > 1 ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, L.half ? 2 * GP_SMS : GP_SMS);
   return L;
+}
+
+// ---- attention of many queries on tcgen05 ---------------------------------------------------------------------------------------
+bool attn_attrs_ready() {
+  static bool done[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (!done[dev])
+    done[dev] = cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_PROMPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_DIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess;
+  return done[dev];
+}
+// What the kernel's 8- and 16-byte accesses ask for.
+bool attn_tc_takes(const AttnArgs& a, const int mode) {
+  auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  return a.H % a.G == 0 && a.H / a.G <= 128 && a.ldk % 8 == 0 && a.ldv % 8 == 0 && a.ldq % 4 == 0 && a.ldo % (a.out_f32 ? 4 : 8) == 0 && !off(a.q) && !off(a.k) &&
+         !off(a.v) && !off(a.out) && !(mode != AT_PROMPT && a.chunk > 0 && a.window > 0 && a.keep > 0) && attn_attrs_ready();
+}
+void launch_attn_tc(const AttnArgs& a, const int mode, cudaStream_t s, const bool after) {
+  const int per = 2 * (128 / (a.H / a.G));
+  const dim3 grid((a.M + per - 1) / per, a.G);
+  if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_PLAIN) launch_after(fq3c_attn_tc_kernel<AT_PLAIN>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_CAP) launch_after(fq3c_attn_tc_kernel<AT_CAP>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else launch_after(fq3c_attn_tc_kernel<AT_DIST>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
 }
 
 // ---- sequence-model ops: launch logic ---------------------------------------------------------------------------------------
@@ -1404,9 +1432,22 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         return fail("cache_attn: pooled blocks go with a window and their pooled rows, not with kept first positions, a chunked mask or a distance penalty");
       if (splits > 64) return fail("cache_attn: at most 64 key splits");
       if (splits > 1 && (!o.ws || o.ws_bytes < (int64_t)o.M * o.i0 * splits * (o.cin + 2) * 4)) return fail("cache_attn: workspace too small for the splits");
-      // bf16 cache and a prompt portion: the tensor-core kernel (FQ3S_ATTN_MMA=0: CUDA cores everywhere)
+      // bf16 cache and a prompt portion: the tensor-core kernels (FQ3S_ATTN_MMA=0: CUDA cores everywhere)
       static int use_mma = -1;
       if (use_mma < 0) { const char* e7 = getenv("FQ3S_ATTN_MMA"); use_mma = (e7 == nullptr || atoi(e7) != 0) ? 1 : 0; }
+      if (use_mma && !(o.flags & FQ3C_F32) && o.M > 8 && o.i2 == 128 && o.cin == 128 && !pool) {
+        AttnArgs a{};
+        a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.B); a.v = reinterpret_cast<const bf16*>(o.p1);
+        a.ldq = o.lda; a.ldk = o.ldr; a.ldv = o.taps; a.H = o.i0; a.G = o.i1; a.M = o.M; a.p0 = reinterpret_cast<const int*>(o.p0);
+        a.scale = o.f0; a.cap = o.f1; a.mult = o.f2; a.window = o.K; a.keep = o.a_rows; a.chunk = o.tap_off[0];
+        a.r12 = reinterpret_cast<const float*>(o.bias); a.sink = reinterpret_cast<const float*>(o.scale); a.gate = reinterpret_cast<const float*>(o.res);
+        a.gate_ld = o.col_mod; a.entry = o.res && (o.flags & FQ3C_GATE_ENTRY); a.out_f32 = (o.flags & FQ3C_OUT_F32) != 0; a.out = o.C; a.ldo = o.ldc;
+        const int mode = o.bias ? AT_DIST : o.f1 > 0.f ? AT_CAP : AT_PLAIN;
+        if (attn_tc_takes(a, mode)) {
+          launch_attn_tc(a, mode, s, false);
+          return 0;
+        }
+      }
       // rows per block: a multiple of 16 (one MMA tile per warp) that whole queries fill, i.e. that the group size divides
       int mma_rows = 0;
       for (const int w : {4, 8, 3, 6, 5, 7, 2, 1})
@@ -1856,7 +1897,17 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
       case FQ3C_ATTN: {
         if (o.i2 > 128) return fail("attn: head_dim > 128");
         static int use_apf = -1;
-        if (use_apf < 0) { const char* e5 = getenv("FQ3C_ATTN_PREFILL"); use_apf = (e5 == nullptr || atoi(e5) != 0) ? 1 : 0; }
+        if (use_apf < 0) { const char* e5 = getenv("FQ3C_ATTN_PREFILL"); use_apf = e5 == nullptr ? 1 : atoi(e5); }
+        if (use_apf && (o.flags & 1) && o.i2 == 128 && o.taps == 0 && !o.p0) {
+          AttnArgs a{};
+          a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
+          a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
+          // up to 80 rows the kernel below is faster (a warp per query and head, no tile to stage): 64 rows 8.0 against 8.8 us, 100 rows 16.0 against 11.8
+          if (use_apf != 2 && o.M > 80 && attn_tc_takes(a, AT_PROMPT)) {
+            launch_attn_tc(a, AT_PROMPT, s, after);
+            break;
+          }
+        }
         if (use_apf && (o.flags & 1) && o.i2 == 128 && o.taps == 0 && !o.p0 && o.M <= 2048 && (o.lda % 8) == 0 && (o.ldc % 4) == 0 &&
             (o.i0 % o.i1) == 0) {
           const int tpad = (o.M + 7) & ~7;

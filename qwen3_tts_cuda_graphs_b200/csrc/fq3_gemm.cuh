@@ -24,21 +24,22 @@ __host__ __device__ constexpr int gp_stage_bytes(int a_rows, int bn) { return gp
 __host__ __device__ constexpr int gp_part_pitch(int bn) { return bn + 4; }   // floats per row of a partial tile: 16-byte rows, 4 banks apart
 
 // A bounded wait of a whole warp.  When the limit (about a second) runs out it sets the error word and `dead`, and this and all later waits of the block
-// return at once: the loops around them keep their counts, so that the compiler sees control flow that is the same for the whole warp (descriptors
-// in uniform registers), and end on whatever is there.
+// return at once: the loops around them keep their counts and end on whatever is there.  (Each lane tries for itself: with a vote per try the waiting
+// warps took issue slots from the working ones.)
 __device__ __forceinline__ void gp_wait(const uint32_t bar, const uint32_t parity, volatile int* dead) {
   int i = 0;
-  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+  while (!mbar_try_wait(bar, parity)) {
     if (++i > 256) {      // (a try suspends the thread for a while by itself)
-      if (__any_sync(0xffffffffu, *dead != 0)) return;
+      if (*dead) break;
       __nanosleep(i > 8192 ? 1000 : 20);
       if (i > (1 << 20)) {
         *dead = 1;
         seq_wait_error = 1;
-        return;
+        break;
       }
     }
   }
+  __syncwarp();
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
@@ -309,8 +310,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int left = g.kpt - kb0 % g.kpt;      // k-blocks to the end of the tap
       for (int kb = kb0; kb < kb1; ++kb) {
-        gp_wait(full + 8u * st, ph, dead);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        gp_wait(full + 8u * st, ph, dead);      // (filled by the copy engine: no tensor-memory fence)
         const uint64_t da = umma_desc_sw128(base + st * sb), db = umma_desc_sw128(base + st * sb + ab);
         const int mmas = --left == 0 ? g.tail : TK / 16;
         if (left == 0) left = g.kpt;

@@ -1,0 +1,104 @@
+"""Attention of many queries on tcgen05 (both of its callers) at the edges of its key tiles, query groups, windows, chunks and kept positions, against float64."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def launch(op):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    lib = K.load_lib()
+    assert lib.fq3c_run((K.Op * 1)(op), 1, torch.cuda.current_stream().cuda_stream) == 0, lib.fq3c_last_error()
+    torch.cuda.synchronize()
+    assert lib.fq3c_wait_errors() == 0
+
+
+def exact(q, k, v, first, scale, cap=0.0, window=0, keep=0, chunk=0, sink=None, r12=None, rounded=False):
+    M, H, _ = q.shape
+    L, G, _ = k.shape
+    i, j = torch.arange(first, first + M, device="cuda")[:, None], torch.arange(L, device="cuda")[None]
+    seen = j <= i
+    if window:
+        seen = seen & ((i - j < window) | (j < keep))
+    if chunk:
+        seen = seen & (j >= i - i % chunk)
+    out = torch.empty(M, H, 128, device="cuda", dtype=torch.float64)
+    for h in range(H):
+        s = q[:, h] @ k[:, h // (H // G)].T
+        s = (s.bfloat16().double() * scale).bfloat16().double() if rounded else s * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        if r12 is not None:
+            s = s - r12[h] * torch.log1p(r12[H + h] * (i - j).clamp(min=0).double())
+        s = s.masked_fill(~seen, -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink[h].expand(M, 1)], 1)
+        out[:, h] = s.softmax(-1)[:, :L] @ v[:, h // (H // G)]
+    return out
+
+
+def rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("rows, heads, kv, window", [(81, 16, 8, 0), (128, 16, 8, 0), (129, 4, 4, 0), (262, 16, 8, 0), (300, 4, 4, 40), (700, 6, 2, 0)])
+def test_prompt_rows(rows, heads, kv, window):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    torch.manual_seed(rows)
+    n = (heads + 2 * kv) * 128
+    a, out = torch.randn(rows, n, device="cuda").bfloat16(), torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16)
+    o = K.Op()
+    o.kind, o.flags, o.M, o.N, o.A, o.lda, o.a_rows = K.K_ATTN, 1, rows, heads * 128, a.data_ptr(), n, rows
+    o.C, o.ldc, o.col_mod, o.i0, o.i1, o.i2, o.K = out.data_ptr(), heads * 128, heads * 128, heads, kv, 128, window or 2048
+    launch(o)
+    d = a.double()
+    want = exact(d[:, :heads * 128].view(rows, heads, 128), d[:, heads * 128:(heads + kv) * 128].view(rows, kv, 128), d[:, (heads + kv) * 128:].view(rows, kv, 128), 0,
+                 128 ** -0.5, window=window, rounded=True)
+    assert rel(out, want.reshape(rows, -1)) < 2.0 ** -9      # one rounding to bf16: 2^-9 at most, about 2^-9.3 on average
+
+
+# rows, positions in front, heads, key heads, options
+CASES = [(9, 0, 4, 2, {}), (100, 0, 4, 1, {}), (300, 77, 6, 2, {}), (128, 128, 16, 4, dict(cap=50.0, sink=True, gate=1)), (513, 300, 16, 4, dict(cap=50.0, sink=True)),
+         (200, 300, 8, 2, dict(window=64)), (200, 300, 8, 2, dict(window=64, keep=5, dist=True, cap=50.0)), (128, 128, 3, 1, dict(window=130, keep=200)), (400, 0, 8, 8, dict(window=1)),
+         (700, 129, 4, 4, dict(chunk=100, sink=True)), (700, 129, 4, 4, dict(chunk=1000, gate=2)), (260, 260, 12, 4, dict(dist=True, spread=4.0)), (300, 0, 2, 2, dict(spread=8.0)), (40, 700, 2, 1, dict(rising=True))]
+
+
+@pytest.mark.parametrize("rows, first, heads, kv, opt", CASES)
+def test_cache_rows(rows, first, heads, kv, opt):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    torch.manual_seed(rows + first + heads)
+    L = first + rows
+    q = torch.randn(rows, heads * 128, device="cuda") * opt.get("spread", 1.0)
+    kc = torch.full((L + 300, kv * 128), float("nan"), device="cuda", dtype=torch.bfloat16)      # rows beyond the last position are never used
+    vc = kc.clone()
+    kc[:L], vc[:L] = torch.randn(L, kv * 128, device="cuda").bfloat16(), torch.randn(L, kv * 128, device="cuda").bfloat16()
+    if opt.get("rising"):      # scores climb from tile to tile, so that a row's reference moves
+        q, kc[:L] = q.abs(), (kc[:L].float().abs() * torch.linspace(0.1, 3.0, L, device="cuda")[:, None]).bfloat16()
+    pos = torch.tensor([first], dtype=torch.int32, device="cuda")
+    out = torch.zeros(rows, heads * 128, device="cuda")
+    o = K.Op()
+    o.kind, o.flags, o.M, o.N, o.i0, o.i1, o.i2, o.cin, o.f0, o.f1 = K.K_CACHE_ATTN, K.F_OUT_F32, rows, heads * 128, heads, kv, 128, 128, 128 ** -0.5, opt.get("cap", 0.0)
+    o.K, o.a_rows, o.tap_off[0], o.m_begin = opt.get("window", 0), opt.get("keep", 0), opt.get("chunk", 0), 1
+    o.A, o.lda, o.B, o.ldr, o.p1, o.taps, o.p0 = q.data_ptr(), heads * 128, kc.data_ptr(), kv * 128, vc.data_ptr(), kv * 128, pos.data_ptr()
+    o.C, o.ldc, o.col_mod = out.data_ptr(), heads * 128, 1
+    sink = torch.randn(heads, device="cuda") if opt.get("sink") else None
+    r12 = torch.rand(2 * heads, device="cuda") if opt.get("dist") else None
+    gate = torch.randn(rows, heads * (128 if opt["gate"] == 2 else 1), device="cuda") if opt.get("gate") else None
+    if sink is not None:
+        o.scale = sink.data_ptr()
+    if r12 is not None:
+        o.bias = r12.data_ptr()
+    if gate is not None:
+        o.res, o.col_mod = gate.data_ptr(), gate.shape[1]
+        o.flags |= K.F_GATE_ENTRY if opt["gate"] == 2 else 0
+    launch(o)
+    want = exact(q.bfloat16().double().view(rows, heads, 128), kc[:L].double().view(L, kv, 128), vc[:L].double().view(L, kv, 128), first, 128 ** -0.5, opt.get("cap", 0.0),
+                 opt.get("window", 0), opt.get("keep", 0), opt.get("chunk", 0), None if sink is None else sink.double(), None if r12 is None else r12.double())
+    if gate is not None:
+        want = want * torch.sigmoid(gate.double()).view(rows, heads, -1)
+    # weights of 16 mantissa bits (2^-17 each, falling either way), scores within 2^-22 of their size through the fast cap and exponential
+    assert rel(out, want.reshape(rows, -1)) < 1.5e-5
