@@ -175,6 +175,17 @@ __device__ __forceinline__ void epilogue_row8(const fq3c_op& o, int row, int col
         make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     return;
   }
+  // the same on rounded sums (the talker's and the codec's feed-forward)
+  if ((o.flags & FQ3C_SWIGLU) && !(o.flags & ~FQ3C_SWIGLU) && col + 8 <= o.N && (o.ldc & 3) == 0 && !(reinterpret_cast<uintptr_t>(o.C) & 7)) {
+    if (row >= o.M) return;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = bf16r(silu_f(bf16r(acc[2 * j]))) * bf16r(acc[2 * j + 1]);
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(o.C) + (size_t)row * o.ldc + (col >> 1)) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    return;
+  }
   const bool vec = (col + 8 <= o.N) && !(o.flags & (FQ3C_SWIGLU | FQ3C_OUT_F32)) && ((o.ldc & 7) == 0) &&
                    (!(o.flags & FQ3C_RESID) || (o.ldr & 7) == 0);
   if (!vec) {
@@ -1011,6 +1022,7 @@ __global__ void fq3c_snake_kernel(const fq3c_op o) {
 }
 
 #include "fq3_seq.cuh"
+#include "fq3_f32.cuh"
 #include "fq3_gemm.cuh"
 #include "fq3_attn.cuh"
 
@@ -1094,7 +1106,8 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
     const int bn = o.N >= 64 ? 64 : 32;
     const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
     const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));
-    if (sp > 1) { g.splits = sp; g.bn = bn; }
+    // (the cluster's two meetings and the sums cost about 5000 cycles: two splits of 16 k-blocks, 6.9 against 5.6 us, do not pay)
+    if (sp > 1 && (long)KT * 430 - (long)((KT + sp - 1) / sp) * 440 > 5000) { g.splits = sp; g.bn = bn; }
   }
   long kl = 0, ep = 0;
   if (g.splits == 1) {
@@ -1116,6 +1129,8 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   g.acc_cols = 32;
   while (g.acc_cols < g.bn) g.acc_cols *= 2;
   g.early_b = o.reserved & 1;
+  // (few rows and a costly epilogue: 39 rows of gated units 8.3 -> 7.5 us; without one the extra meeting costs 1 us more than it saves)
+  g.staged = g.splits > 1 || (g.mt == 1 && g.a_rows <= 64 && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
   g.vec16 = gemm_vec16(o) ? 1 : 0;
   const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = g.splits > 1 ? (g.kb + g.splits - 1) / g.splits : g.kb;
   // Two CTAs per SM: tiles of one wave keep to half of an SM, so that the next launch's CTAs fit beside them and ask for their weights early; tiles
@@ -1126,7 +1141,7 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   const int room = (L.half ? GP_SMEM_HALF : GP_SMEM_MAX) - 1024, fit = std::min((room - GP_BAR_BYTES) / sb, (room - T_A_BYTES) / sb + 1);
   g.stages = std::max(2, std::min(std::min(fit, 16), g.splits > 1 ? n_kb : 16));
   L.smem = (size_t)std::max(g.stages * sb + GP_BAR_BYTES, (g.stages - 1) * sb + T_A_BYTES) + 1024;
-  L.grid = g.splits > 1 ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, L.half ? 2 * GP_SMS : GP_SMS);
+  L.grid = g.staged ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, L.half ? 2 * GP_SMS : GP_SMS);
   return L;
 }
 
@@ -1212,7 +1227,19 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     return 0;
   }
   dim3 grid((g.N + 63) / 64, row_tiles, zcount);
-  if (b_f32) fq3s_gemm_kernel<float, float><<<grid, 256, 0, s>>>(g);
+  // rows of whole 16-byte pieces: the pipelined product (the other one stages element by element)
+  const bool pieces = !((g.K | g.lda | g.ldb | g.a_zstride) & 3) && !((g.b_zstride | g.b_estride) & 3) && !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15);
+  if (b_f32 && pieces) {
+    static bool attr[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr[dev]) {
+      cudaFuncSetAttribute(fq3s_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
+      attr[dev] = true;
+    }
+    fq3s_gemm_f32_kernel<<<grid, 256, FG_SMEM, s>>>(g);
+  }
+  else if (b_f32) fq3s_gemm_kernel<float, float><<<grid, 256, 0, s>>>(g);
   else if (a_f32 && exact) fq3s_gemm_kernel<float, bf16><<<grid, 256, 0, s>>>(g);
   else if (a_f32 && (g.flags & FQ3C_SWIGLU)) fq3s_gemm_mma_kernel<float, true><<<grid, 128, 0, s>>>(g);
   else if (a_f32) fq3s_gemm_mma_kernel<float><<<grid, 128, 0, s>>>(g);
@@ -1478,6 +1505,24 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         } else if (o.cin <= 32) fq3s_cache_attn_mma_kernel<4><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
         else if (o.cin <= 64) fq3s_cache_attn_mma_kernel<8><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
         else fq3s_cache_attn_mma_kernel<16><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
+        return 0;
+      }
+      // an f32 cache and more than a few queries, heads of 128: 32-row blocks with pipelined tiles
+      if ((o.flags & FQ3C_F32) && o.M > 8 && o.i2 == 128 && o.cin == 128 && !pool && HG <= FA_R && !((o.lda | o.ldr | o.taps) & 3) &&
+          !((reinterpret_cast<uintptr_t>(o.A) | reinterpret_cast<uintptr_t>(o.B) | reinterpret_cast<uintptr_t>(o.p1)) & 15)) {
+        static bool fattr[64] = {};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < 64 && !fattr[dev]) {
+          cudaFuncSetAttribute(fq3s_attn_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM);
+          fattr[dev] = true;
+        }
+        const int QB = FA_R / HG;
+        fq3s_attn_f32_kernel<<<dim3((o.M + QB - 1) / QB, o.i1, splits), 128, FA_SMEM, s>>>(o);
+        if (splits > 1) {
+          fq3s_cache_attn_merge_kernel<<<dim3(o.M, o.i0), 128, 0, s>>>(o, splits);
+          count_launches(1);
+        }
         return 0;
       }
       int QB = o.M == 1 ? 1 : std::max(1, std::min(std::min(16, o.M), 16 / HG)), TJ = 32;

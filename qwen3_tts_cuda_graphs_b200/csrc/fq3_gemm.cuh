@@ -16,6 +16,7 @@ struct GemmPlan {
   int acc_cols;  // tensor-memory columns of one accumulator (power of two); two of them unless splits > 1
   int early_b;   // B is not written by the launches in front: its first stages are asked for before they have ended
   int vec16;     // the epilogue may move 16 columns of a row at a time
+  int staged;    // the epilogue takes its tile from shared memory, spread over all threads: split sums, and few rows (a CTA has one tile then)
 };
 constexpr int GP_EPI_WARPS = 8, GP_MMA_WARP = 8, GP_TMA_WARP = 9, GP_THREADS = 320;
 constexpr int GP_BAR_BYTES = 512;   // barriers, tensor-memory address, error word
@@ -232,9 +233,9 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int tiles = g.mt * g.nt, z = g.splits > 1 ? (int)(blockIdx.x % g.splits) : 0;
-  const int t0 = g.splits > 1 ? (int)(blockIdx.x / g.splits) : (int)blockIdx.x, dt = g.splits > 1 ? tiles : (int)gridDim.x;
+  const int t0 = g.splits > 1 ? (int)(blockIdx.x / g.splits) : (int)blockIdx.x, dt = g.staged ? tiles : (int)gridDim.x;
   const int kb0 = (int)(((long)z * g.kb) / g.splits), kb1 = (int)(((long)(z + 1) * g.kb) / g.splits);
-  const int bufs = g.splits > 1 ? 1 : 2;
+  const int bufs = g.staged ? 1 : 2;
   const uint32_t cols = (uint32_t)(g.acc_cols * bufs);
 
   if (tid == 0) {
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
     // warp w reads tensor-memory lanes 32 (w & 3) .. +31 (= rows of the tile); warps 0-3 take the first half of the 16-column pieces, 4-7 the rest
     const int pieces = g.bn / 16, half = (pieces + 1) / 2, p0 = (warp >> 2) * half, p1 = min(pieces, p0 + half);
     const int r_in = (warp & 3) * 32 + lane;
-    const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && g.splits == 1;
+    const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && !g.staged;
     int n = 0;
     for (int t = t0; t < tiles; t += dt, ++n) {
       const int buf = bufs == 1 ? 0 : n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
           }
-          if (g.splits > 1) {
+          if (g.staged) {
             float* part = reinterpret_cast<float*>(gbase) + (size_t)r_in * gp_part_pitch(g.bn);
             if (row < o.M) {
 #pragma unroll
@@ -379,13 +380,16 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
     }
   }
   __syncwarp();
-  if (g.splits > 1) {
-    // every CTA of the cluster comes here, also after a wait that ran out
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (g.staged) {
     const int n0 = (t0 / g.mt) * g.bn, m0 = o.m_begin + (t0 % g.mt) * TM;
     const int pieces = g.bn / 8, items = min(TM, o.M - m0) * pieces;
     const int i0 = (int)((long)items * z / g.splits), i1 = (int)((long)items * (z + 1) / g.splits);
+    if (g.splits > 1) {      // every CTA of the cluster comes here, also after a wait that ran out
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
     for (int i = i0 + tid; i < i1; i += GP_THREADS) {
       const int r = i / pieces, p = i - r * pieces;
       const uint32_t mine = base + (uint32_t)((r * gp_part_pitch(g.bn) + p * 8) * 4);
@@ -393,8 +397,8 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
 #pragma unroll
       for (int s = 0; s < 8; ++s)
         if (s < g.splits) {
-          uint32_t far;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(mine), "r"(s));
+          uint32_t far = mine;
+          if (g.splits > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(mine), "r"(s));
 #pragma unroll
           for (int j = 0; j < 2; ++j)
             asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q[s][j].x), "=f"(q[s][j].y), "=f"(q[s][j].z), "=f"(q[s][j].w) : "r"(far + 16u * j) : "memory");
@@ -410,8 +414,10 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
         }
       epilogue_row8(o, m0 + r, n0 + p * 8, a);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // the others have read this CTA's partial tile
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (g.splits > 1) {      // the others have read this CTA's partial tile (reads only: nothing to publish)
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -382,6 +382,8 @@ class StepBuilder:
         tiles = max(1, -(-span // 32))
         blocks = -(-M // QB) * G
         splits = min(64, tiles) if M <= 8 else (1 if blocks >= 74 else max(1, min(16, tiles, -(-296 // blocks))))
+        if cf32 and M > 8 and d == dv == 128 and HG <= 32 and pool == 0:      # 32-row blocks over 64-position tiles (fq3s_attn_f32_kernel), two per SM
+            splits = max(1, min(16, -(-span // 64), 296 // (-(-M // (32 // HG)) * G)))
         kw = dict(M=M, N=H * dv, i0=H, i1=G, i2=d, cin=dv, f0=c.scale, f1=c.softcap, K=c.window, a_rows=c.keep_first if c.window > 0 else 0,
                   f2=float(mult), A=_ptr(rows, qcol), lda=rows.shape[1], B=kc, ldr=kc.shape[1], p1=vc, taps=vc.shape[1], p0=self.slot.pos, m_begin=splits,
                   C=oa, ldc=oa.shape[1], flags=cf32 | self._oflag(oa))
