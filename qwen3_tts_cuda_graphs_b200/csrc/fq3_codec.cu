@@ -57,6 +57,26 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); 
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
+// sin(x)^2, the periodic half of SnakeBeta: it has period pi, so x is reduced by the nearest multiple of pi (three constants, exact products) to
+// [-pi/2, pi/2] and the sine is an odd polynomial of degree 9 there (Remez fit of sin(r) / r in r^2, relative error 5e-9): no quadrant to choose and no
+// branch.  Within 2.5e-7 of sin^2; arguments the rounding to a multiple does not hold for go through sinf.
+__device__ __forceinline__ float sin_sq_near(const float x) {
+  const float n = fmaf(x, 0.3183098861837907f, 12582912.f) - 12582912.f;
+  float r = fmaf(n, -3.1415927410125732f, x);
+  r = fmaf(n, 8.742277657347586e-08f, r);
+  r = fmaf(n, 3.4302490200117637e-15f, r);
+  const float u = r * r;
+  float q = fmaf(u, 2.6018262815341586e-06f, -0.00019807384524028748f);
+  q = fmaf(u, q, 0.008333024568855762f);
+  q = fmaf(u, q, -0.16666656732559204f);
+  const float s = fmaf(r * u, q, r);
+  return s * s;
+}
+__device__ __noinline__ float sin_sq_far(const float x) {
+  const float s = sinf(x);
+  return s * s;
+}
+__device__ __forceinline__ float sin_sq(const float x) { return fabsf(x) < 1e6f ? sin_sq_near(x) : sin_sq_far(x); }
 // a gated unit: silu(gate) * up, or with FQ3C_GELU_TANH gelu_tanh(gate) * up
 __device__ __forceinline__ float glu_f(const int flags, const float gate, const float up) {
   return (flags & FQ3C_GELU_TANH) ? gelu_tanh_f(gate) * up : silu_f(gate) * up;
@@ -119,12 +139,8 @@ __device__ __forceinline__ void epilogue_pair(const fq3c_op& o, int row, int col
     const float* ea = reinterpret_cast<const float*>(o.p0);
     const float* ib = reinterpret_cast<const float*>(o.p1);
     bf16* c2 = reinterpret_cast<bf16*>(o.C2) + (size_t)row * o.ldc + col;
-    float s0 = sinf(v0 * ea[cm0]);
-    c2[0] = __float2bfloat16_rn(v0 + ib[cm0] * s0 * s0);
-    if (has1) {
-      float s1 = sinf(v1 * ea[cm1]);
-      c2[1] = __float2bfloat16_rn(v1 + ib[cm1] * s1 * s1);
-    }
+    c2[0] = __float2bfloat16_rn(v0 + ib[cm0] * sin_sq(v0 * ea[cm0]));
+    if (has1) c2[1] = __float2bfloat16_rn(v1 + ib[cm1] * sin_sq(v1 * ea[cm1]));
   }
 }
 
@@ -258,8 +274,8 @@ __device__ __forceinline__ void epilogue_row8(const fq3c_op& o, int row, int col
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float s0 = sinf(v[2 * j] * ea[cm[2 * j]]), s1 = sinf(v[2 * j + 1] * ea[cm[2 * j + 1]]);
-      const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j] + ib[cm[2 * j]] * s0 * s0, v[2 * j + 1] + ib[cm[2 * j + 1]] * s1 * s1);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j] + ib[cm[2 * j]] * sin_sq(v[2 * j] * ea[cm[2 * j]]),
+                                                     v[2 * j + 1] + ib[cm[2 * j + 1]] * sin_sq(v[2 * j + 1] * ea[cm[2 * j + 1]]));
       w[j] = *reinterpret_cast<const uint32_t*>(&h);
     }
     *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(o.C2) + (size_t)row * o.ldc + col) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -1016,9 +1032,47 @@ __global__ void fq3c_snake_kernel(const fq3c_op o) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int t = (int)(i / o.N), c = (int)(i - (size_t)t * o.N);
     const float v = __bfloat162float(x[(size_t)t * o.lda + c]);
-    const float s = sinf(v * ea[c]);
-    y[(size_t)t * o.ldc + c] = __float2bfloat16_rn(v + ib[c] * s * s);
+    y[(size_t)t * o.ldc + c] = __float2bfloat16_rn(v + ib[c] * sin_sq(v * ea[c]));
   }
+}
+
+// A convolution to ONE output channel (the vocoder's last layer: 7 taps x 96 channels): a dot product per row, not a matrix product.  A block stages the rows
+// its 256 outputs see once (the 64 x 64 tensor-core tile read them once per tap and threw 63 of 64 columns away) and every thread forms one
+// output, eight channels a step, f32 sums.  Bound by shared memory (one row's 16-byte pieces per lane).  491 520 rows: 178 -> 30 us.
+constexpr int C1_ROWS = 256, C1_SPAN = 64, C1_CIN = 128;
+__global__ void __launch_bounds__(C1_ROWS) fq3c_conv1_kernel(const fq3c_op o, const int lo, const int span) {
+  grid_dep_begin();
+  extern __shared__ __align__(16) unsigned char c1_raw[];
+  const int cin = o.cin, pitch = cin + 8, m0 = o.m_begin + blockIdx.x * C1_ROWS, tid = threadIdx.x, cpr = cin >> 3;
+  float* w = reinterpret_cast<float*>(c1_raw);                         // [taps][cin]
+  bf16* xs = reinterpret_cast<bf16*>(w + o.taps * cin);                // [C1_ROWS + span][cin + 8]: rows 16 bytes apart in banks
+  for (int i = tid; i < o.taps * cin; i += C1_ROWS) w[i] = __bfloat162float(reinterpret_cast<const bf16*>(o.B)[i]);
+  const int rows = min(C1_ROWS, o.M - m0) + span;
+  for (int i = tid; i < rows * cpr; i += C1_ROWS) {
+    const int r = i / cpr, c = i - r * cpr, src = m0 + lo + r;
+    const bool ok = src >= 0 && src < o.a_rows;
+    cp_async16(xs + (size_t)r * pitch + c * 8, reinterpret_cast<const bf16*>(o.A) + (size_t)(ok ? src : 0) * o.lda + c * 8, ok);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int row = m0 + tid;
+  if (row >= o.M) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int t = 0; t < o.taps; ++t) {
+    const uint4* xr = reinterpret_cast<const uint4*>(xs + (size_t)(tid + o.tap_off[t] - lo) * pitch);
+    const float4* wr = reinterpret_cast<const float4*>(w + t * cin);
+#pragma unroll 4
+    for (int c = 0; c < cpr; ++c) {
+      const uint4 x = xr[c];
+      const float4 a = wr[2 * c], b = wr[2 * c + 1];
+      acc[0] = fmaf(__uint_as_float(x.x << 16), a.x, acc[0]); acc[1] = fmaf(__uint_as_float(x.x & 0xffff0000u), a.y, acc[1]);
+      acc[2] = fmaf(__uint_as_float(x.y << 16), a.z, acc[2]); acc[3] = fmaf(__uint_as_float(x.y & 0xffff0000u), a.w, acc[3]);
+      acc[0] = fmaf(__uint_as_float(x.z << 16), b.x, acc[0]); acc[1] = fmaf(__uint_as_float(x.z & 0xffff0000u), b.y, acc[1]);
+      acc[2] = fmaf(__uint_as_float(x.w << 16), b.z, acc[2]); acc[3] = fmaf(__uint_as_float(x.w & 0xffff0000u), b.w, acc[3]);
+    }
+  }
+  epilogue_pair(o, row, 0, (acc[0] + acc[1]) + (acc[2] + acc[3]), 0.f);
 }
 
 #include "fq3_seq.cuh"
@@ -1926,6 +1980,22 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
             count_launches(1);
           }
           break;
+        }
+        // one output channel: rows, pitch and weights in whole 16-byte pieces, the rows a block sees within its shared memory
+        if (o.N == 1 && o.cin % 8 == 0 && o.cin <= C1_CIN && !o.norm_out && !(o.flags & FQ3C_SWIGLU) && o.lda % 8 == 0 && !(reinterpret_cast<uintptr_t>(o.A) & 15)) {
+          const int lo = *std::min_element(o.tap_off, o.tap_off + o.taps), span = *std::max_element(o.tap_off, o.tap_off + o.taps) - lo;
+          if (span <= C1_SPAN) {
+            const size_t smem = (size_t)o.taps * o.cin * 4 + (size_t)(C1_ROWS + span) * (o.cin + 8) * 2;
+            static bool cattr[64] = {};
+            int dev = 0;
+            cudaGetDevice(&dev);
+            if (dev >= 0 && dev < 64 && !cattr[dev]) {
+              cudaFuncSetAttribute(fq3c_conv1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * C1_CIN * 4 + (C1_ROWS + C1_SPAN) * (C1_CIN + 8) * 2);
+              cattr[dev] = true;
+            }
+            launch_after(fq3c_conv1_kernel, (unsigned)((o.M - o.m_begin + C1_ROWS - 1) / C1_ROWS), C1_ROWS, smem, s, after, 1, o, lo, span);
+            break;
+          }
         }
         dim3 grid((o.N + BN - 1) / BN, (o.M - o.m_begin + BM - 1) / BM);
         fq3c_gemm_kernel<<<grid, 128, 0, s>>>(o);

@@ -193,25 +193,38 @@ __device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float4 a = __ldg(ea + j), b = __ldg(ib + j);
-      const float s0 = sinf(v[4 * j] * a.x), s1 = sinf(v[4 * j + 1] * a.y), s2 = sinf(v[4 * j + 2] * a.z), s3 = sinf(v[4 * j + 3] * a.w);
-      v[4 * j] += b.x * s0 * s0; v[4 * j + 1] += b.y * s1 * s1; v[4 * j + 2] += b.z * s2 * s2; v[4 * j + 3] += b.w * s3 * s3;
+      const float x0 = v[4 * j] * a.x, x1 = v[4 * j + 1] * a.y, x2 = v[4 * j + 2] * a.z, x3 = v[4 * j + 3] * a.w;
+      if (fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(x2), fabsf(x3))) < 1e6f) {
+        v[4 * j] = fmaf(b.x, sin_sq_near(x0), v[4 * j]); v[4 * j + 1] = fmaf(b.y, sin_sq_near(x1), v[4 * j + 1]);
+        v[4 * j + 2] = fmaf(b.z, sin_sq_near(x2), v[4 * j + 2]); v[4 * j + 3] = fmaf(b.w, sin_sq_near(x3), v[4 * j + 3]);
+      } else {
+        v[4 * j] = fmaf(b.x, sin_sq_far(x0), v[4 * j]); v[4 * j + 1] = fmaf(b.y, sin_sq_far(x1), v[4 * j + 1]);
+        v[4 * j + 2] = fmaf(b.z, sin_sq_far(x2), v[4 * j + 2]); v[4 * j + 3] = fmaf(b.w, sin_sq_far(x3), v[4 * j + 3]);
+      }
     }
     pack16(v, w);
     st32(reinterpret_cast<bf16*>(o.C2) + at, w);
   }
 }
+// shapes and addresses without whole sectors: out of line, so that the other path's code stays together
+__device__ __noinline__ void epilogue_odd16(const fq3c_op& o, const int row, const int col, const float* acc) {
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = acc[8 * h + j];
+    epilogue_row8(o, row, col + 8 * h, v);
+  }
+}
 __device__ __forceinline__ void gp_epilogue(const fq3c_op& o, const GemmPlan& g, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8]) {
   if (g.vec16) {
     epilogue_row16(o, row, col, acc, r);
-    return;
+  } else {
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc[j]);
+    epilogue_odd16(o, row, col, v);
   }
-  float h[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) h[j] = __uint_as_float(acc[j]);
-  epilogue_row8(o, row, col, h);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) h[j] = __uint_as_float(acc[8 + j]);
-  epilogue_row8(o, row, col + 8, h);
 }
 
 // One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  Warp 9 asks for the operand
