@@ -1131,13 +1131,12 @@ constexpr int GP_SMEM_MAX = 227 * 1024, GP_SMEM_HALF = 112 * 1024;
 // Whether the epilogue may move whole 32-byte sectors (16 columns of bf16, 8 of f32).
 bool gemm_vec16(const fq3c_op& o) {
   auto off = [](const void* p, int a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
-  if (o.N % 16 || o.col_mod % 16) return false;
-  if (((o.flags & FQ3C_BIAS) && off(o.bias, 16)) || ((o.flags & FQ3C_SCALE) && off(o.scale, 16))) return false;
+  if (o.N % 16) return false;
   const bool f32 = (o.flags & FQ3C_OUT_F32) != 0;
   if (o.flags & FQ3C_SWIGLU) return o.ldc % 8 == 0 && !off(o.C, 32);
   if (o.ldc % (f32 && !(o.flags & FQ3C_SNAKE2) ? 8 : 16) || off(o.C, 32)) return false;
   if ((o.flags & FQ3C_RESID) && (o.ldr % 16 || off(o.res, 32))) return false;
-  if ((o.flags & FQ3C_SNAKE2) && (off(o.C2, 32) || off(o.p0, 16) || off(o.p1, 16))) return false;
+  if ((o.flags & FQ3C_SNAKE2) && off(o.C2, 32)) return false;
   return true;
 }
 struct GemmLaunch { GemmPlan g; bool half; unsigned grid; size_t smem; };

@@ -19,7 +19,8 @@ struct GemmPlan {
   int staged;    // the epilogue takes its tile from shared memory, spread over all threads: split sums, and few rows (a CTA has one tile then)
 };
 constexpr int GP_EPI_WARPS = 8, GP_MMA_WARP = 8, GP_TMA_WARP = 9, GP_THREADS = 320;
-constexpr int GP_BAR_BYTES = 512;   // barriers, tensor-memory address, error word
+constexpr int GP_PAR = 256;         // columns of a tile at most: its bias, scale and SnakeBeta parameters lie in shared memory
+constexpr int GP_BAR_BYTES = 512 + 4 * GP_PAR * 4;   // barriers, tensor-memory address, error word; parameters
 __host__ __device__ constexpr int gp_a_bytes(int a_rows) { return (a_rows * TK * 2 + 1023) & ~1023; }
 __host__ __device__ constexpr int gp_stage_bytes(int a_rows, int bn) { return gp_a_bytes(a_rows) + bn * TK * 2; }
 __host__ __device__ constexpr int gp_part_pitch(int bn) { return bn + 4; }   // floats per row of a partial tile: 16-byte rows, 4 banks apart
@@ -107,18 +108,19 @@ __device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
 }
 
 // Epilogue of 16 consecutive columns of one row: the arithmetic and order of epilogue_pair, every access a whole 32-byte sector.  The host
-// has checked sizes, pitches and addresses (gemm_vec16).  r: the residual's 16 entries, asked for before the accumulator was read.
-__device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8]) {
+// has checked sizes, pitches and addresses (gemm_vec16).  r: the residual's 16 entries, asked for before the accumulator was read.  par: the tile's
+// parameters from this column on (bias, scale, SnakeBeta's two, GP_PAR floats apart): from global memory they missed the few KB of L1 that are left
+// beside the stages, behind the streaming residual (72 % of the stalls of a 96-column layer).
+__device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8], const float* par) {
   if (row >= o.M || col >= o.N) return;
   float v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(acc[j]);
-  const int c0 = o.col_mod == o.N ? col : col % o.col_mod;
   if (o.flags & FQ3C_BIAS) {
-    const float4* b = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.bias) + c0);
+    const float4* b = reinterpret_cast<const float4*>(par);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 q = __ldg(b + j);
+      const float4 q = b[j];
       v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
     }
   }
@@ -154,10 +156,10 @@ __device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, 
     round16(v);
   }
   if (o.flags & FQ3C_SCALE) {
-    const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.scale) + c0);
+    const float4* s = reinterpret_cast<const float4*>(par + GP_PAR);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 q = __ldg(s + j);
+      const float4 q = s[j];
       v[4 * j] *= q.x; v[4 * j + 1] *= q.y; v[4 * j + 2] *= q.z; v[4 * j + 3] *= q.w;
     }
     round16(v);
@@ -188,11 +190,11 @@ __device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, 
     st32(reinterpret_cast<bf16*>(o.C) + at, w);
   }
   if (o.flags & FQ3C_SNAKE2) {
-    const float4* ea = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.p0) + c0);
-    const float4* ib = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(o.p1) + c0);
+    const float4* ea = reinterpret_cast<const float4*>(par + 2 * GP_PAR);
+    const float4* ib = reinterpret_cast<const float4*>(par + 3 * GP_PAR);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 a = __ldg(ea + j), b = __ldg(ib + j);
+      const float4 a = ea[j], b = ib[j];
       const float x0 = v[4 * j] * a.x, x1 = v[4 * j + 1] * a.y, x2 = v[4 * j + 2] * a.z, x3 = v[4 * j + 3] * a.w;
       if (fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(x2), fabsf(x3))) < 1e6f) {
         v[4 * j] = fmaf(b.x, sin_sq_near(x0), v[4 * j]); v[4 * j + 1] = fmaf(b.y, sin_sq_near(x1), v[4 * j + 1]);
@@ -216,9 +218,10 @@ __device__ __noinline__ void epilogue_odd16(const fq3c_op& o, const int row, con
     epilogue_row8(o, row, col + 8 * h, v);
   }
 }
-__device__ __forceinline__ void gp_epilogue(const fq3c_op& o, const GemmPlan& g, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8]) {
+__device__ __forceinline__ void gp_epilogue(const fq3c_op& o, const GemmPlan& g, const int row, const int col, const uint32_t (&acc)[16], const uint32_t (&r)[8],
+                                            const float* par) {
   if (g.vec16) {
-    epilogue_row16(o, row, col, acc, r);
+    epilogue_row16(o, row, col, acc, r, par);
   } else {
     float v[16];
 #pragma unroll
@@ -344,21 +347,34 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
     const int pieces = g.bn / 16, half = (pieces + 1) / 2, p0 = (warp >> 2) * half, p1 = min(pieces, p0 + half);
     const int r_in = (warp & 3) * 32 + lane;
     const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && !g.staged;
-    int n = 0;
+    float* par = reinterpret_cast<float*>(gbase + g.stages * sb + 512);
+    const bool params = g.vec16 && !g.staged && (o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_SNAKE2));
+    int n = 0, par_n0 = -1;
     for (int t = t0; t < tiles; t += dt, ++n) {
       const int buf = bufs == 1 ? 0 : n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
+      if (params && n0 != par_n0) {      // another column tile (rows go first): its parameters, when the epilogue warps have left the last one's
+        par_n0 = n0;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const int col = n0 + tid;
+        if (tid < g.bn && col < o.N) {
+          const int c = col % o.col_mod;
+          if (o.flags & FQ3C_BIAS) par[tid] = reinterpret_cast<const float*>(o.bias)[c];
+          if (o.flags & FQ3C_SCALE) par[GP_PAR + tid] = reinterpret_cast<const float*>(o.scale)[c];
+          if (o.flags & FQ3C_SNAKE2) {
+            par[2 * GP_PAR + tid] = reinterpret_cast<const float*>(o.p0)[c];
+            par[3 * GP_PAR + tid] = reinterpret_cast<const float*>(o.p1)[c];
+          }
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+      }
       const int row = m0 + r_in;
       const bool rows = m0 + (warp & 3) * 32 < o.M;      // (warp-uniform)
       uint32_t rx[8], ry[8];
-      // the residual's next two pieces, on their way while the accumulator is waited for or worked on
-      auto ask = [&](const int p) {
-        if (resid && row < o.M) {
-          const bf16* src = reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16;
-          if (n0 + p * 16 < o.N) ld32(src, rx);
-          if (p + 1 < p1 && n0 + p * 16 + 16 < o.N) ld32(src + 16, ry);
-        }
+      // a piece of the residual, on its way while the accumulator is waited for or another piece is worked on
+      auto ask = [&](const int p, uint32_t (&x)[8]) {
+        if (resid && p < p1 && row < o.M && n0 + p * 16 < o.N) ld32(reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16, x);
       };
-      if (rows && p0 < p1) ask(p0);
+      if (rows) { ask(p0, rx); ask(p0 + 1, ry); }
       gp_wait(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ta = tmem + (uint32_t)(buf * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
@@ -385,9 +401,10 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
             }
             continue;
           }
-          gp_epilogue(o, g, row, n0 + p * 16, x, rx);
-          if (two) gp_epilogue(o, g, row, n0 + p * 16 + 16, y, ry);
-          if (p + 2 < p1) ask(p + 2);
+          gp_epilogue(o, g, row, n0 + p * 16, x, rx, par + p * 16);
+          ask(p + 2, rx);
+          if (two) gp_epilogue(o, g, row, n0 + p * 16 + 16, y, ry, par + p * 16 + 16);
+          ask(p + 3, ry);
         }
       if ((!rows || p0 >= p1) && lane == 0) mbar_arrive(acc_empty + 8u * buf);
     }
