@@ -27,9 +27,9 @@ enum fq3c_kind {
   FQ3C_ATTN = 4,      /* A=qkv [M, lda] (q | k | v), i0 heads, i1 kv heads, i2 head_dim, window K; C[M, i0*i2].  Stateful
                          decode: A holds `taps` history rows in front of the M query rows (query m = row taps + m), of
                          which the last min(*p0, taps) are valid (p0 = device int32: positions decoded so far).
-                         flags bit 0 (ABI 5): prompt-prefill form — head_dim 128, no history rows, M <= 2048: a two-phase
-                         kernel (lanes over keys for the scores, lanes over dims for the output) with the same rounding
-                         points; fp32 sums in another order                                                           */
+                         flags bit 0 (ABI 5): prompt-prefill form — head_dim 128, no history rows, the same rounding points,
+                         fp32 sums in another order: tcgen05 above 80 rows (M not limited), below it (and, M <= 2048, for
+                         addresses the former does not take) a two-phase kernel on the CUDA cores                     */
   FQ3C_DWCONV = 5,    /* depthwise causal conv k=taps: C[m,c] = bias[c] + sum_j B(f32)[c,j] A[m-(taps-1)+j, c]; rows down
                          to -i0 in front of A are history rows (stateful decode), further back reads as zero        */
   FQ3C_LAYERNORM = 6, /* C = layernorm(A) * scale + bias (f32), eps=f0                                      */
@@ -263,14 +263,15 @@ typedef struct fq3c_op {
   const void* p1;        /* f32 */
   void* C;
   void* C2;
-  void* ws;              /* GEMM, optional: fp32 workspace for split-K partial tiles (>= splits * M * round8(N) * 4 bytes are used); */
-  int64_t ws_bytes;      /* NULL / 0 = never split.  Ops of one stream-ordered list may share it.                                  */
+  void* ws;              /* GEMM, optional: not NULL = a short product may be split over K.  The splits are summed in a cluster's shared memory; */
+  int64_t ws_bytes;      /* only c_in = 8 modulo 16 over several taps keeps partial tiles here (>= splits * M * round8(N) * 4 bytes are used).
+                            Ops of one stream-ordered list may share it.                                                        */
   int32_t m_begin;       /* GEMM: only output rows [m_begin, M) are computed (tail-only streaming decode); pointers stay at row 0 */
   int32_t reserved;      /* GEMM: 1 = no op of the list writes B, so a launch may read it before the launches in front of it have ended; else 0 */
   /* GEMM, optional (ABI 5): the RMSNorm that reads the finished output rows, fused behind the epilogue — a decoder layer's norm
    * reads exactly the residual stream its o / down projection just wrote.  norm_out bf16 [M, norm_ld] = FQ3C_RMSNORM(C rows)
-   * with weights norm_w (f32 [N]) and eps norm_eps, same arithmetic and summation order as the stand-alone op.  With split-K it
-   * runs inside the reduction kernel (one CTA per row), otherwise as one more launch.  Not with FQ3C_SWIGLU / FQ3C_OUT_F32. */
+   * with weights norm_w (f32 [N]) and eps norm_eps, same arithmetic and summation order as the stand-alone op.  It is one
+   * more launch, which begins while the product still runs and waits for it.  Not with FQ3C_SWIGLU / FQ3C_OUT_F32. */
   void* norm_out;
   const void* norm_w;
   int32_t norm_ld;

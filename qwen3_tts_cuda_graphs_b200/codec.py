@@ -94,8 +94,8 @@ def vocoder_tail_starts(rows0: int, upsample_rates, skip: int, trim: str = "both
 
 def fuse_row_norms(ops: list) -> list:
     """An RMSNORM op that reads exactly the rows the GEMM before it wrote becomes that GEMM's fused norm (fq3c_op.norm_out):
-    inside the split-K reduction when the GEMM is split, one small launch otherwise — same arithmetic, fewer launches (two per
-    transformer layer of the prompt prefill and of the codec).  FQ3C_FUSE_NORM=0 keeps the ops apart."""
+    a small launch that begins while the GEMM still runs and waits for it — same arithmetic (two per transformer layer of the prompt
+    prefill and of the codec).  FQ3C_FUSE_NORM=0 keeps the ops apart."""
     if os.environ.get("FQ3C_FUSE_NORM", "1") == "0":
         return ops
     out = []
@@ -110,7 +110,8 @@ def fuse_row_norms(ops: list) -> list:
 
 
 def attach_splitk_workspace(ops, device, keep) -> None:
-    """One fp32 workspace per stream-ordered op list: every short GEMM of the list may use it for split-K partial tiles."""
+    """One fp32 workspace per stream-ordered op list: it allows every short GEMM of the list to be split over K (most sum their partial tiles in
+    the shared memory of a cluster; the kernel for c_in = 8 modulo 16 over several taps keeps them here)."""
     need = 0
     for o in ops:
         if o.kind == K_GEMM and 0 < o.M <= SPLITK_MAX_ROWS and o.K >= 512:

@@ -67,7 +67,8 @@ __device__ __forceinline__ float ex2f(const float x) {
 // tensor memory.  While one group's threads work, the tensor pipe has the other group's products.  The reference is the first tile's maximum and
 // moves only when a later one is more than 8 above it: then the row's output is rescaled in tensor memory.  Tiles outside every row's window, chunk
 // and kept positions are not fetched.
-// Bound by the tensor pipe (about 115 cycles per 128 x 128 x 16 MMA: 24 of them a tile) and, with a cap, by the special-function unit (three a score).
+// Bound by the chain scores -> maximum -> weights -> output of a group (24 MMAs of 64 cycles a tile are about half of it; the other group fills part of the
+// rest) and, with a cap, by the special-function unit (three a score).
 template <int MODE>
 __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __grid_constant__ AttnArgs a) {
   extern __shared__ unsigned char at_raw[];
