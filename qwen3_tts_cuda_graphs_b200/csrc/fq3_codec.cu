@@ -412,8 +412,8 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 // Split-K (splits > 1, short-and-wide problems that would leave most SMs idle): blockIdx.z takes a contiguous range of
 // k-blocks and stores its raw fp32 tile into the workspace [split][M][Nw]; fq3c_splitk_reduce_kernel adds the splits in
 // order and applies the fused epilogue.
-// This kernel is left for operands that a tensor map does not take (c_in = 8 modulo 16 over several taps); everything else runs on
-// fq3c_gemm_persist_kernel (fq3_gemm.cuh).
+// This kernel is left for c_in = 8 modulo 16 over several taps, where a 16-column MMA step would straddle two taps of a tensor map's row;
+// everything else runs on fq3c_gemm_persist_kernel (fq3_gemm.cuh).
 template <int MINB>  // CTAs per SM the register budget is planned for: 2 with three stages, 1 with six
 __global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3c_op o, const int BN, const int splits, const int Nw, const int NST) {
   extern __shared__ unsigned char tsmem_raw[];
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(TTHREADS, MINB) fq3c_gemm_tc5_kernel(const fq3
 
 // RVQ dequantiser front half: gather + sum codebook rows. C[m, 0:dim] = sum of the first i0 groups, C[m, dim:2dim] = rest.
 // second half of a split-K GEMM: a thread owns eight consecutive columns of a row, adds the splits in order (deterministic)
-// and runs the same fused epilogue the single-pass kernel would have run
+// and runs the same fused epilogue the single-pass kernel would have run.  (Only behind fq3c_gemm_tc5_kernel: the persistent kernel sums in its cluster.)
 __global__ void __launch_bounds__(256) fq3c_splitk_reduce_kernel(const fq3c_op o, const int splits, const int Nw) {
   const int groups = Nw >> 3;
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1038,7 +1038,7 @@ __global__ void fq3c_snake_kernel(const fq3c_op o) {
 
 // A convolution to ONE output channel (the vocoder's last layer: 7 taps x 96 channels): a dot product per row, not a matrix product.  A block stages the rows
 // its 256 outputs see once (the 64 x 64 tensor-core tile read them once per tap and threw 63 of 64 columns away) and every thread forms one
-// output, eight channels a step, f32 sums.  Bound by shared memory (one row's 16-byte pieces per lane).  491 520 rows: 178 -> 30 us.
+// output, eight channels a step, f32 sums.  Bound by shared memory (one row's 16-byte pieces per lane).  491 520 rows: 178 -> 51 us.
 constexpr int C1_ROWS = 256, C1_SPAN = 64, C1_CIN = 128;
 __global__ void __launch_bounds__(C1_ROWS) fq3c_conv1_kernel(const fq3c_op o, const int lo, const int span) {
   grid_dep_begin();
@@ -1164,8 +1164,9 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   }
   long kl = 0, ep = 0;
   if (g.splits == 1) {
-    // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  Measured: a k-block (four MMAs) takes 427 cycles at 32
-    // columns, 458 at 128, 480 at 224, 512 at 256, or its operand bytes at about 60 a cycle; the epilogue about 20 a column, four times that with sines.
+    // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  Measured: a k-block (four MMAs, a
+    // commit, the waits on both sides) takes 427 cycles at 32 columns, 458 at 128, 480 at 224, 512 at 256: the issuing warp's loop, not the tensor pipe, which is
+    // busy for 130-510 of them; or its operand bytes at the 60 a cycle that L2 gives one SM.  The epilogue takes about 20 a column, four times that with sines.
     long best = -1;
     const int per_col = (o.flags & FQ3C_SNAKE2) ? 80 : 20;
     for (int cand = 256; cand >= 16; cand -= 16) {
@@ -1267,6 +1268,22 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     if (b_f32) fq3s_ggemv_kernel<float, float><<<grid, 256, smem, s>>>(g);
     else if (a_f32) fq3s_ggemv_kernel<float, bf16><<<grid, 256, smem, s>>>(g);
     else fq3s_ggemv_kernel<bf16, bf16><<<grid, 256, smem, s>>>(g);
+    return 0;
+  }
+  // bf16 rows of whole 16-byte pieces (what its copies ask for): the pipelined product, faster at every size (figures at the kernel)
+  if (!a_f32 && !b_f32 && !((g.K | g.lda | g.ldb | g.a_zstride) & 7) && !((g.b_zstride | g.b_estride) & 7) &&
+      !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15)) {
+    static bool pattr[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !pattr[dev]) {
+      cudaFuncSetAttribute(fq3s_gemm_pipe_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GQ_SMEM);
+      cudaFuncSetAttribute(fq3s_gemm_pipe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GQ_SMEM);
+      pattr[dev] = true;
+    }
+    const dim3 pgrid((g.N + GQ_BN - 1) / GQ_BN, (g.M + GQ_BM - 1) / GQ_BM + (g.seg ? g.E : 0), zcount);
+    if (g.flags & FQ3C_SWIGLU) fq3s_gemm_pipe_kernel<true><<<pgrid, 256, GQ_SMEM, s>>>(g);
+    else fq3s_gemm_pipe_kernel<false><<<pgrid, 256, GQ_SMEM, s>>>(g);
     return 0;
   }
   // tall bf16 products (many rows per block / per expert, wide enough outputs): 128 x 128 tiles
@@ -1854,14 +1871,14 @@ int fq3c_run(const fq3c_op* ops, int n_ops, void* stream) {
 }
 static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, SideStream*& open) {
   cudaStream_t s = main_stream;
-  // FQ3C_PDL=0: every launch waits for the end of the one in front.  Otherwise a kernel that waits for itself may begin early, as long as the launch in
-  // front of it on its stream belongs to this list (what ran before the list is complete when its first launch begins).
-  static const bool pdl = [] { const char* e = getenv("FQ3C_PDL"); return e == nullptr || atoi(e) != 0; }();
+  // The codec's kernels wait for the launches in front themselves and may begin early, as long as the launch in front on their stream belongs to this list
+  // (what ran before the list is complete when its first launch begins): a prompt of 39 rows through 28 layers 1676 -> 1497 us, a codec window 1059 -> 972.
+  // The sequence models' kernels are launched one behind the other: early launches made their replays slower (a request of 24 tokens 5.4 -> 6.4 ms).
   bool chained = false;
   for (int i = 0; i < n_ops; ++i) {
     const fq3c_op& o = ops[i];
     if (o.M <= 0) continue;
-    const bool after = pdl && chained;
+    const bool after = chained;
     chained = o.kind != FQ3C_BRANCH;
     switch (o.kind) {
       case FQ3C_BRANCH: {
@@ -1919,7 +1936,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
             if (L.half) launch_after(fq3c_gemm_persist_kernel<2>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
             else launch_after(fq3c_gemm_persist_kernel<1>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
             if (o.norm_out) {
-              launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, pdl, 1, o);
+              launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, true, 1, o);
               count_launches(1);
             }
             break;

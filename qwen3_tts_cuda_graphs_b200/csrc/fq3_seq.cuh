@@ -189,6 +189,64 @@ __device__ __forceinline__ void sg_fetch16(const T* p, const bool vec, const int
   r[0] = make_uint4(u[0], u[1], u[2], u[3]);
   r[1] = make_uint4(u[4], u[5], u[6], u[7]);
 }
+// The epilogue of a warp's 32 x 32 quadrant of m16n8k16 accumulators, first row and column r0 and n0.
+template <bool GLU>
+__device__ __forceinline__ void sg_quad_epilogue(const SeqGemm& g, const float (&acc)[2][4][4], const int r0, const int row_end, const int n0, const int ccol, const int lane) {
+  if constexpr (GLU) {      // an accumulator pair (q, q + 1) is one gated unit
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; q += 2) {
+        const int r = r0 + i * 16 + (lane >> 2) + (q >> 1) * 8;
+        if (r >= row_end) continue;
+        const float w = sg_row_scale(g, r);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int n = n0 + j * 8 + (lane & 3) * 2;
+          if (n + 1 < g.N) sg_store_glu(g, r, ccol, n, acc[i][j][q], acc[i][j][q + 1], w);
+        }
+      }
+    return;
+  }
+  const bool pairs = !((g.ldc | ccol | n0) & 1) && !(reinterpret_cast<uintptr_t>(g.C) & 7);      // two columns a store
+  auto fin = [&](float v, const int n) {
+    if (g.flags & FQ3C_BIAS) v += g.bias[ccol + n];
+    if (g.flags & FQ3C_GELU) v = gelu_f(v);
+    if (g.flags & FQ3C_GELU_TANH) v = gelu_tanh_f(v);
+    if (g.flags & FQ3C_SIGMOID) v = sigmoid_f(v);
+    if (g.flags & FQ3C_RELU2) { v = fmaxf(v, 0.f); v *= v; }
+    return v;
+  };
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; q += 2) {
+      const int r = r0 + i * 16 + (lane >> 2) + (q >> 1) * 8;
+      if (r >= row_end) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + j * 8 + (lane & 3) * 2;
+        if (n >= g.N) continue;
+        const size_t ci = (size_t)r * g.ldc + ccol + n;
+        const float v0 = fin(acc[i][j][q], n);
+        if (n + 1 == g.N) {
+          if (g.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(g.C)[ci] = v0;
+          else reinterpret_cast<bf16*>(g.C)[ci] = __float2bfloat16_rn(v0);
+          continue;
+        }
+        const float v1 = fin(acc[i][j][q + 1], n + 1);
+        if (g.flags & FQ3C_OUT_F32) {
+          float* c = reinterpret_cast<float*>(g.C) + ci;
+          if (pairs) *reinterpret_cast<float2*>(c) = make_float2(v0, v1);
+          else { c[0] = v0; c[1] = v1; }
+        } else {
+          bf16* c = reinterpret_cast<bf16*>(g.C) + ci;
+          if (pairs) *reinterpret_cast<__nv_bfloat162*>(c) = __floats2bfloat162_rn(v0, v1);
+          else { c[0] = __float2bfloat16_rn(v0); c[1] = __float2bfloat16_rn(v1); }
+        }
+      }
+    }
+}
 template <typename TA, bool GLU = false>      // GLU: the gated-unit epilogue (a variant of its own, so that the plain one compiles as it always did)
 __global__ void __launch_bounds__(128) fq3s_gemm_mma_kernel(const SeqGemm g) {
   constexpr int LD = 32 + 8;
@@ -268,46 +326,101 @@ __global__ void __launch_bounds__(128) fq3s_gemm_mma_kernel(const SeqGemm g) {
     }
     __syncthreads();
   }
-  const int ccol = z * g.c_zstride;
-  if constexpr (GLU) {      // an accumulator pair (q, q + 1) is one gated unit
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int q = 0; q < 4; q += 2) {
-        const int r = row0 + wm + i * 16 + (lane >> 2) + (q >> 1) * 8;
-        if (r >= row_end) continue;
-        const float w = sg_row_scale(g, r);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = col0 + wn + j * 8 + (lane & 3) * 2;
-          if (n + 1 < g.N) sg_store_glu(g, r, ccol, n, acc[i][j][q], acc[i][j][q + 1], w);
-        }
-      }
-    return;
+  sg_quad_epilogue<GLU>(g, acc, row0 + wm, row_end, col0 + wn, z * g.c_zstride, lane);
+}
+
+// Rows of whole 16-byte pieces, bf16 on both sides (the grouped products of the experts): 128 x 64 tiles, eight warps, each a 32 x 32 quadrant (a quadrant
+// behind the expert's last row does nothing), three stages of 64 k by cp.async, 16-byte pieces exclusive-ored with the row against bank conflicts.  The sums run
+// over k in the other kernels' order.  Bound by the L2 latency of the stages in flight (three blocks per SM, 48 KB each).  A whole layer of 16 experts, two a row (1024 x 768 gated,
+// shared expert and router beside them), against the 64 x 64 and 128 x 128 tiles staged through registers: 33 rows 101 -> 70 us, 701 171 -> 115, 1500 250 -> 165,
+// 3000 360 -> 235, 6000 562 -> 397: at every size, so there is no line between the two.
+constexpr int GQ_BM = 128, GQ_BN = 64, GQ_BK = 64, GQ_ST = 3, GQ_STAGE = (GQ_BM + GQ_BN) * GQ_BK * 2, GQ_SMEM = GQ_ST * GQ_STAGE;
+template <bool GLU>
+__global__ void __launch_bounds__(256, 3) fq3s_gemm_pipe_kernel(const SeqGemm g) {
+  extern __shared__ __align__(128) unsigned char gq[];
+  const int tid = threadIdx.x, z = blockIdx.z, warp = tid >> 5, lane = tid & 31;
+  int row0, row_end;
+  const bf16* Bp = reinterpret_cast<const bf16*>(g.B) + (size_t)z * g.b_zstride;
+  if (g.seg) {
+    int t = blockIdx.y, e = 0;
+    row0 = -1; row_end = 0;
+    for (; e < g.E; ++e) {
+      const int s0 = g.seg[e], s1 = g.seg[e + 1], nt = (s1 - s0 + GQ_BM - 1) / GQ_BM;
+      if (t < nt) { row0 = s0 + t * GQ_BM; row_end = s1; break; }
+      t -= nt;
+    }
+    if (row0 < 0) return;
+    Bp += (size_t)e * g.b_estride;
+  } else {
+    row0 = blockIdx.y * GQ_BM; row_end = g.M;
   }
+  const int col0 = blockIdx.x * GQ_BN;
+  const bf16* Ap = reinterpret_cast<const bf16*>(g.A) + (size_t)(z % g.a_mod) * g.a_zstride;
+  // loaders: thread -> piece tid % 8 of rows tid / 8 + 32 i
+  const int piece = tid & 7, lr = tid >> 3;
+  int a_row[4];                                  // -1: behind the expert's last row
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = row0 + lr + 32 * i;
+    a_row[i] = r < row_end ? (g.rows ? g.rows[r] : r) : -1;
+  }
+  const int swz = (piece ^ (lr & 7)) * 16;      // (rows 32 apart share it)
+  auto load = [&](const int kt) {
+    unsigned char* st = gq + (kt % GQ_ST) * GQ_STAGE + lr * 128 + swz;
+    const int k = kt * GQ_BK + piece * 8;
+    const bool in = k < g.K;
+    const int kk = in ? k : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cp_async16(st + i * 32 * 128, Ap + (size_t)max(a_row[i], 0) * g.lda + kk, in && a_row[i] >= 0);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int n = col0 + lr + 32 * i;
+      cp_async16(st + GQ_BM * 128 + i * 32 * 128, Bp + (size_t)min(n, g.N - 1) * g.ldb + kk, in && n < g.N);
+    }
+  };
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const bool work = row0 + wm < row_end && col0 + wn < g.N;
+  float acc[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = row0 + wm + i * 16 + (lane >> 2) + (q >> 1) * 8;
-        const int n = col0 + wn + j * 8 + (lane & 3) * 2 + (q & 1);
-        if (r >= row_end || n >= g.N) continue;
-        float v = acc[i][j][q];
-        if (g.flags & FQ3C_BIAS) v += g.bias[ccol + n];
-        if (g.flags & FQ3C_GELU) v = gelu_f(v);
-        if (g.flags & FQ3C_GELU_TANH) v = gelu_tanh_f(v);
-        if (g.flags & FQ3C_SIGMOID) v = sigmoid_f(v);
-        if (g.flags & FQ3C_RELU2) { v = fmaxf(v, 0.f); v *= v; }
-        const size_t ci = (size_t)r * g.ldc + ccol + n;
-        if (g.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(g.C)[ci] = v;
-        else reinterpret_cast<bf16*>(g.C)[ci] = __float2bfloat16_rn(v);
-      }
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+  // ldmatrix lanes.  A (row-major [m][k]): matrices rows 0-7 / 8-15 at k, then at k + 8.  B ([n][k]): columns n 0-7 at k, k + 8, then n 8-15.
+  const int ar = wm + (lane & 15), ap = lane >> 4, br = wn + (lane & 7) + ((lane >> 4) << 3), bp = (lane >> 3) & 1;
+  const int KT = (g.K + GQ_BK - 1) / GQ_BK;
+#pragma unroll
+  for (int t = 0; t < GQ_ST - 1; ++t) {
+    if (t < KT) load(t);
+    cp_async_commit();
+  }
+  for (int kt = 0; kt < KT; ++kt) {
+    cp_async_wait<GQ_ST - 2>();
+    __syncthreads();                            // the stage has landed for all, and everyone is done with the one that is filled next
+    if (kt + GQ_ST - 1 < KT) load(kt + GQ_ST - 1);
+    cp_async_commit();
+    if (!work) continue;
+    const unsigned char* as = gq + (kt % GQ_ST) * GQ_STAGE;
+    const unsigned char* bs = as + GQ_BM * 128;
+#pragma unroll
+    for (int kk = 0; kk < GQ_BK / 16; ++kk) {
+      uint32_t a[2][4], b[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldmatrix_x4(a[i], as + (ar + 16 * i) * 128 + (((2 * kk + ap) ^ (ar & 7)) * 16));
+#pragma unroll
+      for (int j = 0; j < 2; ++j) ldmatrix_x4(b[j], bs + (br + 16 * j) * 128 + (((2 * kk + bp) ^ (br & 7)) * 16));
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma16816(acc[i][j], a[i], b[j >> 1][(j & 1) * 2], b[j >> 1][(j & 1) * 2 + 1]);
+    }
+  }
+  if (work) sg_quad_epilogue<GLU>(g, acc, row0 + wm, row_end, col0 + wn, z * g.c_zstride, lane);
 }
 
 // The same product for tall operands (hundreds of rows per block / expert): 128 x 128 x 32 tiles, eight warps of 64 x 32 each, fragments
-// by ldmatrix.  Halves the operand traffic per output of the 64 x 64 kernel and runs 16 MMAs per warp between two barriers.
+// by ldmatrix (f32 rows, or rows that are not whole 16-byte pieces).  Halves the operand traffic per output of the 64 x 64 kernel and runs 16 MMAs per warp between two barriers.
 template <typename TA, bool GLU = false>
 __global__ void __launch_bounds__(256) fq3s_gemm_mma128_kernel(const SeqGemm g) {
   constexpr int LD = 32 + 8, BM = 128, BN = 128;
