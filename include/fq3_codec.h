@@ -267,7 +267,9 @@ typedef struct fq3c_op {
   int64_t ws_bytes;      /* only c_in = 8 modulo 16 over several taps keeps partial tiles here (>= splits * M * round8(N) * 4 bytes are used).
                             Ops of one stream-ordered list may share it.                                                        */
   int32_t m_begin;       /* GEMM: only output rows [m_begin, M) are computed (tail-only streaming decode); pointers stay at row 0 */
-  int32_t reserved;      /* GEMM: 1 = no op of the list writes B, so a launch may read it before the launches in front of it have ended; else 0 */
+  int32_t reserved;      /* GEMM, bit 0: no op of the list writes B, so a launch may read it before the launches in front of it have ended.  GEMM,
+                            ATTN and CACHE_ATTN on tcgen05, bit 1: the first operand tile is never asked for and the waits are short, so
+                            that one runs out (tests of the error path: NaN outputs, fq3c_wait_errors) */
   /* GEMM, optional (ABI 5): the RMSNorm that reads the finished output rows, fused behind the epilogue — a decoder layer's norm
    * reads exactly the residual stream its o / down projection just wrote.  norm_out bf16 [M, norm_ld] = FQ3C_RMSNORM(C rows)
    * with weights norm_w (f32 [N]) and eps norm_eps, same arithmetic and summation order as the stand-alone op.  It is one
@@ -285,8 +287,10 @@ const char* fq3c_last_error(void);
 int fq3c_run(const fq3c_op* ops, int n_ops, void* stream);
 /* number of kernel launches issued so far by this process through fq3c_run / fq3c_graph_launch */
 int64_t fq3c_launch_count(void);
-/* ABI 11: nonzero when a kernel's bounded wait for its own copy ran out on the current device (its outputs are NaN); synchronises */
+/* ABI 11: nonzero when a kernel's bounded wait for its own copies or products ran out on the current device (its outputs are NaN); synchronises */
 int fq3c_wait_errors(void);
+/* the same for any device and without synchronising: what launches that have ended by now left (stays set) */
+int fq3c_wait_failed(void);
 /* A decode plan is static for a given frame count: capture its launches once (stream capture of fq3c_run) and replay
  * them as one CUDA graph.  The ops' buffers must stay alive and at the same addresses for the life of the graph. */
 int fq3c_graph_create(const fq3c_op* ops, int n_ops, void** out_graph);

@@ -149,6 +149,7 @@ def load_lib():
     lib.fq3c_run.argtypes = [C.POINTER(Op), C.c_int, C.c_void_p]
     lib.fq3c_launch_count.restype = C.c_int64
     lib.fq3c_wait_errors.restype = C.c_int
+    lib.fq3c_wait_failed.restype = C.c_int
     lib.fq3c_graph_create.restype = C.c_int
     lib.fq3c_graph_create.argtypes = [C.POINTER(Op), C.c_int, C.POINTER(C.c_void_p)]
     lib.fq3c_graph_launch.restype = C.c_int
@@ -263,9 +264,17 @@ class _Plan:
         self.graph_failed = False
 
 
+def check_waits() -> None:
+    """Raises when a kernel of an earlier launch gave up a bounded wait (its outputs are NaN).  Does not synchronise: where results of
+    launches reach the host, it is asked behind the synchronisation that is there anyway."""
+    if _lib is not None and _lib.fq3c_wait_failed() != 0:
+        raise CodecError("a kernel's wait for its own copies or products ran out: the outputs since then are not valid")
+
+
 def run_op_plan(lib, plan: _Plan, use_graphs: bool = True):
     """Launch a plan's op list on the current stream; from its second use on a plan replays as one CUDA graph (its launches are
     static: same ops, same buffers).  Shared by the codec decoder and the sequence-model engine."""
+    check_waits()
     if plan.arr is None:
         plan.arr = (Op * len(plan.ops))(*plan.ops)
     stream = torch.cuda.current_stream().cuda_stream

@@ -16,6 +16,8 @@ struct AttnArgs {
   int gate_ld, entry, out_f32;
   void* out;
   long ldo;
+  int tries;                // of a wait before it gives up
+  int lost;                 // 1: the first key tile is never asked for (tests of the error path)
 };
 enum { AT_PROMPT, AT_PLAIN, AT_CAP, AT_DIST };   // AT_PROMPT: scores rounded to bf16 before and behind the scale; AT_DIST: cap and distance penalty, both optional
 constexpr int AT_KEYS = 128, AT_THREADS = 640, AT_LOADERS = 96;
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   const uint32_t raw = smem_u32(at_raw), base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - raw);
   const uint32_t q_s = base, k_s = base + 2 * AT_TILE, v_s = base + 4 * AT_TILE, bars = base + 6 * AT_TILE;
-  const uint32_t q_full = bars, k_full = bars + 16, k_empty = bars + 32, v_full = bars + 48, v_empty = bars + 64, s_full = bars + 80, p_full = bars + 96, o_done = bars + 112;
+  const uint32_t q_full = bars, k_full = bars + 16, k_empty = bars + 32, v_full = bars + 48, v_empty = bars + 64, s_full = bars + 80, p_full = bars + 96, o_done = bars + 112, drain = bars + 144;      // (behind the words)
   uint32_t* words = reinterpret_cast<uint32_t*>(gbase + 6 * AT_TILE + 128);
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       mbar_init(v_full + 8u * i, AT_LOADERS); mbar_init(v_empty + 8u * i, 1);
       mbar_init(s_full + 8u * i, 1); mbar_init(p_full + 8u * i, 8); mbar_init(o_done + 8u * i, 1);
     }
+    mbar_init(drain, 1);
     words[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -96,6 +99,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const bool leader = elect_one();
   const uint32_t tmem = __shfl_sync(0xffffffffu, words[0], 0);   // S0 | S1 | O0 | O1, 128 columns each
   grid_dep_launch();
   grid_dep_wait();
@@ -119,20 +123,20 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
 
   if (warp == 19) {
-    const bool leader = elect_one();
     const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);   // F32 += BF16 x BF16, both K-major
     const uint32_t idesc_o = idesc_s | (1u << 16);                                                        // B (values: rows = keys) MN-major
     bool pend[2] = {false, false}, begun[2] = {false, false};
     int prev = 0;
-    gp_wait(q_full, 0, dead);
-    if (nq[1] > 0) gp_wait(q_full + 8, 0, dead);
+    bool gone = false;      // a wait gave up: nothing more is issued
+    if (!gp_wait(q_full, 0, dead, a.tries)) gone = true;
+    if (nq[1] > 0 && !gp_wait(q_full + 8, 0, dead, a.tries)) gone = true;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     // O[g] += P[g] V of the tile in stage st
     auto values = [&](const int g, const int st) {
       const uint32_t pa = tmem + g * 128, d = tmem + 256 + g * 128;
       // MN-major, 128-byte swizzle: 64 columns further is a half tile further, eight keys further 1024 bytes
       const uint64_t vd = (uint64_t)(((v_s + st * AT_TILE) & 0x3ffffu) >> 4) | ((uint64_t)(AT_TILE / 2 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-      if (leader) {
+      if (leader && !gone) {
 #pragma unroll
         for (int part = 0; part < 2; ++part)
 #pragma unroll
@@ -148,23 +152,23 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       if (more && !n0 && !n1) continue;
       const int st = n & 1;
       if (more) {
-        gp_wait(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead);
+        if (!gp_wait(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead, a.tries)) gone = true;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       if (pend[0] || pend[1]) {
-        gp_wait(v_full + 8u * (st ^ 1), (uint32_t)(((n - 1) >> 1) & 1), dead);
+        if (!gp_wait(v_full + 8u * (st ^ 1), (uint32_t)(((n - 1) >> 1) & 1), dead, a.tries)) gone = true;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         if (pend[g]) {
-          gp_wait(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead);
+          if (!gp_wait(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead, a.tries)) gone = true;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           values(g, st ^ 1);
           pend[g] = false;
         }
         if (g ? n1 : n0) {
-          if (leader) {
+          if (leader && !gone) {
             const uint64_t qd = umma_desc_sw128(q_s + g * AT_TILE), kd = umma_desc_sw128(k_s + st * AT_TILE);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           pend[g] = true;
         }
       }
-      if (leader) {
+      if (leader && !gone) {
         if (n > 0) umma_commit(v_empty + 8u * (st ^ 1));
         if (more) umma_commit(k_empty + 8u * st);
       }
@@ -186,8 +190,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   } else if (warp >= 16) {
     // ---- key and value tiles ----
     const int lt = tid - 512;
+    bool gone = false;
     const bf16 *kc = a.k + (size_t)kvh * 128, *vc = a.v + (size_t)kvh * 128;
     auto stage = [&](const bf16* src, const long ld, const uint32_t dst, const int j0, const uint32_t bar) {
+      if (gone) return;
       for (int i = lt; i < 128 * 16; i += AT_LOADERS) {      // 16 lanes read a row
         const int r = i >> 4, c = i & 15, j = j0 + r;
         const bool ok = j <= jend;
@@ -201,9 +207,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       if (!need(0, t) && !need(1, t)) continue;
       const int st = n & 1;
       const uint32_t ph = (uint32_t)(((n >> 1) - 1) & 1);
-      if (n >= 2) gp_wait(k_empty + 8u * st, ph, dead);
-      stage(kc, a.ldk, k_s + st * AT_TILE, t * AT_KEYS, k_full + 8u * st);
-      if (n >= 2) gp_wait(v_empty + 8u * st, ph, dead);
+      if (n >= 2 && !gp_wait(k_empty + 8u * st, ph, dead, a.tries)) gone = true;
+      if (n > 0 || !a.lost) stage(kc, a.ldk, k_s + st * AT_TILE, t * AT_KEYS, k_full + 8u * st);
+      if (n >= 2 && !gp_wait(v_empty + 8u * st, ph, dead, a.tries)) gone = true;
       stage(vc, a.ldv, v_s + st * AT_TILE, t * AT_KEYS, v_full + 8u * st);
       ++n;
     }
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       int c = 0;
       for (int t = 0; t < tilesg; ++t) {
         if (!need(g, t)) continue;
-        gp_wait(s_full + 8u * g, (uint32_t)(c & 1), dead);
+        gp_wait(s_full + 8u * g, (uint32_t)(c & 1), dead, a.tries);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int j0 = t * AT_KEYS, k0 = j0 + half * 64;
         // tiles that every row of the warp sees whole need no per-score test
@@ -336,7 +342,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         if (lane == 0) mbar_arrive(p_full + 8u * g);
         ++c;
       }
-      gp_wait(o_done + 8u * g, 0, dead);
+      gp_wait(o_done + 8u * g, 0, dead, a.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float f = 1.f, den = sum + meet(sum, c & 1);
       if (MODE != AT_PROMPT && a.sink && live) {
@@ -383,5 +389,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*dead) {      // products still on their way end before the memory they use is given back (every loading thread has waited for its own copies)
+    if (warp == 19 && leader) {
+      umma_commit(drain);
+      mbar_wait_bounded(drain, 0u, 1 << 14);
+    }
+    const int n = (nq[0] + nq[1]) * HG * 128;
+    for (int i = tid; i < n; i += AT_THREADS) {
+      const size_t at = (size_t)(m0 + i / (HG * 128)) * a.ldo + (size_t)kvh * HG * 128 + i % (HG * 128);
+      if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = __int_as_float(0x7fffffff);
+      else reinterpret_cast<uint16_t*>(a.out)[at] = 0x7fff;
+    }
+    __syncthreads();
+  }
   if (warp == 19) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }

@@ -11,6 +11,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "../../include/fq3_codec.h"
@@ -1183,6 +1184,8 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   g.acc_cols = 32;
   while (g.acc_cols < g.bn) g.acc_cols *= 2;
   g.early_b = o.reserved & 1;
+  g.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES;
+  g.lost = o.reserved & 2 ? 0 : -1;
   // (few rows and a costly epilogue: 39 rows of gated units 8.3 -> 7.5 us; without one the extra meeting costs 1 us more than it saves)
   g.staged = g.splits > 1 || (g.mt == 1 && g.a_rows <= 64 && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
   g.vec16 = gemm_vec16(o) ? 1 : 0;
@@ -1535,6 +1538,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       if (use_mma && !(o.flags & FQ3C_F32) && o.M > 8 && o.i2 == 128 && o.cin == 128 && !pool) {
         AttnArgs a{};
         a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.B); a.v = reinterpret_cast<const bf16*>(o.p1);
+        a.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES; a.lost = (o.reserved >> 1) & 1;
         a.ldq = o.lda; a.ldk = o.ldr; a.ldv = o.taps; a.H = o.i0; a.G = o.i1; a.M = o.M; a.p0 = reinterpret_cast<const int*>(o.p0);
         a.scale = o.f0; a.cap = o.f1; a.mult = o.f2; a.window = o.K; a.keep = o.a_rows; a.chunk = o.tap_off[0];
         a.r12 = reinterpret_cast<const float*>(o.bias); a.sink = reinterpret_cast<const float*>(o.scale); a.gate = reinterpret_cast<const float*>(o.res);
@@ -1827,6 +1831,43 @@ int fq3c_wait_errors(void) {
   return cudaMemcpyFromSymbol(&v, seq_wait_error, sizeof v) == cudaSuccess ? v : -1;
 }
 
+// The host's error words, one per device, made before a device's first launch (also when that one is captured: the calls are exempt from the capture).
+static std::atomic<volatile int*> wait_words[64];
+static bool wait_word_ready() {
+  static std::mutex making;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (wait_words[dev].load(std::memory_order_acquire)) return true;
+  std::lock_guard<std::mutex> lock(making);
+  if (wait_words[dev].load(std::memory_order_relaxed)) return true;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+  int* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool ok = cudaHostAlloc(reinterpret_cast<void**>(&p), 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess;
+  if (ok) {
+    *p = 0;
+    ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess &&
+         cudaMemcpyToSymbolAsync(seq_wait_host, &p, sizeof p, 0, cudaMemcpyHostToDevice, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+    if (s) cudaStreamDestroy(s);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ok) {
+    if (p) cudaFreeHost(p);
+    cudaGetLastError();
+    return false;
+  }
+  wait_words[dev].store(p, std::memory_order_release);
+  return true;
+}
+int fq3c_wait_failed(void) {
+  for (auto& w : wait_words) {
+    const volatile int* p = w.load(std::memory_order_acquire);
+    if (p && *p) return 1;
+  }
+  return 0;
+}
+
 // Opt-in shared-memory sizes are a per-DEVICE function attribute: a process that serves several GPUs (server.py --gpus N: one scheduler
 // thread per device) must set them on each device it launches on, not once per process.
 static bool device_attrs_ready() {
@@ -1863,6 +1904,7 @@ static SideStream* side_stream() {
 }
 static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, SideStream*& open);
 int fq3c_run(const fq3c_op* ops, int n_ops, void* stream) {
+  if (!wait_word_ready()) return fail("cannot make the error word of bounded waits");
   SideStream* open = nullptr;
   const int rc = run_ops(ops, n_ops, (cudaStream_t)stream, open);
   if (open && (cudaEventRecord(open->done, open->stream) != cudaSuccess || cudaStreamWaitEvent((cudaStream_t)stream, open->done, 0) != cudaSuccess))
@@ -2032,6 +2074,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         if (use_apf && (o.flags & 1) && o.i2 == 128 && o.taps == 0 && !o.p0) {
           AttnArgs a{};
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
+          a.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES; a.lost = (o.reserved >> 1) & 1;
           a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
           // up to 80 rows the kernel below is faster (a warp per query and head, no tile to stage): 64 rows 8.0 against 8.8 us, 100 rows 16.0 against 11.8
           if (use_apf != 2 && o.M > 80 && attn_tc_takes(a, AT_PROMPT)) {

@@ -17,6 +17,8 @@ struct GemmPlan {
   int early_b;   // B is not written by the launches in front: its first stages are asked for before they have ended
   int vec16;     // the epilogue may move 16 columns of a row at a time
   int staged;    // the epilogue takes its tile from shared memory, spread over all threads: split sums, and few rows (a CTA has one tile then)
+  int tries;     // of a wait before it gives up
+  int lost;      // k-block whose rows are never asked for (tests of the error path), else -1
 };
 constexpr int GP_EPI_WARPS = 8, GP_MMA_WARP = 8, GP_TMA_WARP = 9, GP_THREADS = 320;
 constexpr int GP_PAR = 256;         // columns of a tile at most: its bias, scale and SnakeBeta parameters lie in shared memory
@@ -25,23 +27,27 @@ __host__ __device__ constexpr int gp_a_bytes(int a_rows) { return (a_rows * TK *
 __host__ __device__ constexpr int gp_stage_bytes(int a_rows, int bn) { return gp_a_bytes(a_rows) + bn * TK * 2; }
 __host__ __device__ constexpr int gp_part_pitch(int bn) { return bn + 4; }   // floats per row of a partial tile: 16-byte rows, 4 banks apart
 
-// A bounded wait of a whole warp.  When the limit (about a second) runs out it sets the error word and `dead`, and this and all later waits of the block
-// return at once: the loops around them keep their counts and end on whatever is there.  (Each lane tries for itself: with a vote per try the waiting
-// warps took issue slots from the working ones.)
-__device__ __forceinline__ void gp_wait(const uint32_t bar, const uint32_t parity, volatile int* dead) {
+// A bounded wait of a whole warp.  When its tries run out (about a second) it sets the block's word `dead` and the error words; the block's other waits give up
+// when they see `dead`.  A lane whose wait gave up (false) issues no more copies, products or commits, so that no barrier gets an arrival that its phase does not
+// expect; at its end the kernel waits for what had been issued and fills its outputs with NaN.  (Each lane tries for itself: with a vote per try the
+// waiting warps took issue slots from the working ones.)
+constexpr int GP_TRIES = 1 << 20, GP_TRIES_TEST = 4096;
+__device__ __forceinline__ bool gp_wait(const uint32_t bar, const uint32_t parity, volatile int* dead, const int tries) {
+  bool there = true;
   int i = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if (++i > 256) {      // (a try suspends the thread for a while by itself)
-      if (*dead) break;
-      __nanosleep(i > 8192 ? 1000 : 20);
-      if (i > (1 << 20)) {
+    if (++i > 256 || i > tries) {      // (a try suspends the thread for a while by itself)
+      if (*dead || i > tries) {
         *dead = 1;
-        seq_wait_error = 1;
+        wait_ran_out();
+        there = false;
         break;
       }
+      __nanosleep(i > 8192 ? 1000 : 20);
     }
   }
   __syncwarp();
+  return there;
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
@@ -230,6 +236,18 @@ __device__ __forceinline__ void gp_epilogue(const fq3c_op& o, const GemmPlan& g,
   }
 }
 
+// NaN in place of `n` (even) columns of an output row, both outputs: a wait ran out
+__device__ __noinline__ void poison(const fq3c_op& o, const int row, const int col, const int n) {
+  if (row >= o.M) return;
+  const bool glu = o.flags & FQ3C_SWIGLU, f32 = (o.flags & FQ3C_OUT_F32) && (!glu || (o.flags & FQ3C_NOROUND));
+  for (int c = col; c < min(col + n, o.N); c += glu ? 2 : 1) {
+    const size_t at = (size_t)row * o.ldc + (glu ? c >> 1 : c);
+    if (f32) reinterpret_cast<float*>(o.C)[at] = __int_as_float(0x7fffffff);
+    else reinterpret_cast<uint16_t*>(o.C)[at] = 0x7fff;
+    if (o.flags & FQ3C_SNAKE2) reinterpret_cast<uint16_t*>(o.C2)[at] = 0x7fff;
+  }
+}
+
 // One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  Warp 9 asks for the operand
 // boxes up to `stages` k-blocks ahead, across tiles; warp 8 issues the MMAs of tile n + 1 into the second accumulator while warps 0-7 take tile n
 // through the epilogue.  With splits > 1 a cluster of CTAs shares one tile: each takes a run of k-blocks, leaves its f32 partial tile in its
@@ -247,6 +265,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   const uint32_t full = bars, empty = bars + 8u * g.stages, acc_full = bars + 16u * g.stages, acc_empty = acc_full + 16;
   uint32_t* words = reinterpret_cast<uint32_t*>(gbase + g.stages * sb + 16 * g.stages + 32);   // tensor-memory address | dead | k-blocks asked for
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
+  const uint32_t drain = acc_empty + 32;      // (behind the words)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int tiles = g.mt * g.nt, z = g.splits > 1 ? (int)(blockIdx.x % g.splits) : 0;
   const int t0 = g.splits > 1 ? (int)(blockIdx.x / g.splits) : (int)blockIdx.x, dt = g.staged ? tiles : (int)gridDim.x;
@@ -257,6 +276,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   if (tid == 0) {
     for (int s = 0; s < g.stages; ++s) { mbar_init(full + 8u * s, 1); mbar_init(empty + 8u * s, 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, GP_EPI_WARPS); }
+    mbar_init(drain, 1);
     words[1] = 0;
     words[2] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -277,10 +297,11 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
 
   // The two issuing warps run their loops whole, with one elected lane at the copies and MMAs: in code of a single lane every descriptor goes through
   // per-lane registers (a k-block took 700-800 cycles to issue that way, whatever its size).
+  const bool leader = elect_one();
   if (warp == GP_TMA_WARP) {
-    const bool leader = elect_one();
     const uint32_t tx = (uint32_t)(g.a_rows * TK * 2 + g.bn * TK * 2);
-    int it = 0, early = 0, st = 0;
+    int it = 0, early = 0, st = 0, asked = 0;
+    bool gone = false;
     uint32_t ph = 0;      // parity of the stage's current use
     if (g.early_b && t0 < tiles) {   // the first tile's weights
       early = min(g.stages, kb1 - kb0);
@@ -299,39 +320,40 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       const int n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
       int tap = kb0 / g.kpt, c = kb0 - tap * g.kpt;
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        if (it >= g.stages) gp_wait(empty + 8u * st, ph ^ 1u, dead);
+        if (it >= g.stages && !gp_wait(empty + 8u * st, ph ^ 1u, dead, g.tries)) gone = true;
         const uint32_t fb = full + 8u * st, a_dst = base + st * sb;
-        if (leader) {
+        if (leader && !gone) {
           if (it >= early) {
             mbar_expect(fb, tx);
             tma_2d(a_dst + ab, &tmB, tap * o.cin + c * TK, n0, fb);
           }
-          tma_2d(a_dst, &tmA, c * TK, m0 + o.tap_off[tap], fb);
+          if (it != g.lost) tma_2d(a_dst, &tmA, c * TK, m0 + o.tap_off[tap], fb);
+          asked = it + 1;
         }
         if (++c == g.kpt) { c = 0; ++tap; }
         if (++st == g.stages) { st = 0; ph ^= 1u; }
       }
     }
-    if (leader) words[2] = (uint32_t)max(it, early);
+    if (leader) words[2] = (uint32_t)max(asked, early);
   } else if (warp == GP_MMA_WARP) {
     grid_dep_wait();
-    const bool leader = elect_one();
     // instruction descriptor: D = F32, A = B = BF16, both K-major, N = bn, M = 128
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bn >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
     int st = 0, n = 0;
+    bool gone = false;
     uint32_t ph = 0;
     for (int t = t0; t < tiles; t += dt, ++n) {
       const int buf = n & 1;
       const uint32_t d = tmem + (uint32_t)(buf * g.acc_cols);
-      if (n >= 2) gp_wait(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead);
+      if (n >= 2 && !gp_wait(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead, g.tries)) gone = true;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int left = g.kpt - kb0 % g.kpt;      // k-blocks to the end of the tap
       for (int kb = kb0; kb < kb1; ++kb) {
-        gp_wait(full + 8u * st, ph, dead);      // (filled by the copy engine: no tensor-memory fence)
+        if (!gp_wait(full + 8u * st, ph, dead, g.tries)) gone = true;      // (filled by the copy engine: no tensor-memory fence)
         const uint64_t da = umma_desc_sw128(base + st * sb), db = umma_desc_sw128(base + st * sb + ab);
         const int mmas = --left == 0 ? g.tail : TK / 16;
         if (left == 0) left = g.kpt;
-        if (leader) {
+        if (leader && !gone) {
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk)
             if (kk < mmas) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);      // 16 columns = 32 bytes further
@@ -339,7 +361,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
         }
         if (++st == g.stages) { st = 0; ph ^= 1u; }
       }
-      if (leader) umma_commit(acc_full + 8u * buf);
+      if (leader && !gone) umma_commit(acc_full + 8u * buf);
     }
   } else {
     grid_dep_wait();
@@ -375,7 +397,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
         if (resid && p < p1 && row < o.M && n0 + p * 16 < o.N) ld32(reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16, x);
       };
       if (rows) { ask(p0, rx); ask(p0 + 1, ry); }
-      gp_wait(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead);
+      gp_wait(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead, g.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ta = tmem + (uint32_t)(buf * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
       if (rows)
@@ -414,11 +436,18 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
     const int n0 = (t0 / g.mt) * g.bn, m0 = o.m_begin + (t0 % g.mt) * TM;
     const int pieces = g.bn / 8, items = min(TM, o.M - m0) * pieces;
     const int i0 = (int)((long)items * z / g.splits), i1 = (int)((long)items * (z + 1) / g.splits);
+    int lost = 0;
     if (g.splits > 1) {      // every CTA of the cluster comes here, also after a wait that ran out
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (tid < g.splits) {      // whether that CTA's part can be used; looked at behind the sums
+        uint32_t far;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(smem_u32(words + 1)), "r"(tid));
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(lost) : "r"(far) : "memory");
+      }
     } else {
       __syncthreads();
+      lost = *dead;
     }
     for (int i = i0 + tid; i < i1; i += GP_THREADS) {
       const int r = i / pieces, p = i - r * pieces;
@@ -444,6 +473,8 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
         }
       epilogue_row8(o, m0 + r, n0 + p * 8, a);
     }
+    if (__syncthreads_or(lost))
+      for (int i = i0 + tid; i < i1; i += GP_THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
     if (g.splits > 1) {      // the others have read this CTA's partial tile (reads only: nothing to publish)
       asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -451,8 +482,20 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (*dead && tid == 0) {      // copies still on their way land before the shared memory is given back
-    for (int i = max(0, (int)words[2] - g.stages); i < (int)words[2]; ++i) mbar_wait_bounded(full + 8u * (i % g.stages), (uint32_t)((i / g.stages) & 1));
+  if (*dead) {      // copies and products still on their way end before the memory they use is given back
+    if (warp == GP_MMA_WARP && leader) {
+      umma_commit(drain);
+      mbar_wait_bounded(drain, 0u, 1 << 14);
+    }
+    if (tid < g.stages && tid < (int)words[2]) {
+      const int i = (int)words[2] - 1 - tid;
+      mbar_wait_bounded(full + 8u * (i % g.stages), (uint32_t)((i / g.stages) & 1), 1 << 14);
+    }
+    if (!g.staged)
+      for (int t = t0; t < tiles; t += dt) {
+        const int n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM, pieces = g.bn / 8;
+        for (int i = tid; i < TM * pieces; i += GP_THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
+      }
   }
   __syncthreads();
   if (warp == GP_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");

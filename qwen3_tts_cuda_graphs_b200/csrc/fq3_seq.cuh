@@ -2956,11 +2956,20 @@ __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(cons
   }
 }
 
-// set by a kernel whose bounded wait for its own copy ran out; its outputs are then NaN
+// set by a kernel whose bounded wait for its own copies or products ran out; its outputs are then NaN.  The second word is the same for the host: an int in pinned
+// memory (null until fq3c_run has made it), which can be looked at without a synchronisation.
 __device__ int seq_wait_error;
+__device__ volatile int* seq_wait_host;
+__device__ __noinline__ void wait_ran_out() {
+  seq_wait_error = 1;
+  if (seq_wait_host) {
+    *seq_wait_host = 1;
+    __threadfence_system();
+  }
+}
 // true when the barrier's phase completed, false when the limit ran out (about a second)
-__device__ __forceinline__ bool mbar_wait_bounded(const uint32_t bar, const uint32_t parity) {
-  for (int i = 0; i < (1 << 20); ++i) {
+__device__ __forceinline__ bool mbar_wait_bounded(const uint32_t bar, const uint32_t parity, const int tries = 1 << 20) {
+  for (int i = 0; i < tries; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if (i > 64) __nanosleep(256);
   }
@@ -3043,7 +3052,7 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
     const bool there = mbar_wait_bounded(smem_u32(&full[n & 1]), (uint32_t)((n >> 1) & 1));
     // the record is there, the transposed state too; everyone is done with the other buffer
     if (__syncthreads_or(!there)) {
-      if (tid == 0) { seq_wait_error = 1; mbar_wait_bounded(smem_u32(&full[n & 1]), (uint32_t)((n >> 1) & 1)); }
+      if (tid == 0) { wait_ran_out(); mbar_wait_bounded(smem_u32(&full[n & 1]), (uint32_t)((n >> 1) & 1)); }
       for (int i = tid; i < o.M * DVT; i += 128)
         if (j0 + i % DVT < dv) reinterpret_cast<float*>(o.C)[(size_t)(i / DVT) * o.ldc + (size_t)h * dv + j0 + i % DVT] = __int_as_float(0x7fc00000);
       return;

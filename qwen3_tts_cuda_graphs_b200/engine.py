@@ -266,6 +266,8 @@ class Engine:
     def status(self, idx: int = 0) -> _lib.Status:
         st = _lib.Status()
         _lib.check(self.lib.fq3_get_status(self.h, idx, C.byref(st), _stream()))
+        if self._dense:      # a prompt went through the op lists
+            self._dense.check_waits()
         return st
 
     def read_codes(self, idx: int, first: int, n: int) -> torch.Tensor:

@@ -18,6 +18,7 @@ from typing import Generator, List, Optional, Tuple, Union
 import numpy as np
 import torch
 
+from . import codec as _codec
 from .base_model import Qwen3TTSBaseModel
 from .predictor_graph import PredictorGraph
 from .sampling import set_default_engine
@@ -408,7 +409,9 @@ class FasterQwen3TTS:
     @staticmethod
     def _to_numpy(a) -> np.ndarray:
         if hasattr(a, "cpu"):
-            return a.flatten().float().cpu().numpy()
+            out = a.flatten().float().cpu().numpy()
+            _codec.check_waits()
+            return out
         return a.flatten() if hasattr(a, "flatten") else a
 
     def _decode_full(self, m, codec_ids, ref_codes=None) -> Tuple[List[np.ndarray], int]:

@@ -134,6 +134,8 @@ class DensePrefill:
         self.cap = cap
         self.cur_stream = 0
 
+    check_waits = staticmethod(_codec.check_waits)
+
     def close(self):
         for h in self.graphs.values():
             self.lib.fq3c_graph_destroy(h)
@@ -141,6 +143,7 @@ class DensePrefill:
 
     def run(self, stream_idx: int, embeds: torch.Tensor, R: int):
         """rows [0, R) of `embeds` (bf16 [T, H], device): fills the K/V cache of every layer for positions [0, R)."""
+        _codec.check_waits()
         if R > self.cap:
             self._build(max(64, (R + 63) // 64 * 64))
         arr = self.arr
