@@ -23,7 +23,7 @@ enum { AT_PROMPT, AT_PLAIN, AT_CAP, AT_DIST };   // AT_PROMPT: scores rounded to
 constexpr int AT_KEYS = 128, AT_THREADS = 640, AT_LOADERS = 96;
 constexpr int AT_TILE = 128 * 128 * 2;           // a query, key or value tile: two halves of 64 columns, 128-byte lines, 128-byte swizzle
 constexpr int AT_SMEM = 6 * AT_TILE + 1024 + 256 + 2 * 2 * 256 * 4;   // tiles, alignment, barriers, the half rows' maxima (two tiles in turn)
-constexpr float AT_SLACK = 8.f;                  // a row's reference score moves when its maximum is further above it than this
+constexpr float AT_SLACK = 11.f;                 // a row's reference moves when its maximum is further above it than this (in powers of two)
 
 __device__ __forceinline__ void tmem_ld32(const uint32_t a, float* f) {
   uint32_t v[32];
@@ -39,6 +39,8 @@ __device__ __forceinline__ void tmem_ld32(const uint32_t a, float* f) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
 }
+// 2^n for a whole number n <= 0, exactly (0 below the normal range)
+__device__ __forceinline__ float pow2_down(const float n) { return n < -126.f ? 0.f : __int_as_float(((int)n + 127) << 23); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(const uint32_t a, const uint32_t (&v)[16]) {
   asm volatile(
@@ -65,10 +67,11 @@ __device__ __forceinline__ float ex2f(const float x) {
 // A CTA takes two groups of 128 rows of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
 // staged tile.  Warps 0-7 and 8-15: two threads per row of group 0 and 1, 64 keys of a tile each; warps 16-18 stage key and value tiles of 128 positions (two
 // stages); warp 19 issues the MMAs.  Per group and tile: S = Q K^T into tensor memory; the row's threads scale, cap and mask its 128 scores, agree on the
-// maximum, take e^(score - reference) and write every weight as a bf16 pair hi + lo (16 mantissa bits) over S; O += hi V + lo V with the weights read from
-// tensor memory.  While one group's threads work, the tensor pipe has the other group's products.  The reference is the first tile's maximum and
-// moves only when a later one is more than 8 above it: then the row's output is rescaled in tensor memory.  Tiles outside every row's window, chunk
-// and kept positions are not fetched.
+// maximum, take 2^(score log2 e - reference) and write every weight as a bf16 pair hi + mid (16 mantissa bits) over S; O += hi V + mid V with the weights read from
+// tensor memory.  AT_PROMPT's weights keep their 24 bits: what the pair lacks goes over the hi parts as soon as the products with those have ended, while the ones
+// with the mid parts run, and makes a third product.  While one group's threads work, the tensor pipe has the other group's products.  The reference is a whole
+// number next to the first tile's maximum, so that neither it nor a rescaling rounds anything, and moves only when a later maximum is more than 2^11 above it: then
+// the row's output is rescaled in tensor memory.  Tiles outside every row's window, chunk and kept positions are not fetched.
 // Bound by the chain scores -> maximum -> weights -> output of a group (24 MMAs of 64 cycles a tile are about half of it; the other group fills part of the
 // rest) and, with a cap, by the special-function unit (three a score).
 template <int MODE>
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   const uint32_t raw = smem_u32(at_raw), base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - raw);
   const uint32_t q_s = base, k_s = base + 2 * AT_TILE, v_s = base + 4 * AT_TILE, bars = base + 6 * AT_TILE;
-  const uint32_t q_full = bars, k_full = bars + 16, k_empty = bars + 32, v_full = bars + 48, v_empty = bars + 64, s_full = bars + 80, p_full = bars + 96, o_done = bars + 112, drain = bars + 144;      // (behind the words)
+  const uint32_t q_full = bars, k_full = bars + 16, k_empty = bars + 32, v_full = bars + 48, v_empty = bars + 64, s_full = bars + 80, p_full = bars + 96, o_done = bars + 112, drain = bars + 144, h_done = bars + 152, l_full = bars + 168;      // (behind the words)
   uint32_t* words = reinterpret_cast<uint32_t*>(gbase + 6 * AT_TILE + 128);
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -87,6 +90,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       mbar_init(k_full + 8u * i, AT_LOADERS); mbar_init(k_empty + 8u * i, 1);
       mbar_init(v_full + 8u * i, AT_LOADERS); mbar_init(v_empty + 8u * i, 1);
       mbar_init(s_full + 8u * i, 1); mbar_init(p_full + 8u * i, 8); mbar_init(o_done + 8u * i, 1);
+      mbar_init(h_done + 8u * i, 1); mbar_init(l_full + 8u * i, 8);
     }
     mbar_init(drain, 1);
     words[1] = 0;
@@ -131,6 +135,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     if (!gp_wait(q_full, 0, dead, a.tries)) gone = true;
     if (nq[1] > 0 && !gp_wait(q_full + 8, 0, dead, a.tries)) gone = true;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    int nl[2] = {0, 0};
     // O[g] += P[g] V of the tile in stage st
     auto values = [&](const int g, const int st) {
       const uint32_t pa = tmem + g * 128, d = tmem + 256 + g * 128;
@@ -138,11 +143,21 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       const uint64_t vd = (uint64_t)(((v_s + st * AT_TILE) & 0x3ffffu) >> 4) | ((uint64_t)(AT_TILE / 2 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
       if (leader && !gone) {
 #pragma unroll
-        for (int part = 0; part < 2; ++part)
+        for (int part = 0; part < 2; ++part) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) umma_bf16_ta(d, pa + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, (begun[g] || part || kk) ? 1u : 0u);
-        if (prev == tiles[g] - 1) umma_commit(o_done + 8u * g);
+          if (MODE == AT_PROMPT && part == 0) umma_commit(h_done + 8u * g);
+        }
       }
+      if (MODE == AT_PROMPT) {
+        if (!gp_wait(l_full + 8u * g, (uint32_t)(nl[g]++ & 1), dead, a.tries)) gone = true;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (leader && !gone) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) umma_bf16_ta(d, pa + (kk >> 1) * 32 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, 1u);
+        }
+      }
+      if (leader && !gone && prev == tiles[g] - 1) umma_commit(o_done + 8u * g);
       begun[g] = true;
     };
     int n = 0, np[2] = {0, 0};
@@ -306,11 +321,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           if (h == 0) tmem_ld_wait();
         }
         mx = fmaxf(mx, meet(mx, c & 1));
-        if (c == 0) ref = mx;
-        else if (__any_sync(0xffffffffu, mx > ref + AT_SLACK)) {      // (from -inf too: nothing summed yet)
-          const bool up = mx > ref + AT_SLACK;
-          const float al = up ? (ref == -INFINITY ? 0.f : expf(ref - mx)) : 1.f;
-          if (up) ref = mx;
+        const float mk = rintf(mx * L2E);
+        if (c == 0) ref = mk;
+        else if (__any_sync(0xffffffffu, mk > ref + AT_SLACK)) {      // (from -inf too: nothing summed yet)
+          const bool up = mk > ref + AT_SLACK;
+          const float al = up ? (ref == -INFINITY ? 0.f : pow2_down(ref - mk)) : 1.f;
+          if (up) ref = mk;
           sum *= al;
 #pragma unroll 1
           for (int i = 0; i < 4; ++i) {      // the product in front has ended: this tile's scores were issued behind it
@@ -322,7 +338,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
             tmem_st16(o_t + i * 16, x);
           }
         }
-        const float u = ref == -INFINITY ? 0.f : -ref * L2E;
+        const float u = ref == -INFINITY ? 0.f : -ref;
+        uint32_t rest[2][16];      // AT_PROMPT
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t hi[16], lw[16];
@@ -331,7 +348,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
             const float p = ex2f(fmaf(s[h][2 * j], L2E, u)), q = ex2f(fmaf(s[h][2 * j + 1], L2E, u));
             sum += p + q;
             hi[j] = bf_pair(p, q);
-            lw[j] = bf_pair(p - __uint_as_float(hi[j] << 16), q - __uint_as_float(hi[j] & 0xffff0000u));
+            const float p1 = p - __uint_as_float(hi[j] << 16), q1 = q - __uint_as_float(hi[j] & 0xffff0000u);
+            lw[j] = bf_pair(p1, q1);
+            if (MODE == AT_PROMPT) rest[h][j] = bf_pair(p1 - __uint_as_float(lw[j] << 16), q1 - __uint_as_float(lw[j] & 0xffff0000u));
           }
           tmem_st16(s_t + h * 32, hi);
           tmem_st16(s_t + h * 32 + 16, lw);
@@ -340,15 +359,25 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full + 8u * g);
+        if (MODE == AT_PROMPT) {
+          gp_wait(h_done + 8u * g, (uint32_t)(c & 1), dead, a.tries);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          tmem_st16(s_t, rest[0]);
+          tmem_st16(s_t + 32, rest[1]);
+          tmem_st_wait();
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(l_full + 8u * g);
+        }
         ++c;
       }
       gp_wait(o_done + 8u * g, 0, dead, a.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float f = 1.f, den = sum + meet(sum, c & 1);
       if (MODE != AT_PROMPT && a.sink && live) {
-        const float sk = a.sink[head], mm = fmaxf(ref, sk);
-        f = ref == -INFINITY ? 0.f : expf(ref - mm);
-        den = den * f + expf(sk - mm);
+        const float sk = a.sink[head], mm = fmaxf(ref, rintf(sk * L2E));
+        f = ref == -INFINITY ? 0.f : pow2_down(ref - mm);
+        den = den * f + exp2f(fmaf(sk, L2E, -mm));
       }
       const int m = pos - P;
       float sc = f / den;

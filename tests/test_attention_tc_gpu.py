@@ -60,6 +60,37 @@ def test_prompt_rows(rows, heads, kv, window):
     assert rel(out, want.reshape(rows, -1)) < 2.0 ** -9      # one rounding to bf16: 2^-9 at most, about 2^-9.3 on average
 
 
+def test_prompt_weights_keep_32_bits():
+    """Outputs that are small differences of large terms show the weights' own error past the rounding of the output: v = 1 behind one score and -e^(difference),
+    as the sum of three bf16 values, behind another."""
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    torch.manual_seed(3)
+    rows, scale = 384, 128 ** -0.5
+    a = torch.zeros(rows, 3 * 128, device="cuda", dtype=torch.bfloat16)
+    q, k, v = a[:, :128], a[:, 128:256], a[:, 256:]
+    q[:, 0], q[:, 1], q[:, 2] = torch.rand(rows, device="cuda").bfloat16() * 30, torch.rand(rows, device="cuda").bfloat16() * 30, 1.0
+    k[0, 0], k[1:4, 1], k[4:, 2] = 1.0, 1.0, -400.0      # the other keys' weights are nothing
+    s = lambda x: (x.double() * scale).bfloat16().double()
+    s1, s2 = s(q[:, 0]), s(q[:, 1])
+    t = torch.arange(256, 384, device="cuda")      # the rows looked at, one column each
+    rest = -torch.exp(s1 - s2)[t]
+    v[0] = 1.0
+    for j in (1, 2, 3):
+        v[j, t - 256] = rest.bfloat16()
+        rest = rest - v[j, t - 256].double()
+    out = torch.zeros(rows, 128, device="cuda", dtype=torch.bfloat16)
+    o = K.Op()
+    o.kind, o.flags, o.M, o.N, o.A, o.lda, o.a_rows = K.K_ATTN, 1, rows, 128, a.data_ptr(), 384, rows
+    o.C, o.ldc, o.col_mod, o.i0, o.i1, o.i2, o.K = out.data_ptr(), 128, 128, 1, 1, 128, 2048
+    launch(o)
+    w1, w2 = torch.exp(s1)[t], torch.exp(s2)[t]
+    vs = v[:4, t - 256].double()
+    want = (w1 * vs[0] + w2 * vs[1:].sum(0)) / (w1 + 3 * w2)
+    err = (out[t, t - 256].double() - want).abs() / ((w1 + w2 * vs[1:].abs().sum(0)) / (w1 + 3 * w2))
+    assert float(err.max()) < 2.0 ** -20      # two weights: an exponential within 2^-22 of an argument within 2^-22 (16 bits would be 2^-17)
+
+
 # rows, positions in front, heads, key heads, options
 CASES = [(9, 0, 4, 2, {}), (100, 0, 4, 1, {}), (300, 77, 6, 2, {}), (128, 128, 16, 4, dict(cap=50.0, sink=True, gate=1)), (513, 300, 16, 4, dict(cap=50.0, sink=True)),
          (200, 300, 8, 2, dict(window=64)), (200, 300, 8, 2, dict(window=64, keep=5, dist=True, cap=50.0)), (128, 128, 3, 1, dict(window=130, keep=200)), (400, 0, 8, 8, dict(window=1)),
