@@ -23,6 +23,7 @@ enum { AT_PROMPT, AT_PLAIN, AT_CAP, AT_DIST };   // AT_PROMPT: scores rounded to
 constexpr int AT_KEYS = 128, AT_THREADS = 640, AT_LOADERS = 96;
 constexpr int AT_TILE = 128 * 128 * 2;           // a query, key or value tile: two halves of 64 columns, 128-byte lines, 128-byte swizzle
 constexpr int AT_SMEM = 6 * AT_TILE + 1024 + 256 + 2 * 2 * 256 * 4;   // tiles, alignment, barriers, the half rows' maxima (two tiles in turn)
+constexpr float AT_L2E = 1.4426950408889634f;
 constexpr float AT_SLACK = 11.f;                 // a row's reference moves when its maximum is further above it than this (in powers of two)
 
 __device__ __forceinline__ void tmem_ld32(const uint32_t a, float* f) {
@@ -62,6 +63,34 @@ __device__ __forceinline__ float ex2f(const float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Sixteen columns of an unnormalised output row over the keys that the row sees, and no others.  The products above multiply the weight 0 of an unseen key with
+// its value, which is no 0 where the value is infinite or NaN: a row that came out so is formed again here, one thread per row.
+template <int MODE>
+__device__ __noinline__ void at_row_again(const AttnArgs& a, const int m, const int head, const int col, const int pos, const int lo, const int keep, const float ref, float* out) {
+  const int HG = a.H / a.G, kvh = head / HG;
+  for (int j = 0; j < 16; ++j) out[j] = 0.f;
+  const size_t qat = (size_t)m * a.ldq + (size_t)head * 128;
+  for (int key = 0; key <= pos; ++key) {
+    if (key < lo && key >= keep) { key = lo - 1; continue; }
+    const bf16* k = a.k + (size_t)key * a.ldk + kvh * 128;
+    float s = 0.f;
+    for (int c = 0; c < 128; ++c) {
+      const float q = MODE == AT_PROMPT ? __bfloat162float(reinterpret_cast<const bf16*>(a.q)[qat + c]) : bf16r(reinterpret_cast<const float*>(a.q)[qat + c]);
+      s = fmaf(q, __bfloat162float(k[c]), s);
+    }
+    if (MODE == AT_PROMPT) {
+      s = bf16r(bf16r(s) * a.scale);
+    } else {
+      s *= a.scale;
+      if (a.cap > 0.f) s = a.cap * fast_tanh(s / a.cap);
+      if (MODE == AT_DIST && a.r12) s -= a.r12[head] * __logf(fmaf(a.r12[a.H + head], (float)(pos - key), 1.f));
+    }
+    const float w = exp2f(fmaf(s, AT_L2E, -ref));
+    const bf16* v = a.v + (size_t)key * a.ldv + kvh * 128 + col;
+    for (int j = 0; j < 16; ++j) out[j] = fmaf(w, __bfloat162float(v[j]), out[j]);
+  }
 }
 
 // A CTA takes two groups of 128 rows of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
@@ -261,7 +290,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       const bool wfull = (wq * 32 + 31) / HG < nqg;
       const int lo = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 ? pos - pos % a.chunk : 0);
       const int keep = a.window > 0 && a.chunk <= 0 ? a.keep : 0;
-      constexpr float L2E = 1.4426950408889634f;
       const float icap = a.cap > 0.f ? 1.f / a.cap : 0.f;
       float r1 = 0.f, r2 = 0.f;
       if (MODE == AT_DIST && a.r12) { r1 = a.r12[head]; r2 = a.r12[a.H + head]; }
@@ -321,7 +349,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           if (h == 0) tmem_ld_wait();
         }
         mx = fmaxf(mx, meet(mx, c & 1));
-        const float mk = rintf(mx * L2E);
+        const float mk = rintf(mx * AT_L2E);
         if (c == 0) ref = mk;
         else if (__any_sync(0xffffffffu, mk > ref + AT_SLACK)) {      // (from -inf too: nothing summed yet)
           const bool up = mk > ref + AT_SLACK;
@@ -345,7 +373,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           uint32_t hi[16], lw[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float p = ex2f(fmaf(s[h][2 * j], L2E, u)), q = ex2f(fmaf(s[h][2 * j + 1], L2E, u));
+            const float p = ex2f(fmaf(s[h][2 * j], AT_L2E, u)), q = ex2f(fmaf(s[h][2 * j + 1], AT_L2E, u));
             sum += p + q;
             hi[j] = bf_pair(p, q);
             const float p1 = p - __uint_as_float(hi[j] << 16), q1 = q - __uint_as_float(hi[j] & 0xffff0000u);
@@ -375,9 +403,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float f = 1.f, den = sum + meet(sum, c & 1);
       if (MODE != AT_PROMPT && a.sink && live) {
-        const float sk = a.sink[head], mm = fmaxf(ref, rintf(sk * L2E));
+        const float sk = a.sink[head], mm = fmaxf(ref, rintf(sk * AT_L2E));
         f = ref == -INFINITY ? 0.f : pow2_down(ref - mm);
-        den = den * f + exp2f(fmaf(sk, L2E, -mm));
+        den = den * f + exp2f(fmaf(sk, AT_L2E, -mm));
       }
       const int m = pos - P;
       float sc = f / den;
@@ -395,7 +423,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         if (live) {
           float v[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]) * sc;
+          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]);
+          float far = 0.f;      // NaN as soon as one of them is not finite
+#pragma unroll
+          for (int j = 0; j < 16; ++j) far = fmaf(v[j], 0.f, far);
+          if (far != 0.f && fabsf(sc) < INFINITY) at_row_again<MODE>(a, m, head, half * 64 + i * 16, pos, lo, keep, ref == -INFINITY ? 0.f : ref, v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] *= sc;
           if (ge) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] *= sigmoid_f(ge[i * 16 + j]);

@@ -117,6 +117,27 @@ __global__ void __launch_bounds__(256) fq3s_gemm_f32_kernel(const SeqGemm g) {
 // takes 32 (query, head of the group) rows of one key / value head and tiles of 64 positions: S [32 x 64] with 4 x 4 scores a thread, an online softmax over
 // half-warps, O [32 x 128] += P V with 4 x 8 outputs a thread.  Keys of the next tile arrive while this one's weights and outputs are formed, values while
 // its scores are.  384 rows of 8 heads behind 300 positions, window 512: 235 -> 56 us with three key splits and their merge.
+// Eight columns (4 tx .. + 3 and 64 + 4 tx .. + 3) of an unnormalised output row over the keys first .. last that the row sees, and no others: formed again
+// where the weight 0 of an unseen key met an infinite or NaN value of the tile.
+__device__ __noinline__ void fa_row_again(const fq3c_op& o, const CacheAttnMask& mask, const int m, const int head, const int tx, const int pos, const int first, const int last,
+                                          const float mx, float* out) {
+  const int kvh = head / (o.i0 / o.i1);
+  const float* q = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + (size_t)head * 128;
+  const float* r12 = reinterpret_cast<const float*>(o.bias);
+  for (int j = 0; j < 8; ++j) out[j] = 0.f;
+  for (int key = first; key <= min(last, pos); ++key) {
+    if (!mask.sees(pos, key)) continue;
+    const float* k = reinterpret_cast<const float*>(o.B) + (size_t)key * o.ldr + kvh * 128;
+    float s = 0.f;
+    for (int c = 0; c < 128; ++c) s = fmaf(q[c], k[c], s);
+    s *= o.f0;
+    if (o.f1 > 0.f) s = o.f1 * tanhf(s / o.f1);
+    if (r12) s -= r12[head] * log1pf(r12[o.i0 + head] * (float)(pos - key));
+    const float w = expf(s - mx);
+    const float* v = reinterpret_cast<const float*>(o.p1) + (size_t)key * o.taps + kvh * 128 + 4 * tx;
+    for (int j = 0; j < 8; ++j) out[j] = fmaf(w, v[(j >> 2) * 64 + (j & 3)], out[j]);
+  }
+}
 constexpr int FA_R = 32, FA_T = 64, FA_P = 132, FA_PP = FA_T + 4;
 constexpr int FA_SMEM = (FA_R * FA_P + 2 * FA_T * FA_P + FA_R * FA_PP) * 4;
 __global__ void __launch_bounds__(128) fq3s_attn_f32_kernel(const fq3c_op o) {
@@ -180,6 +201,8 @@ __global__ void __launch_bounds__(128) fq3s_attn_f32_kernel(const fq3c_op o) {
     count = ntiles;
   }
   if (count == 0) t = ntiles;
+  const int tfirst = t;
+  int tlast = t;
   if (t < ntiles) fetch(o.B, o.ldr, ks, t);
   if (t < ntiles) fetch(o.p1, o.taps, vs, t);
   while (t < ntiles) {
@@ -263,6 +286,7 @@ __global__ void __launch_bounds__(128) fq3s_attn_f32_kernel(const fq3c_op o) {
     __syncthreads();
     if (tn < ntiles) fetch(o.p1, o.taps, vs, tn);
     else cp_async_commit();
+    tlast = t;
     t = tn;
   }
   cp_async_wait<0>();
@@ -273,6 +297,15 @@ __global__ void __launch_bounds__(128) fq3s_attn_f32_kernel(const fq3c_op o) {
   for (int e = 0; e < 4; ++e) {
     if (!live[e]) continue;
     const int m = pos[e] - P, h = head[e];
+    f32x2 far = 0ull;      // NaN as soon as one of the sums is not finite
+#pragma unroll
+    for (int j = 0; j < 4; ++j) far = fma2<true>(acc[e][j], pack2(0.f, 0.f), far);
+    if (lo2(far) + hi2(far) != 0.f && sum[e] < INFINITY) {
+      float v[8];
+      fa_row_again(o, mask, m, h, tx, pos[e], tfirst * FA_T, tlast * FA_T + FA_T - 1, mx[e], v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[e][j] = pack2(v[2 * j], v[2 * j + 1]);
+    }
     if (splits > 1) {      // (maximum, sum, unnormalised output): fq3s_cache_attn_merge_kernel adds the splits
       float* dst = reinterpret_cast<float*>(o.ws) + (((size_t)m * H + h) * splits + blockIdx.z) * 130;
       if (tx == 0) { dst[0] = mx[e]; dst[1] = sum[e]; }

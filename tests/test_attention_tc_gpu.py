@@ -133,3 +133,74 @@ def test_cache_rows(rows, first, heads, kv, opt):
         want = want * torch.sigmoid(gate.double()).view(rows, heads, -1)
     # weights of 16 mantissa bits (2^-17 each, falling either way), scores within 2^-22 of their size through the fast cap and exponential
     assert rel(out, want.reshape(rows, -1)) < 1.5e-5
+
+
+def spoil(v, rows_bad):
+    """Infinite and NaN values of the first key head in some rows; where they may show: a position, and the columns."""
+    v[rows_bad[0], 3], v[rows_bad[1], 70], v[rows_bad[2], 127] = math.inf, math.nan, -math.inf
+    return [(rows_bad[0], 3), (rows_bad[1], 70), (rows_bad[2], 127)]
+
+
+def check_spoiled(got, clean, heads_of, bad, first, tol):
+    """got [M, H, 128] with spoiled values, clean without: what does not see a spoiled row is as without it, what sees it is not finite."""
+    M = got.shape[0]
+    for row, col in bad:
+        sees = torch.arange(first, first + M, device="cuda") >= row
+        hit = got[:, :heads_of, col]
+        assert not hit[sees].isfinite().any() and hit[~sees].isfinite().all()
+        if col != 70:      # an infinite value stays one
+            assert hit[sees].isinf().all()
+    keep = torch.ones_like(clean, dtype=torch.bool)
+    for row, col in bad:
+        keep[max(0, row - first):, :heads_of, col] = False
+    assert float((got.double() - clean.double())[keep].norm() / clean.double()[keep].norm()) < tol
+
+
+def test_prompt_values_past_the_causal_edge():
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    torch.manual_seed(5)
+    rows, heads, kv = 450, 4, 2
+    n = (heads + 2 * kv) * 128
+    a = torch.randn(rows, n, device="cuda").bfloat16()
+    outs = []
+    bad = []
+    for spoiled in (False, True):
+        if spoiled:
+            bad = spoil(a[:, (heads + kv) * 128:], (130, 255, 400))
+        out = torch.zeros(rows, heads * 128, device="cuda", dtype=torch.bfloat16)
+        o = K.Op()
+        o.kind, o.flags, o.M, o.N, o.A, o.lda, o.a_rows = K.K_ATTN, 1, rows, heads * 128, a.data_ptr(), n, rows
+        o.C, o.ldc, o.col_mod, o.i0, o.i1, o.i2, o.K = out.data_ptr(), heads * 128, heads * 128, heads, kv, 128, 2048
+        launch(o)
+        outs.append(out.view(rows, heads, 128).float())
+    check_spoiled(outs[1], outs[0], heads // kv, bad, 0, 2.0 ** -8)
+
+
+@pytest.mark.parametrize("f32, splits", [(False, 1), (True, 1), (True, 3)])
+@pytest.mark.parametrize("opt", [{}, dict(window=2000, keep=3), dict(cap=20.0), dict(dist=True)])
+def test_cache_values_past_the_causal_edge(f32, splits, opt):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    torch.manual_seed(6)
+    rows, first, heads, kv = 300, 70, 6, 2
+    L = first + rows
+    q = torch.randn(rows, heads * 128, device="cuda")
+    kc, vc = (torch.randn(L, kv * 128, device="cuda").to(torch.float32 if f32 else torch.bfloat16) for _ in range(2))
+    pos, r12 = torch.tensor([first], dtype=torch.int32, device="cuda"), torch.rand(2 * heads, device="cuda")
+    ws = torch.zeros(rows * heads * splits * 130, device="cuda")
+    outs, bad = [], []
+    for spoiled in (False, True):
+        if spoiled:
+            bad = spoil(vc, (100, 201, 350))
+        out = torch.zeros(rows, heads * 128, device="cuda")
+        o = K.Op()
+        o.kind, o.flags, o.M, o.N, o.i0, o.i1, o.i2, o.cin = K.K_CACHE_ATTN, K.F_OUT_F32 | (K.F_F32 if f32 else 0), rows, heads * 128, heads, kv, 128, 128
+        o.f0, o.f1, o.K, o.a_rows, o.m_begin = 128 ** -0.5, opt.get("cap", 0.0), opt.get("window", 0), opt.get("keep", 0), splits
+        o.A, o.lda, o.B, o.ldr, o.p1, o.taps, o.p0 = q.data_ptr(), heads * 128, kc.data_ptr(), kv * 128, vc.data_ptr(), kv * 128, pos.data_ptr()
+        o.C, o.ldc, o.col_mod, o.ws, o.ws_bytes = out.data_ptr(), heads * 128, 1, ws.data_ptr(), ws.numel() * 4
+        if opt.get("dist"):
+            o.bias = r12.data_ptr()
+        launch(o)
+        outs.append(out.view(rows, heads, 128))
+    check_spoiled(outs[1], outs[0], heads // kv, bad, first, 1e-5)
