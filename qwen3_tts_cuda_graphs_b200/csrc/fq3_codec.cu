@@ -58,26 +58,28 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); 
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
-// sin(x)^2, the periodic half of SnakeBeta: it has period pi, so x is reduced by the nearest multiple of pi (three constants, exact products) to
-// [-pi/2, pi/2] and the sine is an odd polynomial of degree 9 there (Remez fit of sin(r) / r in r^2, relative error 5e-9): no quadrant to choose and no
-// branch.  Within 2.5e-7 of sin^2; arguments the rounding to a multiple does not hold for go through sinf.
+// sin(x)^2, the periodic half of SnakeBeta.  x is reduced by the nearest multiple of pi / 2 (Cody and Waite: three parts, exact products) to [-pi/4, pi/4],
+// where the sine is an odd polynomial of degree 7 (least-maximum fit of sin(r) / r in r^2, relative error 5e-9); behind an odd multiple the square
+// is 1 - sin^2(r), so that no sum near 1 loses what the square of a rounded sine loses.  Within 1.2e-7 of sin^2, 2.1e-8 root mean square (the square of
+// a correctly rounded sine: 2.7e-8), and within 4e-7 of its own size.  Beyond SIN_SQ_NEAR, where the multiple's own rounding leaves the fitted range, through sinf.
+constexpr float SIN_SQ_NEAR = 2.5e5f;
 __device__ __forceinline__ float sin_sq_near(const float x) {
-  const float n = fmaf(x, 0.3183098861837907f, 12582912.f) - 12582912.f;
-  float r = fmaf(n, -3.1415927410125732f, x);
-  r = fmaf(n, 8.742277657347586e-08f, r);
-  r = fmaf(n, 3.4302490200117637e-15f, r);
+  const float m = fmaf(x, 0.6366197723675814f, 12582912.f), n = m - 12582912.f;      // the multiple in m's low bits
+  float r = fmaf(n, -1.5707963705062866f, x);
+  r = fmaf(n, 4.371138828673793e-08f, r);
+  r = fmaf(n, 1.7151245100058819e-15f, r);
   const float u = r * r;
-  float q = fmaf(u, 2.6018262815341586e-06f, -0.00019807384524028748f);
-  q = fmaf(u, q, 0.008333024568855762f);
-  q = fmaf(u, q, -0.16666656732559204f);
+  float q = fmaf(u, -0.00019498496840242296f, 0.008332036435604095f);
+  q = fmaf(u, q, -0.16666652262210846f);
   const float s = fmaf(r * u, q, r);
-  return s * s;
+  const bool odd = __float_as_int(m) & 1;
+  return fmaf(s, odd ? -s : s, odd ? 1.f : 0.f);
 }
 __device__ __noinline__ float sin_sq_far(const float x) {
   const float s = sinf(x);
   return s * s;
 }
-__device__ __forceinline__ float sin_sq(const float x) { return fabsf(x) < 1e6f ? sin_sq_near(x) : sin_sq_far(x); }
+__device__ __forceinline__ float sin_sq(const float x) { return fabsf(x) < SIN_SQ_NEAR ? sin_sq_near(x) : sin_sq_far(x); }
 // a gated unit: silu(gate) * up, or with FQ3C_GELU_TANH gelu_tanh(gate) * up
 __device__ __forceinline__ float glu_f(const int flags, const float gate, const float up) {
   return (flags & FQ3C_GELU_TANH) ? gelu_tanh_f(gate) * up : silu_f(gate) * up;

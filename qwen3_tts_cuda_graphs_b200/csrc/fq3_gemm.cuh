@@ -202,7 +202,7 @@ __device__ __forceinline__ void epilogue_row16(const fq3c_op& o, const int row, 
     for (int j = 0; j < 4; ++j) {
       const float4 a = ea[j], b = ib[j];
       const float x0 = v[4 * j] * a.x, x1 = v[4 * j + 1] * a.y, x2 = v[4 * j + 2] * a.z, x3 = v[4 * j + 3] * a.w;
-      if (fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(x2), fabsf(x3))) < 1e6f) {
+      if (fmaxf(fmaxf(fabsf(x0), fabsf(x1)), fmaxf(fabsf(x2), fabsf(x3))) < SIN_SQ_NEAR) {
         v[4 * j] = fmaf(b.x, sin_sq_near(x0), v[4 * j]); v[4 * j + 1] = fmaf(b.y, sin_sq_near(x1), v[4 * j + 1]);
         v[4 * j + 2] = fmaf(b.z, sin_sq_near(x2), v[4 * j + 2]); v[4 * j + 3] = fmaf(b.w, sin_sq_near(x3), v[4 * j + 3]);
       } else {
