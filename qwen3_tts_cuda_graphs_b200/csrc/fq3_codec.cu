@@ -58,22 +58,22 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); 
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
-// sin(x)^2, the periodic half of SnakeBeta.  x is reduced by the nearest multiple of pi / 2 (Cody and Waite: three parts, exact products) to [-pi/4, pi/4],
-// where the sine is an odd polynomial of degree 7 (least-maximum fit of sin(r) / r in r^2, relative error 5e-9); behind an odd multiple the square
-// is 1 - sin^2(r), so that no sum near 1 loses what the square of a rounded sine loses.  Within 1.2e-7 of sin^2, 2.1e-8 root mean square (the square of
-// a correctly rounded sine: 2.7e-8), and within 4e-7 of its own size.  Beyond SIN_SQ_NEAR, where the multiple's own rounding leaves the fitted range, through sinf.
+// sin(x)^2, the periodic half of SnakeBeta.  x is reduced by the nearest multiple of pi / 2 (Cody and Waite: two parts, the first product exact) to
+// [-pi/4, pi/4], where sin^2 = u + u^2 Q(u), u = r^2, with a cubic Q (least-maximum fit of sin^2, error 2.4e-10); behind an odd multiple it is 1 - sin^2(r).
+// Within 1.1e-7 of sin^2, 1.9e-8 root mean square (the square of a correctly rounded sine: 0.9e-7 and 2.7e-8).  Beyond SIN_SQ_NEAR, where the multiple's own
+// rounding leaves the fitted range, through sinf.
 constexpr float SIN_SQ_NEAR = 2.5e5f;
 __device__ __forceinline__ float sin_sq_near(const float x) {
   const float m = fmaf(x, 0.6366197723675814f, 12582912.f), n = m - 12582912.f;      // the multiple in m's low bits
   float r = fmaf(n, -1.5707963705062866f, x);
   r = fmaf(n, 4.371138828673793e-08f, r);
-  r = fmaf(n, 1.7151245100058819e-15f, r);
   const float u = r * r;
-  float q = fmaf(u, -0.00019498496840242296f, 0.008332036435604095f);
-  q = fmaf(u, q, -0.16666652262210846f);
-  const float s = fmaf(r * u, q, r);
-  const bool odd = __float_as_int(m) & 1;
-  return fmaf(s, odd ? -s : s, odd ? 1.f : 0.f);
+  float q = fmaf(u, 0.0001339026930509135f, -0.0031702169217169285f);
+  q = fmaf(u, q, 0.04444332420825958f);
+  q = fmaf(u, q, -0.33333322405815125f);
+  const float sg = __uint_as_float(__float_as_uint(m) * 0x80000000u + 0x3f800000u);      // -1 behind an odd multiple, else 1
+  const float su = sg * u;
+  return fmaf(su * u, q, su) + fmaf(sg, -0.5f, 0.5f);
 }
 __device__ __noinline__ float sin_sq_far(const float x) {
   const float s = sinf(x);
