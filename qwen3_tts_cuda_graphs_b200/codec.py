@@ -110,19 +110,19 @@ def fuse_row_norms(ops: list) -> list:
 
 
 def attach_splitk_workspace(ops, device, keep) -> None:
-    """One fp32 workspace per stream-ordered op list: it allows every short GEMM of the list to be split over K (most sum their partial tiles in
-    the shared memory of a cluster; the kernel for c_in = 8 modulo 16 over several taps keeps them here)."""
-    need = 0
-    for o in ops:
-        if o.kind == K_GEMM and 0 < o.M <= SPLITK_MAX_ROWS and o.K >= 512:
-            need = max(need, 8 * o.M * ((o.N + 7) // 8 * 8) * 4)
+    """Allows every short GEMM of a stream-ordered op list to be split over K.  The partial tiles are summed in the shared memory of a cluster; only the kernel
+    for c_in = 8 modulo 16 over several taps keeps them in an fp32 workspace, which the list's ops share."""
+    short = [o for o in ops if o.kind == K_GEMM and 0 < o.M <= SPLITK_MAX_ROWS and o.K >= 512]
+    for o in short:
+        o.reserved |= 4
+    short = [o for o in short if o.taps > 1 and o.cin % 16]
+    need = max((8 * o.M * ((o.N + 7) // 8 * 8) * 4 for o in short), default=0)
     if need == 0:
         return
     ws = torch.empty(min(need, SPLITK_WS_CAP) // 4, dtype=torch.float32, device=device)
     keep.append(ws)
-    for o in ops:
-        if o.kind == K_GEMM and 0 < o.M <= SPLITK_MAX_ROWS and o.K >= 512:
-            o.ws, o.ws_bytes = ws.data_ptr(), ws.numel() * 4
+    for o in short:
+        o.ws, o.ws_bytes = ws.data_ptr(), ws.numel() * 4
 
 
 _lib = None
@@ -511,9 +511,10 @@ class CodecDecoder:
         self._gemm(plan, xs, g["final.w"], rows, 1, out_dim, taps=7, tap_off=[j - 6 for j in range(7)], bias=g["final.b"],
                    flags=F_CLAMP, out=plan.wav, out_f32=True, m_begin=fin_begin)
         plan.n_samples = rows
+        # Nothing is split over K here.  A streamed window runs beside the frame loop, on 20 SMs that lie here and there, and a split's CTAs are a cluster,
+        # which wants its SMs free at once and next to each other: with clusters the whole window waited for the chunk of frames beside it to
+        # end (32 chunks: 31 ms outside the frame loop's launches, 7 without).  Alone it costs a window of 33 frames 4 %.
         plan.ops = fuse_row_norms(plan.ops)
-        if os.environ.get("FQ3C_SPLITK", "1") != "0":
-            attach_splitk_workspace(plan.ops, self.device, plan.keep)
         plan.arr = (Op * len(plan.ops))(*plan.ops)
         return plan
 
@@ -580,8 +581,8 @@ class CodecStream:
     (offset + history) >= 0, so rows of earlier chunks take the place of the causal zero padding, and the last ops of a
     chunk's list roll every buffer's tail into its history rows.  A chunk of n frames costs n frames and returns exactly
     n * total_upsample samples; the concatenation over chunks equals the full, non-streaming decode of all frames bit for
-    bit when neither side splits its GEMMs over K (FQ3C_SPLITK=0, or split_k=False here), because every output element then
-    accumulates the same products in the same order; with split-K (the default, faster) the two agree up to fp32 summation order.
+    bit, because every output element accumulates the same products in the same order.  split_k=True splits the short GEMMs over K
+    (for a stream that has the GPU to itself): then the two agree up to fp32 summation order.
     """
 
     def __init__(self, dec: "CodecDecoder", max_chunk_frames: int = 8, split_k: Optional[bool] = None):
@@ -590,9 +591,7 @@ class CodecStream:
                              '("both") makes every vocoder block look one input row ahead')
         self.dec, self.cfg, self.device = dec, dec.cfg, dec.device
         self.max_frames = int(max_chunk_frames)
-        # short GEMMs with a long reduction may be split over K like the full decode's (faster: 8 rows cover few tiles); the chunks
-        # then equal the full decode up to fp32 summation order instead of bit for bit.  FQ3C_SPLITK=0 / split_k=False: exact.
-        self.split_k = (os.environ.get("FQ3C_SPLITK", "1") != "0") if split_k is None else bool(split_k)
+        self.split_k = bool(split_k)      # (None: not, like the full decode)
         self.hist: List[tuple] = []          # (buffer [hist + rows_max, cols], hist rows, name)
         self.rows_of: Dict[str, int] = {}    # new rows per frame of every history buffer
         self._plans: Dict[int, _Plan] = {}

@@ -1158,7 +1158,7 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   // the same partial sums in the same order.
   const int KT = (o.K + TK - 1) / TK;
   g.splits = 1;
-  if (o.ws && o.M <= 4 * TM && KT >= 8) {
+  if ((o.ws || (o.reserved & 4)) && o.M <= 4 * TM && KT >= 8) {
     const int bn = o.N >= 64 ? 64 : 32;
     const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
     const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));

@@ -143,7 +143,7 @@ class BatchScheduler:
         """codec_mode: "windowed" (default, = "auto") — the reference's 25-frame left-context re-decode (model.py:737-826): the
         audio is bit for bit what the single-stream streaming API returns for the same codes; "stateful" — one
         codec.CodecStream per slot: a chunk costs its own frames and the audio is the full non-streaming decode of the
-        utterance's codes (bit for bit with codec_split_k=False, up to fp32 summation order otherwise).
+        utterance's codes, bit for bit (up to fp32 summation order with codec_split_k=True).
         codec_lanes: CUDA streams the utterances' codec decodes of one chunk are spread over (16 windowed decodes: 23 ms on one
         stream, 11 ms on four, profiles/r02k_codec_lanes_probe.log).
         emit_every: after an utterance's first chunk (time to first audio is not touched) hand audio out every `emit_every`
