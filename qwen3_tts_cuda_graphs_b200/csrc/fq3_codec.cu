@@ -1973,12 +1973,17 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         static int tc5_min_k = -1;
         if (tc5_min_k < 0) { const char* e3 = getenv("FQ3C_TC5_MINK"); tc5_min_k = e3 ? atoi(e3) : TK; }  // one k-block is enough: the vectorised epilogue beats the mma.sync kernel even at K = 96
         if (use_tc5 && o.N >= 16 && o.K >= tc5_min_k && (o.taps == 1 || o.cin % 16 == 0)) {
-          const GemmLaunch L = gemm_plan(o);
+          // Columns behind N that are scratch make a width of whole 16-column pieces (B's missing rows arrive as zeros): the epilogue of any other width stores every
+          // entry by itself (1501 rows of 643 columns 31 us, of 656 9.3).
+          fq3c_op w = o;
+          if ((o.reserved & 8) && !(o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_RESID | FQ3C_SWIGLU | FQ3C_SNAKE2)) && o.ldc >= (o.N + 15) / 16 * 16 && !o.norm_out)
+            w.N = (o.N + 15) / 16 * 16;
+          const GemmLaunch L = gemm_plan(w);
           CUtensorMap tmA, tmB;
           if (make_map(&tmA, o.A, (uint64_t)o.cin, (uint64_t)o.a_rows, (uint64_t)o.lda, (uint32_t)L.g.a_rows) &&
               make_map(&tmB, o.B, (uint64_t)o.K, (uint64_t)o.N, (uint64_t)o.K, (uint32_t)L.g.bn)) {
-            if (L.half) launch_after(fq3c_gemm_persist_kernel<2>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
-            else launch_after(fq3c_gemm_persist_kernel<1>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, o, L.g, tmA, tmB);
+            if (L.half) launch_after(fq3c_gemm_persist_kernel<2>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
+            else launch_after(fq3c_gemm_persist_kernel<1>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
             if (o.norm_out) {
               launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, true, 1, o);
               count_launches(1);

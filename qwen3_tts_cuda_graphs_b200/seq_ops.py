@@ -48,6 +48,7 @@ class StepBuilder:
         self.adt = torch.float32 if f32 else torch.bfloat16     # dtype of product operands
         self.plan = _Plan()
         self._pool: Dict[tuple, torch.Tensor] = {}
+        self._wide: set = set()      # buffers whose last columns are scratch
 
     # ---- buffers --------------------------------------------------------------------------------
     def buf(self, name: str, rows: int, cols: int, dtype=torch.float32) -> torch.Tensor:
@@ -57,6 +58,13 @@ class StepBuilder:
         if t is None:
             t = self._pool[key] = torch.zeros(max(rows, 1), cols, dtype=dtype, device=self.device)
             self.plan.keep.append(t)
+        return t
+
+    def wide(self, name: str, cols: int) -> torch.Tensor:
+        """A scratch buffer for projections with a few gate columns behind the heads': the pitch is rounded up to 16 entries, which the product may fill, so that
+        every row begins on whole 64 bytes, as its epilogue and the attention's loads ask for."""
+        t = self.buf(name, self.M, (cols + 15) // 16 * 16)
+        self._wide.add(t.data_ptr())
         return t
 
     def _op(self, kind: int, **kw) -> Op:
@@ -178,8 +186,8 @@ class StepBuilder:
             flags |= F_NOROUND      # f32 results and the activation's argument stay unrounded; with a few rows the flag also picks the weight-streaming product
         if glu:
             flags |= F_SWIGLU | (F_GELU_TANH if glu_gelu else 0)
-        # reserved = 1: w is written by no op of the list
-        kw = dict(M=M, N=N, K=K, taps=1, cin=K, a_rows=x.shape[0], lda=x.shape[1], ldc=out.shape[1], col_mod=N, A=x, B=w, C=out, flags=flags, reserved=1)
+        # reserved: w is written by no op of the list (1); the columns behind N are scratch (8)
+        kw = dict(M=M, N=N, K=K, taps=1, cin=K, a_rows=x.shape[0], lda=x.shape[1], ldc=out.shape[1], col_mod=N, A=x, B=w, C=out, flags=flags, reserved=1 | (8 if out.data_ptr() in self._wide else 0))
         if bias is not None:
             kw["bias"] = bias
         o = self._op(K_GEMM, **kw)
@@ -212,7 +220,7 @@ class StepBuilder:
         M, H, R, E = self.M, c.heads, c.kv_rank, c.rot_dim
         nq = H * (c.dim + E)
         qcols = c.q_rank if c.q_rank > 0 else nq
-        qd = self.linear(h, w["wqd"], self.buf("la.qd", M, w["wqd"].shape[0]))
+        qd = self.linear(h, w["wqd"], self.wide("la.qd", w["wqd"].shape[0]))
         ctab = self.slot.cur[cache]
         cf32 = F_F32 if ctab.dtype == torch.float32 else 0
         self.group_norm(qd, w["dkv_norm"], 1, eps, ctab, n=R, col=qcols, append_at_position=True)
@@ -335,7 +343,7 @@ class StepBuilder:
         kcol = H * d
         vcol = kcol + (G * d if own and not c.keys_as_values else 0)
         gcol = kcol + (G * d + (0 if c.keys_as_values else G * dv) if own else 0)
-        proj = self.linear(h, w["wqkv"], self.buf("sa.proj", M, w["wqkv"].shape[0]), bias=w.get("bqkv"))
+        proj = self.linear(h, w["wqkv"], self.wide("sa.proj", w["wqkv"].shape[0]), bias=w.get("bqkv"))
         rows = self.time_conv(proj, w["conv"], kcache + ".conv", self.buf("sa.cv", M, gcol), channels=gcol) if c.conv > 0 else proj
         oa = self.buf("sa.o", M, H * dv, self.adt)
         self._attend(c, w, rows, 0, kcol, vcol, (proj, gcol), kcache, vcache, eps, oa)
@@ -437,7 +445,7 @@ class StepBuilder:
         write-strength input), conv f32 [2 G dim + H vdim, taps], A_log, dt_bias f32 [H], norm f32 [vdim], o [width, H vdim]."""
         M, H, G, d, dv = self.M, c.heads, c.kv_heads, c.dim, c.vdim
         nconv = 2 * G * d + H * dv
-        raw = self.linear(h, w["win"], self.buf("dr.raw", M, nconv + H * dv + 2 * H))
+        raw = self.linear(h, w["win"], self.wide("dr.raw", nconv + H * dv + 2 * H))
         cv = self.time_conv(raw, w["conv"], state + ".conv", self.buf("dr.cv", M, nconv), channels=nconv, silu=True)
         y = self._mstate(0, cv, raw, H, G, d, dv, G * d, 2 * G * d, nconv + H * dv, nconv + H * dv + H, w, state + ".s", self.buf("dr.y", M, H * dv))
         yn = self.group_norm(y, w["norm"], H, eps, self.buf("dr.yn", M, H * dv, self.adt), n=H * dv, gate=raw, gate_col=nconv, weight_period=dv)
@@ -448,7 +456,7 @@ class StepBuilder:
         conv_b f32 or None, A_log, dt_bias, D f32 [H], norm f32 [inner], o [width, inner]."""
         M, H, P, N, G = self.M, c.heads, c.vdim, c.state, c.groups
         inner, nconv = H * P, H * P + 2 * G * N
-        raw = self.linear(h, w["win"], self.buf("ss.raw", M, inner + nconv + H))
+        raw = self.linear(h, w["win"], self.wide("ss.raw", inner + nconv + H))
         cv = self.time_conv(raw, w["conv"], state + ".conv", self.buf("ss.cv", M, nconv), bias=w.get("conv_b"), col=inner, channels=nconv,
                             silu=True)
         y = self._mstate(1, cv, raw, H, G, N, P, inner, inner + G * N, inner + nconv, 0, w, state + ".s", self.buf("ss.y", M, inner))
@@ -464,7 +472,7 @@ class StepBuilder:
         acol = gcol + H * dv
         rank = w["a2"].shape[1]
         assert w["win"].shape[0] == acol + rank and w["a2"].shape[0] == H * d
-        raw = self.linear(h, w["win"], self.buf("cd.raw", M, acol + rank))
+        raw = self.linear(h, w["win"], self.wide("cd.raw", acol + rank))
         y = self.buf("cd.y", M, H * dv)
         ws = self._scan_ws(-(-(H * d) // 4) * 4, H, d, dv)
         self._op(K_MSTATE_SCAN, M=M, N=H * dv, taps=2, i0=H, i1=H, i2=d, cin=dv, K=H * d, a_rows=2 * H * d, A=raw, lda=raw.shape[1],
@@ -480,7 +488,7 @@ class StepBuilder:
         [H dim], A_log f32 [H], g2 [gate rank, H vdim] (transposed), norm f32 [vdim], o [width, H vdim].  Per head S <- diag(g) S, g = exp(-exp(A_log) softplus(z));
         u = beta (v - S^T k); S <- S + k u^T; o = S^T q, on unit queries (times dim^(-1/2)) and keys.  States: state + ".conv", state + ".s"."""
         M, n = self.M, 2 * c.kv_heads * c.dim + c.heads * c.vdim
-        raw = self.linear(h, w["win"], self.buf("kd.raw", M, w["win"].shape[0]))
+        raw = self.linear(h, w["win"], self.wide("kd.raw", w["win"].shape[0]))
         cv = self.time_conv(raw, w["conv"], state + ".conv", self.buf("kd.cv", M, n), channels=n, silu=True)
         yn = self.buf("kd.yn", M, c.heads * c.vdim, self.adt)
         self._channel_delta(c, w, cv, 0, raw, n, state + ".s", eps, yn, 0)
@@ -511,7 +519,7 @@ class StepBuilder:
         M, H, G, d, dv = self.M, left.heads, left.kv_heads, left.dim, left.vdim
         nl = (H + G) * d + G * dv
         n = nl + 2 * right.kv_heads * right.dim + right.heads * right.vdim
-        raw = self.linear(h, w["win"], self.buf("pd.raw", M, w["win"].shape[0]))
+        raw = self.linear(h, w["win"], self.wide("pd.raw", w["win"].shape[0]))
         cv = self.time_conv(raw, w["conv"], state + ".conv", self.buf("pd.cv", M, n), channels=n, silu=True, silu_from=nl)
         heads = self.buf("pd.heads", M, H * dv + right.heads * right.vdim, self.adt)
         self.branch(0)         # the two mixers run side by side
@@ -527,7 +535,7 @@ class StepBuilder:
         S <- decay S + (k dim^(-1/2)) v^T, o = S^T q; the read-out is divided by its root mean square per head (no weights)."""
         M, H, d, dv = self.M, c.heads, c.dim, c.vdim
         gcol = 2 * H * d + H * dv
-        raw = self.linear(h, w["win"], self.buf("rt.raw", M, w["win"].shape[0]))
+        raw = self.linear(h, w["win"], self.wide("rt.raw", w["win"].shape[0]))
         if c.rot_dims > 0:      # 2 H heads (queries, then keys) turn where they lie; nothing is appended
             self._op(K_ROT_APPEND, M=M, i0=2 * H, i1=0, i2=d, cin=0, taps=c.rot_dims, K=0, a_rows=0, A=raw, lda=raw.shape[1], B=w["freq"],
                      p0=self.slot.pos, flags=F_ROT_HALF)
@@ -544,7 +552,7 @@ class StepBuilder:
         gate's, zeros elsewhere), lower f32 [H dim], norm f32 [vdim], o [width, H vdim].  Per head, with f = l + (1 - l) sigmoid(gate):
         S <- diag(f) S + (1 - f) v^T, o = S^T silu(q)."""
         M, H, d, dv = self.M, c.heads, c.dim, c.vdim
-        raw = self.linear(h, w["win"], self.buf("fg.raw", M, w["win"].shape[0]), bias=w["bin"])
+        raw = self.linear(h, w["win"], self.wide("fg.raw", w["win"].shape[0]), bias=w["bin"])
         y = self.buf("fg.y", M, H * dv)
         ws = self._scan_ws(-(-(3 * H * d) // 4) * 4, H, d, dv)
         self._op(K_MSTATE_SCAN, M=M, N=H * dv, taps=4, i0=H, i1=H, i2=d, cin=dv, K=0, a_rows=2 * H * d, A=raw, lda=raw.shape[1], col_mod=H * d,
@@ -561,7 +569,7 @@ class StepBuilder:
         and state + ".m" [1, H]."""
         M, H, d, dv = self.M, c.heads, c.dim, c.vdim
         gcol = 2 * H * d + H * dv
-        raw = self.linear(h, w["win"], self.buf("mm.raw", M, w["win"].shape[0]), bias=w["bin"])
+        raw = self.linear(h, w["win"], self.wide("mm.raw", w["win"].shape[0]), bias=w["bin"])
         y, den = self.buf("mm.y", M, H * dv), self.buf("mm.den", M, H)
         ws = self._scan_ws(-(-(3 * H) // 4) * 4, H, d, dv + 1)
         S, mx = state + ".s", state + ".m"

@@ -111,3 +111,23 @@ def test_a_chain_of_products_reads_what_the_one_in_front_wrote():
             for i in range(40):
                 want, mag = product(x[i], W[i], rows, 512, (0,))
                 assert ((x[i + 1].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -15 * mag).all(), i
+
+
+@pytest.mark.parametrize("M, N, K", [(9, 643, 256), (33, 20, 128), (701, 1286, 192), (260, 17, 64), (1501, 385, 72)])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_widths_between_whole_pieces(M, N, K, scratch):
+    """A product whose width is no multiple of 16: with scratch columns behind it only those are written, without none."""
+    from qwen3_tts_cuda_graphs_b200 import codec as C
+
+    torch.manual_seed(M)
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    want, mag = product(A, B, M, K, (0,))
+    wide = (N + 15) // 16 * 16
+    for dtype, flags in ((torch.float32, C.F_OUT_F32 | C.F_NOROUND), (torch.bfloat16, 0)):
+        out = torch.full((M + 1, wide + 16), 7.0, device="cuda", dtype=dtype)
+        o = make_op(A, B, out, M, N, K, flags=flags)
+        o.reserved = 9 if scratch else 1
+        launch([o])
+        err = K * 2.0 ** -24 * mag + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+        assert ((out[:M, :N].double() - want).abs() <= err).all()
+        assert (out[:, wide if scratch else N:] == 7).all() and (out[M] == 7).all()
