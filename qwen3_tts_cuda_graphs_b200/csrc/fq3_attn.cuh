@@ -9,6 +9,7 @@ struct AttnArgs {
   const bf16 *k, *v;        // row j of key / value head g at j * ld + g * 128
   long ldq, ldk, ldv;
   int H, G, M;
+  int groups;               // row groups per CTA: 2, or 1 while the CTAs of one group each are a single wave
   const int* p0;            // position of query 0 (device), or null: 0
   float scale, cap, mult;   // mult != 0 multiplies the output
   int window, keep, chunk;  // 0: none
@@ -40,6 +41,8 @@ __device__ __forceinline__ void tmem_ld32(const uint32_t a, float* f) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
 }
+// the lowest n bits (none below 0, all from 32 on)
+__device__ __forceinline__ uint32_t first_bits(const int n) { return n >= 32 ? 0xffffffffu : (1u << max(n, 0)) - 1u; }
 // 2^n for a whole number n <= 0, exactly (0 below the normal range)
 __device__ __forceinline__ float pow2_down(const float n) { return n < -126.f ? 0.f : __int_as_float(((int)n + 127) << 23); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -93,7 +96,7 @@ __device__ __noinline__ void at_row_again(const AttnArgs& a, const int m, const 
   }
 }
 
-// A CTA takes two groups of 128 rows of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
+// A CTA takes two groups of 128 rows (a.groups = 1: one) of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
 // staged tile.  Warps 0-7 and 8-15: two threads per row of group 0 and 1, 64 keys of a tile each; warps 16-18 stage key and value tiles of 128 positions (two
 // stages); warp 19 issues the MMAs.  Per group and tile: S = Q K^T into tensor memory; the row's threads scale, cap and mask its 128 scores, agree on the
 // maximum, take 2^(score log2 e - reference) and write every weight as a bf16 pair hi + mid (16 mantissa bits) over S; O += hi V + mid V with the weights read from
@@ -138,12 +141,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   grid_dep_wait();
 
   const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
-  const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * QB;   // the last queries (most keys) start first
+  const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * a.groups * QB;   // the last queries (most keys) start first
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
-    nq[g] = max(0, min(QB, a.M - m0 - g * QB));
+    nq[g] = g < a.groups ? max(0, min(QB, a.M - m0 - g * QB)) : 0;
     first[g] = P + m0 + g * QB;
     last[g] = first[g] + nq[g] - 1;
     tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
@@ -152,12 +155,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     tlo[g] = lo / AT_KEYS;
   }
   const int tkeep = a.window > 0 && a.chunk <= 0 ? (a.keep + AT_KEYS - 1) / AT_KEYS : 0;
-  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + 2 * QB) - 1;
+  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + a.groups * QB) - 1;
   auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
 
   if (warp == 19) {
-    const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);   // F32 += BF16 x BF16, both K-major
-    const uint32_t idesc_o = idesc_s | (1u << 16);                                                        // B (values: rows = keys) MN-major
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);   // F32 += BF16 x BF16, both K-major; columns: bits 17..
+    const uint32_t idesc_o = idesc | ((128u >> 3) << 17) | (1u << 16);                                                        // B (values: rows = keys) MN-major
     bool pend[2] = {false, false}, begun[2] = {false, false};
     int prev = 0;
     bool gone = false;      // a wait gave up: nothing more is issued
@@ -165,16 +168,20 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     if (nq[1] > 0 && !gp_wait(q_full + 8, 0, dead, a.tries)) gone = true;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     int nl[2] = {0, 0};
+    // steps of 16 keys of tile t up to the group's last position: what lies behind is neither scored nor multiplied
+    auto steps = [&](const int g, const int t) { return min(8, (last[g] - t * AT_KEYS) / 16 + 1); };
     // O[g] += P[g] V of the tile in stage st
     auto values = [&](const int g, const int st) {
       const uint32_t pa = tmem + g * 128, d = tmem + 256 + g * 128;
+      const int ks = steps(g, prev);
       // MN-major, 128-byte swizzle: 64 columns further is a half tile further, eight keys further 1024 bytes
       const uint64_t vd = (uint64_t)(((v_s + st * AT_TILE) & 0x3ffffu) >> 4) | ((uint64_t)(AT_TILE / 2 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
       if (leader && !gone) {
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) umma_bf16_ta(d, pa + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, (begun[g] || part || kk) ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk)
+            if (kk < ks) umma_bf16_ta(d, pa + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, (begun[g] || part || kk) ? 1u : 0u);
           if (MODE == AT_PROMPT && part == 0) umma_commit(h_done + 8u * g);
         }
       }
@@ -183,7 +190,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (leader && !gone) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) umma_bf16_ta(d, pa + (kk >> 1) * 32 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, 1u);
+          for (int kk = 0; kk < 8; ++kk)
+            if (kk < ks) umma_bf16_ta(d, pa + (kk >> 1) * 32 + (kk & 1) * 8, vd + kk * (2048 >> 4), idesc_o, 1u);
         }
       }
       if (leader && !gone && prev == tiles[g] - 1) umma_commit(o_done + 8u * g);
@@ -213,6 +221,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         }
         if (g ? n1 : n0) {
           if (leader && !gone) {
+            const uint32_t idesc_s = idesc | ((uint32_t)steps(g, t) << 18);
             const uint64_t qd = umma_desc_sw128(q_s + g * AT_TILE), kd = umma_desc_sw128(k_s + st * AT_TILE);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
@@ -238,7 +247,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     const bf16 *kc = a.k + (size_t)kvh * 128, *vc = a.v + (size_t)kvh * 128;
     auto stage = [&](const bf16* src, const long ld, const uint32_t dst, const int j0, const uint32_t bar) {
       if (gone) return;
-      for (int i = lt; i < 128 * 16; i += AT_LOADERS) {      // 16 lanes read a row
+      const int n16 = min(8, (jend - j0) / 16 + 1) * 256;      // 16 lanes read a row; rows behind the last steps of 16 keys are not looked at
+      for (int i = lt; i < n16; i += AT_LOADERS) {
         const int r = i >> 4, c = i & 15, j = j0 + r;
         const bool ok = j <= jend;
         const uint32_t at = dst + (uint32_t)((c >> 3) * (AT_TILE / 2) + r * 128 + (((c & 7) ^ (r & 7)) << 4));
@@ -265,7 +275,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     if (nqg > 0) {
       {   // the group's queries: a warp per row, rounded to bf16 once
         unsigned char* qt = gbase + g * AT_TILE;
-#pragma unroll 8
+#pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int r = (half * 4 + wq) * 16 + i, qi = r / HG, hh = r - qi * HG;
           uint2 w = make_uint2(0u, 0u);
@@ -335,14 +345,15 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (h == 0) tmem_ld32(s_t + 32, s[1]);      // on its way while the first half is worked on
+          if (k0 + h * 32 <= wlast) {      // (keys behind every row of the warp: masked below, whatever they are)
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i);
+            for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i);
+          }
           if (!whole) {
+            // which of the 32 keys the row sees, as bits: conditions per score became divergent branches (8 400 cycles a tile)
+            const uint32_t sees = first_bits(hi_k + 1 - h * 32) & (~first_bits(lo_k - h * 32) | first_bits(kp_k - h * 32));
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int k = h * 32 + i;
-              if (!(k <= hi_k && (k >= lo_k || k < kp_k))) s[h][i] = -INFINITY;
-            }
+            for (int i = 0; i < 32; ++i) s[h][i] = (sees >> i) & 1u ? s[h][i] : -INFINITY;
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[h][i]);
@@ -399,8 +410,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         }
         ++c;
       }
-      gp_wait(o_done + 8u * g, 0, dead, a.tries);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // what the output is divided and multiplied by, while the last product runs
       float f = 1.f, den = sum + meet(sum, c & 1);
       if (MODE != AT_PROMPT && a.sink && live) {
         const float sk = a.sink[head], mm = fmaxf(ref, rintf(sk * AT_L2E));
@@ -413,6 +423,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         if (a.gate && !a.entry) sc *= sigmoid_f(a.gate[(size_t)m * a.gate_ld + head]);
         if (a.mult != 0.f) sc *= a.mult;
       }
+      gp_wait(o_done + 8u * g, 0, dead, a.tries);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float* ge = MODE != AT_PROMPT && a.entry ? a.gate + (size_t)m * a.gate_ld + (size_t)head * 128 + half * 64 : nullptr;
       const size_t at = (size_t)m * a.ldo + (size_t)head * 128 + half * 64;
 #pragma unroll 1

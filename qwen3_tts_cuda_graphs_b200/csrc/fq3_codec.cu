@@ -1222,8 +1222,10 @@ bool attn_tc_takes(const AttnArgs& a, const int mode) {
   return a.H % a.G == 0 && a.H / a.G <= 128 && a.ldk % 8 == 0 && a.ldv % 8 == 0 && a.ldq % 4 == 0 && a.ldo % (a.out_f32 ? 4 : 8) == 0 && !off(a.q) && !off(a.k) &&
          !off(a.v) && !off(a.out) && !(mode != AT_PROMPT && a.chunk > 0 && a.window > 0 && a.keep > 0) && attn_attrs_ready();
 }
-void launch_attn_tc(const AttnArgs& a, const int mode, cudaStream_t s, const bool after) {
-  const int per = 2 * (128 / (a.H / a.G));
+void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after) {
+  const int group = 128 / (a.H / a.G);
+  a.groups = (long)((a.M + group - 1) / group) * a.G <= GP_SMS ? 1 : 2;
+  const int per = a.groups * group;
   const dim3 grid((a.M + per - 1) / per, a.G);
   if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
   else if (mode == AT_PLAIN) launch_after(fq3c_attn_tc_kernel<AT_PLAIN>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
@@ -2083,8 +2085,9 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
           a.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES; a.lost = (o.reserved >> 1) & 1;
           a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
-          // up to 80 rows the kernel below is faster (a warp per query and head, no tile to stage): 64 rows 8.0 against 8.8 us, 100 rows 16.0 against 11.8
-          if (use_apf != 2 && o.M > 80 && attn_tc_takes(a, AT_PROMPT)) {
+          // Up to 112 rows the kernel below is faster (a warp per query and head, no tile to stage).  It against this one, heads 16 / 8, 14 / 2, 1 / 1: 81 rows
+          // 9.1, 8.7, 7.9 against 10.9, 11.0, 9.7 us; 100 rows 11.1, 10.5, 9.2 against 10.9, 11.2, 10.3; 128 rows 13.8, 13.2, 11.3 against 11.4, 11.4, 11.3
+          if (use_apf != 2 && o.M > 112 && attn_tc_takes(a, AT_PROMPT)) {
             launch_attn_tc(a, AT_PROMPT, s, after);
             break;
           }

@@ -43,7 +43,7 @@ def rel(got, want):
     return float((got.double() - want).norm() / want.norm())
 
 
-@pytest.mark.parametrize("rows, heads, kv, window", [(81, 16, 8, 0), (128, 16, 8, 0), (129, 4, 4, 0), (262, 16, 8, 0), (300, 4, 4, 40), (700, 6, 2, 0)])
+@pytest.mark.parametrize("rows, heads, kv, window", [(81, 16, 8, 0), (128, 16, 8, 0), (129, 4, 4, 0), (262, 16, 8, 0), (300, 4, 4, 40), (700, 6, 2, 0), (1300, 16, 16, 0), (1290, 12, 12, 200)])      # (the last two: two row groups a CTA)
 def test_prompt_rows(rows, heads, kv, window):
     from qwen3_tts_cuda_graphs_b200 import codec as K
 
@@ -94,7 +94,8 @@ def test_prompt_weights_keep_32_bits():
 # rows, positions in front, heads, key heads, options
 CASES = [(9, 0, 4, 2, {}), (100, 0, 4, 1, {}), (300, 77, 6, 2, {}), (128, 128, 16, 4, dict(cap=50.0, sink=True, gate=1)), (513, 300, 16, 4, dict(cap=50.0, sink=True)),
          (200, 300, 8, 2, dict(window=64)), (200, 300, 8, 2, dict(window=64, keep=5, dist=True, cap=50.0)), (128, 128, 3, 1, dict(window=130, keep=200)), (400, 0, 8, 8, dict(window=1)),
-         (700, 129, 4, 4, dict(chunk=100, sink=True)), (700, 129, 4, 4, dict(chunk=1000, gate=2)), (260, 260, 12, 4, dict(dist=True, spread=4.0)), (300, 0, 2, 2, dict(spread=8.0)), (40, 700, 2, 1, dict(rising=True))]
+         (700, 129, 4, 4, dict(chunk=100, sink=True)), (700, 129, 4, 4, dict(chunk=1000, gate=2)), (260, 260, 12, 4, dict(dist=True, spread=4.0)), (300, 0, 2, 2, dict(spread=8.0)), (40, 700, 2, 1, dict(rising=True)),
+         (1300, 100, 16, 16, {}), (1285, 33, 16, 16, dict(window=300, keep=2)), (33, 0, 8, 2, dict(cap=50.0)), (17, 111, 4, 4, {}), (9, 7, 1, 1, {})]
 
 
 @pytest.mark.parametrize("rows, first, heads, kv, opt", CASES)
