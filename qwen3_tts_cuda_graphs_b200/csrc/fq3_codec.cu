@@ -1162,8 +1162,9 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
     const int bn = o.N >= 64 ? 64 : 32;
     const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
     const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));
-    // (the cluster's two meetings and the sums cost about 5000 cycles: two splits of 16 k-blocks, 6.9 against 5.6 us, do not pay)
-    if (sp > 1 && (long)KT * 430 - (long)((KT + sp - 1) / sp) * 440 > 5000) { g.splits = sp; g.bn = bn; }
+    // The cluster's two meetings and the sums cost about 3700 cycles and 90 for each row of the tile.  Split against whole: 72 x 1024 x 2048 8.1 and 8.7 us,
+    // 100 rows 9.1 and 8.7, 130 x 1024 x 1024 9.5 and 6.0, 262 x 1024 x 2048 12.4 and 9.1, 130 x 2048 x 6144 17.8 and 21.0.
+    if (sp > 1 && (long)KT * 430 - (long)((KT + sp - 1) / sp) * 440 > 3700 + 90L * std::min(o.M, TM)) { g.splits = sp; g.bn = bn; }
   }
   long kl = 0, ep = 0;
   if (g.splits == 1) {
