@@ -1920,7 +1920,8 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
   cudaStream_t s = main_stream;
   // The codec's kernels wait for the launches in front themselves and may begin early, as long as the launch in front on their stream belongs to this list
   // (what ran before the list is complete when its first launch begins): a prompt of 39 rows through 28 layers 1676 -> 1497 us, a codec window 1059 -> 972.
-  // The sequence models' kernels are launched one behind the other: early launches made their replays slower (a request of 24 tokens 5.4 -> 6.4 ms).
+  // The sequence models' own kernels are launched one behind the other (their GEMMs are not): early launches made their replays slower (a request of 24
+  // tokens 5.4 -> 6.4 ms).
   bool chained = false;
   for (int i = 0; i < n_ops; ++i) {
     const fq3c_op& o = ops[i];
@@ -2080,7 +2081,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
       case FQ3C_ATTN: {
         if (o.i2 > 128) return fail("attn: head_dim > 128");
         static int use_apf = -1;
-        if (use_apf < 0) { const char* e5 = getenv("FQ3C_ATTN_PREFILL"); use_apf = e5 == nullptr ? 1 : atoi(e5); }
+        if (use_apf < 0) { const char* e5 = getenv("FQ3C_ATTN_PREFILL"); use_apf = (e5 == nullptr || atoi(e5) != 0) ? 1 : 0; }
         if (use_apf && (o.flags & 1) && o.i2 == 128 && o.taps == 0 && !o.p0) {
           AttnArgs a{};
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
@@ -2088,7 +2089,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
           // Up to 112 rows the kernel below is faster (a warp per query and head, no tile to stage).  It against this one, heads 16 / 8, 14 / 2, 1 / 1: 81 rows
           // 9.1, 8.7, 7.9 against 10.9, 11.0, 9.7 us; 100 rows 11.1, 10.5, 9.2 against 10.9, 11.2, 10.3; 128 rows 13.8, 13.2, 11.3 against 11.4, 11.4, 11.3
-          if (use_apf != 2 && o.M > 112 && attn_tc_takes(a, AT_PROMPT)) {
+          if (o.M > 112 && attn_tc_takes(a, AT_PROMPT)) {
             launch_attn_tc(a, AT_PROMPT, s, after);
             break;
           }

@@ -84,7 +84,10 @@ def test_product_and_epilogues(name):
             launch([make_op(A, B, out, M, N, cin, offs, flags, ws=ws)])
             gate, up = want[:, 0::2], want[:, 1::2]
             unit = gate * torch.sigmoid(gate) * up
-            assert ((out.double() - unit).abs() <= 2.0 ** -8 * (2 + gate.abs()) * 2 * (unit.abs() + up.abs() * 2.0 ** -8 + gate.abs() * 2.0 ** -8) + 1e-5).all()
+            # silu's slope is at most 1.1; rounded sums: gate, silu, up and the product are each rounded, else the result alone
+            sums = len(offs) * cin * 2.0 ** -24 * (1.1 * mag[:, 0::2] * up.abs() + (gate * torch.sigmoid(gate)).abs() * mag[:, 1::2])
+            rounds = unit.abs() if flags & K.F_NOROUND else 1.1 * (gate * up).abs() + 4 * unit.abs()
+            assert ((out.double() - unit).abs() <= 1.01 * 2.0 ** -9 * rounds + sums + 2.0 ** -20 * unit.abs() + 1e-6).all()
 
 
 def test_rows_from_m_begin_on_are_the_full_products_rows():
@@ -131,3 +134,63 @@ def test_widths_between_whole_pieces(M, N, K, scratch):
         err = K * 2.0 ** -24 * mag + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
         assert ((out[:M, :N].double() - want).abs() <= err).all()
         assert (out[:, wide if scratch else N:] == 7).all() and (out[M] == 7).all()
+
+
+# 39 rows: staged, from shared memory; 9000 rows of 768 columns: a CTA goes on to another column tile; 300 x 200: a last piece of eight columns
+@pytest.mark.parametrize("M, N, cin, col_mod", [(39, 384, 128, 384), (300, 200, 64, 200), (300, 768, 64, 192), (9000, 768, 64, 256)])
+@pytest.mark.parametrize("what", ["gelu", "silu", "clamp", "relu2", "snake"])
+def test_vector_epilogues(M, N, cin, col_mod, what):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    A, B = torch.randn(M, cin, device="cuda", generator=g).bfloat16(), (torch.randn(N, cin, device="cuda", generator=g) / cin ** 0.5).bfloat16()
+    bias, res = torch.randn(col_mod, device="cuda", generator=g), torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    want, mag = product(A, B, M, cin, (0,))
+    z = want + bias.double().repeat(N // col_mod)
+    err = 2.0 ** -20 * mag + 1e-6
+    out = torch.zeros(M, N, device="cuda", dtype=torch.float32 if what == "relu2" else torch.bfloat16)
+    flags = dict(gelu=K.F_GELU, silu=K.F_SILU, clamp=K.F_CLAMP, relu2=K.F_RELU2 | K.F_OUT_F32 | K.F_NOROUND, snake=K.F_SNAKE2)[what]
+    o = make_op(A, B, out, M, N, cin, flags=flags, bias=bias, res=res if what == "snake" else None)
+    o.col_mod = col_mod
+    if what == "snake":
+        out2 = torch.zeros_like(out)
+        ea, ib = torch.rand(col_mod, device="cuda", generator=g) * 4, torch.rand(col_mod, device="cuda", generator=g)
+        ea[3], ea[7] = 2e5, 1e6      # far from zero, and beyond the range of the reduction
+        o.C2, o.p0, o.p1 = out2.data_ptr(), ea.data_ptr(), ib.data_ptr()
+    launch([o])
+    r = 1.01 * 2.0 ** -9
+    if what == "gelu":
+        y = torch.nn.functional.gelu(z)
+        assert ((out.double() - y).abs() <= r * (1.13 * z.abs() + y.abs()) + err).all()
+    elif what == "silu":
+        y = z * torch.sigmoid(z)
+        assert ((out.double() - y).abs() <= r * (1.1 * z.abs() + y.abs()) + err).all()
+    elif what == "clamp":
+        assert ((out.double() - z.clamp(-1, 1)).abs() <= r * z.abs() + err).all()
+    elif what == "relu2":
+        y = z.clamp(min=0)
+        assert ((out.double() - y * y).abs() <= 2 * y * err + err ** 2 + 2.0 ** -23 * y * y).all()
+    else:
+        y = z + res.double()
+        assert ((out.double() - y).abs() <= r * (z.abs() + y.abs()) + err).all()
+        x = (out.float() * ea.repeat(N // col_mod)).double()      # what the kernel takes the sine of
+        y = out.double() + ib.double().repeat(N // col_mod) * torch.sin(x) ** 2
+        assert ((out2.double() - y).abs() <= r * y.abs() + 4e-7).all()
+
+
+@pytest.mark.parametrize("M, m_begin", [(1, 0), (255, 0), (256, 0), (257, 0), (257, 256), (700, 130)])
+@pytest.mark.parametrize("offs", [SEVEN, tuple(9 * t for t in SEVEN), (1, 0), (-3, 4)])
+def test_one_output_channel(M, m_begin, offs):
+    """The convolution to a single channel: last blocks, rows in front of and behind the input, spread taps, rows from m_begin on."""
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for cin in (8, 96, 128):
+        A, B = torch.randn(M, cin, device="cuda", generator=g).bfloat16(), (torch.randn(1, len(offs) * cin, device="cuda", generator=g) / 20).bfloat16()
+        bias = torch.randn(1, device="cuda", generator=g)
+        want, mag = product(A, B, M, cin, offs)
+        out = torch.full((M + 1, 1), 7.0, device="cuda")
+        launch([make_op(A, B, out, M, 1, cin, offs, K.F_OUT_F32 | K.F_CLAMP, bias=bias, m_begin=m_begin)])
+        z = want + bias.double()
+        assert ((out[:M].double() - z.clamp(-1, 1)).abs() <= 1.01 * 2.0 ** -9 * z.abs() + 2.0 ** -20 * mag + 1e-6)[m_begin:].all()
+        assert (out[:m_begin] == 7).all() and out[M] == 7
