@@ -20,6 +20,7 @@ def test_a_window_ends_beside_the_frame_loop():
         eng.prefill(0, rows(120), 0, policy, dense=False)
         hidden, codes = rows(), torch.randint(0, 2048, (33, 16), device="cuda", generator=g)
         alone = dec.decode(codes, 25 * 1920)
+        torch.cuda.synchronize()      # (a plan's buffers belong to one stream at a time)
         side = torch.cuda.Stream()
         with torch.cuda.stream(side):
             for _ in range(3):      # (from the second use on a graph; the stream's memory is there too)

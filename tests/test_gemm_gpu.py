@@ -87,7 +87,7 @@ def test_product_and_epilogues(name):
             # silu's slope is at most 1.1; rounded sums: gate, silu, up and the product are each rounded, else the result alone
             sums = len(offs) * cin * 2.0 ** -24 * (1.1 * mag[:, 0::2] * up.abs() + (gate * torch.sigmoid(gate)).abs() * mag[:, 1::2])
             rounds = unit.abs() if flags & K.F_NOROUND else 1.1 * (gate * up).abs() + 4 * unit.abs()
-            assert ((out.double() - unit).abs() <= 1.01 * 2.0 ** -9 * rounds + sums + 2.0 ** -20 * unit.abs() + 1e-6).all()
+            assert ((out.double() - unit).abs() <= 1.01 * 2.0 ** -8 * rounds + sums + 2.0 ** -20 * unit.abs() + 1e-6).all()
 
 
 def test_rows_from_m_begin_on_are_the_full_products_rows():
@@ -158,7 +158,7 @@ def test_vector_epilogues(M, N, cin, col_mod, what):
         ea[3], ea[7] = 2e5, 1e6      # far from zero, and beyond the range of the reduction
         o.C2, o.p0, o.p1 = out2.data_ptr(), ea.data_ptr(), ib.data_ptr()
     launch([o])
-    r = 1.01 * 2.0 ** -9
+    r = 1.01 * 2.0 ** -8      # bf16 keeps 8 bits: half of the last one
     if what == "gelu":
         y = torch.nn.functional.gelu(z)
         assert ((out.double() - y).abs() <= r * (1.13 * z.abs() + y.abs()) + err).all()
@@ -192,5 +192,5 @@ def test_one_output_channel(M, m_begin, offs):
         out = torch.full((M + 1, 1), 7.0, device="cuda")
         launch([make_op(A, B, out, M, 1, cin, offs, K.F_OUT_F32 | K.F_CLAMP, bias=bias, m_begin=m_begin)])
         z = want + bias.double()
-        assert ((out[:M].double() - z.clamp(-1, 1)).abs() <= 1.01 * 2.0 ** -9 * z.abs() + 2.0 ** -20 * mag + 1e-6)[m_begin:].all()
+        assert ((out[:M].double() - z.clamp(-1, 1)).abs() <= 1.01 * 2.0 ** -8 * z.abs() + 2.0 ** -20 * mag + 1e-6)[m_begin:].all()
         assert (out[:m_begin] == 7).all() and out[M] == 7
