@@ -1537,7 +1537,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         return fail("cache_attn: pooled blocks go with a window and their pooled rows, not with kept first positions, a chunked mask or a distance penalty");
       if (splits > 64) return fail("cache_attn: at most 64 key splits");
       if (splits > 1 && (!o.ws || o.ws_bytes < (int64_t)o.M * o.i0 * splits * (o.cin + 2) * 4)) return fail("cache_attn: workspace too small for the splits");
-      // bf16 cache and a prompt portion: the tensor-core kernels (FQ3S_ATTN_MMA=0: CUDA cores everywhere)
+      // bf16 cache and a prompt portion: the tensor-core kernels (FQ3S_ATTN_MMA=0: CUDA cores everywhere).  Heads of 128 on tcgen05 from 9 rows on: against the
+      // mma.sync kernel 9 rows of 16 heads over 4 behind 2000 positions 185 and 51 us, 1000 rows 303 and 76; only short portions at the very
+      // beginning are slower (33-64 rows at position 0: 10.7-11.5 and 12.9), and the host does not know where a portion begins.
       static int use_mma = -1;
       if (use_mma < 0) { const char* e7 = getenv("FQ3S_ATTN_MMA"); use_mma = (e7 == nullptr || atoi(e7) != 0) ? 1 : 0; }
       if (use_mma && !(o.flags & FQ3C_F32) && o.M > 8 && o.i2 == 128 && o.cin == 128 && !pool) {
@@ -2087,9 +2089,11 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
           a.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES; a.lost = (o.reserved >> 1) & 1;
           a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
-          // Up to 112 rows the kernel below is faster (a warp per query and head, no tile to stage).  It against this one, heads 16 / 8, 14 / 2, 1 / 1: 81 rows
-          // 9.1, 8.7, 7.9 against 10.9, 11.0, 9.7 us; 100 rows 11.1, 10.5, 9.2 against 10.9, 11.2, 10.3; 128 rows 13.8, 13.2, 11.3 against 11.4, 11.4, 11.3
-          if (o.M > 112 && attn_tc_takes(a, AT_PROMPT)) {
+          // Few rows are faster in the kernel below (a warp per query and head, no tile to stage), whose time grows with rows^2 x heads.  Launched early as both
+          // are, it against this one: 81 rows of 16 heads 10.2 and 10.9 us, of 32 14.1 and 10.9, of 14 9.8 and 11.0; 90 of 16 11.5 and 10.9, of 14 10.0 and 11.1;
+          // 100 of 14 12.0 and 11.2, of 8 10.7 and 10.3, of 1 8.9 and 10.3; 128 of 8 12.4 (not early) and 11.3
+          const bool many = o.M > 112 || (o.M > 64 && (long)o.M * o.M * o.i0 > 115000);
+          if (many && attn_tc_takes(a, AT_PROMPT)) {
             launch_attn_tc(a, AT_PROMPT, s, after);
             break;
           }
