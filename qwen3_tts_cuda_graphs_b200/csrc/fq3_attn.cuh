@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     bool pend[2] = {false, false}, begun[2] = {false, false};
     int prev = 0;
     bool gone = false;      // a wait gave up: nothing more is issued
-    if (!gp_wait(q_full, 0, dead, a.tries)) gone = true;
-    if (nq[1] > 0 && !gp_wait(q_full + 8, 0, dead, a.tries)) gone = true;
+    if (!gp_wait_warp(q_full, 0, dead, a.tries)) gone = true;
+    if (nq[1] > 0 && !gp_wait_warp(q_full + 8, 0, dead, a.tries)) gone = true;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     int nl[2] = {0, 0};
     // steps of 16 keys of tile t up to the group's last position: what lies behind is neither scored nor multiplied
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         part(16, true);
       }
       if (MODE == AT_PROMPT) {
-        if (!gp_wait(l_full + 8u * g, (uint32_t)(nl[g]++ & 1), dead, a.tries)) gone = true;
+        if (!gp_wait_warp(l_full + 8u * g, (uint32_t)(nl[g]++ & 1), dead, a.tries)) gone = true;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (leader && !gone) part(0, true);
       }
@@ -207,17 +207,17 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       if (more && !n0 && !n1) continue;
       const int st = n & 1;
       if (more) {
-        if (!gp_wait(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead, a.tries)) gone = true;
+        if (!gp_wait_warp(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead, a.tries)) gone = true;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       if (pend[0] || pend[1]) {
-        if (!gp_wait(v_full + 8u * (st ^ 1), (uint32_t)(((n - 1) >> 1) & 1), dead, a.tries)) gone = true;
+        if (!gp_wait_warp(v_full + 8u * (st ^ 1), (uint32_t)(((n - 1) >> 1) & 1), dead, a.tries)) gone = true;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         if (pend[g]) {
-          if (!gp_wait(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead, a.tries)) gone = true;
+          if (!gp_wait_warp(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead, a.tries)) gone = true;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           values(g, st ^ 1);
           pend[g] = false;
@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       if (!need(0, t) && !need(1, t)) continue;
       const int st = n & 1;
       const uint32_t ph = (uint32_t)(((n >> 1) - 1) & 1);
-      if (n >= 2 && !gp_wait(k_empty + 8u * st, ph, dead, a.tries)) gone = true;
+      if (n >= 2 && !gp_wait_warp(k_empty + 8u * st, ph, dead, a.tries)) gone = true;
       if (n > 0 || !a.lost) stage(kc, a.ldk, k_s + st * AT_TILE, t * AT_KEYS, k_full + 8u * st);
-      if (n >= 2 && !gp_wait(v_empty + 8u * st, ph, dead, a.tries)) gone = true;
+      if (n >= 2 && !gp_wait_warp(v_empty + 8u * st, ph, dead, a.tries)) gone = true;
       stage(vc, a.ldv, v_s + st * AT_TILE, t * AT_KEYS, v_full + 8u * st);
       ++n;
     }
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       int c = 0;
       for (int t = 0; t < tilesg; ++t) {
         if (!need(g, t)) continue;
-        gp_wait(s_full + 8u * g, (uint32_t)(c & 1), dead, a.tries);
+        gp_wait_warp(s_full + 8u * g, (uint32_t)(c & 1), dead, a.tries);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int j0 = t * AT_KEYS, k0 = j0 + half * 64;
         // tiles that every row of the warp sees whole need no per-score test
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full + 8u * g);
         if (MODE == AT_PROMPT) {
-          gp_wait(h_done + 8u * g, (uint32_t)(c & 1), dead, a.tries);
+          gp_wait_warp(h_done + 8u * g, (uint32_t)(c & 1), dead, a.tries);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           tmem_st16(s_t, rest[0]);
           tmem_st16(s_t + 32, rest[1]);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         if (a.gate && !a.entry) sc *= sigmoid_f(a.gate[(size_t)m * a.gate_ld + head]);
         if (a.mult != 0.f) sc *= a.mult;
       }
-      gp_wait(o_done + 8u * g, 0, dead, a.tries);
+      gp_wait_warp(o_done + 8u * g, 0, dead, a.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float* ge = MODE != AT_PROMPT && a.entry ? a.gate + (size_t)m * a.gate_ld + (size_t)head * 128 + half * 64 : nullptr;
       const size_t at = (size_t)m * a.ldo + (size_t)head * 128 + half * 64;

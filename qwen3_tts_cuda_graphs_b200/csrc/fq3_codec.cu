@@ -1142,7 +1142,13 @@ bool gemm_vec16(const fq3c_op& o) {
   if ((o.flags & FQ3C_SNAKE2) && off(o.C2, 32)) return false;
   return true;
 }
-struct GemmLaunch { GemmPlan g; bool half; unsigned grid; size_t smem; };
+// A tile's epilogue, in cycles for 16 columns of its 128 rows with sixteen warps at work on an SM (two CTAs of eight or one of sixteen; fitted to 75776 x 384 x 64,
+// where it is all there is: bf16 18 us, residual 34 - 42, GELU 43, gated units 38, residual and SnakeBeta 59 - 65).
+long epilogue_piece(const int flags) {
+  return 290 + (flags & FQ3C_RESID ? 310 : 0) + (flags & FQ3C_SNAKE2 ? 480 : 0) + (flags & (FQ3C_GELU | FQ3C_SILU) ? 560 : 0) + (flags & FQ3C_SWIGLU ? 510 : 0);
+}
+enum GemmShape { GS_WIDE, GS_FEW, GS_HALF };      // one CTA per SM with sixteen epilogue warps, one with eight, two with eight each
+struct GemmLaunch { GemmPlan g; GemmShape shape; unsigned grid; size_t smem; };
 GemmLaunch gemm_plan(const fq3c_op& o) {
   GemmLaunch L{};
   GemmPlan& g = L.g;
@@ -1153,34 +1159,41 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   g.kb = o.taps == 1 ? g.kpt : g.kpt * o.taps;
   const int last = (o.taps == 1 ? o.K : o.cin) - (g.kpt - 1) * TK;
   g.tail = (last + 15) / 16;
-  // Split over K when the tiles would cover less than half of the SMs and the reduction is long (the transformer's o / down projections at 8-240
-  // rows: 16-48 tiles of 32-48 k-blocks): up to eight CTAs per tile, a cluster.  The count must not depend on m_begin: a tail-only decode has to add
-  // the same partial sums in the same order.
+  // 64 rows and fewer: half of sixteen warps would have no rows, and the smaller block starts sooner (39 x 4096 x 1024: 5.0 and 5.3 us)
+  const bool few = g.a_rows <= 64;
+  L.shape = few ? GS_FEW : GS_WIDE;
+  const int groups = few ? 2 : 4;
+  // Split over K when the tiles would cover less than half of the SMs and the reduction is long (the transformer's o / down projections of few rows: 16-32 tiles of
+  // 32-48 k-blocks): two or four CTAs per tile, a cluster; six, eight and more than 128 CTAs in clusters do not find room at the same time (17 x 1024 x 2048: four
+  // 5.7 us, six 6.3, eight 11.3).  The count must not depend on m_begin: a tail-only decode has to add the same partial sums in the same order.
   const int KT = (o.K + TK - 1) / TK;
   g.splits = 1;
   if ((o.ws || (o.reserved & 4)) && o.M <= 4 * TM && KT >= 8) {
     const int bn = o.N >= 64 ? 64 : 32;
     const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
-    const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));
-    // The cluster's two meetings and the sums cost about 3700 cycles and 90 for each row of the tile.  Split against whole: 72 x 1024 x 2048 8.1 and 8.7 us,
-    // 100 rows 9.1 and 8.7, 130 x 1024 x 1024 9.5 and 6.0, 262 x 1024 x 2048 12.4 and 9.1, 130 x 2048 x 6144 17.8 and 21.0.
-    if (sp > 1 && (long)KT * 430 - (long)((KT + sp - 1) / sp) * 440 > 3700 + 90L * std::min(o.M, TM)) { g.splits = sp; g.bn = bn; }
+    const int sp = tiles * 4 <= 128 && KT >= 16 ? 4 : tiles * 2 <= 128 ? 2 : 1;
+    // The cluster's two meetings and the sums cost about 5000 cycles and 30 for each row of the tile, a k-block 300.  Whole against split: 17 x 1024 x 2048 6.6 and
+    // 5.7 us, 64 rows 6.6 and 6.4, 100 rows 6.7 and 7.0; 39 x 1024 x 3072 9.1 and 6.7, 130 rows 9.4 and 9.0, 262 rows 9.8 and 10.0; 39 x 2048 x 6144 15.7 and 10.0.
+    if (sp > 1 && (long)(KT - (KT + sp - 1) / sp) * 300 > 5000 + 30L * std::min(o.M, TM)) { g.splits = sp; g.bn = bn; }
   }
-  long kl = 0, ep = 0;
   if (g.splits == 1) {
-    // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  Measured: a k-block (four MMAs, a
-    // commit, the waits on both sides) takes 427 cycles at 32 columns, 458 at 128, 480 at 224, 512 at 256: the issuing warp's loop, not the tensor pipe, which is
-    // busy for 130-510 of them; or its operand bytes at the 60 a cycle that L2 gives one SM.  The epilogue takes about 20 a column, four times that with sines.
+    // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  A k-block takes what its instructions take (300), its four products
+    // (two cycles a column), or its operand bytes at the 60 a cycle that L2 gives one SM.  The operand bytes of all tiles count a little by themselves: of two widths
+    // that cost the same the wider one reads A less often (491520 x 96 x 96 with SnakeBeta: 16 columns 264 us, 96 columns 87).
+    // Two CTAs per SM overlap their epilogues with each other's waits, but share the stages: only where a tile's few k-blocks fit in them (the same product over seven
+    // taps: 143 us against 126).
     long best = -1;
-    const int per_col = (o.flags & FQ3C_SNAKE2) ? 80 : 20;
+    const long piece = epilogue_piece(o.flags);
     for (int cand = 256; cand >= 16; cand -= 16) {
       const int nt = (o.N + cand - 1) / cand;
-      const int bn = std::min(256, ((o.N + nt - 1) / nt + 15) / 16 * 16);
+      const int bn = std::min(256, ((o.N + nt - 1) / nt + 15) / 16 * 16), pieces = bn / 16;
       if (bn != cand && cand != 16) continue;
-      const long tiles = (long)nt * g.mt, waves = (tiles + GP_SMS - 1) / GP_SMS;
-      const long k = (long)g.kb * std::max(420 + bn / 3, (g.a_rows + bn) * 128 / 60), e = (long)bn * per_col;
-      const long cost = waves * std::max(k, e) + std::min(k, e);
-      if (best < 0 || cost < best) { best = cost; g.bn = bn; kl = k; ep = e; }
+      const long tiles = (long)nt * g.mt, bytes = (g.a_rows + bn) * 128L, reads = tiles * g.kb * bytes / (4 * 60 * GP_SMS);
+      auto cost = [&](const long rounds, const long k, const long e) { return rounds * std::max(k, e) + std::min(k, e) + reads; };
+      const long c1 = cost((tiles + GP_SMS - 1) / GP_SMS, g.kb * std::max({300L, 2L * bn + 20, bytes / 60}), 700 + (pieces + groups - 1) / groups * groups * piece);
+      const long c2 = cost(2 * ((tiles + 2 * GP_SMS - 1) / (2 * GP_SMS)), g.kb * std::max({160L, 2L * bn + 20, bytes / 60}), 500 + pieces * piece);
+      const bool half = bn <= 128 && g.kb <= 4 && gp_stage_bytes(g.a_rows, bn) * std::max(2, g.kb) + GP_BAR_BYTES + 1024 <= GP_SMEM_HALF && c2 < c1;
+      if (best < 0 || (half ? c2 : c1) < best) { best = half ? c2 : c1; g.bn = bn; L.shape = half ? GS_HALF : few ? GS_FEW : GS_WIDE; }
     }
   }
   g.nt = (o.N + g.bn - 1) / g.bn;
@@ -1190,18 +1203,18 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   g.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES;
   g.lost = o.reserved & 2 ? 0 : -1;
   // (few rows and a costly epilogue: 39 rows of gated units 8.3 -> 7.5 us; without one the extra meeting costs 1 us more than it saves)
-  g.staged = g.splits > 1 || (g.mt == 1 && g.a_rows <= 64 && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
+  g.staged = g.splits > 1 || (g.mt == 1 && few && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
   g.vec16 = gemm_vec16(o) ? 1 : 0;
-  const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = g.splits > 1 ? (g.kb + g.splits - 1) / g.splits : g.kb;
-  // Two CTAs per SM: tiles of one wave keep to half of an SM, so that the next launch's CTAs fit beside them and ask for their weights early; tiles
-  // bound by their epilogue get twice the epilogue warps.
-  L.half = g.acc_cols <= 128 && ((sb * 4 + 2048 <= GP_SMEM_HALF && tiles * g.splits <= 2 * GP_SMS) || (sb * 3 + 2048 <= GP_SMEM_HALF && g.splits == 1 && ep > kl));
-  // The MMA reads 128 rows of A also where the box has fewer: the last stage's are inside the allocation.  A partial tile (at least four k-blocks
-  // per split, 4 x 128 bytes a row against 4 x (bn + 4)) fits in the stages.
-  const int room = (L.half ? GP_SMEM_HALF : GP_SMEM_MAX) - 1024, fit = std::min((room - GP_BAR_BYTES) / sb, (room - T_A_BYTES) / sb + 1);
-  g.stages = std::max(2, std::min(std::min(fit, 16), g.splits > 1 ? n_kb : 16));
+  const bool half = L.shape == GS_HALF;
+  const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = (g.kb + g.splits - 1) / g.splits;
+  // The MMA reads 128 rows of A also where the box has fewer: the last stage's are inside the allocation.  One tile per CTA needs no more stages than k-blocks,
+  // and a staged one's partial tile has to fit in them.
+  const int room = (half ? GP_SMEM_HALF : GP_SMEM_MAX) - 1024, fit = std::min((room - GP_BAR_BYTES) / sb, (room - T_A_BYTES) / sb + 1);
+  const int part = (g.a_rows * gp_part_pitch(g.bn) * 4 + sb - 1) / sb;
+  const bool once = g.staged || tiles <= GP_SMS * (half ? 2 : 1);
+  g.stages = std::max(2, std::min(std::min(fit, 16), once ? std::max(n_kb, g.staged ? part : 0) : 16));
   L.smem = (size_t)std::max(g.stages * sb + GP_BAR_BYTES, (g.stages - 1) * sb + T_A_BYTES) + 1024;
-  L.grid = g.staged ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, L.half ? 2 * GP_SMS : GP_SMS);
+  L.grid = g.staged ? (unsigned)(tiles * g.splits) : (unsigned)std::min(tiles, half ? 2 * GP_SMS : GP_SMS);
   return L;
 }
 
@@ -1884,8 +1897,9 @@ static bool device_attrs_ready() {
   if (done[dev]) return true;
   if (cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, T_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_gemm_tc5_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, t_smem(3)) != cudaSuccess ||
-      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
-      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_HALF) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_gemm_persist_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_HALF) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, APF_WARPS * (128 + 2048) * 4) != cudaSuccess)
     return false;
   done[dev] = true;
@@ -1988,8 +2002,9 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           CUtensorMap tmA, tmB;
           if (make_map(&tmA, o.A, (uint64_t)o.cin, (uint64_t)o.a_rows, (uint64_t)o.lda, (uint32_t)L.g.a_rows) &&
               make_map(&tmB, o.B, (uint64_t)o.K, (uint64_t)o.N, (uint64_t)o.K, (uint32_t)L.g.bn)) {
-            if (L.half) launch_after(fq3c_gemm_persist_kernel<2>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
-            else launch_after(fq3c_gemm_persist_kernel<1>, L.grid, GP_THREADS, L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
+            if (L.shape == GS_HALF) launch_after(fq3c_gemm_persist_kernel<2, 8>, L.grid, gp_threads(8), L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
+            else if (L.shape == GS_FEW) launch_after(fq3c_gemm_persist_kernel<1, 8>, L.grid, gp_threads(8), L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
+            else launch_after(fq3c_gemm_persist_kernel<1, 16>, L.grid, gp_threads(16), L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
             if (o.norm_out) {
               launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, true, 1, o);
               count_launches(1);

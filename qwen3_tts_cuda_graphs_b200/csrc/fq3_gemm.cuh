@@ -20,34 +20,40 @@ struct GemmPlan {
   int tries;     // of a wait before it gives up
   int lost;      // k-block whose rows are never asked for (tests of the error path), else -1
 };
-constexpr int GP_EPI_WARPS = 8, GP_MMA_WARP = 8, GP_TMA_WARP = 9, GP_THREADS = 320;
+__host__ __device__ constexpr int gp_threads(int epi_warps) { return (epi_warps + 2) * 32; }
 constexpr int GP_PAR = 256;         // columns of a tile at most: its bias, scale and SnakeBeta parameters lie in shared memory
 constexpr int GP_BAR_BYTES = 512 + 4 * GP_PAR * 4;   // barriers, tensor-memory address, error word; parameters
 __host__ __device__ constexpr int gp_a_bytes(int a_rows) { return (a_rows * TK * 2 + 1023) & ~1023; }
 __host__ __device__ constexpr int gp_stage_bytes(int a_rows, int bn) { return gp_a_bytes(a_rows) + bn * TK * 2; }
 __host__ __device__ constexpr int gp_part_pitch(int bn) { return bn + 4; }   // floats per row of a partial tile: 16-byte rows, 4 banks apart
 
-// A bounded wait of a whole warp.  When its tries run out (about a second) it sets the block's word `dead` and the error words; the block's other waits give up
+// A bounded wait.  When its tries run out (about a second) it sets the block's word `dead`; the block's other waits give up
 // when they see `dead`.  A lane whose wait gave up (false) issues no more copies, products or commits, so that no barrier gets an arrival that its phase does not
-// expect; at its end the kernel waits for what had been issued and fills its outputs with NaN.  (Each lane tries for itself: with a vote per try the
-// waiting warps took issue slots from the working ones.)
+// expect; it sets the error words behind its loop (a call inside would keep the loop's operands out of the uniform registers), and at its end the kernel waits
+// for what had been issued and fills its outputs with NaN.
 constexpr int GP_TRIES = 1 << 20, GP_TRIES_TEST = 4096;
 __device__ __forceinline__ bool gp_wait(const uint32_t bar, const uint32_t parity, volatile int* dead, const int tries) {
-  bool there = true;
-  int i = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if (++i > 256 || i > tries) {      // (a try suspends the thread for a while by itself)
+  if (mbar_try_wait(bar, parity)) return true;
+  for (int i = 1; !mbar_try_wait(bar, parity); ++i)
+    if (i > 256 || i > tries) {      // (a try suspends the thread for a while by itself)
       if (*dead || i > tries) {
         *dead = 1;
-        wait_ran_out();
-        there = false;
-        break;
+        return false;
       }
       __nanosleep(i > 8192 ? 1000 : 20);
     }
-  }
+  return true;
+}
+// the same for a whole warp that goes on together: each lane tries for itself (with a vote per try the waiting warps took issue slots from the working ones)
+__device__ __forceinline__ bool gp_wait_warp(const uint32_t bar, const uint32_t parity, volatile int* dead, const int tries) {
+  const bool there = gp_wait(bar, parity, dead, tries);
+  if (!there) wait_ran_out();
   __syncwarp();
   return there;
+}
+// and for the issuing warps: one answer for all lanes, so that they leave their loops together
+__device__ __forceinline__ bool gp_wait_all(const uint32_t bar, const uint32_t parity, volatile int* dead, const int tries) {
+  return __all_sync(0xffffffffu, gp_wait(bar, parity, dead, tries));
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
@@ -248,15 +254,17 @@ __device__ __noinline__ void poison(const fq3c_op& o, const int row, const int c
   }
 }
 
-// One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  Warp 9 asks for the operand
-// boxes up to `stages` k-blocks ahead, across tiles; warp 8 issues the MMAs of tile n + 1 into the second accumulator while warps 0-7 take tile n
-// through the epilogue.  With splits > 1 a cluster of CTAs shares one tile: each takes a run of k-blocks, leaves its f32 partial tile in its
+// One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  The last warp asks for the operand
+// boxes up to `stages` k-blocks ahead, across tiles; the one before it issues the MMAs of tile n + 1 into the second accumulator while the others take tile n
+// through the epilogue.  What bounds that is latency (accumulator, residual, a chain of conversions per row), so an SM has sixteen such warps, of one CTA or of two:
+// with eight, 1900 x 6144 x 1024 with gated units took 33 us, with sixteen 24.  With splits > 1 a cluster of CTAs shares one tile: each takes a run of k-blocks, leaves its f32 partial tile in its
 // shared memory, and each then adds the partial tiles of a part of the rows in split order.
 // The launch may begin before the ones in front of it have ended (programmatic dependent launch): nothing but B (early_b) is touched before
 // grid_dep_wait.
-template <int MINB>
-__global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ GemmPlan g,
+template <int MINB, int EPI_WARPS>
+__global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ GemmPlan g,
                                                                               const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+  constexpr int MMA_WARP = EPI_WARPS, TMA_WARP = EPI_WARPS + 1, THREADS = gp_threads(EPI_WARPS), GROUPS = EPI_WARPS / 4;
   extern __shared__ unsigned char gp_raw[];
   const uint32_t raw = smem_u32(gp_raw), base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = gp_raw + (base - raw);
@@ -275,17 +283,17 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
 
   if (tid == 0) {
     for (int s = 0; s < g.stages; ++s) { mbar_init(full + 8u * s, 1); mbar_init(empty + 8u * s, 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, GP_EPI_WARPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, EPI_WARPS); }
     mbar_init(drain, 1);
     words[1] = 0;
     words[2] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == GP_MMA_WARP) {
+  if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(words)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (warp == GP_TMA_WARP && lane == 0) {
+  if (warp == TMA_WARP && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
   }
@@ -295,14 +303,14 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   const uint32_t tmem = __shfl_sync(0xffffffffu, words[0], 0);
   grid_dep_launch();
 
-  // The two issuing warps run their loops whole, with one elected lane at the copies and MMAs: in code of a single lane every descriptor goes through
-  // per-lane registers (a k-block took 700-800 cycles to issue that way, whatever its size).
+  // The two issuing warps run their loops whole, with one elected lane at the copies, products and commits: in code of a single lane every operand goes
+  // through per-lane registers (700 - 800 cycles a k-block with `lane == 0`, 380 with the election around the loop).  What bounds a k-block of narrow tiles is
+  // the chain of instructions from one issue to the next, so the inner loops hold no more than a pointer's step each: taps and their last, shorter k-blocks are
+  // outside of them.  347 -> 270 cycles a k-block (40 x 1024 x 8192: 25.9 -> 22.9 us); the tensor pipe needs 160 - 256 up to 128 columns.
   const bool leader = elect_one();
-  if (warp == GP_TMA_WARP) {
-    const uint32_t tx = (uint32_t)(g.a_rows * TK * 2 + g.bn * TK * 2);
-    int it = 0, early = 0, st = 0, asked = 0;
-    bool gone = false;
-    uint32_t ph = 0;      // parity of the stage's current use
+  if (warp == TMA_WARP) {
+    const uint32_t tx = (uint32_t)(g.a_rows * TK * 2 + g.bn * TK * 2), ring = 8u * g.stages;
+    int it = 0, early = 0;
     if (g.early_b && t0 < tiles) {   // the first tile's weights
       early = min(g.stages, kb1 - kb0);
       const int n0 = (t0 / g.mt) * g.bn;
@@ -316,57 +324,86 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       }
     }
     grid_dep_wait();
-    for (int t = t0; t < tiles; t += dt) {
+    bool there = true, wrapped = false;
+    uint32_t st8 = 0, dst = base, ph = 1;      // 8 x stage, its memory, the parity that the end of its last use has
+    for (int t = t0; t < tiles && there; t += dt) {
       const int n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
       int tap = kb0 / g.kpt, c = kb0 - tap * g.kpt;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        if (it >= g.stages && !gp_wait(empty + 8u * st, ph ^ 1u, dead, g.tries)) gone = true;
-        const uint32_t fb = full + 8u * st, a_dst = base + st * sb;
-        if (leader && !gone) {
-          if (it >= early) {
-            mbar_expect(fb, tx);
-            tma_2d(a_dst + ab, &tmB, tap * o.cin + c * TK, n0, fb);
+      for (int m = kb1 - kb0; m > 0 && there; ++tap, c = 0) {
+        const int run = min(g.kpt - c, m), row = m0 + o.tap_off[tap];
+        int x = c * TK, xb = tap * o.cin + x;
+#pragma unroll 1
+        for (int i = run; i > 0; --i) {
+          if (wrapped && !gp_wait_all(empty + st8, ph, dead, g.tries)) { there = false; break; }
+          if (leader) {
+            if (it >= early) {
+              mbar_expect(full + st8, tx);
+              tma_2d(dst + ab, &tmB, xb, n0, full + st8);
+            }
+            if (it != g.lost) tma_2d(dst, &tmA, x, row, full + st8);
           }
-          if (it != g.lost) tma_2d(a_dst, &tmA, c * TK, m0 + o.tap_off[tap], fb);
-          asked = it + 1;
+          ++it;
+          x += TK; xb += TK; st8 += 8; dst += sb;
+          if (st8 == ring) { st8 = 0; dst = base; ph ^= 1u; wrapped = true; }
         }
-        if (++c == g.kpt) { c = 0; ++tap; }
-        if (++st == g.stages) { st = 0; ph ^= 1u; }
+        m -= run;
       }
     }
-    if (leader) words[2] = (uint32_t)max(asked, early);
-  } else if (warp == GP_MMA_WARP) {
+    if (leader) words[2] = (uint32_t)max(it, early);
+    if (!there) wait_ran_out();
+  } else if (warp == MMA_WARP) {
     grid_dep_wait();
     // instruction descriptor: D = F32, A = B = BF16, both K-major, N = bn, M = 128
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bn >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-    int st = 0, n = 0;
-    bool gone = false;
-    uint32_t ph = 0;
-    for (int t = t0; t < tiles; t += dt, ++n) {
+    const uint64_t d0 = umma_desc_sw128(base);
+    const uint32_t ring = 8u * g.stages, sb16 = (uint32_t)sb >> 4, ab16 = (uint32_t)ab >> 4;
+    uint32_t st8 = 0, off = 0, ph = 0;      // 8 x stage, its memory / 16, parity
+    bool there = true;
+    int n = 0;
+    for (int t = t0; t < tiles && there; t += dt, ++n) {
       const int buf = n & 1;
       const uint32_t d = tmem + (uint32_t)(buf * g.acc_cols);
-      if (n >= 2 && !gp_wait(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead, g.tries)) gone = true;
+      if (n >= 2 && !gp_wait_all(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead, g.tries)) { there = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      int left = g.kpt - kb0 % g.kpt;      // k-blocks to the end of the tap
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!gp_wait(full + 8u * st, ph, dead, g.tries)) gone = true;      // (filled by the copy engine: no tensor-memory fence)
-        const uint64_t da = umma_desc_sw128(base + st * sb), db = umma_desc_sw128(base + st * sb + ab);
-        const int mmas = --left == 0 ? g.tail : TK / 16;
-        if (left == 0) left = g.kpt;
-        if (leader && !gone) {
+      uint32_t acc = 0;
+      for (int m = kb1 - kb0, c = kb0 % g.kpt; m > 0 && there; c = 0) {
+        const int run = min(g.kpt - c, m);
+        const bool tail = c + run == g.kpt && g.tail != TK / 16;      // the tap's last k-block has fewer columns
+#pragma unroll 1
+        for (int i = run - (tail ? 1 : 0); i > 0; --i) {
+          if (!gp_wait_all(full + st8, ph, dead, g.tries)) { there = false; break; }      // (filled by the copy engine: no tensor-memory fence)
+          const uint64_t da = d0 + off, db = da + ab16;
+          if (leader) {
+            umma_bf16(d, da, db, idesc, acc);
 #pragma unroll
-          for (int kk = 0; kk < TK / 16; ++kk)
-            if (kk < mmas) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);      // 16 columns = 32 bytes further
-          umma_commit(empty + 8u * st);
+            for (int kk = 1; kk < TK / 16; ++kk) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, 1u);      // 16 columns = 32 bytes further
+            umma_commit(empty + st8);
+          }
+          __syncwarp();
+          acc = 1; st8 += 8; off += sb16;
+          if (st8 == ring) { st8 = 0; off = 0; ph ^= 1u; }
         }
-        if (++st == g.stages) { st = 0; ph ^= 1u; }
+        if (tail && there) {
+          there = gp_wait_all(full + st8, ph, dead, g.tries);
+          const uint64_t da = d0 + off, db = da + ab16;
+          if (leader && there) {
+            for (int kk = 0; kk < g.tail; ++kk) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, kk ? 1u : acc);
+            umma_commit(empty + st8);
+          }
+          __syncwarp();
+          acc = 1; st8 += 8; off += sb16;
+          if (st8 == ring) { st8 = 0; off = 0; ph ^= 1u; }
+        }
+        m -= run;
       }
-      if (leader && !gone) umma_commit(acc_full + 8u * buf);
+      if (leader && there) umma_commit(acc_full + 8u * buf);
+      __syncwarp();
     }
+    if (!there) wait_ran_out();
   } else {
     grid_dep_wait();
-    // warp w reads tensor-memory lanes 32 (w & 3) .. +31 (= rows of the tile); warps 0-3 take the first half of the 16-column pieces, 4-7 the rest
-    const int pieces = g.bn / 16, half = (pieces + 1) / 2, p0 = (warp >> 2) * half, p1 = min(pieces, p0 + half);
+    // warp w reads tensor-memory lanes 32 (w & 3) .. +31 (= rows of the tile); each four warps take a run of the 16-column pieces
+    const int pieces = g.bn / 16, p0 = (warp >> 2) * pieces / GROUPS, p1 = ((warp >> 2) + 1) * pieces / GROUPS;
     const int r_in = (warp & 3) * 32 + lane;
     const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && !g.staged;
     float* par = reinterpret_cast<float*>(gbase + g.stages * sb + 512);
@@ -376,7 +413,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       const int buf = bufs == 1 ? 0 : n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
       if (params && n0 != par_n0) {      // another column tile (rows go first): its parameters, when the epilogue warps have left the last one's
         par_n0 = n0;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
         const int col = n0 + tid;
         if (tid < g.bn && col < o.N) {
           const int c = col % o.col_mod;
@@ -387,7 +424,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
             par[3 * GP_PAR + tid] = reinterpret_cast<const float*>(o.p1)[c];
           }
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
       }
       const int row = m0 + r_in;
       const bool rows = m0 + (warp & 3) * 32 < o.M;      // (warp-uniform)
@@ -397,7 +434,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
         if (resid && p < p1 && row < o.M && n0 + p * 16 < o.N) ld32(reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16, x);
       };
       if (rows) { ask(p0, rx); ask(p0 + 1, ry); }
-      gp_wait(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead, g.tries);
+      gp_wait_warp(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead, g.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ta = tmem + (uint32_t)(buf * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
       if (rows)
@@ -449,7 +486,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       __syncthreads();
       lost = *dead;
     }
-    for (int i = i0 + tid; i < i1; i += GP_THREADS) {
+    for (int i = i0 + tid; i < i1; i += THREADS) {
       const int r = i / pieces, p = i - r * pieces;
       const uint32_t mine = base + (uint32_t)((r * gp_part_pitch(g.bn) + p * 8) * 4);
       float4 q[8][2];      // every split's part is on its way before the first is added
@@ -474,7 +511,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
       epilogue_row8(o, m0 + r, n0 + p * 8, a);
     }
     if (__syncthreads_or(lost))
-      for (int i = i0 + tid; i < i1; i += GP_THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
+      for (int i = i0 + tid; i < i1; i += THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
     if (g.splits > 1) {      // the others have read this CTA's partial tile (reads only: nothing to publish)
       asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -483,7 +520,7 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (*dead) {      // copies and products still on their way end before the memory they use is given back
-    if (warp == GP_MMA_WARP && leader) {
+    if (warp == MMA_WARP && leader) {
       umma_commit(drain);
       mbar_wait_bounded(drain, 0u, 1 << 14);
     }
@@ -494,9 +531,9 @@ __global__ void __launch_bounds__(GP_THREADS, MINB) fq3c_gemm_persist_kernel(con
     if (!g.staged)
       for (int t = t0; t < tiles; t += dt) {
         const int n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM, pieces = g.bn / 8;
-        for (int i = tid; i < TM * pieces; i += GP_THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
+        for (int i = tid; i < TM * pieces; i += THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);
       }
   }
   __syncthreads();
-  if (warp == GP_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  if (warp == MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }

@@ -1,0 +1,45 @@
+"""The tcgen05 GEMM on both sides of the lines between its launch shapes (few rows, one wide CTA per SM, two CTAs per SM, split sums)."""
+import pytest
+import torch
+
+from test_gemm_gpu import SEVEN, launch, make_op, product
+
+pytestmark = pytest.mark.gpu
+
+# rows, columns, inputs per tap, taps, split allowed
+CASES = [(64, 512, 256, (0,), False), (65, 512, 256, (0,), False),                       # eight and sixteen epilogue warps
+         (20000, 96, 96, (0,), False), (9600, 192, 256, (0,), False), (9600, 192, 320, (0,), False), (20000, 96, 40, (-1, 0), False),      # two CTAs per SM: up to four k-blocks
+         (700, 208, 192, (0,), False), (1900, 176, 64, (0,), False), (2500, 256, 128, (0,), False),      # column pieces that four groups of warps share unevenly
+         (64, 1024, 1536, (0,), True), (64, 1024, 2048, (0,), True), (100, 1024, 3072, (0,), True), (130, 1024, 3072, (0,), True), (40, 2048, 1024, (0,), True),
+         (17, 48, 2048, (0,), True), (200, 512, 512, SEVEN, True)]
+
+
+@pytest.mark.parametrize("M,N,cin,offs,split", CASES)
+def test_product_residual_snake_and_units(M, N, cin, offs, split):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + N)
+    A = torch.randn(M, cin, device="cuda", generator=g).bfloat16()
+    B = (torch.randn(N, len(offs) * cin, device="cuda", generator=g) / (len(offs) * cin) ** 0.5).bfloat16()
+    ws = torch.zeros(8 * M * (N + 8), device="cuda") if split else None
+    want, mag = product(A, B, M, cin, offs)
+    sums = len(offs) * cin * 2.0 ** -24 * mag      # f32 sums in any order
+    out = torch.full((M + 1, N), 7.0, device="cuda")
+    launch([make_op(A, B, out, M, N, cin, offs, K.F_OUT_F32 | K.F_NOROUND, ws=ws)])
+    assert ((out[:M].double() - want).abs() <= sums).all() and (out[M] == 7).all()
+    # residual and SnakeBeta: the sum is rounded, its sum with the residual is rounded, and the second output is that value's own, rounded
+    res, freq, inv = torch.randn(M, N, device="cuda", generator=g).bfloat16(), torch.rand(N, device="cuda", generator=g) + 0.5, torch.rand(N, device="cuda", generator=g)
+    out, out2 = (torch.zeros(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    o = make_op(A, B, out, M, N, cin, offs, K.F_SNAKE2, res=res, ws=ws)
+    o.p0, o.p1, o.C2 = freq.data_ptr(), inv.data_ptr(), out2.data_ptr()
+    launch([o])
+    exact = want + res.double()
+    assert ((out.double() - exact).abs() <= 1.01 * 2.0 ** -8 * (want.abs() + exact.abs()) + 2 * sums).all()
+    snake = out.double() + inv.double() * torch.sin(out.double() * freq.double()) ** 2
+    assert ((out2.double() - snake).abs() <= 1.01 * 2.0 ** -8 * snake.abs() + 2.0 ** -20).all()
+    out = torch.zeros(M, N // 2, device="cuda", dtype=torch.bfloat16)
+    launch([make_op(A, B, out, M, N, cin, offs, K.F_SWIGLU | K.F_NOROUND, ws=ws)])
+    gate, up = want[:, 0::2], want[:, 1::2]
+    unit = gate * torch.sigmoid(gate) * up
+    slack = 1.1 * sums[:, 0::2] * up.abs() + (gate * torch.sigmoid(gate)).abs() * sums[:, 1::2]      # silu's slope is at most 1.1
+    assert ((out.double() - unit).abs() <= 1.01 * 2.0 ** -8 * unit.abs() + slack + 2.0 ** -20 * unit.abs() + 1e-6).all()
