@@ -13,10 +13,15 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "../../include/fq3_codec.h"
 
 typedef __nv_bfloat16 bf16;
+
+extern "C" {
+static bool device_attrs_ready();      // shared-memory limits of the kernels, once per device
+}
 
 namespace {
 
@@ -974,6 +979,173 @@ __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
   }
 }
 
+// Attention of a few rows or of a short window, FQ3C_ATTN with heads of D entries: a CTA takes RB query rows of one key / value head, stages the keys and values that they
+// see in shared memory once, and then
+//   scores: a warp per (row, head, 32 keys), a lane per key - q is a broadcast, keys lie 16 bytes apart in banks, no shuffles;
+//   sums:   a warp per (row, head), the exponentials once per key, then a lane per D / 32 entries walks the keys in order.
+// A row's sums do not depend on the rows beside it, so a window of a stream gives the bits of the whole decode.  Rounding points of fq3c_attn_kernel: score -> bf16 ->
+// x scale -> bf16, softmax and sums f32, output bf16.
+// What bounds it is latency: one round trip to L2, a few thousand cycles of dependent work and a launch; the kernels with a warp per (row, head) make
+// a round trip for every four to sixteen keys.
+// PROMPT: `n` is the FQ3C_QKNORM_ROPE_KV op in front.  Every CTA norms and turns the keys it stages (again for each RB rows: 60 instructions a key), its queries, and
+// writes its own rows of the cache: one launch in place of two, and the rows in `A` stay as the product left them.  39 rows of
+// 16 heads 8.1 -> 5.7 us; the codec's attention (16 heads of 64, window 72) 33 rows 7.6 -> 3.8, 256 rows 31.8 -> 16.1, one row
+// 1.7 -> 2.5 (kept there too: a stream's rows and the whole decode's have the same sums).
+constexpr int GP_SMS = 148;
+constexpr int AR_PROMPT_ROWS = 144, AR_WARPS = 16, AR_SMEM_MAX = 128 * 1024;
+struct AttnRows { int rb, span, sp; size_t smem; };      // rows of a CTA, keys it may stage, pitch of its scores
+__host__ __device__ constexpr int ar_k_pitch(int d) { return d * 2 + 16; }      // bytes
+AttnRows attn_rows_plan(const fq3c_op& o) {
+  AttnRows r;
+  const int hg = o.i0 / o.i1;
+  r.rb = 1;      // as few rows as one CTA per SM allows: 100 rows of 16 heads with 160 CTAs 16.5 us
+  while (r.rb < 16 && (long)((o.M + r.rb - 1) / r.rb) * o.i1 > GP_SMS) ++r.rb;
+  r.span = (int)std::min<long>((long)o.K + r.rb - 1, (long)o.M + o.taps);
+  r.sp = (r.span + 31) / 32 * 32;
+  r.smem = (size_t)r.span * (ar_k_pitch(o.i2) + o.i2 * 2) + (size_t)r.rb * hg * (o.i2 + r.sp) * 4;
+  return r;
+}
+// a head's row of 128, four entries a lane: RMSNorm and rotation with the rounding points of fq3c_qknorm_rope_kv_kernel
+__device__ __forceinline__ uint2 norm_turn(const uint2 raw, const float eps, const uint2 gamma, const uint2 cosr, const uint2 sinr, const int lane) {
+  float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)};
+  const float ga[4] = {__uint_as_float(gamma.x << 16), __uint_as_float(gamma.x & 0xffff0000u), __uint_as_float(gamma.y << 16), __uint_as_float(gamma.y & 0xffff0000u)};
+  const float co[4] = {__uint_as_float(cosr.x << 16), __uint_as_float(cosr.x & 0xffff0000u), __uint_as_float(cosr.y << 16), __uint_as_float(cosr.y & 0xffff0000u)};
+  const float si[4] = {__uint_as_float(sinr.x << 16), __uint_as_float(sinr.x & 0xffff0000u), __uint_as_float(sinr.y << 16), __uint_as_float(sinr.y & 0xffff0000u)};
+  float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  const float rs = rsqrtf(ss * (1.f / 128.f) + eps);
+  float y[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) y[i] = bf16r(bf16r(x[i] * rs) * ga[i]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float partner = __shfl_xor_sync(0xffffffffu, y[i], 16);
+    x[i] = bf16r(y[i] * co[i]) + bf16r((lane < 16 ? -partner : partner) * si[i]);
+  }
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+template <int D, bool PROMPT>
+__global__ void __launch_bounds__(AR_WARPS * 32) fq3c_attn_rows_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op n, const int RB, const int span_max, const int SP) {
+  extern __shared__ __align__(16) unsigned char ar_raw[];
+  constexpr int PER = D / 32, KP = ar_k_pitch(D);      // entries of a lane; bytes of a staged key
+  typedef typename std::conditional<PER == 4, uint2, uint32_t>::type Vec;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nh = o.i0, G = o.i1, HG = nh / G, g = blockIdx.y, win = o.K, hist = PROMPT ? 0 : o.taps;
+  const int r0 = blockIdx.x * RB, rows = min(RB, o.M - r0);
+  grid_dep_begin();
+  uint2 gk = make_uint2(0u, 0u), gq = make_uint2(0u, 0u);
+  if (PROMPT) {
+    gk = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(n.p1) + lane * 4);
+    gq = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(n.p0) + lane * 4);
+  }
+  const int first = (!PROMPT && o.p0) ? hist - min(*reinterpret_cast<const int*>(o.p0), hist) : 0;
+  const int j_lo = max(first, r0 + hist - win + 1), span = r0 + rows + hist - j_lo, items = span + rows * HG;
+  unsigned char* ks = ar_raw;                                              // [span][KP]
+  unsigned char* vs = ks + (size_t)span_max * KP;                          // [span][2 D]
+  float* qs = reinterpret_cast<float*>(vs + (size_t)span_max * 2 * D);     // [RB HG][D]
+  float* sc = qs + RB * HG * D;                                            // [RB HG][SP]
+  const bf16* base = reinterpret_cast<const bf16*>(o.A) + lane * PER;
+  const size_t lda = (size_t)o.lda;
+  const bf16* cosp = reinterpret_cast<const bf16*>(n.B) + lane * 4;
+  const bf16* sinp = reinterpret_cast<const bf16*>(n.bias) + lane * 4;
+  // the keys with their values, then the queries: U of a warp's items on their way together
+  constexpr int U = 4;
+  for (int ib = warp; ib < items; ib += AR_WARPS * U) {
+    Vec x[U], v[U];
+    uint2 c[U], si[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = min(ib + u * AR_WARPS, items - 1), qi = i - span;
+      const int row = qi < 0 ? j_lo + i : r0 + hist + qi / HG, head = qi < 0 ? nh + g : g * HG + qi % HG;
+      x[u] = *reinterpret_cast<const Vec*>(base + row * lda + head * D);
+      if (qi < 0) v[u] = *reinterpret_cast<const Vec*>(base + row * lda + (head + G) * D);
+      if constexpr (PROMPT) {
+        c[u] = *reinterpret_cast<const uint2*>(cosp + (size_t)(n.i2 + row) * 128);
+        si[u] = *reinterpret_cast<const uint2*>(sinp + (size_t)(n.i2 + row) * 128);
+      }
+    }
+    if constexpr (PROMPT) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = norm_turn(x[u], n.f0, ib + u * AR_WARPS < span ? gk : gq, c[u], si[u], lane);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = ib + u * AR_WARPS, qi = i - span;
+      if (qi < 0) {
+        *reinterpret_cast<Vec*>(ks + (size_t)i * KP + lane * PER * 2) = x[u];
+        *reinterpret_cast<Vec*>(vs + (size_t)i * 2 * D + lane * PER * 2) = v[u];
+        if constexpr (PROMPT) {
+          if (j_lo + i >= r0) {
+            const size_t at = ((size_t)g * n.ldc + n.i2 + j_lo + i) * 128 + lane * 4;
+            *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(n.C) + at) = x[u];
+            *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(n.C2) + at) = v[u];
+          }
+        }
+      } else if (i < items) {
+        float* q = qs + qi * D + lane * PER;
+        if constexpr (PER == 4) *reinterpret_cast<float4*>(q) = make_float4(__uint_as_float(x[u].x << 16), __uint_as_float(x[u].x & 0xffff0000u), __uint_as_float(x[u].y << 16), __uint_as_float(x[u].y & 0xffff0000u));
+        else *reinterpret_cast<float2*>(q) = make_float2(__uint_as_float(x[u] << 16), __uint_as_float(x[u] & 0xffff0000u));
+      }
+    }
+  }
+  __syncthreads();
+  const float scale = rsqrtf((float)D);
+  const int chunks = (span + 31) >> 5;
+  for (int it = warp; it < rows * HG * chunks; it += AR_WARPS) {
+    const int i = it / chunks, ch = it - i * chunks, j = ch * 32 + lane, t = r0 + i / HG + hist - j_lo;      // the row's own key
+    if (ch * 32 > t || ch * 32 + 31 <= t - win) continue;
+    const uint4* kp = reinterpret_cast<const uint4*>(ks + (size_t)min(j, span - 1) * KP);
+    const float4* qa = reinterpret_cast<const float4*>(qs + i * D);
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < D / 8; ++c) {
+      const uint4 k = kp[c];
+      const float4 x = qa[2 * c], y = qa[2 * c + 1];
+      a[0] = fmaf(x.x, __uint_as_float(k.x << 16), a[0]); a[1] = fmaf(x.y, __uint_as_float(k.x & 0xffff0000u), a[1]);
+      a[2] = fmaf(x.z, __uint_as_float(k.y << 16), a[2]); a[3] = fmaf(x.w, __uint_as_float(k.y & 0xffff0000u), a[3]);
+      a[0] = fmaf(y.x, __uint_as_float(k.z << 16), a[0]); a[1] = fmaf(y.y, __uint_as_float(k.z & 0xffff0000u), a[1]);
+      a[2] = fmaf(y.z, __uint_as_float(k.w << 16), a[2]); a[3] = fmaf(y.w, __uint_as_float(k.w & 0xffff0000u), a[3]);
+    }
+    sc[i * SP + j] = bf16r(bf16r((a[0] + a[1]) + (a[2] + a[3])) * scale);
+  }
+  __syncthreads();
+  for (int i = warp; i < rows * HG; i += AR_WARPS) {
+    const int row = i / HG, h = g * HG + i - row * HG, je = r0 + row + hist - j_lo, jb = max(0, je - win + 1);
+    float* s = sc + (size_t)i * SP;
+    float mx = -INFINITY;
+    for (int j = jb + lane; j <= je; j += 32) mx = fmaxf(mx, s[j]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    for (int j = jb + lane; j <= je; j += 32) s[j] = expf(s[j] - mx);
+    __syncwarp();
+    float l = 0.f, acc[PER];
+#pragma unroll
+    for (int e = 0; e < PER; ++e) acc[e] = 0.f;
+    const unsigned char* vp = vs + lane * PER * 2;
+#pragma unroll 8
+    for (int j = jb; j <= je; ++j) {
+      const float p = s[j];
+      const Vec v = *reinterpret_cast<const Vec*>(vp + (size_t)j * 2 * D);
+      l += p;
+      if constexpr (PER == 4) {
+        acc[0] = fmaf(p, __uint_as_float(v.x << 16), acc[0]); acc[1] = fmaf(p, __uint_as_float(v.x & 0xffff0000u), acc[1]);
+        acc[2] = fmaf(p, __uint_as_float(v.y << 16), acc[2]); acc[3] = fmaf(p, __uint_as_float(v.y & 0xffff0000u), acc[3]);
+      } else {
+        acc[0] = fmaf(p, __uint_as_float(v << 16), acc[0]); acc[1] = fmaf(p, __uint_as_float(v & 0xffff0000u), acc[1]);
+      }
+    }
+    bf16* out = reinterpret_cast<bf16*>(o.C) + (size_t)(r0 + row) * o.ldc + h * D + lane * PER;
+    if constexpr (PER == 4) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0] / l, acc[1] / l), hi = __floats2bfloat162_rn(acc[2] / l, acc[3] / l);
+      *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    } else {
+      *reinterpret_cast<__nv_bfloat162*>(out) = __floats2bfloat162_rn(acc[0] / l, acc[1] / l);
+    }
+  }
+}
+
 __global__ void fq3c_dwconv_kernel(const fq3c_op o) {
   grid_dep_begin();
   const size_t n = (size_t)o.M * o.N;
@@ -1129,7 +1301,6 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 }
 
 // ---- the tcgen05 GEMM: what a launch looks like ------------------------------------------------------------------------------
-constexpr int GP_SMS = 148;
 constexpr int GP_SMEM_MAX = 227 * 1024, GP_SMEM_HALF = 112 * 1024;
 // Whether the epilogue may move whole 32-byte sectors (16 columns of bf16, 8 of f32).
 bool gemm_vec16(const fq3c_op& o) {
@@ -1245,6 +1416,23 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
   else if (mode == AT_PLAIN) launch_after(fq3c_attn_tc_kernel<AT_PLAIN>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
   else if (mode == AT_CAP) launch_after(fq3c_attn_tc_kernel<AT_CAP>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
   else launch_after(fq3c_attn_tc_kernel<AT_DIST>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+}
+
+// ---- attention of few rows or a short window -----------------------------------------------------------------------------------
+// What fq3c_attn_rows_kernel's vector accesses and shared memory ask for; grid.y is the head.
+bool attn_rows_takes(const fq3c_op& o) {
+  auto off = [](const void* p, int a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
+  const int vec = o.i2 / 32;      // entries a lane moves at a time
+  return (o.i2 == 64 || o.i2 == 128) && o.i1 > 0 && o.i0 > 0 && o.i0 % o.i1 == 0 && o.i1 <= 65535 && o.K > 0 && o.taps >= 0 && o.lda % vec == 0 && o.ldc % vec == 0 &&
+         !off(o.A, 2 * vec) && !off(o.C, 2 * vec) && attn_rows_plan(o).smem <= AR_SMEM_MAX && device_attrs_ready();
+}
+// `n` (q / k norm, rotation, cache rows) and the prompt attention `o` behind it, where the rows that `n` would rewrite are scratch to everyone else (reserved bit 0)
+// Against two launches (behind these lines the second is the kernel on tcgen05): 39 rows of 16 heads 5.7 and 8.1 us, 100 11.6 and 13.1, 112 14.3 and 13.3; 64 of 32 11.0
+// and 14.8, 80 15.2 and 13.5; 144 of 8 14.2 and 14.5, of 4 11.7 and 12.9.
+bool attn_rows_takes_prompt(const fq3c_op& n, const fq3c_op& o) {
+  auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) != 0; };
+  return (n.reserved & 1) && o.kind == FQ3C_ATTN && (o.flags & 1) && o.A == n.A && o.lda == n.lda && o.M == n.M && o.i0 == n.i0 && o.i1 == n.i1 && o.i2 == 128 && o.taps == 0 && !o.p0 &&
+         o.M <= AR_PROMPT_ROWS && (long)o.M * o.M * o.i0 <= 165000 && !off(n.p0) && !off(n.p1) && !off(n.B) && !off(n.bias) && !off(n.C) && !off(n.C2) && attn_rows_takes(o);
 }
 
 // ---- sequence-model ops: launch logic ---------------------------------------------------------------------------------------
@@ -1900,6 +2088,9 @@ static bool device_attrs_ready() {
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_HALF) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_attn_rows_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_attn_rows_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3c_attn_rows_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, APF_WARPS * (128 + 2048) * 4) != cudaSuccess)
     return false;
   done[dev] = true;
@@ -2122,6 +2313,13 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           launch_after(fq3c_attn_prefill_kernel, (warps + APF_WARPS - 1) / APF_WARPS, APF_WARPS * 32, smem, s, after, 1, o, tpad);
           break;
         }
+        if (attn_rows_takes(o)) {
+          const AttnRows r = attn_rows_plan(o);
+          const dim3 grid((unsigned)((o.M + r.rb - 1) / r.rb), (unsigned)o.i1);
+          if (o.i2 == 64) launch_after(fq3c_attn_rows_kernel<64, false>, grid, AR_WARPS * 32, r.smem, s, after, 1, o, o, r.rb, r.span, r.sp);
+          else launch_after(fq3c_attn_rows_kernel<128, false>, grid, AR_WARPS * 32, r.smem, s, after, 1, o, o, r.rb, r.span, r.sp);
+          break;
+        }
         const int warps = o.M * o.i0;
         launch_after(fq3c_attn_kernel, (warps + 7) / 8, 256, 0, s, after, 1, o);
         break;
@@ -2133,6 +2331,12 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
       }
       case FQ3C_QKNORM_ROPE_KV: {
         if (o.lda % 4 || !o.C || !o.C2 || !o.p0 || !o.p1 || !o.B || !o.bias) return fail("qknorm_rope_kv: missing operand");
+        if (i + 1 < n_ops && attn_rows_takes_prompt(o, ops[i + 1])) {      // with the attention behind it in one launch
+          const fq3c_op& at = ops[++i];
+          const AttnRows r = attn_rows_plan(at);
+          launch_after(fq3c_attn_rows_kernel<128, true>, dim3((unsigned)((at.M + r.rb - 1) / r.rb), (unsigned)at.i1), AR_WARPS * 32, r.smem, s, after, 1, at, o, r.rb, r.span, r.sp);
+          break;
+        }
         const int warps = o.M * (o.i0 + 2 * o.i1);
         launch_after(fq3c_qknorm_rope_kv_kernel, (warps + 7) / 8, 256, 0, s, after, 1, o);
         break;

@@ -98,6 +98,7 @@ class DensePrefill:
             gemm(h, self.off(f"{p}.wqkv"), Q, H, qkv)
             o = Op()
             o.kind, o.M, o.N = K_QKNORM_ROPE_KV, cap, Q
+            o.reserved = 1      # the rows of qkv are read by the attention behind it alone
             o.A, o.lda, o.a_rows = qkv.data_ptr(), Q, cap
             o.i0, o.i1, o.i2, o.f0 = nq, nkv, 0, t.rms_norm_eps
             o.p0, o.p1 = self.off(f"{p}.qn"), self.off(f"{p}.kn")
