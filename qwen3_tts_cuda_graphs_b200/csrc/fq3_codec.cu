@@ -1619,11 +1619,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
     }
     case FQ3C_MOE_SORT: {
       if (o.i1 < 1 || !o.A || !o.C || !o.C2 || !o.ws) return fail("moe_sort: missing operand");
-      int nth = (int)std::min<long>(1024, ((48 * 1024) / 4 - o.i1 - 1) / o.i1);
-      if (nth < 1) return fail("moe_sort: too many experts");
-      if (nth >= 32) nth &= ~31;
-      nth = std::min(nth, std::max(32, ((o.M * o.i0 + 31) / 32) * 32));
-      fq3s_moe_sort_kernel<<<1, nth, (size_t)(o.i1 + 1 + (size_t)nth * o.i1) * 4, s>>>(o);
+      const int warps = std::min(std::min(32, ((48 * 1024) / 4 - o.i1 - 1) / o.i1), std::max(1, (o.M * o.i0 + 31) / 32));
+      if (warps < 1) return fail("moe_sort: too many experts");
+      fq3s_moe_sort_kernel<<<1, warps * 32, (size_t)(o.i1 + 1 + warps * o.i1) * 4, s>>>(o);
       return 0;
     }
     case FQ3C_MOE_COMBINE:

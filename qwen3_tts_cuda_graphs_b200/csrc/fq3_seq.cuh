@@ -1087,45 +1087,63 @@ __global__ void fq3s_router_kernel(const fq3c_op o) {
     if (i < n && lid[i] >= E) pos[i] = -1;
 }
 
-// One block.  Counting sort of the (token, choice) pairs by expert, token order kept inside an expert.
+// One block.  Counting sort of the (token, choice) pairs by expert, token order kept inside an expert.  A warp takes a run of the pairs, 32 at a time: lanes with the
+// same expert find each other with one match, so that only a count per (warp, expert) is walked serially - with one per (thread, expert) that walk over 1024 shares was
+// all the time there is.  1402 pairs of 16 experts 12.5 -> 4.6 us, 8192 of 32 25.6 -> 16.7; what is left are two passes over the pairs and four block barriers.
 __global__ void __launch_bounds__(1024) fq3s_moe_sort_kernel(const fq3c_op o) {
-  extern __shared__ int ssm[];   // [E + 1] starts, then [nchunk][E] counts
-  const int E = o.i1, n = o.M * o.i0, nth = blockDim.x;
+  extern __shared__ int ssm[];   // [E + 1] starts, then [warps][E] counts
+  const int E = o.i1, n = o.M * o.i0, nth = blockDim.x, warps = nth >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* ids = reinterpret_cast<const int*>(o.A);
   int* seg = reinterpret_cast<int*>(o.C);
   int* rows = reinterpret_cast<int*>(o.C2);
   int* pos = reinterpret_cast<int*>(o.ws);
   int* start = ssm;
-  int* cnt = ssm + E + 1;        // cnt[t * E + e]: entries of expert e in thread t's contiguous share
-  const int per = (n + nth - 1) / nth;
-  const int i0 = threadIdx.x * per, i1 = min(n, i0 + per);
-  for (int e = 0; e < E; ++e) cnt[threadIdx.x * E + e] = 0;
-  for (int i = i0; i < i1; ++i) { const int e = ids[i]; if (e < E) cnt[threadIdx.x * E + e] += 1; }
+  int* cnt = ssm + E + 1;        // cnt[w * E + e]: entries of expert e in warp w's share, then in front of it
+  const int per = ((n + warps - 1) / warps + 31) / 32 * 32;
+  const int i0 = warp * per, i1 = min(n, i0 + per);
+  for (int i = threadIdx.x; i < warps * E; i += nth) cnt[i] = 0;
   __syncthreads();
-  // per expert: exclusive scan over the threads' shares (thread e walks column e)
+  for (int b = i0; b < i1; b += 32) {
+    const int e = b + lane < i1 ? min(ids[b + lane], E) : E;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    if (e < E && lane == __ffs(same) - 1) cnt[warp * E + e] += __popc(same);
+    __syncwarp();
+  }
+  __syncthreads();
   for (int e = threadIdx.x; e < E; e += nth) {
     int run = 0;
-    for (int t = 0; t < nth; ++t) { const int v = cnt[t * E + e]; cnt[t * E + e] = run; run += v; }
+    for (int w = 0; w < warps; ++w) { const int v = cnt[w * E + e]; cnt[w * E + e] = run; run += v; }
     start[e + 1] = run;   // total, turned into starts below
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == 0) {
     int run = 0;
-    start[0] = 0;
-    for (int e = 0; e < E; ++e) { const int v = start[e + 1]; start[e] = run; run += v; }
-    start[E] = run;
+    for (int b = 0; b < E; b += 32) {
+      int sum = b + lane < E ? start[b + lane + 1] : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += u;
+      }
+      if (b + lane < E) start[b + lane + 1] = run + sum;
+      run += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) start[0] = 0;
   }
   __syncthreads();
   for (int e = threadIdx.x; e <= E; e += nth) seg[e] = start[e];
-  for (int i = i0; i < i1; ++i) {
-    const int e = ids[i];
+  for (int b = i0; b < i1; b += 32) {
+    const int i = b + lane, e = i < i1 ? min(ids[i], E) : E;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    int p = -1;
     if (e < E) {
-      const int p = start[e] + cnt[threadIdx.x * E + e]++;
+      p = start[e] + cnt[warp * E + e] + __popc(same & ((1u << lane) - 1u));
       rows[p] = i / o.i0;
-      pos[i] = p;
-    } else {
-      pos[i] = -1;
     }
+    if (i < i1) pos[i] = p;
+    __syncwarp();
+    if (e < E && lane == __ffs(same) - 1) cnt[warp * E + e] += __popc(same);
+    __syncwarp();
   }
 }
 
