@@ -622,6 +622,18 @@ class StepBuilder:
         width = x32.shape[1]
         zc = w["router"].shape[0]        # n, or n + 1 with the shared expert's gate row
         assert zc == n + (1 if c.shared_gate else 0)
+        sh = None
+        if w.get("shared_up") is not None:      # beside the router, the sort and the experts: 701 rows 103 -> 93 us
+            self.branch(0)
+        if w.get("shared_up") is not None and c.gated:
+            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0] // 2, self.adt), glu=True)
+            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
+        elif w.get("shared_up") is not None:
+            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0], self.adt), gelu=c.act != "relu2",
+                             relu2=c.act == "relu2")
+            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
+        if sh is not None:
+            self.branch(1)
         z = self.linear(x32 if w["router"].dtype == torch.float32 else xop, w["router"], self.buf("moe.z", M, zc),
                         bias=w.get("router_b") if c.router_bias else None)
         ids = self.buf("moe.ids", M, top, torch.int32)
@@ -652,14 +664,8 @@ class StepBuilder:
         y = self.buf("moe.y", M * top, width)
         self._op(K_GGEMM, M=M * top, N=width, K=ff, i0=E, A=act, lda=ff, B=w["down"], p0=seg, C=y, ldc=width,
                  flags=F_OUT_F32 | (F_F32 if f32 else 0))
-        sh = None
-        if w.get("shared_up") is not None and c.gated:
-            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0] // 2, self.adt), glu=True)
-            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
-        elif w.get("shared_up") is not None:
-            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0], self.adt), gelu=c.act != "relu2",
-                             relu2=c.act == "relu2")
-            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
+        if sh is not None:
+            self.branch(2)
         kw = dict(M=M, N=width, i0=top, i1=E, A=y, lda=width, B=x32, ldr=width, p0=ids, ws=pos, C=out, ldc=out.shape[1])
         if not c.weight_input:
             kw["p1"] = wt
