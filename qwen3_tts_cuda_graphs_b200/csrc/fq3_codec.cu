@@ -624,6 +624,66 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return t;
 }
 
+// RMSNorm of a row by a warp, eight entries a lane and load: the reciprocal root of the mean square, and eight normed entries.
+__device__ __forceinline__ float sq8(const uint4 x, float ss) {
+  const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float a = __uint_as_float(u[q] << 16), b = __uint_as_float(u[q] & 0xffff0000u);
+    ss = fmaf(a, a, ss);
+    ss = fmaf(b, b, ss);
+  }
+  return ss;
+}
+__device__ __forceinline__ float rms_of(float ss, const int N, const float eps) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  return rsqrtf(ss / N + eps);
+}
+__device__ __forceinline__ uint4 norm8(const uint4 x, const float rs, const float* w) {
+  const float4 a = *reinterpret_cast<const float4*>(w), b = *(reinterpret_cast<const float4*>(w) + 1);
+  const float wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+  uint32_t r[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(bf16r(__uint_as_float(u[q] << 16) * rs) * wv[2 * q], bf16r(__uint_as_float(u[q] & 0xffff0000u) * rs) * wv[2 * q + 1]);
+    r[q] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+// rows of whole 16-byte pieces
+bool norm_vec_ok(const void* x, const void* y, const void* w, const int N, const int ldx, const int ldy) {
+  return ((N | ldx | ldy) & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+// FQ3C_RMSNORM and the norm behind a product (fq3c_op.norm_out), the same bits either way.  Bound by latency for few rows (a launch, a trip to L2), by its bytes for
+// many.  A block per row with two-byte loads and two block-wide sums took 2.6 us for 39 rows of 1024 and 5.5 for 1900; so 2.2 and 3.5.  (Normed by the product behind
+// it instead, in each of its CTAs: a layer of a 39-row prompt 38.7 -> 43.3 us.)
+constexpr int RN_WARPS = 4;
+__global__ void __launch_bounds__(RN_WARPS * 32) fq3c_rownorm_vec_kernel(const bf16* x, const int ldx, bf16* y, const int ldy, const float* w, const float eps, const int row0, const int rows,
+                                                                         const int N) {
+  grid_dep_begin();
+  const int row = blockIdx.x * RN_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(row0 + row) * ldx);
+  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)(row0 + row) * ldy);
+  constexpr int C = 4;      // pieces of a lane kept from the sum to the norm; longer rows are read again
+  uint4 v[C];
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (lane + 32 * c < N / 8) v[c] = xr[lane + 32 * c];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (lane + 32 * c < N / 8) ss = sq8(v[c], ss);
+  for (int p = lane + 32 * C; p < N / 8; p += 32) ss = sq8(xr[p], ss);
+  const float rs = rms_of(ss, N, eps);
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (lane + 32 * c < N / 8) yr[lane + 32 * c] = norm8(v[c], rs, w + 8 * (lane + 32 * c));
+  for (int p = lane + 32 * C; p < N / 8; p += 32) yr[p] = norm8(xr[p], rs, w + 8 * p);
+}
+// rows without whole pieces
 __global__ void fq3c_rmsnorm_kernel(const fq3c_op o) {
   grid_dep_begin();
   __shared__ float red[32];
@@ -638,7 +698,7 @@ __global__ void fq3c_rmsnorm_kernel(const fq3c_op o) {
     y[c] = __float2bfloat16_rn(bf16r(bf16r(__bfloat162float(x[c]) * rs) * w[c]));
 }
 
-// RMSNorm of the rows a GEMM just finished (fq3c_op.norm_out), with the arithmetic of fq3c_rmsnorm_kernel: same column-strided
+// RMSNorm of the rows a GEMM just finished in rows without whole pieces, with the arithmetic of fq3c_rmsnorm_kernel: same column-strided
 // partial sums, same block tree, same rounding points — the fused form changes the launch count, not a bit of the result.
 __device__ __forceinline__ void row_rmsnorm(const fq3c_op& o, int row, float* red) {
   const bf16* x = reinterpret_cast<const bf16*>(o.C) + (size_t)row * o.ldc;
@@ -1298,6 +1358,15 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
   if (cluster > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; ++n; }
   cfg.attrs = at; cfg.numAttrs = n;
   cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// the norm of a finished product's rows
+void launch_rownorm(const fq3c_op& o, cudaStream_t s, const bool after) {
+  const int rows = o.M - o.m_begin;
+  if (norm_vec_ok(o.C, o.norm_out, o.norm_w, o.N, o.ldc, o.norm_ld))
+    launch_after(fq3c_rownorm_vec_kernel, (unsigned)((rows + RN_WARPS - 1) / RN_WARPS), RN_WARPS * 32, 0, s, after, 1, reinterpret_cast<const bf16*>(o.C), o.ldc,
+                 reinterpret_cast<bf16*>(o.norm_out), o.norm_ld, reinterpret_cast<const float*>(o.norm_w), o.norm_eps, o.m_begin, rows, o.N);
+  else launch_after(fq3c_rownorm_kernel, (unsigned)rows, 256, 0, s, after, 1, o);
 }
 
 // ---- the tcgen05 GEMM: what a launch looks like ------------------------------------------------------------------------------
@@ -2195,7 +2264,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
             else if (L.shape == GS_FEW) launch_after(fq3c_gemm_persist_kernel<1, 8>, L.grid, gp_threads(8), L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
             else launch_after(fq3c_gemm_persist_kernel<1, 16>, L.grid, gp_threads(16), L.smem, s, after, L.g.splits, w, L.g, tmA, tmB);
             if (o.norm_out) {
-              launch_after(fq3c_rownorm_kernel, (unsigned)(o.M - o.m_begin), 256, 0, s, true, 1, o);
+              launch_rownorm(o, s, true);
               count_launches(1);
             }
             break;
@@ -2251,7 +2320,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
             }
             count_launches(1);
           } else if (o.norm_out) {
-            fq3c_rownorm_kernel<<<(unsigned)(o.M - o.m_begin), 256, 0, s>>>(o);
+            launch_rownorm(o, s, false);
             count_launches(1);
           }
           break;
@@ -2275,13 +2344,18 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         dim3 grid((o.N + BN - 1) / BN, (o.M - o.m_begin + BM - 1) / BM);
         fq3c_gemm_kernel<<<grid, 128, 0, s>>>(o);
         if (o.norm_out) {
-          fq3c_rownorm_kernel<<<(unsigned)(o.M - o.m_begin), 256, 0, s>>>(o);
+          launch_rownorm(o, s, false);
           count_launches(1);
         }
         break;
       }
       case FQ3C_RVQ: launch_after(fq3c_rvq_kernel, o.M, 128, 0, s, after, 1, o); break;
-      case FQ3C_RMSNORM: launch_after(fq3c_rmsnorm_kernel, o.M, 256, 0, s, after, 1, o); break;
+      case FQ3C_RMSNORM:
+        if (norm_vec_ok(o.A, o.C, o.scale, o.N, o.lda, o.ldc))
+          launch_after(fq3c_rownorm_vec_kernel, (unsigned)((o.M + RN_WARPS - 1) / RN_WARPS), RN_WARPS * 32, 0, s, after, 1, reinterpret_cast<const bf16*>(o.A), o.lda,
+                       reinterpret_cast<bf16*>(o.C), o.ldc, reinterpret_cast<const float*>(o.scale), o.f0, 0, o.M, o.N);
+        else launch_after(fq3c_rmsnorm_kernel, o.M, 256, 0, s, after, 1, o);
+        break;
       case FQ3C_LAYERNORM: launch_after(fq3c_layernorm_kernel, o.M, 256, 0, s, after, 1, o); break;
       case FQ3C_ROPE: launch_after(fq3c_rope_kernel, o.M, 256, 0, s, after, 1, o); break;
       case FQ3C_ATTN: {
