@@ -1508,14 +1508,16 @@ bool attn_rows_takes_prompt(const fq3c_op& n, const fq3c_op& o) {
 constexpr int SEQ_GEMM_FLAGS = FQ3C_BIAS | FQ3C_GELU | FQ3C_GELU_TANH | FQ3C_SIGMOID | FQ3C_OUT_F32 | FQ3C_F32 | FQ3C_NOROUND | FQ3C_A_F32 | FQ3C_SWIGLU | FQ3C_RELU2;
 
 // a_f32 / b_f32: operand types.  exact: keep f32 A values as they are (CUDA cores) instead of rounding them onto the tensor cores.
-int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zcount, int row_tiles, cudaStream_t s) {
+// tail: ops that go on with the product's entries, where it takes the few-row kernel (gemv_tail).
+bool takes_gemv(const SeqGemm& g) { return !g.seg && g.M <= 8 && (size_t)g.M * g.K * sizeof(float) <= 96 * 1024; }
+int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zcount, int row_tiles, cudaStream_t s, const SeqTail* tail = nullptr) {
   if (g.flags & ~SEQ_GEMM_FLAGS) return fail("sequence product: unsupported epilogue flag");
   if (b_f32 && !a_f32) return fail("sequence product: f32 weights need f32 rows");
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || zcount <= 0) return 0;
   if ((g.flags & FQ3C_SWIGLU) && ((g.N & 1) || (g.flags & (FQ3C_BIAS | FQ3C_GELU | FQ3C_SIGMOID | FQ3C_RELU2)) || zcount != 1))
     return fail("sequence product: a gated-unit epilogue takes an even number of alternating gate / up columns and no other epilogue");
   const size_t gemv_smem = (size_t)g.M * g.K * sizeof(float);
-  if (!g.seg && g.M <= 8 && gemv_smem <= 96 * 1024) {
+  if (takes_gemv(g)) {
     static bool attr[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1523,12 +1525,20 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       cudaFuncSetAttribute(fq3s_gemv_kernel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
       cudaFuncSetAttribute(fq3s_gemv_kernel<float, bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
       cudaFuncSetAttribute(fq3s_gemv_kernel<bf16, bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+      cudaFuncSetAttribute(fq3s_gemv_kernel<float, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+      cudaFuncSetAttribute(fq3s_gemv_kernel<bf16, bf16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
       attr[dev] = true;
     }
     dim3 grid((g.N + 7) / 8, 1, zcount);
-    if (b_f32) fq3s_gemv_kernel<float, float><<<grid, 256, gemv_smem, s>>>(g);
-    else if (a_f32) fq3s_gemv_kernel<float, bf16><<<grid, 256, gemv_smem, s>>>(g);
-    else fq3s_gemv_kernel<bf16, bf16><<<grid, 256, gemv_smem, s>>>(g);
+    static const SeqTail none{};
+    if (tail && tail->n > 0 && a_f32 == b_f32) {
+      if (b_f32) fq3s_gemv_kernel<float, float, true><<<grid, 256, gemv_smem, s>>>(g, *tail);
+      else fq3s_gemv_kernel<bf16, bf16, true><<<grid, 256, gemv_smem, s>>>(g, *tail);
+      return 0;
+    }
+    if (b_f32) fq3s_gemv_kernel<float, float><<<grid, 256, gemv_smem, s>>>(g, none);
+    else if (a_f32) fq3s_gemv_kernel<float, bf16><<<grid, 256, gemv_smem, s>>>(g, none);
+    else fq3s_gemv_kernel<bf16, bf16><<<grid, 256, gemv_smem, s>>>(g, none);
     return 0;
   }
   if (g.seg && zcount == 1 && g.M <= 16 && (size_t)g.K * sizeof(float) <= 96 * 1024) {
@@ -1607,6 +1617,71 @@ bool tconv_vec_ok(const fq3c_op& o) {
 }
 
 // returns 1 when the kind is not a sequence-model op
+const char* entry_op_error(const fq3c_op& o) {      // of DYT, DEPTH_MIX and XIELU
+  if (o.kind == FQ3C_DYT) {
+    if (!o.A || !o.scale || !o.C || ((o.flags & FQ3C_RESID) && !o.res)) return "dyt: missing operand";
+    if (o.norm_out && (!o.norm_w || !(o.flags & FQ3C_OUT_F32))) return "dyt: a chained norm needs its weights and an f32 result";
+  } else if (o.kind == FQ3C_DEPTH_MIX) {
+    if (o.i0 < 1 || !o.A || !o.p0 || !o.C || (o.norm_out && !o.norm_w)) return "depth_mix: missing operand";
+  } else if (!o.A || !o.p0 || !o.C) {
+    return "xielu: missing operand";
+  }
+  return nullptr;
+}
+// Which of the ops behind a product of few rows go on with its entries in the same launch.  As launches of their own they see everything that the ones in front wrote; in one launch
+// entry (m, n) sees what itself did, and nothing about other entries.  So no op may write what the product reads, and where an op writes what another one of them reads or
+// writes, it has to be the same entry: the same rows (address, pitch, type), or memory apart.
+void gemv_tail(const fq3c_op& o, const SeqGemm& g, const fq3c_op* next, const int n_next, SeqTail& t) {
+  t.n = 0;
+  if ((o.flags & ~(FQ3C_OUT_F32 | FQ3C_NOROUND | FQ3C_F32)) || !(o.flags & FQ3C_OUT_F32) || !takes_gemv(g) || o.N < 1 || o.K < 1) return;
+  struct Rows { uintptr_t at, end; long pitch; int size; };
+  const int M = o.M, N = o.N;
+  auto rows = [&](const void* p, const long ld, const int size, const int cols) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    return p ? Rows{a, a + (uintptr_t)((long)(M - 1) * ld + cols) * size, M > 1 ? ld : 0, size} : Rows{0, 0, 0, 0};
+  };
+  auto apart = [](const Rows& a, const Rows& b) { return a.end <= b.at || b.end <= a.at; };
+  auto same = [](const Rows& a, const Rows& b) { return a.at == b.at && a.pitch == b.pitch && a.size == b.size; };
+  const int in = o.flags & FQ3C_F32 ? 4 : 2;
+  const Rows from[2] = {rows(o.A, o.lda, in, o.K), Rows{reinterpret_cast<uintptr_t>(o.B), reinterpret_cast<uintptr_t>(o.B) + (uintptr_t)N * o.K * in, 0, in}};
+  Rows reads[80], writes[8], fixed[16];      // entries read and written so far; parameters, which nothing may write
+  int nr = 0, nw = 0, nf = 0;
+  writes[nw++] = rows(o.C, o.ldc, 4, N);
+  for (int k = 0; k < 2 && k < n_next; ++k) {
+    const fq3c_op& q = next[k];
+    const bool first = k == 0 && (q.kind == FQ3C_DYT || q.kind == FQ3C_XIELU), mix = k == 1 && next[0].kind == FQ3C_DYT && q.kind == FQ3C_DEPTH_MIX && q.i0 <= 64;
+    if (!(first || mix) || q.M != M || q.N != N || entry_op_error(q)) return;
+    if (first && (q.A != o.C || (M > 1 && q.lda != o.ldc))) return;
+    int r = nr, w = nw, f = nf;
+    auto param = [&](const void* p, const int n) {
+      if (p) fixed[f++] = Rows{reinterpret_cast<uintptr_t>(p), reinterpret_cast<uintptr_t>(p) + (uintptr_t)n * 4, 0, 4};
+    };
+    if (mix) {
+      for (int j = 0; j < q.i0; ++j) reads[r++] = rows(reinterpret_cast<const float*>(q.A) + (size_t)j * (size_t)q.K, q.lda, 4, N);
+      param(q.p0, q.i0);
+    } else if (q.kind == FQ3C_XIELU) {
+      param(q.p0, 2);
+    } else {
+      if (q.flags & FQ3C_RESID) reads[r++] = rows(q.res, q.ldr, 4, N);
+      param(q.scale, N);
+      param(q.bias, N);
+    }
+    const bool out32 = mix || (q.flags & FQ3C_OUT_F32);
+    writes[w++] = rows(q.C, q.ldc, out32 ? 4 : 2, N);
+    if (q.kind != FQ3C_XIELU && out32 && q.C2) writes[w++] = rows(q.C2, q.ldc, 2, N);
+    if (q.kind != FQ3C_XIELU && out32 && q.norm_out) { writes[w++] = rows(q.norm_out, q.norm_ld, q.flags & FQ3C_F32 ? 4 : 2, N); param(q.norm_w, 2 * N); }
+    for (int a = 0; a < w; ++a) {
+      if (a >= nw && (!apart(writes[a], from[0]) || !apart(writes[a], from[1]))) return;
+      for (int b = 0; b < r; ++b) if (!apart(writes[a], reads[b]) && !same(writes[a], reads[b])) return;
+      for (int b = 0; b < a; ++b) if (!apart(writes[a], writes[b]) && !same(writes[a], writes[b])) return;
+      for (int b = 0; b < f; ++b) if (!apart(writes[a], fixed[b])) return;
+    }
+    nr = r; nw = w; nf = f;
+    t.op[k] = q;
+    t.n = k + 1;
+    if (q.kind == FQ3C_XIELU) return;
+  }
+}
 int seq_run(const fq3c_op& o, cudaStream_t s) {
   switch (o.kind) {
     case FQ3C_EMBED:
@@ -1765,18 +1840,15 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       return 0;
     }
     case FQ3C_DYT:
-      if (!o.A || !o.scale || !o.C || ((o.flags & FQ3C_RESID) && !o.res)) return fail("dyt: missing operand");
-      if (o.norm_out && (!o.norm_w || !(o.flags & FQ3C_OUT_F32))) return fail("dyt: a chained norm needs its weights and an f32 result");
-      fq3s_dyt_kernel<<<dim3((o.N + 255) / 256, o.M), 256, 0, s>>>(o);
-      return 0;
     case FQ3C_DEPTH_MIX:
-      if (o.i0 < 1 || !o.A || !o.p0 || !o.C || (o.norm_out && !o.norm_w)) return fail("depth_mix: missing operand");
-      fq3s_depth_mix_kernel<<<dim3((o.N + 255) / 256, o.M), 256, 0, s>>>(o);
+    case FQ3C_XIELU: {
+      if (const char* e = entry_op_error(o)) return fail(e);
+      const dim3 grid((o.N + 255) / 256, o.M);
+      if (o.kind == FQ3C_DYT) fq3s_dyt_kernel<<<grid, 256, 0, s>>>(o);
+      else if (o.kind == FQ3C_DEPTH_MIX) fq3s_depth_mix_kernel<<<grid, 256, 0, s>>>(o);
+      else fq3s_xielu_kernel<<<grid, 256, 0, s>>>(o);
       return 0;
-    case FQ3C_XIELU:
-      if (!o.A || !o.p0 || !o.C) return fail("xielu: missing operand");
-      fq3s_xielu_kernel<<<dim3((o.N + 255) / 256, o.M), 256, 0, s>>>(o);
-      return 0;
+    }
     case FQ3C_ROT_APPEND: {
       if (!o.A || o.i0 < 0 || o.i1 < 0 || o.i2 < 1 || o.taps < 0 || (o.taps & 1) || o.taps > o.i2 || (o.taps > 0 && !o.B) ||
           (o.i1 > 0 && (!o.C || (o.cin > 0 && !o.C2))))
@@ -2235,7 +2307,10 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           g.M = o.M; g.N = o.N; g.K = o.K; g.lda = o.lda; g.ldb = o.K; g.ldc = o.ldc; g.flags = o.flags;
           g.a_mod = 1;
           const bool f32 = (o.flags & FQ3C_F32) != 0;
-          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s) != 0) return -1;
+          SeqTail tail{};
+          gemv_tail(o, g, ops + i + 1, n_ops - i - 1, tail);
+          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s, &tail) != 0) return -1;
+          i += tail.n;
           break;
         }
         if (o.K % 8 || o.cin % 8 || o.taps > 8 || o.col_mod <= 0) return fail("gemm: K and cin must be multiples of 8, taps <= 8");

@@ -552,10 +552,49 @@ __device__ __forceinline__ void stage_row_f32(float* dst, const TA* src, const i
   }
 }
 
+// ---- ops on single entries of finished f32 rows: kernels of their own, or the tail of a product of few rows --------------------
+// what follows a finished f32 value of the residual stream: the stream itself, its bf16 copy, and the next norm's output
+__device__ __forceinline__ void stream_out(const fq3c_op& o, const int m, const int c, const float v) {
+  reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
+  if (o.C2) reinterpret_cast<bf16*>(o.C2)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+  if (o.norm_out) {
+    const float* w = reinterpret_cast<const float*>(o.norm_w);
+    const float n = fmaf(tanhf(o.norm_eps * v), w[c], w[o.N + c]);
+    if (o.flags & FQ3C_F32) reinterpret_cast<float*>(o.norm_out)[(size_t)m * o.norm_ld + c] = n;
+    else reinterpret_cast<bf16*>(o.norm_out)[(size_t)m * o.norm_ld + c] = __float2bfloat16_rn(n);
+  }
+}
+__device__ __forceinline__ void dyt_at(const fq3c_op& o, const int m, const int c, const float x) {
+  float v = tanhf(o.f0 * x) * reinterpret_cast<const float*>(o.scale)[c];
+  if (o.bias) v += reinterpret_cast<const float*>(o.bias)[c];
+  if (o.flags & FQ3C_RESID) v += reinterpret_cast<const float*>(o.res)[(size_t)m * o.ldr + c];
+  if (o.flags & FQ3C_OUT_F32) stream_out(o, m, c, v);
+  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+}
+__device__ __forceinline__ void depth_mix_at(const fq3c_op& o, const int m, const int c) {
+  const float* a = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + c;
+  const float* w = reinterpret_cast<const float*>(o.p0);
+  float v = 0.f;
+  for (int j = 0; j < o.i0; ++j) v = fmaf(w[j], a[(size_t)j * (size_t)o.K], v);
+  stream_out(o, m, c, v);
+}
+__device__ __forceinline__ void xielu_at(const fq3c_op& o, const int m, const int c, const float z) {
+  const float* p = reinterpret_cast<const float*>(o.p0);
+  const float ap = softplus_f(p[0]), aq = 0.5f + softplus_f(p[1]);
+  const float v = z > 0.f ? fmaf(ap * z, z, 0.5f * z) : fmaf(aq, expm1f(z) - z, 0.5f * z);
+  if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
+  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+}
+// Up to two such ops behind a product of few rows: DYT, DYT and DEPTH_MIX, or XIELU.
+struct SeqTail { int n; fq3c_op op[2]; };
+
 // One output row with few rows in flight (decode: M <= 8): a warp per output column streams its weight row once, 16 bytes per
-// lane and load, and dots it with every A row (f32 or bf16 in shared memory as f32).  Weight-streaming bound.
-template <typename TA, typename TB>
-__global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g) {
+// lane and load, and dots it with every A row (f32 or bf16 in shared memory as f32).  Bound by latency up to a few MB of weights: the launch, one trip to the weights
+// (two batches of loads leave before the rows are staged) and the reduction.
+// TAIL: lane m goes on with entry (m, n) of row m through the ops of `tail`, with their own arithmetic: each was a launch of its own of 2 us, of which a decoded token of
+// four layers had sixteen.
+template <typename TA, typename TB, bool TAIL = false>
+__global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const __grid_constant__ SeqTail tail) {
   extern __shared__ float xs[];  // [M][K]
   const int z = blockIdx.z;
   const TA* Ap = reinterpret_cast<const TA*>(g.A) + (size_t)(z % g.a_mod) * g.a_zstride;
@@ -566,13 +605,18 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g) {
   constexpr int VEC = 16 / sizeof(TB);
   constexpr int U = 4;                 // 16-byte weight loads a lane keeps in flight
   const bool vec = ((reinterpret_cast<uintptr_t>(w) & 15) == 0) && (g.K % VEC == 0);
-  // the first weight loads leave before the rows are staged: the two latencies overlap
-  uint4 raw[U];
+  // the first weight loads leave before the rows are staged: the latencies overlap
+  uint4 raw[U], nxt[U];
   if (vec && n < g.N) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = (lane + 32 * u) * VEC;
       raw[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (lane + 32 * (U + u)) * VEC;
+      nxt[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
     }
   }
   for (int m = 0; m < g.M; ++m) stage_row_f32<TA>(xs + (size_t)m * g.K, Ap + (size_t)m * g.lda, g.K, threadIdx.x, blockDim.x);
@@ -583,11 +627,11 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g) {
   for (int m = 0; m < 8; ++m) acc[m] = 0.f;
   if (vec) {
     for (int k0 = lane * VEC; k0 < g.K; k0 += 32 * U * VEC) {
-      uint4 nxt[U];
+      uint4 fut[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {      // the next batch is on its way while this one is used
-        const int k = k0 + 32 * (U + u) * VEC;
-        nxt[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+      for (int u = 0; u < U; ++u) {      // the batch behind the next is on its way while this one is used
+        const int k = k0 + 32 * (2 * U + u) * VEC;
+        fut[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -610,7 +654,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g) {
         }
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) raw[u] = nxt[u];
+      for (int u = 0; u < U; ++u) { raw[u] = nxt[u]; nxt[u] = fut[u]; }
     }
   } else {
     for (int k = lane; k < g.K; k += 32) {
@@ -619,6 +663,22 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g) {
       for (int m = 0; m < 8; ++m)
         if (m < g.M) acc[m] = fmaf(wv, xs[m * g.K + k], acc[m]);
     }
+  }
+  if (TAIL) {
+    float v = 0.f;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      if (m >= g.M) break;
+      const float t = warp_sum(acc[m]);
+      if (lane == m) v = t;
+    }
+    if (lane < g.M) {
+      reinterpret_cast<float*>(g.C)[(size_t)lane * g.ldc + n] = v;
+      if (tail.op[0].kind == FQ3C_XIELU) xielu_at(tail.op[0], lane, n, v);
+      else dyt_at(tail.op[0], lane, n, v);
+      if (tail.n > 1) depth_mix_at(tail.op[1], lane, n);
+    }
+    return;
   }
   const int ccol = z * g.c_zstride;
   if (g.flags & FQ3C_SWIGLU) {      // warps (2k, 2k + 1) hold a unit's gate and up columns: the odd one hands its sums over
@@ -1529,50 +1589,22 @@ __global__ void __launch_bounds__(256) fq3s_latent_attn_mma_kernel(const fq3c_op
 // distance penalties / output gates, and recurrences with a matrix state per head (gated delta rule, state-space scan).
 // ===========================================================================================================================
 
-// what follows a finished f32 value of the residual stream: the stream itself, its bf16 copy, and the next norm's output
-__device__ __forceinline__ void stream_out(const fq3c_op& o, const int m, const int c, const float v) {
-  reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
-  if (o.C2) reinterpret_cast<bf16*>(o.C2)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
-  if (o.norm_out) {
-    const float* w = reinterpret_cast<const float*>(o.norm_w);
-    const float n = fmaf(tanhf(o.norm_eps * v), w[c], w[o.N + c]);
-    if (o.flags & FQ3C_F32) reinterpret_cast<float*>(o.norm_out)[(size_t)m * o.norm_ld + c] = n;
-    else reinterpret_cast<bf16*>(o.norm_out)[(size_t)m * o.norm_ld + c] = __float2bfloat16_rn(n);
-  }
-}
-
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_dyt_kernel(const fq3c_op o) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c >= o.N) return;
-  float v = tanhf(o.f0 * reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c]) * reinterpret_cast<const float*>(o.scale)[c];
-  if (o.bias) v += reinterpret_cast<const float*>(o.bias)[c];
-  if (o.flags & FQ3C_RESID) v += reinterpret_cast<const float*>(o.res)[(size_t)m * o.ldr + c];
-  if (o.flags & FQ3C_OUT_F32) stream_out(o, m, c, v);
-  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+  if (c < o.N) dyt_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c]);
 }
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_depth_mix_kernel(const fq3c_op o) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c >= o.N) return;
-  const float* a = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + c;
-  const float* w = reinterpret_cast<const float*>(o.p0);
-  float v = 0.f;
-  for (int j = 0; j < o.i0; ++j) v = fmaf(w[j], a[(size_t)j * (size_t)o.K], v);
-  stream_out(o, m, c, v);
+  if (c < o.N) depth_mix_at(o, m, c);
 }
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_xielu_kernel(const fq3c_op o) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c >= o.N) return;
-  const float* p = reinterpret_cast<const float*>(o.p0);
-  const float ap = softplus_f(p[0]), aq = 0.5f + softplus_f(p[1]);
-  const float z = reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c];
-  const float v = z > 0.f ? fmaf(ap * z, z, 0.5f * z) : fmaf(aq, expm1f(z) - z, 0.5f * z);
-  if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
-  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+  if (c < o.N) xielu_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c]);
 }
 
 // the mean of the P rows of block b of a cache -> row b of its pooled rows, for columns c0, c0 + step, .. below c1
