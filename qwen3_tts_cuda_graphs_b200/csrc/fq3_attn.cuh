@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   grid_dep_wait();
 
   const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
+  const bool one = a.groups == 1;      // its tiles take the score columns of both groups in turn
   const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * a.groups * QB;   // the last queries (most keys) start first
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
@@ -195,9 +196,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     // steps of 16 keys of tile t up to the group's last position: what lies behind is neither scored nor multiplied
     auto steps = [&](const int g, const int t) { return min(8, (last[g] - t * AT_KEYS) / 16 + 1); };
     // O[g] += P[g] V of the tile in stage st
-    auto values = [&](const int g, const int st) {
-      const uint32_t pa = tmem + g * 128, d = tmem + 256 + g * 128;
-      const int ks = steps(g, prev);
+    auto values = [&](const int g, const int st, const int tile) {
+      const uint32_t pa = tmem + (one ? st : g) * 128, d = tmem + 256 + g * 128;
+      const int ks = steps(g, tile);
       // MN-major, 128-byte swizzle: 64 columns further is a half tile further, eight keys further 1024 bytes
       const uint64_t vd = (uint64_t)(((v_s + st * AT_TILE) & 0x3ffffu) >> 4) | ((uint64_t)(AT_TILE / 2 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
       auto part = [&](const uint32_t col, const bool later) {      // (a whole tile: no condition per step)
@@ -219,10 +220,47 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (leader && !gone) part(0, true);
       }
-      if (leader && !gone && prev == tiles[g] - 1) umma_commit(o_done + 8u * g);
+      if (leader && !gone && tile == tiles[g] - 1) umma_commit(o_done + 8u * g);
       begun[g] = true;
     };
+    auto scores = [&](const int g, const int st, const int t, const int buf) {
+      if (leader && !gone) {
+        const uint32_t idesc_s = idesc | ((uint32_t)steps(g, t) << 18);
+        const uint64_t qd = umma_desc_sw128(q_s + g * AT_TILE), kd = umma_desc_sw128(k_s + st * AT_TILE);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint32_t off = (kk >> 2) * (AT_TILE / 2 >> 4) + (kk & 3) * 2;
+          umma_bf16(tmem + buf * 128, qd + off, kd + off, idesc_s, kk ? 1u : 0u);
+        }
+        umma_commit(s_full + 8u * buf);
+      }
+    };
     int n = 0, np[2] = {0, 0};
+    if (one) {
+      // One group: the next tile's scores are issued in front of this one's values, into the other score columns, so that its threads go on without waiting for the products
+      // (5 600 cycles a tile when they did).  Score columns, weights and stages of tile n have the parity of n; barriers of their own each, since two tiles may be ahead.
+      auto finish = [&](const int k, const int tile) {
+        const int st = k & 1;
+        if (!gp_wait_warp(v_full + 8u * st, (uint32_t)((k >> 1) & 1), dead, a.tries)) gone = true;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (!gp_wait_warp(p_full + 8u * st, (uint32_t)((k >> 1) & 1), dead, a.tries)) gone = true;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        values(0, st, tile);
+        if (leader && !gone) umma_commit(v_empty + 8u * st);
+      };
+      for (int t = 0; t < ntiles; ++t) {
+        if (!need(0, t)) continue;
+        const int st = n & 1;
+        if (!gp_wait_warp(k_full + 8u * st, (uint32_t)((n >> 1) & 1), dead, a.tries)) gone = true;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        scores(0, st, t, st);
+        if (leader && !gone) umma_commit(k_empty + 8u * st);
+        if (n > 0) finish(n - 1, prev);
+        prev = t;
+        ++n;
+      }
+      finish(n - 1, prev);
+    } else {
     for (int t = 0; t <= ntiles; ++t) {
       const bool more = t < ntiles;
       const bool n0 = more && need(0, t), n1 = more && need(1, t);
@@ -241,20 +279,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         if (pend[g]) {
           if (!gp_wait_warp(p_full + 8u * g, (uint32_t)(np[g]++ & 1), dead, a.tries)) gone = true;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          values(g, st ^ 1);
+          values(g, st ^ 1, prev);
           pend[g] = false;
         }
         if (g ? n1 : n0) {
-          if (leader && !gone) {
-            const uint32_t idesc_s = idesc | ((uint32_t)steps(g, t) << 18);
-            const uint64_t qd = umma_desc_sw128(q_s + g * AT_TILE), kd = umma_desc_sw128(k_s + st * AT_TILE);
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-              const uint32_t off = (kk >> 2) * (AT_TILE / 2 >> 4) + (kk & 3) * 2;
-              umma_bf16(tmem + g * 128, qd + off, kd + off, idesc_s, kk ? 1u : 0u);
-            }
-            umma_commit(s_full + 8u * g);
-          }
+          scores(g, st, t, g);
           pend[g] = true;
         }
       }
@@ -264,6 +293,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       }
       prev = t;
       ++n;
+    }
     }
   } else if (warp >= 16) {
     // ---- key and value tiles ----
@@ -334,7 +364,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       const float icap = a.cap > 0.f ? 1.f / a.cap : 0.f;
       float r1 = 0.f, r2 = 0.f;
       if (MODE == AT_DIST && a.r12) { r1 = a.r12[head]; r2 = a.r12[a.H + head]; }
-      const uint32_t lanes = (uint32_t)(wq * 32) << 16, s_t = tmem + lanes + g * 128 + half * 64, o_t = tmem + lanes + 256 + g * 128 + half * 64;
+      const uint32_t lanes = (uint32_t)(wq * 32) << 16, s_0 = tmem + lanes + g * 128 + half * 64, o_t = tmem + lanes + 256 + g * 128 + half * 64;
       // where this thread and the row's other one leave a number for each other, two tiles in turn; the two warps meet at a barrier of their own
       float* mine = reinterpret_cast<float*>(gbase + 6 * AT_TILE + 256) + g * 256 + half * 128 + r;
       const float* other = reinterpret_cast<float*>(gbase + 6 * AT_TILE + 256) + g * 256 + (half ^ 1) * 128 + r;
@@ -363,7 +393,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
       int c = 0;
       for (int t = 0; t < tilesg; ++t) {
         if (!need(g, t)) continue;
-        gp_wait_warp(s_full + 8u * g, (uint32_t)(c & 1), dead, a.tries);
+        const int buf = one ? c & 1 : g;
+        const uint32_t s_t = one ? s_0 + buf * 128 : s_0;
+        gp_wait_warp(s_full + 8u * buf, (uint32_t)((one ? c >> 1 : c) & 1), dead, a.tries);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int j0 = t * AT_KEYS, k0 = j0 + half * 64;
         // tiles that every row of the warp sees whole need no per-score test
@@ -398,8 +430,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           const float al = up ? (ref == -INFINITY ? 0.f : pow2_down(ref - mk)) : 1.f;
           if (up) ref = mk;
           sum *= al;
+          if (one) {      // the product in front ends (of two groups it has: this tile's scores were issued behind it)
+            gp_wait_warp(v_empty + 8u * (buf ^ 1), (uint32_t)(((c - 1) >> 1) & 1), dead, a.tries);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
 #pragma unroll 1
-          for (int i = 0; i < 4; ++i) {      // the product in front has ended: this tile's scores were issued behind it
+          for (int i = 0; i < 4; ++i) {
             uint32_t x[16];
             tmem_ld16(o_t + i * 16, x);
             tmem_ld_wait();
@@ -428,7 +464,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         tmem_st_wait();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full + 8u * g);
+        if (lane == 0) mbar_arrive(p_full + 8u * buf);
         if (MODE == AT_PROMPT) {
           gp_wait_warp(h_done + 8u * g, (uint32_t)(c & 1), dead, a.tries);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

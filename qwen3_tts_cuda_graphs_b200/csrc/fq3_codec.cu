@@ -1478,7 +1478,8 @@ bool attn_tc_takes(const AttnArgs& a, const int mode) {
 }
 void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after) {
   const int group = 128 / (a.H / a.G);
-  a.groups = (long)((a.M + group - 1) / group) * a.G <= GP_SMS ? 1 : 2;
+  // (with a cap the special-function unit sets the pace, which a second group cannot fill: 2048 rows of 16 heads over 4, 256 CTAs of one group 87 us, 128 of two 96)
+  a.groups = (long)((a.M + group - 1) / group) * a.G <= (mode == AT_CAP ? 2 * GP_SMS : GP_SMS) ? 1 : 2;
   const int per = a.groups * group;
   const dim3 grid((a.M + per - 1) / per, a.G);
   if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
