@@ -624,21 +624,32 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return t;
 }
 
-// RMSNorm of a row by a warp, eight entries a lane and load: the reciprocal root of the mean square, and eight normed entries.
-__device__ __forceinline__ float sq8(const uint4 x, float ss) {
+// RMSNorm of a row by a warp, eight entries a lane and load, with the sums of fq3c_rmsnorm_kernel's 256 threads in their order: lane l's pieces 8 l + 256 c .. + 7 are the
+// entries of its threads 8 l .. 8 l + 7, and thread t of a warp of the block is entry t & 7 of lane t >> 3.  sq8 adds a piece to those eight sums; rms_of adds them as
+// block_sum does (threads 16, 8, 4, 2, 1 apart, then the eight warps one by one) and gives the reciprocal root of the mean square.
+__device__ __forceinline__ void sq8(const uint4 x, float (&ss)[8]) {
   const uint32_t u[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const float a = __uint_as_float(u[q] << 16), b = __uint_as_float(u[q] & 0xffff0000u);
-    ss = fmaf(a, a, ss);
-    ss = fmaf(b, b, ss);
+    ss[2 * q] = fmaf(a, a, ss[2 * q]);
+    ss[2 * q + 1] = fmaf(b, b, ss[2 * q + 1]);
   }
-  return ss;
 }
-__device__ __forceinline__ float rms_of(float ss, const int N, const float eps) {
+__device__ __forceinline__ float rms_of(const float (&ss)[8], const int lane, const int N, const float eps) {
+  const bool b4 = lane & 2, b3 = lane & 1;      // bits 4 and 3 of the lane's threads; each meeting keeps half of the entries
+  float a[4], b[2];
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-  return rsqrtf(ss / N + eps);
+  for (int i = 0; i < 4; ++i) a[i] = (b4 ? ss[i + 4] : ss[i]) + __shfl_xor_sync(0xffffffffu, b4 ? ss[i] : ss[i + 4], 2);      // 16 apart
+#pragma unroll
+  for (int i = 0; i < 2; ++i) b[i] = (b3 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, b3 ? a[i] : a[i + 2], 1);          // 8 apart
+  float t = (b4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b4 ? b[0] : b[1], 2);      // entries 4 apart, between the lanes that kept them
+  t += __shfl_xor_sync(0xffffffffu, t, 1);      // 2 apart
+  t += __shfl_xor_sync(0xffffffffu, t, 2);      // 1 apart
+  float sum = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) sum += __shfl_sync(0xffffffffu, t, 4 * w);
+  return rsqrtf(sum / N + eps);
 }
 __device__ __forceinline__ uint4 norm8(const uint4 x, const float rs, const float* w) {
   const float4 a = *reinterpret_cast<const float4*>(w), b = *(reinterpret_cast<const float4*>(w) + 1);
@@ -657,7 +668,7 @@ bool norm_vec_ok(const void* x, const void* y, const void* w, const int N, const
   return ((N | ldx | ldy) & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 // FQ3C_RMSNORM and the norm behind a product (fq3c_op.norm_out), the same bits either way.  Bound by latency for few rows (a launch, a trip to L2), by its bytes for
-// many.  A block per row with two-byte loads and two block-wide sums took 2.6 us for 39 rows of 1024 and 5.5 for 1900; so 2.2 and 3.5.  (Normed by the product behind
+// many.  A block per row with two-byte loads and block-wide sums takes 2.6 us for 39 rows of 1024 and 5.5 for 1900, this 2.2 and 3.9.  (Normed by the product behind
 // it instead, in each of its CTAs: a layer of a 39-row prompt 38.7 -> 43.3 us.)
 constexpr int RN_WARPS = 4;
 __global__ void __launch_bounds__(RN_WARPS * 32) fq3c_rownorm_vec_kernel(const bf16* x, const int ldx, bf16* y, const int ldy, const float* w, const float eps, const int row0, const int rows,
@@ -669,15 +680,15 @@ __global__ void __launch_bounds__(RN_WARPS * 32) fq3c_rownorm_vec_kernel(const b
   uint4* yr = reinterpret_cast<uint4*>(y + (size_t)(row0 + row) * ldy);
   constexpr int C = 4;      // pieces of a lane kept from the sum to the norm; longer rows are read again
   uint4 v[C];
-  float ss = 0.f;
+  float ss[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if (lane + 32 * c < N / 8) v[c] = xr[lane + 32 * c];
 #pragma unroll
   for (int c = 0; c < C; ++c)
-    if (lane + 32 * c < N / 8) ss = sq8(v[c], ss);
-  for (int p = lane + 32 * C; p < N / 8; p += 32) ss = sq8(xr[p], ss);
-  const float rs = rms_of(ss, N, eps);
+    if (lane + 32 * c < N / 8) sq8(v[c], ss);
+  for (int p = lane + 32 * C; p < N / 8; p += 32) sq8(xr[p], ss);
+  const float rs = rms_of(ss, lane, N, eps);
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if (lane + 32 * c < N / 8) yr[lane + 32 * c] = norm8(v[c], rs, w + 8 * (lane + 32 * c));
