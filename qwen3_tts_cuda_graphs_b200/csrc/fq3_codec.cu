@@ -798,6 +798,8 @@ __device__ __forceinline__ void attn_load(const bf16* p, float (&v)[4]) {
     v[0] = __bfloat162float(p[0]); v[1] = 0.f; v[2] = 0.f; v[3] = 0.f;
   }
 }
+// A key's share p v joins a sum that shrinks by corr.  The product is rounded before the sum, in every kernel that adds key by key: their results are the same bits.
+__device__ __forceinline__ float attn_add(const float acc, const float corr, const float p, const float v) { return fmaf(acc, corr, __fmul_rn(p, v)); }
 template <int PER>
 __device__ __forceinline__ void attn_warp(const fq3c_op& o, int t_out, int h, int lane) {
   const int nh = o.i0, nkv = o.i1, d = o.i2, win = o.K;
@@ -819,7 +821,8 @@ __device__ __forceinline__ void attn_warp(const fq3c_op& o, int t_out, int h, in
       float k[4];
       attn_load<PER>(base + (size_t)j * o.lda + koff, k);
       attn_load<PER>(base + (size_t)j * o.lda + voff, v[u]);
-      s[u] = q[0] * k[0] + q[1] * k[1] + q[2] * k[2] + q[3] * k[3];
+      s[u] = fmaf(q[0], k[0], __fmul_rn(q[1], k[1]));
+      if (PER == 4) s[u] = fmaf(q[3], k[3], fmaf(q[2], k[2], s[u]));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -831,9 +834,9 @@ __device__ __forceinline__ void attn_warp(const fq3c_op& o, int t_out, int h, in
       if (jb + u <= t) {
         const float su = bf16r(bf16r(s[u]) * scale);
         const float mn = fmaxf(m, su), corr = expf(m - mn), p = expf(su - mn);
-        l = l * corr + p;
+        l = fmaf(l, corr, p);
 #pragma unroll
-        for (int i = 0; i < PER; ++i) acc[i] = acc[i] * corr + p * v[u][i];
+        for (int i = 0; i < PER; ++i) acc[i] = attn_add(acc[i], corr, p, v[u][i]);
         m = mn;
       }
     }
@@ -1054,26 +1057,26 @@ __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
 // see in shared memory once, and then
 //   scores: a warp per (row, head, 32 keys), a lane per key - q is a broadcast, keys lie 16 bytes apart in banks, no shuffles;
 //   sums:   a warp per (row, head), the exponentials once per key, then a lane per D / 32 entries walks the keys in order.
-// A row's sums do not depend on the rows beside it, so a window of a stream gives the bits of the whole decode.  Rounding points of fq3c_attn_kernel: score -> bf16 ->
-// x scale -> bf16, softmax and sums f32, output bf16.
+// Its bits are those of the kernels with a warp per (row, head), infinities and NaN among them: fq3c_attn_kernel's, and with PROMPT fq3c_attn_prefill_kernel's.  A dot
+// product is added up as their lanes and shuffles do, the running maximum of the one is a scan over the keys, its sums shrink key by key.  So a
+// stream and the whole decode agree whichever kernel each of their sizes comes to.
 // What bounds it is latency: one round trip to L2, a few thousand cycles of dependent work and a launch; the kernels with a warp per (row, head) make
 // a round trip for every four to sixteen keys.
 // PROMPT: `n` is the FQ3C_QKNORM_ROPE_KV op in front.  Every CTA norms and turns the keys it stages (again for each RB rows: 60 instructions a key), its queries, and
 // writes its own rows of the cache: one launch in place of two, and the rows in `A` stay as the product left them.  39 rows of
-// 16 heads 8.1 -> 5.7 us; the codec's attention (16 heads of 64, window 72) 33 rows 7.6 -> 3.8, 256 rows 31.8 -> 16.1, one row
-// 1.7 -> 2.5 (kept there too: a stream's rows and the whole decode's have the same sums).
+// 16 heads 8.2 -> 5.6 us; the codec's attention (16 heads of 64, window 72) 33 rows 7.6 -> 3.8, 256 rows 32.0 -> 12.9, one row behind 71 others 14.4 -> 4.3.
 constexpr int GP_SMS = 148;
 constexpr int AR_PROMPT_ROWS = 144, AR_WARPS = 16, AR_SMEM_MAX = 128 * 1024;
 struct AttnRows { int rb, span, sp; size_t smem; };      // rows of a CTA, keys it may stage, pitch of its scores
 __host__ __device__ constexpr int ar_k_pitch(int d) { return d * 2 + 16; }      // bytes
-AttnRows attn_rows_plan(const fq3c_op& o) {
+AttnRows attn_rows_plan(const fq3c_op& o, const bool prompt) {
   AttnRows r;
   const int hg = o.i0 / o.i1;
   r.rb = 1;      // as few rows as one CTA per SM allows: 100 rows of 16 heads with 160 CTAs 16.5 us
   while (r.rb < 16 && (long)((o.M + r.rb - 1) / r.rb) * o.i1 > GP_SMS) ++r.rb;
   r.span = (int)std::min<long>((long)o.K + r.rb - 1, (long)o.M + o.taps);
   r.sp = (r.span + 31) / 32 * 32;
-  r.smem = (size_t)r.span * (ar_k_pitch(o.i2) + o.i2 * 2) + (size_t)r.rb * hg * (o.i2 + r.sp) * 4;
+  r.smem = (size_t)r.span * (ar_k_pitch(o.i2) + o.i2 * 2) + (size_t)r.rb * hg * (o.i2 + (prompt ? 1 : 2) * r.sp) * 4;
   return r;
 }
 // a head's row of 128, four entries a lane: RMSNorm and rotation with the rounding points of fq3c_qknorm_rope_kv_kernel
@@ -1096,6 +1099,35 @@ __device__ __forceinline__ uint2 norm_turn(const uint2 raw, const float eps, con
   }
   const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
   return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+__device__ __forceinline__ float dot2(const float x, const float y, const uint32_t a) { return fmaf(x, __uint_as_float(a << 16), __fmul_rn(y, __uint_as_float(a & 0xffff0000u))); }
+__device__ __forceinline__ float dot4(const float4 q, const uint32_t a, const uint32_t b) {
+  return fmaf(q.w, __uint_as_float(b & 0xffff0000u), fmaf(q.z, __uint_as_float(b << 16), dot2(q.x, q.y, a)));
+}
+// The D / 32 entries of each lane of attn_warp, summed in the order of its shuffles (lanes 16, 8, 4, 2, 1 apart): pieces of eight entries hold 256 / D lanes' shares, and
+// here the pieces C, C + STRIDE, .. have met.  (Products of two bf16 are exact in f32 up to its largest value: only the order of the sums counts, and which product of a pair
+// overflows by itself.)
+template <int D, int C, int STRIDE>
+__device__ __forceinline__ void lane_sums(const uint4* kp, const float4* qa, float (&sum)[256 / D]) {
+  if constexpr (STRIDE == D / 8) {
+    const uint4 k = kp[C];
+    const float4 x = qa[2 * C], y = qa[2 * C + 1];
+    if constexpr (D == 128) {
+      sum[0] = dot4(x, k.x, k.y);
+      sum[1] = dot4(y, k.z, k.w);
+    } else {
+      sum[0] = dot2(x.x, x.y, k.x);
+      sum[1] = dot2(x.z, x.w, k.y);
+      sum[2] = dot2(y.x, y.y, k.z);
+      sum[3] = dot2(y.z, y.w, k.w);
+    }
+  } else {
+    float far[256 / D];
+    lane_sums<D, C, 2 * STRIDE>(kp, qa, sum);
+    lane_sums<D, C + STRIDE, 2 * STRIDE>(kp, qa, far);
+#pragma unroll
+    for (int i = 0; i < 256 / D; ++i) sum[i] += far[i];
+  }
 }
 template <int D, bool PROMPT>
 __global__ void __launch_bounds__(AR_WARPS * 32) fq3c_attn_rows_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op n, const int RB, const int span_max, const int SP) {
@@ -1169,50 +1201,107 @@ __global__ void __launch_bounds__(AR_WARPS * 32) fq3c_attn_rows_kernel(const __g
     if (ch * 32 > t || ch * 32 + 31 <= t - win) continue;
     const uint4* kp = reinterpret_cast<const uint4*>(ks + (size_t)min(j, span - 1) * KP);
     const float4* qa = reinterpret_cast<const float4*>(qs + i * D);
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    float dot;
+    if constexpr (PROMPT) {      // the shares of four lanes, every fourth piece each, its first and its last four entries apart
+      float part[4];
 #pragma unroll
-    for (int c = 0; c < D / 8; ++c) {
-      const uint4 k = kp[c];
-      const float4 x = qa[2 * c], y = qa[2 * c + 1];
-      a[0] = fmaf(x.x, __uint_as_float(k.x << 16), a[0]); a[1] = fmaf(x.y, __uint_as_float(k.x & 0xffff0000u), a[1]);
-      a[2] = fmaf(x.z, __uint_as_float(k.y << 16), a[2]); a[3] = fmaf(x.w, __uint_as_float(k.y & 0xffff0000u), a[3]);
-      a[0] = fmaf(y.x, __uint_as_float(k.z << 16), a[0]); a[1] = fmaf(y.y, __uint_as_float(k.z & 0xffff0000u), a[1]);
-      a[2] = fmaf(y.z, __uint_as_float(k.w << 16), a[2]); a[3] = fmaf(y.w, __uint_as_float(k.w & 0xffff0000u), a[3]);
+      for (int l = 0; l < 4; ++l) {
+        float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+        for (int c = l; c < D / 8; c += 4) {
+          const uint4 k = kp[c];
+          d0 += dot4(qa[2 * c], k.x, k.y);
+          d1 += dot4(qa[2 * c + 1], k.z, k.w);
+        }
+        part[l] = d0 + d1;
+      }
+      dot = (part[0] + part[1]) + (part[2] + part[3]);
+    } else {
+      float sum[256 / D];
+      lane_sums<D, 0, 1>(kp, qa, sum);
+      if constexpr (D == 128) dot = sum[0] + sum[1];
+      else dot = (sum[0] + sum[2]) + (sum[1] + sum[3]);
     }
-    sc[i * SP + j] = bf16r(bf16r((a[0] + a[1]) + (a[2] + a[3])) * scale);
+    const float x = bf16r(bf16r(dot) * scale);
+    if constexpr (PROMPT) sc[i * SP + j] = x;
+    else reinterpret_cast<float2*>(sc)[i * SP + j].x = x;
   }
   __syncthreads();
   for (int i = warp; i < rows * HG; i += AR_WARPS) {
     const int row = i / HG, h = g * HG + i - row * HG, je = r0 + row + hist - j_lo, jb = max(0, je - win + 1);
-    float* s = sc + (size_t)i * SP;
-    float mx = -INFINITY;
-    for (int j = jb + lane; j <= je; j += 32) mx = fmaxf(mx, s[j]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    for (int j = jb + lane; j <= je; j += 32) s[j] = expf(s[j] - mx);
-    __syncwarp();
     float l = 0.f, acc[PER];
 #pragma unroll
     for (int e = 0; e < PER; ++e) acc[e] = 0.f;
     const unsigned char* vp = vs + lane * PER * 2;
+    if constexpr (PROMPT) {
+      float* s = sc + (size_t)i * SP;
+      float mx = -INFINITY;
+      for (int j = jb + lane; j <= je; j += 32) mx = fmaxf(mx, s[j]);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      for (int j = jb + lane; j <= je; j += 32) s[j] = expf(s[j] - mx);
+      __syncwarp();
 #pragma unroll 8
-    for (int j = jb; j <= je; ++j) {
-      const float p = s[j];
-      const Vec v = *reinterpret_cast<const Vec*>(vp + (size_t)j * 2 * D);
-      l += p;
-      if constexpr (PER == 4) {
+      for (int j = jb; j <= je; ++j) {
+        const float p = s[j];
+        const Vec v = *reinterpret_cast<const Vec*>(vp + (size_t)j * 2 * D);
+        l += p;
         acc[0] = fmaf(p, __uint_as_float(v.x << 16), acc[0]); acc[1] = fmaf(p, __uint_as_float(v.x & 0xffff0000u), acc[1]);
         acc[2] = fmaf(p, __uint_as_float(v.y << 16), acc[2]); acc[3] = fmaf(p, __uint_as_float(v.y & 0xffff0000u), acc[3]);
-      } else {
-        acc[0] = fmaf(p, __uint_as_float(v << 16), acc[0]); acc[1] = fmaf(p, __uint_as_float(v & 0xffff0000u), acc[1]);
       }
+    } else {
+      // the highest score up to each key, four times 32 keys at a time: a key's weight, and what the sums in front of it shrink by
+      float2* s = reinterpret_cast<float2*>(sc) + (size_t)i * SP;
+      float m = -INFINITY;
+      for (int b = jb + lane; b - lane <= je; b += 128) {
+        float x[4], top[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) top[u] = x[u] = b + 32 * u <= je ? s[b + 32 * u].x : -INFINITY;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float y = __shfl_up_sync(0xffffffffu, top[u], d);
+            if (lane >= d) top[u] = fmaxf(top[u], y);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          top[u] = fmaxf(m, top[u]);
+          float before = __shfl_up_sync(0xffffffffu, top[u], 1);
+          if (lane == 0) before = m;
+          m = __shfl_sync(0xffffffffu, top[u], 31);
+          if (b + 32 * u <= je) s[b + 32 * u] = make_float2(expf(x[u] - top[u]), expf(before - top[u]));
+        }
+      }
+      __syncwarp();
+#pragma unroll 8
+      for (int j = jb; j <= je; ++j) {
+        const float2 w = s[j];
+        const Vec v = *reinterpret_cast<const Vec*>(vp + (size_t)j * 2 * D);
+        l = fmaf(l, w.y, w.x);
+        if constexpr (PER == 4) {
+          acc[0] = attn_add(acc[0], w.y, w.x, __uint_as_float(v.x << 16)); acc[1] = attn_add(acc[1], w.y, w.x, __uint_as_float(v.x & 0xffff0000u));
+          acc[2] = attn_add(acc[2], w.y, w.x, __uint_as_float(v.y << 16)); acc[3] = attn_add(acc[3], w.y, w.x, __uint_as_float(v.y & 0xffff0000u));
+        } else {
+          acc[0] = attn_add(acc[0], w.y, w.x, __uint_as_float(v << 16)); acc[1] = attn_add(acc[1], w.y, w.x, __uint_as_float(v & 0xffff0000u));
+        }
+      }
+    }
+    if constexpr (PROMPT) {
+      const float inv = 1.f / l;
+#pragma unroll
+      for (int e = 0; e < PER; ++e) acc[e] *= inv;
+    } else {
+#pragma unroll
+      for (int e = 0; e < PER; ++e) acc[e] /= l;
     }
     bf16* out = reinterpret_cast<bf16*>(o.C) + (size_t)(r0 + row) * o.ldc + h * D + lane * PER;
     if constexpr (PER == 4) {
-      const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0] / l, acc[1] / l), hi = __floats2bfloat162_rn(acc[2] / l, acc[3] / l);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0], acc[1]), hi = __floats2bfloat162_rn(acc[2], acc[3]);
       *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     } else {
-      *reinterpret_cast<__nv_bfloat162*>(out) = __floats2bfloat162_rn(acc[0] / l, acc[1] / l);
+      *reinterpret_cast<__nv_bfloat162*>(out) = __floats2bfloat162_rn(acc[0], acc[1]);
     }
   }
 }
@@ -1501,11 +1590,11 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
 
 // ---- attention of few rows or a short window -----------------------------------------------------------------------------------
 // What fq3c_attn_rows_kernel's vector accesses and shared memory ask for; grid.y is the head.
-bool attn_rows_takes(const fq3c_op& o) {
+bool attn_rows_takes(const fq3c_op& o, const bool prompt) {
   auto off = [](const void* p, int a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
   const int vec = o.i2 / 32;      // entries a lane moves at a time
   return (o.i2 == 64 || o.i2 == 128) && o.i1 > 0 && o.i0 > 0 && o.i0 % o.i1 == 0 && o.i1 <= 65535 && o.K > 0 && o.taps >= 0 && o.lda % vec == 0 && o.ldc % vec == 0 &&
-         !off(o.A, 2 * vec) && !off(o.C, 2 * vec) && attn_rows_plan(o).smem <= AR_SMEM_MAX && device_attrs_ready();
+         !off(o.A, 2 * vec) && !off(o.C, 2 * vec) && attn_rows_plan(o, prompt).smem <= AR_SMEM_MAX && device_attrs_ready();
 }
 // `n` (q / k norm, rotation, cache rows) and the prompt attention `o` behind it, where the rows that `n` would rewrite are scratch to everyone else (reserved bit 0)
 // Against two launches (behind these lines the second is the kernel on tcgen05): 39 rows of 16 heads 5.7 and 8.1 us, 100 11.6 and 13.1, 112 14.3 and 13.3; 64 of 32 11.0
@@ -1513,7 +1602,7 @@ bool attn_rows_takes(const fq3c_op& o) {
 bool attn_rows_takes_prompt(const fq3c_op& n, const fq3c_op& o) {
   auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) != 0; };
   return (n.reserved & 1) && o.kind == FQ3C_ATTN && (o.flags & 1) && o.A == n.A && o.lda == n.lda && o.M == n.M && o.i0 == n.i0 && o.i1 == n.i1 && o.i2 == 128 && o.taps == 0 && !o.p0 &&
-         o.M <= AR_PROMPT_ROWS && (long)o.M * o.M * o.i0 <= 165000 && !off(n.p0) && !off(n.p1) && !off(n.B) && !off(n.bias) && !off(n.C) && !off(n.C2) && attn_rows_takes(o);
+         o.M <= AR_PROMPT_ROWS && (long)o.M * o.M * o.i0 <= 165000 && !off(n.p0) && !off(n.p1) && !off(n.B) && !off(n.bias) && !off(n.C) && !off(n.C2) && attn_rows_takes(o, true);
 }
 
 // ---- sequence-model ops: launch logic ---------------------------------------------------------------------------------------
@@ -2472,8 +2561,8 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           launch_after(fq3c_attn_prefill_kernel, (warps + APF_WARPS - 1) / APF_WARPS, APF_WARPS * 32, smem, s, after, 1, o, tpad);
           break;
         }
-        if (attn_rows_takes(o)) {
-          const AttnRows r = attn_rows_plan(o);
+        if (attn_rows_takes(o, false)) {
+          const AttnRows r = attn_rows_plan(o, false);
           const dim3 grid((unsigned)((o.M + r.rb - 1) / r.rb), (unsigned)o.i1);
           if (o.i2 == 64) launch_after(fq3c_attn_rows_kernel<64, false>, grid, AR_WARPS * 32, r.smem, s, after, 1, o, o, r.rb, r.span, r.sp);
           else launch_after(fq3c_attn_rows_kernel<128, false>, grid, AR_WARPS * 32, r.smem, s, after, 1, o, o, r.rb, r.span, r.sp);
@@ -2492,7 +2581,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         if (o.lda % 4 || !o.C || !o.C2 || !o.p0 || !o.p1 || !o.B || !o.bias) return fail("qknorm_rope_kv: missing operand");
         if (i + 1 < n_ops && attn_rows_takes_prompt(o, ops[i + 1])) {      // with the attention behind it in one launch
           const fq3c_op& at = ops[++i];
-          const AttnRows r = attn_rows_plan(at);
+          const AttnRows r = attn_rows_plan(at, true);
           launch_after(fq3c_attn_rows_kernel<128, true>, dim3((unsigned)((at.M + r.rb - 1) / r.rb), (unsigned)at.i1), AR_WARPS * 32, r.smem, s, after, 1, at, o, r.rb, r.span, r.sp);
           break;
         }

@@ -86,3 +86,57 @@ def test_norm_rotation_and_cache_in_the_same_launch(M, H, G, pos0):
     assert torch.equal(ck, ck1) and torch.equal(cv, cv1)
     want, bound = exact(turned, M, H, G, 128, 4096)
     assert ((out.double() - want).abs() <= bound).all()
+
+
+def streamed(x, M, H, G, d, window, chunk):
+    """The rows in chunks, each behind the window's earlier rows, as a stateful stream decodes them."""
+    out = torch.zeros(M, H * d, device="cuda", dtype=torch.bfloat16)
+    for at in range(0, M, chunk):
+        hist, rows = min(window - 1, at), min(chunk, M - at)
+        launch(attn_op(x[at - hist:at + rows], out[at:at + rows], rows, H, G, d, window, hist))
+    return out
+
+
+# windows on both sides of what a CTA's shared memory holds: whole decode and stream do not come to the same kernel at 400 (460 rows), 480 and 1024
+@pytest.mark.parametrize("M,H,G,d,window,chunk", [(100, 16, 16, 64, 72, 1), (256, 16, 16, 64, 72, 9), (460, 16, 16, 64, 400, 33), (256, 16, 16, 64, 480, 8), (300, 16, 16, 64, 1024, 33), (90, 4, 2, 64, 8, 3),
+                                                  (260, 8, 8, 128, 130, 20), (300, 8, 2, 128, 300, 50)])
+def test_a_stream_has_the_bits_of_the_whole_decode(M, H, G, d, window, chunk):
+    g = torch.Generator(device="cuda").manual_seed(M + window)
+    x = (1.5 * torch.randn(M, (H + 2 * G) * d, device="cuda", generator=g)).bfloat16()
+    out = torch.zeros(M, H * d, device="cuda", dtype=torch.bfloat16)
+    launch(attn_op(x, out, M, H, G, d, window))
+    assert torch.equal(out, streamed(x, M, H, G, d, window, chunk))
+
+
+@pytest.mark.parametrize("M,H,G,d,window,hist,known", [c for c in CASES if c[0] * c[1] * c[3] <= 400000] + [(33, 16, 16, 64, 72, 71, 71), (100, 16, 8, 128, 72, 0, None)])
+def test_the_general_kernel_has_the_same_bits(M, H, G, d, window, hist, known):
+    """Outputs one entry off an even address go through the kernel with a warp per row and head; infinite scores among the keys."""
+    g = torch.Generator(device="cuda").manual_seed(M * 3 + d)
+    x = (1.5 * torch.randn(hist + M, (H + 2 * G) * d, device="cuda", generator=g)).bfloat16()
+    x[(hist + M) // 2, H * d:H * d + 8] = 3e38      # scores of both signs beyond bf16 (and NaN, where they meet)
+    n = None if known is None else torch.tensor([known], dtype=torch.int32, device="cuda")
+    out, wide = torch.zeros(M, H * d, device="cuda", dtype=torch.bfloat16), torch.zeros(M, H * d + 4, device="cuda", dtype=torch.bfloat16)
+    launch(attn_op(x, out, M, H, G, d, window, hist, n))
+    launch(attn_op(x, wide[:, 1:], M, H, G, d, window, hist, n))
+    got, want = out.float(), wide[:, 1:1 + H * d].float()
+    assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)) and torch.equal(got.isnan(), want.isnan())
+
+
+@pytest.mark.parametrize("M,H,G", [(17, 16, 8), (39, 16, 8), (64, 4, 4), (84, 16, 8), (30, 14, 2), (64, 4, 1), (39, 32, 8)])
+def test_prompt_in_one_launch_has_the_bits_of_two(M, H, G):
+    """Rows that tcgen05 does not take yet: norm, rotation, cache and attention together, and the attention behind them by itself."""
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    g = torch.Generator(device="cuda").manual_seed(M * H + 1)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g).bfloat16()  # noqa: E731
+    x, gq, gk, ang = rand(M, (H + 2 * G) * 128), rand(128), rand(128), torch.rand(M, 64, device="cuda", generator=g) * 6.28
+    cos, sin = torch.cat([ang, ang], -1).cos().bfloat16(), torch.cat([ang, ang], -1).sin().bfloat16()
+    got = []
+    for scratch in (0, 1):
+        rows, ck, cv, out = x.clone(), *(torch.zeros(G, M, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2)), torch.zeros(M, H * 128, device="cuda", dtype=torch.bfloat16)
+        n = K.Op()
+        n.kind, n.M, n.N, n.A, n.lda, n.a_rows, n.i0, n.i1, n.f0, n.reserved = 8, M, x.shape[1], rows.data_ptr(), x.shape[1], M, H, G, 1e-6, scratch
+        n.p0, n.p1, n.B, n.bias, n.C, n.C2, n.ldc, n.col_mod = (*(t.data_ptr() for t in (gq, gk, cos, sin, ck, cv)), M, x.shape[1])
+        assert launch(n, attn_op(rows, out, M, H, G, 128, 4096, flags=1)) == 2 - scratch
+        got.append((ck, cv, out))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
