@@ -1589,10 +1589,14 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
 }
 
 // ---- attention of few rows or a short window -----------------------------------------------------------------------------------
-// What fq3c_attn_rows_kernel's vector accesses and shared memory ask for; grid.y is the head.
+// What fq3c_attn_rows_kernel's vector accesses and shared memory ask for; grid.y is the head.  By itself it pays from nine keys in sight on: fq3c_attn_kernel fetches up to
+// eight in two trips (16 heads of 64: 1 row 1.7 and 2.7 us, 8 rows 2.8 and 3.2, 9 rows 3.3 and 3.2; a window of 8, 33 rows 3.0 and 3.6, 600 rows 8.9 and 13.0), and from
+// sixteen where the rows make more than one CTA per SM (600 rows, a window of 12 11.6 and 13.7, of 16 14.2 and 14.0).
 bool attn_rows_takes(const fq3c_op& o, const bool prompt) {
   auto off = [](const void* p, int a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; };
   const int vec = o.i2 / 32;      // entries a lane moves at a time
+  const long keys = std::min<long>(o.K, (long)o.M + o.taps);
+  if (!prompt && (keys <= 8 || (keys < 16 && (long)((o.M + 15) / 16) * o.i1 > GP_SMS))) return false;
   return (o.i2 == 64 || o.i2 == 128) && o.i1 > 0 && o.i0 > 0 && o.i0 % o.i1 == 0 && o.i1 <= 65535 && o.K > 0 && o.taps >= 0 && o.lda % vec == 0 && o.ldc % vec == 0 &&
          !off(o.A, 2 * vec) && !off(o.C, 2 * vec) && attn_rows_plan(o, prompt).smem <= AR_SMEM_MAX && device_attrs_ready();
 }

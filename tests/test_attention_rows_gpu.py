@@ -108,7 +108,8 @@ def test_a_stream_has_the_bits_of_the_whole_decode(M, H, G, d, window, chunk):
     assert torch.equal(out, streamed(x, M, H, G, d, window, chunk))
 
 
-@pytest.mark.parametrize("M,H,G,d,window,hist,known", [c for c in CASES if c[0] * c[1] * c[3] <= 400000] + [(33, 16, 16, 64, 72, 71, 71), (100, 16, 8, 128, 72, 0, None)])
+@pytest.mark.parametrize("M,H,G,d,window,hist,known", [c for c in CASES if c[0] * c[1] * c[3] <= 400000] + [(33, 16, 16, 64, 72, 71, 71), (100, 16, 8, 128, 72, 0, None)] +
+                         [(8, 16, 16, 64, 72, 0, None), (9, 16, 8, 128, 72, 0, None), (33, 16, 16, 64, 9, 0, None), (300, 16, 16, 64, 15, 0, None), (300, 16, 16, 64, 16, 0, None)])      # lines between the kernels
 def test_the_general_kernel_has_the_same_bits(M, H, G, d, window, hist, known):
     """Outputs one entry off an even address go through the kernel with a warp per row and head; infinite scores among the keys."""
     g = torch.Generator(device="cuda").manual_seed(M * 3 + d)
