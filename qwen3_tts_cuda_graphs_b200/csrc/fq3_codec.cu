@@ -1503,20 +1503,29 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   const bool few = g.a_rows <= 64;
   L.shape = few ? GS_FEW : GS_WIDE;
   const int groups = few ? 2 : 4;
-  // Split over K when the tiles would cover less than half of the SMs and the reduction is long (the transformer's o / down projections of few rows: 16-32 tiles of
-  // 32-48 k-blocks): two or four CTAs per tile, a cluster; six, eight and more than 128 CTAs in clusters do not find room at the same time (17 x 1024 x 2048: four
-  // 5.7 us, six 6.3, eight 11.3).  The count must not depend on m_begin: a tail-only decode has to add the same partial sums in the same order.
+  // Sums in parts, where the tiles would cover less than half of the SMs and the reduction is long (the transformer's o / down projections of few rows): up to eight parts of
+  // at least four k-blocks, as many as there are SMs for.  The parts are the order of the sums and their exactness: against float64, 39 x 1024 x 2048 is off by 2.4e-7 of its
+  // norm in eight parts, by 4.7e-7 in four and by 2.1e-6 whole (the tensor pipe drops what lies below its accumulator's last place, once per product).  So they do not follow
+  // what a launch costs, nor m_begin: a tail-only decode has to add the same partial sums in the same order.
   const int KT = (o.K + TK - 1) / TK;
-  g.splits = 1;
+  g.parts = 1;
   if ((o.ws || (o.reserved & 4)) && o.M <= 4 * TM && KT >= 8) {
     const int bn = o.N >= 64 ? 64 : 32;
     const int tiles = ((o.N + bn - 1) / bn) * ((o.M + TM - 1) / TM);
-    const int sp = tiles * 4 <= 128 && KT >= 16 ? 4 : tiles * 2 <= 128 ? 2 : 1;
-    // The cluster's two meetings and the sums cost about 5000 cycles and 30 for each row of the tile, a k-block 300.  Whole against split: 17 x 1024 x 2048 6.6 and
-    // 5.7 us, 64 rows 6.6 and 6.4, 100 rows 6.7 and 7.0; 39 x 1024 x 3072 9.1 and 6.7, 130 rows 9.4 and 9.0, 262 rows 9.8 and 10.0; 39 x 2048 x 6144 15.7 and 10.0.
-    if (sp > 1 && (long)(KT - (KT + sp - 1) / sp) * 300 > 5000 + 30L * std::min(o.M, TM)) { g.splits = sp; g.bn = bn; }
+    const int sp = std::min(std::min(8, KT / 4), GP_SMS / std::max(1, tiles));
+    if (sp > 1 && (long)KT * 430 - (long)((KT + sp - 1) / sp) * 440 > 3700 + 90L * std::min(o.M, TM)) {
+      g.parts = sp;
+      g.bn = bn;
+      // Clusters of more than four CTAs, or of more than 128 in all, do not find room at the same time, nor beside the launches around them: their CTAs take two parts each
+      // (eight parts in a prompt of 39 rows through 28 layers: clusters of eight 1203 us, of four 1125).  An SM's sixteen epilogue warps are of no use to a single tile: 73 x 1024 x
+      // 3072 8.6 us, with eight 7.9; 200 rows 8.7 and 7.8.
+      g.per = sp > 4 || tiles * sp > 128 ? 2 : 1;
+      L.shape = GS_FEW;
+    }
   }
-  if (g.splits == 1) {
+  if (g.parts == 1) g.per = 1;
+  g.splits = (g.parts + g.per - 1) / g.per;
+  if (g.parts == 1) {
     // The width with the least waves x slower of (k loop, epilogue) + the other one once, in cycles.  A k-block takes what its instructions take (300), its four products
     // (two cycles a column), or its operand bytes at the 60 a cycle that L2 gives one SM.  The operand bytes of all tiles count a little by themselves: of two widths
     // that cost the same the wider one reads A less often (491520 x 96 x 96 with SnakeBeta: 16 columns 264 us, 96 columns 87).
@@ -1543,14 +1552,14 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   g.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES;
   g.lost = o.reserved & 2 ? 0 : -1;
   // (few rows and a costly epilogue: 39 rows of gated units 8.3 -> 7.5 us; without one the extra meeting costs 1 us more than it saves)
-  g.staged = g.splits > 1 || (g.mt == 1 && few && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
+  g.staged = g.parts > 1 || (g.mt == 1 && few && g.nt <= 2 * GP_SMS && (o.flags & (FQ3C_SWIGLU | FQ3C_GELU | FQ3C_SILU | FQ3C_SNAKE2)));
   g.vec16 = gemm_vec16(o) ? 1 : 0;
   const bool half = L.shape == GS_HALF;
-  const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = (g.kb + g.splits - 1) / g.splits;
+  const int sb = gp_stage_bytes(g.a_rows, g.bn), tiles = g.mt * g.nt, n_kb = (g.kb + g.parts - 1) / g.parts * g.per;
   // The MMA reads 128 rows of A also where the box has fewer: the last stage's are inside the allocation.  One tile per CTA needs no more stages than k-blocks,
-  // and a staged one's partial tile has to fit in them.
+  // and a staged one's partial tiles have to fit in them.
   const int room = (half ? GP_SMEM_HALF : GP_SMEM_MAX) - 1024, fit = std::min((room - GP_BAR_BYTES) / sb, (room - T_A_BYTES) / sb + 1);
-  const int part = (g.a_rows * gp_part_pitch(g.bn) * 4 + sb - 1) / sb;
+  const int part = (g.per * g.a_rows * gp_part_pitch(g.bn) * 4 + sb - 1) / sb;
   const bool once = g.staged || tiles <= GP_SMS * (half ? 2 : 1);
   g.stages = std::max(2, std::min(std::min(fit, 16), once ? std::max(n_kb, g.staged ? part : 0) : 16));
   L.smem = (size_t)std::max(g.stages * sb + GP_BAR_BYTES, (g.stages - 1) * sb + T_A_BYTES) + 1024;

@@ -10,10 +10,12 @@ struct GemmPlan {
   int stages;    // operand stages in shared memory
   int a_rows;    // rows of the A box: 128, or what a single row tile needs (multiple of 8; the accumulator rows behind it are never read)
   int mt, nt;    // row and column tiles
-  int splits;    // CTAs that share a tile's k-blocks: a cluster, its partial tiles meet in shared memory
+  int parts;     // runs of a tile's k-blocks that are summed by themselves, each in an accumulator of its own, and then added in order
+  int splits;    // CTAs that share a tile's parts: a cluster, its partial tiles meet in shared memory
+  int per;       // parts of a CTA: one or two (the last CTA may have one less)
   int kpt, kb;   // k-blocks per tap, in all
   int tail;      // MMAs (16 columns each) of a tap's last k-block
-  int acc_cols;  // tensor-memory columns of one accumulator (power of two); two of them unless splits > 1
+  int acc_cols;  // tensor-memory columns of one accumulator (power of two); two of them, of a staged tile as many as the CTA has parts
   int early_b;   // B is not written by the launches in front: its first stages are asked for before they have ended
   int vec16;     // the epilogue may move 16 columns of a row at a time
   int staged;    // the epilogue takes its tile from shared memory, spread over all threads: split sums, and few rows (a CTA has one tile then)
@@ -257,8 +259,8 @@ __device__ __noinline__ void poison(const fq3c_op& o, const int row, const int c
 // One CTA per SM (or two small ones) walks the tiles t = blockIdx.x, + gridDim.x, ..; a tile is 128 rows x bn columns.  The last warp asks for the operand
 // boxes up to `stages` k-blocks ahead, across tiles; the one before it issues the MMAs of tile n + 1 into the second accumulator while the others take tile n
 // through the epilogue.  What bounds that is latency (accumulator, residual, a chain of conversions per row), so an SM has sixteen such warps, of one CTA or of two:
-// with eight, 1900 x 6144 x 1024 with gated units took 33 us, with sixteen 24.  With splits > 1 a cluster of CTAs shares one tile: each takes a run of k-blocks, leaves its f32 partial tile in its
-// shared memory, and each then adds the partial tiles of a part of the rows in split order.
+// with eight, 1900 x 6144 x 1024 with gated units took 33 us, with sixteen 24.  A tile whose sums come in parts is a cluster's: each CTA takes one or two parts, leaves their f32 partial tiles in its
+// shared memory, and each then adds the partial tiles of a share of the rows in the parts' order.
 // The launch may begin before the ones in front of it have ended (programmatic dependent launch): nothing but B (early_b) is touched before
 // grid_dep_wait.
 template <int MINB, int EPI_WARPS>
@@ -277,8 +279,10 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int tiles = g.mt * g.nt, z = g.splits > 1 ? (int)(blockIdx.x % g.splits) : 0;
   const int t0 = g.splits > 1 ? (int)(blockIdx.x / g.splits) : (int)blockIdx.x, dt = g.staged ? tiles : (int)gridDim.x;
-  const int kb0 = (int)(((long)z * g.kb) / g.splits), kb1 = (int)(((long)(z + 1) * g.kb) / g.splits);
-  const int bufs = g.staged ? 1 : 2;
+  const int part0 = z * g.per, own = min(g.per, g.parts - part0);      // this CTA's parts: k-blocks kb0 .. kbm and, of two, kbm .. kb1
+  auto part_at = [&](const int p) { return p * g.kb / g.parts; };
+  const int kb0 = part_at(part0), kbm = part_at(part0 + 1), kb1 = part_at(part0 + own);
+  const int bufs = g.staged ? g.per : 2;
   const uint32_t cols = (uint32_t)(g.acc_cols * bufs);
 
   if (tid == 0) {
@@ -360,13 +364,13 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
     uint32_t st8 = 0, off = 0, ph = 0;      // 8 x stage, its memory / 16, parity
     bool there = true;
     int n = 0;
-    for (int t = t0; t < tiles && there; t += dt, ++n) {
+    for (int t = t0, k0 = kb0, k1 = kbm; t < tiles && there; ++n) {
       const int buf = n & 1;
       const uint32_t d = tmem + (uint32_t)(buf * g.acc_cols);
       if (n >= 2 && !gp_wait_all(acc_empty + 8u * buf, (uint32_t)((n / 2 - 1) & 1), dead, g.tries)) { there = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t acc = 0;
-      for (int m = kb1 - kb0, c = kb0 % g.kpt; m > 0 && there; c = 0) {
+      for (int m = k1 - k0, c = k0 % g.kpt; m > 0 && there; c = 0) {
         const int run = min(g.kpt - c, m);
         const bool tail = c + run == g.kpt && g.tail != TK / 16;      // the tap's last k-block has fewer columns
 #pragma unroll 1
@@ -398,6 +402,8 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
       }
       if (leader && there) umma_commit(acc_full + 8u * buf);
       __syncwarp();
+      if (k1 < kb1) { k0 = k1; k1 = kb1; }      // the CTA's other part
+      else t += dt;
     }
     if (!there) wait_ran_out();
   } else {
@@ -405,12 +411,35 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
     // warp w reads tensor-memory lanes 32 (w & 3) .. +31 (= rows of the tile); each four warps take a run of the 16-column pieces
     const int pieces = g.bn / 16, p0 = (warp >> 2) * pieces / GROUPS, p1 = ((warp >> 2) + 1) * pieces / GROUPS;
     const int r_in = (warp & 3) * 32 + lane;
-    const bool resid = g.vec16 && (o.flags & FQ3C_RESID) && !g.staged;
+    const bool resid = g.vec16 && (o.flags & FQ3C_RESID);
     float* par = reinterpret_cast<float*>(gbase + g.stages * sb + 512);
-    const bool params = g.vec16 && !g.staged && (o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_SNAKE2));
+    const bool params = g.vec16 && (o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_SNAKE2));
     int n = 0, par_n0 = -1;
+    if (g.staged) {      // the CTA's tile, once every product of it has ended: the partial tiles lie where its operands did
+      const bool rows = o.m_begin + (t0 % g.mt) * TM + (warp & 3) * 32 < o.M;
+      for (int h = 0; h < own; ++h) gp_wait_warp(acc_full + 8u * h, 0u, dead, g.tries);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int h = 0; h < own && rows; ++h) {
+        float* part = reinterpret_cast<float*>(gbase) + (size_t)(h * g.a_rows + r_in) * gp_part_pitch(g.bn);
+        const uint32_t ta = tmem + (uint32_t)(h * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int p = p0; p < p1; p += 2) {
+          uint32_t x[16], y[16];
+          const bool two = p + 1 < p1;
+          tmem_ld16(ta + p * 16, x);
+          if (two) tmem_ld16(ta + p * 16 + 16, y);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (r_in < g.a_rows) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              *reinterpret_cast<uint4*>(part + p * 16 + 4 * j) = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+              if (two) *reinterpret_cast<uint4*>(part + p * 16 + 16 + 4 * j) = make_uint4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+            }
+          }
+        }
+      }
+    } else
     for (int t = t0; t < tiles; t += dt, ++n) {
-      const int buf = bufs == 1 ? 0 : n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
+      const int buf = n & 1, n0 = (t / g.mt) * g.bn, m0 = o.m_begin + (t % g.mt) * TM;
       if (params && n0 != par_n0) {      // another column tile (rows go first): its parameters, when the epilogue warps have left the last one's
         par_n0 = n0;
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
@@ -434,7 +463,7 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
         if (resid && p < p1 && row < o.M && n0 + p * 16 < o.N) ld32(reinterpret_cast<const bf16*>(o.res) + (size_t)row * o.ldr + n0 + p * 16, x);
       };
       if (rows) { ask(p0, rx); ask(p0 + 1, ry); }
-      gp_wait_warp(acc_full + 8u * buf, (uint32_t)((bufs == 1 ? n : n / 2) & 1), dead, g.tries);
+      gp_wait_warp(acc_full + 8u * buf, (uint32_t)((n / 2) & 1), dead, g.tries);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ta = tmem + (uint32_t)(buf * g.acc_cols) + ((uint32_t)((warp & 3) * 32) << 16);
       if (rows)
@@ -449,17 +478,6 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
           }
-          if (g.staged) {
-            float* part = reinterpret_cast<float*>(gbase) + (size_t)r_in * gp_part_pitch(g.bn);
-            if (row < o.M) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                *reinterpret_cast<uint4*>(part + p * 16 + 4 * j) = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
-                if (two) *reinterpret_cast<uint4*>(part + p * 16 + 16 + 4 * j) = make_uint4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
-              }
-            }
-            continue;
-          }
           gp_epilogue(o, g, row, n0 + p * 16, x, rx, par + p * 16);
           ask(p + 2, rx);
           if (two) gp_epilogue(o, g, row, n0 + p * 16 + 16, y, ry, par + p * 16 + 16);
@@ -472,7 +490,7 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
   if (g.staged) {
     const int n0 = (t0 / g.mt) * g.bn, m0 = o.m_begin + (t0 % g.mt) * TM;
     const int pieces = g.bn / 8, items = min(TM, o.M - m0) * pieces;
-    const int i0 = (int)((long)items * z / g.splits), i1 = (int)((long)items * (z + 1) / g.splits);
+    const int i0 = items / 2 * z / g.splits * 2, i1 = items / 2 * (z + 1) / g.splits * 2;      // (a row has an even number of pieces)
     int lost = 0;
     if (g.splits > 1) {      // every CTA of the cluster comes here, also after a wait that ran out
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -486,29 +504,36 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
       __syncthreads();
       lost = *dead;
     }
-    for (int i = i0 + tid; i < i1; i += THREADS) {
-      const int r = i / pieces, p = i - r * pieces;
-      const uint32_t mine = base + (uint32_t)((r * gp_part_pitch(g.bn) + p * 8) * 4);
-      float4 q[8][2];      // every split's part is on its way before the first is added
+    // Two lanes share two pieces: each adds up the lower or the upper four columns of both, so that a warp reads whole rows, and they swap the finished sums
+    // (39 x 1024 x 2048 in eight parts 6.9 -> 6.3 us).
+    for (int b = i0 + warp * 32; b < i1; b += THREADS) {
+      const int i = min(b + lane, i1 - 1), r = i / pieces, p = i - r * pieces;
+      const uint32_t mine = base + (uint32_t)((r * gp_part_pitch(g.bn) + (p & ~1) * 8 + (lane & 1) * 4) * 4), slot = (uint32_t)(g.a_rows * gp_part_pitch(g.bn) * 4);
+      float4 q[8][2];      // every part is on its way before the first is added
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        if (s < g.splits) {
-          uint32_t far = mine;
-          if (g.splits > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(mine), "r"(s));
+        if (s < g.parts) {
+          uint32_t far = g.per == 2 && (s & 1) ? mine + slot : mine;
+          if (g.splits > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(far), "r"(g.per == 2 ? s >> 1 : s));
 #pragma unroll
           for (int j = 0; j < 2; ++j)
-            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q[s][j].x), "=f"(q[s][j].y), "=f"(q[s][j].z), "=f"(q[s][j].w) : "r"(far + 16u * j) : "memory");
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q[s][j].x), "=f"(q[s][j].y), "=f"(q[s][j].z), "=f"(q[s][j].w) : "r"(far + 32u * j) : "memory");
         }
       float a[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) a[j] = 0.f;
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        if (s < g.splits) {
+        if (s < g.parts) {
 #pragma unroll
           for (int j = 0; j < 2; ++j) { a[4 * j] += q[s][j].x; a[4 * j + 1] += q[s][j].y; a[4 * j + 2] += q[s][j].z; a[4 * j + 3] += q[s][j].w; }
         }
-      epilogue_row8(o, m0 + r, n0 + p * 8, a);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {      // the even lane keeps the first piece: its lower half, and the odd lane's upper one
+        const float got = __shfl_xor_sync(0xffffffffu, lane & 1 ? a[j] : a[4 + j], 1);
+        if (lane & 1) a[j] = got; else a[4 + j] = got;
+      }
+      if (b + lane < i1) epilogue_row8(o, m0 + r, n0 + p * 8, a);
     }
     if (__syncthreads_or(lost))
       for (int i = i0 + tid; i < i1; i += THREADS) poison(o, m0 + i / pieces, n0 + i % pieces * 8, 8);

@@ -43,3 +43,22 @@ def test_product_residual_snake_and_units(M, N, cin, offs, split):
     unit = gate * torch.sigmoid(gate) * up
     slack = 1.1 * sums[:, 0::2] * up.abs() + (gate * torch.sigmoid(gate)).abs() * sums[:, 1::2]      # silu's slope is at most 1.1
     assert ((out.double() - unit).abs() <= 1.01 * 2.0 ** -8 * unit.abs() + slack + 2.0 ** -20 * unit.abs() + 1e-6).all()
+
+
+# rows, columns, inputs, parts: two to eight of them, one and two to a CTA, runs of k-blocks of unequal length, the last CTA with one part less
+@pytest.mark.parametrize("M,N,K,parts", [(39, 1024, 2048, 8), (90, 1024, 2048, 8), (73, 1024, 3072, 8), (128, 1024, 3072, 8), (33, 1024, 1792, 7), (33, 1024, 1536, 6), (17, 1024, 1280, 5), (140, 1024, 3072, 4), (64, 2048, 6144, 4),
+                                         (262, 1024, 8192, 3), (33, 4096, 2048, 2), (200, 2048, 6144, 2), (8, 40, 1536, 6), (5, 1000, 2000, 8)])
+def test_sums_come_in_parts_and_in_their_order(M, N, K, parts):
+    """A split product is the f32 sum, in order, of the whole products of its runs of 64 inputs."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    A, B = torch.randn(M, K, device="cuda", generator=g).bfloat16(), (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).bfloat16()
+    flags = 64 | 1024      # f32, as it is
+    split, whole = torch.zeros(M, N, device="cuda"), torch.zeros(M, N, device="cuda")
+    launch([make_op(A, B, split, M, N, K, flags=flags, ws=torch.zeros(8 * M * (N + 8), device="cuda"))])
+    blocks = (K + 63) // 64
+    for p in range(parts):
+        lo, hi = 64 * (p * blocks // parts), min(K, 64 * ((p + 1) * blocks // parts))
+        part = torch.zeros(M, N, device="cuda")
+        launch([make_op(A[:, lo:hi].contiguous(), B[:, lo:hi].contiguous(), part, M, N, hi - lo, flags=flags)])
+        whole += part
+    assert torch.equal(split, whole)
