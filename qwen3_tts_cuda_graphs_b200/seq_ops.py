@@ -49,6 +49,7 @@ class StepBuilder:
         self.plan = _Plan()
         self._pool: Dict[tuple, torch.Tensor] = {}
         self._wide: set = set()      # buffers whose last columns are scratch
+        self._branched = False       # between branch(0) and branch(2)
 
     # ---- buffers --------------------------------------------------------------------------------
     def buf(self, name: str, rows: int, cols: int, dtype=torch.float32) -> torch.Tensor:
@@ -617,22 +618,26 @@ class StepBuilder:
         f32 router weights take the f32 rows (true 32-bit product); bf16 ones take the bf16 rows, whose products with the weights
         are exact in f32 and are summed in f32.  c.act == "relu2": max(., 0)^2 instead of gelu.  c.router_bias: router_b f32 added
         to the logits.  c.shared_gate: the router matrix carries one more row (and router_b one more entry, zero) whose product, through
-        a sigmoid, multiplies the shared expert's output."""
+        a sigmoid, multiplies the shared expert's output.  The shared expert runs on the list's side stream, beside the router, the grouping and
+        the experts, unless a branch of the caller's has taken it: then it follows the experts."""
         M, n, top, E = self.M, c.routed, c.top, c.experts
         width = x32.shape[1]
         zc = w["router"].shape[0]        # n, or n + 1 with the shared expert's gate row
         assert zc == n + (1 if c.shared_gate else 0)
+
+        def shared():
+            up = w["shared_up"]
+            if c.gated:
+                sa = self.linear(xop, up, self.buf("moe.sa", M, up.shape[0] // 2, self.adt), glu=True)
+            else:
+                sa = self.linear(xop, up, self.buf("moe.sa", M, up.shape[0], self.adt), gelu=c.act != "relu2", relu2=c.act == "relu2")
+            return self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
+
         sh = None
-        if w.get("shared_up") is not None:      # beside the router, the sort and the experts: 701 rows 103 -> 93 us
+        beside = w.get("shared_up") is not None and not self._branched      # 701 rows 103 -> 93 us
+        if beside:
             self.branch(0)
-        if w.get("shared_up") is not None and c.gated:
-            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0] // 2, self.adt), glu=True)
-            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
-        elif w.get("shared_up") is not None:
-            sa = self.linear(xop, w["shared_up"], self.buf("moe.sa", M, w["shared_up"].shape[0], self.adt), gelu=c.act != "relu2",
-                             relu2=c.act == "relu2")
-            sh = self.linear(sa, w["shared_down"], self.buf("moe.sh", M, width))
-        if sh is not None:
+            sh = shared()
             self.branch(1)
         z = self.linear(x32 if w["router"].dtype == torch.float32 else xop, w["router"], self.buf("moe.z", M, zc),
                         bias=w.get("router_b") if c.router_bias else None)
@@ -664,8 +669,10 @@ class StepBuilder:
         y = self.buf("moe.y", M * top, width)
         self._op(K_GGEMM, M=M * top, N=width, K=ff, i0=E, A=act, lda=ff, B=w["down"], p0=seg, C=y, ldc=width,
                  flags=F_OUT_F32 | (F_F32 if f32 else 0))
-        if sh is not None:
+        if beside:
             self.branch(2)
+        elif w.get("shared_up") is not None:
+            sh = shared()
         kw = dict(M=M, N=width, i0=top, i1=E, A=y, lda=width, B=x32, ldr=width, p0=ids, ws=pos, C=out, ldc=out.shape[1])
         if not c.weight_input:
             kw["p1"] = wt
@@ -692,7 +699,9 @@ class StepBuilder:
 
     def branch(self, what: int):
         """0: the following ops go to a side stream; 1: to the main stream again, beside it; 2: the main stream waits for the side stream.
-        The two parts must not share scratch buffers."""
+        The two parts must not share scratch buffers.  A list has one side stream: a mechanism that would branch by itself (moe_ff) stays on the stream
+        it is called on between 0 and 2."""
+        self._branched = what == 0 or (what == 1 and self._branched)
         self._op(K_BRANCH, M=1, i0=what)
 
     def commit(self):
