@@ -590,7 +590,7 @@ struct SeqTail { int n; fq3c_op op[2]; };
 
 // One output row with few rows in flight (decode: M <= 8): a warp per output column streams its weight row once, 16 bytes per
 // lane and load, and dots it with every A row (f32 or bf16 in shared memory as f32).  Bound by latency up to a few MB of weights: the launch, one trip to the weights
-// (two batches of loads leave before the rows are staged) and the reduction.
+// (the first loads leave before the rows are staged) and the reduction.
 // TAIL: lane m goes on with entry (m, n) of row m through the ops of `tail`, with their own arithmetic: each was a launch of its own of 2 us, of which a decoded token of
 // four layers had sixteen.
 template <typename TA, typename TB, bool TAIL = false>
@@ -605,18 +605,13 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
   constexpr int VEC = 16 / sizeof(TB);
   constexpr int U = 4;                 // 16-byte weight loads a lane keeps in flight
   const bool vec = ((reinterpret_cast<uintptr_t>(w) & 15) == 0) && (g.K % VEC == 0);
-  // the first weight loads leave before the rows are staged: the latencies overlap
-  uint4 raw[U], nxt[U];
+  // the first weight loads leave before the rows are staged: the two latencies overlap
+  uint4 raw[U];
   if (vec && n < g.N) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = (lane + 32 * u) * VEC;
       raw[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = (lane + 32 * (U + u)) * VEC;
-      nxt[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
     }
   }
   for (int m = 0; m < g.M; ++m) stage_row_f32<TA>(xs + (size_t)m * g.K, Ap + (size_t)m * g.lda, g.K, threadIdx.x, blockDim.x);
@@ -627,11 +622,11 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
   for (int m = 0; m < 8; ++m) acc[m] = 0.f;
   if (vec) {
     for (int k0 = lane * VEC; k0 < g.K; k0 += 32 * U * VEC) {
-      uint4 fut[U];
+      uint4 nxt[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {      // the batch behind the next is on its way while this one is used
-        const int k = k0 + 32 * (2 * U + u) * VEC;
-        fut[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+      for (int u = 0; u < U; ++u) {      // the next batch is on its way while this one is used (and the one behind it, too: 1 x 4096 x 2048 of f32 8.5 -> 12.2 us)
+        const int k = k0 + 32 * (U + u) * VEC;
+        nxt[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -654,7 +649,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
         }
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) { raw[u] = nxt[u]; nxt[u] = fut[u]; }
+      for (int u = 0; u < U; ++u) raw[u] = nxt[u];
     }
   } else {
     for (int k = lane; k < g.K; k += 32) {
