@@ -1066,7 +1066,7 @@ __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
 // writes its own rows of the cache: one launch in place of two, and the rows in `A` stay as the product left them.  39 rows of
 // 16 heads 8.2 -> 5.6 us; the codec's attention (16 heads of 64, window 72) 33 rows 7.6 -> 3.8, 256 rows 32.0 -> 12.9, one row behind 71 others 14.4 -> 4.3.
 constexpr int GP_SMS = 148;
-constexpr int AR_PROMPT_ROWS = 144, AR_WARPS = 16, AR_SMEM_MAX = 128 * 1024;
+constexpr int AR_WARPS = 16, AR_SMEM_MAX = 128 * 1024;
 struct AttnRows { int rb, span, sp; size_t smem; };      // rows of a CTA, keys it may stage, pitch of its scores
 __host__ __device__ constexpr int ar_k_pitch(int d) { return d * 2 + 16; }      // bytes
 AttnRows attn_rows_plan(const fq3c_op& o, const bool prompt) {
@@ -1609,13 +1609,16 @@ bool attn_rows_takes(const fq3c_op& o, const bool prompt) {
   return (o.i2 == 64 || o.i2 == 128) && o.i1 > 0 && o.i0 > 0 && o.i0 % o.i1 == 0 && o.i1 <= 65535 && o.K > 0 && o.taps >= 0 && o.lda % vec == 0 && o.ldc % vec == 0 &&
          !off(o.A, 2 * vec) && !off(o.C, 2 * vec) && attn_rows_plan(o, prompt).smem <= AR_SMEM_MAX && device_attrs_ready();
 }
+// The rows of a prompt from which its attention goes to tcgen05, where that takes the addresses.  Below them it is on the CUDA cores, by itself (fq3c_attn_prefill_kernel) or, where
+// the rows are scratch, in one launch with the norm in front: the same bits, so that they do not depend on who else reads the rows.  One launch against the two with tcgen05:
+// 64 rows of 16 heads over 8 8.0 and 10.8 us, 84 10.8 and 11.0, 90 11.0 and 11.0, 97 11.6 and 11.1, 112 14.5 and 11.3; of 32 over 8 64 rows 11.0 and 14.8 (the kernel by itself),
+// 80 15.3 and 11.6; of 14 over 2 66 rows 8.8 and 10.3, 80 12.3 and 10.4 (15.2 by itself); of 8 112 rows 10.4 and 11.2, 128 12.5 and 11.6; of 4 112 rows 8.7 and 10.5.
+bool attn_prompt_many(const fq3c_op& o) { return o.M > 112 || (o.M > 64 && (long)o.M * o.M * o.i0 > 115000); }
 // `n` (q / k norm, rotation, cache rows) and the prompt attention `o` behind it, where the rows that `n` would rewrite are scratch to everyone else (reserved bit 0)
-// Against two launches (behind these lines the second is the kernel on tcgen05): 39 rows of 16 heads 5.7 and 8.1 us, 100 11.6 and 13.1, 112 14.3 and 13.3; 64 of 32 11.0
-// and 14.8, 80 15.2 and 13.5; 144 of 8 14.2 and 14.5, of 4 11.7 and 12.9.
 bool attn_rows_takes_prompt(const fq3c_op& n, const fq3c_op& o) {
   auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) != 0; };
   return (n.reserved & 1) && o.kind == FQ3C_ATTN && (o.flags & 1) && o.A == n.A && o.lda == n.lda && o.M == n.M && o.i0 == n.i0 && o.i1 == n.i1 && o.i2 == 128 && o.taps == 0 && !o.p0 &&
-         o.M <= AR_PROMPT_ROWS && (long)o.M * o.M * o.i0 <= 165000 && !off(n.p0) && !off(n.p1) && !off(n.B) && !off(n.bias) && !off(n.C) && !off(n.C2) && attn_rows_takes(o, true);
+         !attn_prompt_many(o) && !off(n.p0) && !off(n.p1) && !off(n.B) && !off(n.bias) && !off(n.C) && !off(n.C2) && attn_rows_takes(o, true);
 }
 
 // ---- sequence-model ops: launch logic ---------------------------------------------------------------------------------------
@@ -2556,11 +2559,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
           a.tries = o.reserved & 2 ? GP_TRIES_TEST : GP_TRIES; a.lost = (o.reserved >> 1) & 1;
           a.ldq = a.ldk = a.ldv = o.lda; a.H = o.i0; a.G = o.i1; a.M = o.M; a.scale = 0.08838834764831845f; a.window = o.K < o.M ? o.K : 0; a.out = o.C; a.ldo = o.ldc;
-          // Few rows are faster in the kernel below (a warp per query and head, no tile to stage), whose time grows with rows^2 x heads.  Launched early as both
-          // are, it against this one: 81 rows of 16 heads 10.2 and 10.9 us, of 32 14.1 and 10.9, of 14 9.8 and 11.0; 90 of 16 11.5 and 10.9, of 14 10.0 and 11.1;
-          // 100 of 14 12.0 and 11.2, of 8 10.7 and 10.3, of 1 8.9 and 10.3; 128 of 8 12.4 (not early) and 11.3
-          const bool many = o.M > 112 || (o.M > 64 && (long)o.M * o.M * o.i0 > 115000);
-          if (many && attn_tc_takes(a, AT_PROMPT)) {
+          if (attn_prompt_many(o) && attn_tc_takes(a, AT_PROMPT)) {
             launch_attn_tc(a, AT_PROMPT, s, after);
             break;
           }

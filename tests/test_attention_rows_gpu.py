@@ -64,7 +64,7 @@ def test_windows_and_history(M, H, G, d, window, hist, known):
         assert torch.equal(tail, out[cut:M])
 
 
-@pytest.mark.parametrize("M,H,G,pos0", [(1, 16, 8, 0), (17, 16, 8, 0), (39, 16, 8, 3), (64, 4, 4, 0), (100, 14, 2, 0), (101, 16, 8, 0), (102, 16, 8, 0), (130, 9, 1, 0), (144, 4, 4, 0), (145, 4, 4, 0), (30, 3, 1, 0)])
+@pytest.mark.parametrize("M,H,G,pos0", [(1, 16, 8, 0), (17, 16, 8, 0), (39, 16, 8, 3), (64, 4, 4, 0), (84, 16, 8, 0), (85, 16, 8, 0), (90, 14, 2, 0), (91, 14, 2, 0), (112, 8, 8, 0), (113, 4, 4, 0), (64, 32, 8, 0), (65, 32, 8, 0), (100, 14, 2, 0), (101, 16, 8, 0), (102, 16, 8, 0), (130, 9, 1, 0), (144, 4, 4, 0), (145, 4, 4, 0), (30, 3, 1, 0)])
 def test_norm_rotation_and_cache_in_the_same_launch(M, H, G, pos0):
     from qwen3_tts_cuda_graphs_b200 import codec as K
 
@@ -80,10 +80,10 @@ def test_norm_rotation_and_cache_in_the_same_launch(M, H, G, pos0):
         n.kind, n.M, n.N, n.A, n.lda, n.a_rows, n.i0, n.i1, n.i2, n.f0, n.reserved = 8, M, x.shape[1], rows.data_ptr(), x.shape[1], M, H, G, pos0, 1e-6, scratch
         n.p0, n.p1, n.B, n.bias, n.C, n.C2, n.ldc, n.col_mod = (*(t.data_ptr() for t in (gq, gk, cos, sin, ck, cv)), ck.shape[1], x.shape[1])
         launches = launch(n, attn_op(rows, out, M, H, G, 128, 4096, flags=1))
-        assert launches == (1 if scratch and M <= 144 and M * M * H <= 165000 else 2)
+        assert launches == (1 if scratch and (M <= 64 or (M <= 112 and M * M * H <= 115000)) else 2)      # behind that line tcgen05 takes the rows, scratch or not
         got.append((rows, ck, cv, out))
-    (turned, ck, cv, _), (_, ck1, cv1, out) = got
-    assert torch.equal(ck, ck1) and torch.equal(cv, cv1)
+    (turned, ck, cv, apart), (_, ck1, cv1, out) = got
+    assert torch.equal(ck, ck1) and torch.equal(cv, cv1) and torch.equal(apart, out)
     want, bound = exact(turned, M, H, G, 128, 4096)
     assert ((out.double() - want).abs() <= bound).all()
 
