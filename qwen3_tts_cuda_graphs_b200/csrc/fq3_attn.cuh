@@ -9,7 +9,8 @@ struct AttnArgs {
   const bf16 *k, *v;        // row j of key / value head g at j * ld + g * 128
   long ldq, ldk, ldv;
   int H, G, M;
-  int groups;               // row groups per CTA: 2, or 1 while the CTAs of one group each are a single wave
+  int groups;               // row groups per CTA: 1 or 2
+  int two_from;             // > 0: launched with one, but behind more positions than these a CTA takes two and every other one leaves
   const int* p0;            // position of query 0 (device), or null: 0
   float scale, cap, mult;   // mult != 0 multiplies the output
   int window, keep, chunk;  // 0: none
@@ -118,7 +119,7 @@ __device__ __noinline__ void at_row_again(const AttnArgs& a, const int m, const 
   at_store(a, (size_t)m * a.ldo + (size_t)head * 128 + col, out);
 }
 
-// A CTA takes two groups of 128 rows (a.groups = 1: one) of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
+// A CTA takes two groups of 128 rows (or one: launch_attn_tc) of one key / value head; a row is a (query, head of the group) pair, so that all heads sharing the keys score the same
 // staged tile.  Warps 0-7 and 8-15: two threads per row of group 0 and 1, 64 keys of a tile each; warps 16-18 stage key and value tiles of 128 positions (two
 // stages); warp 19 issues the MMAs.  Per group and tile: S = Q K^T into tensor memory; the row's threads scale, cap and mask its 128 scores, agree on the
 // maximum, take 2^(score log2 e - reference) and write every weight as a bf16 pair hi + mid (16 mantissa bits) over S; O += hi V + mid V with the weights read from
@@ -128,8 +129,8 @@ __device__ __noinline__ void at_row_again(const AttnArgs& a, const int m, const 
 // the row's output is rescaled in tensor memory.  Tiles outside every row's window, chunk and kept positions are not fetched.
 // Bound by the chain scores -> maximum -> weights -> output of a group (24 MMAs of 64 cycles a tile are about half of it; the other group fills part of the
 // rest) and, with a cap, by the special-function unit (three a score).
-// Without a wave's worth of row groups a CTA has one, so that no group waits for the other's issue slots.  128 prompt rows of 16 heads over 8 11.3 us, 262 14.9,
-// 700 26 (a warp per query and head: 13.8, 36, 184).
+// Without a wave's worth of row groups a CTA has one, so that no group waits for the other's issue slots; one group's next scores are issued in front of its values.
+// A tile takes one group some 3.7 us with a cap, two 6.0.  Norm and attention of 85 prompt rows of 16 heads over 8 10.9 us, 144 13.3, 262 17.0.
 template <int MODE>
 __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __grid_constant__ AttnArgs a) {
   extern __shared__ unsigned char at_raw[];
@@ -140,6 +141,15 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   uint32_t* words = reinterpret_cast<uint32_t*>(gbase + 6 * AT_TILE + 128);
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  int groups = a.groups, gx = gridDim.x;
+  if (a.two_from > 0) {
+    grid_dep_wait();
+    if (*a.p0 > a.two_from) {
+      groups = 2;
+      gx = (gx + 1) / 2;
+      if ((int)blockIdx.x >= gx) return;
+    }
+  }
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(q_full + 8u * i, 8);
@@ -165,13 +175,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   grid_dep_wait();
 
   const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
-  const bool one = a.groups == 1;      // its tiles take the score columns of both groups in turn
-  const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * a.groups * QB;   // the last queries (most keys) start first
+  const bool one = groups == 1;      // its tiles take the score columns of both groups in turn
+  const int m0 = (gx - 1 - (int)blockIdx.x) * groups * QB;   // the last queries (most keys) start first
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
-    nq[g] = g < a.groups ? max(0, min(QB, a.M - m0 - g * QB)) : 0;
+    nq[g] = g < groups ? max(0, min(QB, a.M - m0 - g * QB)) : 0;
     first[g] = P + m0 + g * QB;
     last[g] = first[g] + nq[g] - 1;
     tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
@@ -180,7 +190,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     tlo[g] = lo / AT_KEYS;
   }
   const int tkeep = a.window > 0 && a.chunk <= 0 ? (a.keep + AT_KEYS - 1) / AT_KEYS : 0;
-  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + a.groups * QB) - 1;
+  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + groups * QB) - 1;
   auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
 
   if (warp == 19) {

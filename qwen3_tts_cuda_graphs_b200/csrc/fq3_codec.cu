@@ -1587,8 +1587,17 @@ bool attn_tc_takes(const AttnArgs& a, const int mode) {
 }
 void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after) {
   const int group = 128 / (a.H / a.G);
-  // (with a cap the special-function unit sets the pace, which a second group cannot fill: 2048 rows of 16 heads over 4, 256 CTAs of one group 87 us, 128 of two 96)
-  a.groups = (long)((a.M + group - 1) / group) * a.G <= (mode == AT_CAP ? 2 * GP_SMS : GP_SMS) ? 1 : 2;
+  const long ctas = (long)((a.M + group - 1) / group) * a.G;      // of one group each
+  a.groups = ctas <= GP_SMS ? 1 : 2;
+  a.two_from = 0;
+  // With a cap the special-function unit sets the pace, which a second group fills little: two groups take 1.55 times one's time.  So one pays for some more CTAs than SMs, where
+  // the first rows' short ones make room for the others: without a window, few positions in front of the rows, and the more so the fewer key heads the rows are spread over.  Two
+  // groups against one, 16 heads over 4: 1300 rows (164 CTAs) 67 and 44 us, behind 1500 positions 132 and 112, behind 4000 238 and 246; 2048 (256) 101 and 91, behind 500 122 and
+  // 118, behind 1500 166 and 172; of 32 heads over 8 1100 rows (280) 61 and 66, of 16 over 16 1900 (240) 85 and 94; under a window of 256 1800 rows (228) 31 and 36.
+  if (mode == AT_CAP && a.groups == 2 && a.window <= 0 && a.chunk <= 0 && ctas <= (a.G <= 4 ? 256 : 168)) {
+    a.groups = 1;
+    if (a.p0) a.two_from = a.G <= 4 && ctas <= 200 ? a.M / 4 * 3 : a.M / 4;
+  }
   const int per = a.groups * group;
   const dim3 grid((a.M + per - 1) / per, a.G);
   if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);

@@ -95,7 +95,10 @@ def test_prompt_weights_keep_32_bits():
 CASES = [(9, 0, 4, 2, {}), (100, 0, 4, 1, {}), (300, 77, 6, 2, {}), (128, 128, 16, 4, dict(cap=50.0, sink=True, gate=1)), (513, 300, 16, 4, dict(cap=50.0, sink=True)),
          (200, 300, 8, 2, dict(window=64)), (200, 300, 8, 2, dict(window=64, keep=5, dist=True, cap=50.0)), (128, 128, 3, 1, dict(window=130, keep=200)), (400, 0, 8, 8, dict(window=1)),
          (700, 129, 4, 4, dict(chunk=100, sink=True)), (700, 129, 4, 4, dict(chunk=1000, gate=2)), (260, 260, 12, 4, dict(dist=True, spread=4.0)), (300, 0, 2, 2, dict(spread=8.0)), (40, 700, 2, 1, dict(rising=True)),
-         (1300, 100, 16, 16, {}), (1285, 33, 16, 16, dict(window=300, keep=2)), (33, 0, 8, 2, dict(cap=50.0)), (17, 111, 4, 4, {}), (9, 7, 1, 1, {})]
+         (1300, 100, 16, 16, {}), (1285, 33, 16, 16, dict(window=300, keep=2)), (33, 0, 8, 2, dict(cap=50.0)), (17, 111, 4, 4, {}), (9, 7, 1, 1, {}),
+         # with a cap and more row groups than SMs: one a CTA, two because of the positions in front, two from the start (a window; too many), an odd number of them, scores that climb
+         (2048, 0, 16, 4, dict(cap=50.0)), (2048, 513, 16, 4, dict(cap=50.0)), (1300, 200, 16, 4, dict(cap=50.0, rising=True)), (1185, 900, 16, 4, dict(cap=50.0, sink=True, gate=2)),
+         (1500, 300, 16, 4, dict(cap=50.0, window=700)), (1300, 0, 32, 32, dict(cap=50.0)), (2433, 100, 8, 2, dict(cap=50.0)), (1210, 20, 8, 8, dict(cap=50.0, gate=1)), (600, 151, 32, 8, dict(cap=50.0, rising=True))]
 
 
 @pytest.mark.parametrize("rows, first, heads, kv, opt", CASES)
