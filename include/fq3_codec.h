@@ -29,7 +29,9 @@ enum fq3c_kind {
                          which the last min(*p0, taps) are valid (p0 = device int32: positions decoded so far).
                          flags bit 0 (ABI 5): prompt-prefill form — head_dim 128, no history rows, the same rounding points,
                          fp32 weights (24 bits), exponentials within 2 ulp, fp32 sums in another order: tcgen05 above 64-112 rows, by heads (M not
-                         limited), below that (and, M <= 2048, for addresses the former does not take) a two-phase kernel on the CUDA cores */
+                         limited), below that (and, M <= 2048, for addresses the former does not take) a two-phase kernel on the CUDA cores, or, behind a
+                         QKNORM_ROPE_KV whose rows are scratch, one launch for both ops with the same bits.  FQ3C_ATTN_PREFILL=0 in the environment: none of
+                         these, the kernels of every other FQ3C_ATTN */
   FQ3C_DWCONV = 5,    /* depthwise causal conv k=taps: C[m,c] = bias[c] + sum_j B(f32)[c,j] A[m-(taps-1)+j, c]; rows down
                          to -i0 in front of A are history rows (stateful decode), further back reads as zero        */
   FQ3C_LAYERNORM = 6, /* C = layernorm(A) * scale + bias (f32), eps=f0                                      */

@@ -1606,6 +1606,12 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
   else launch_after(fq3c_attn_tc_kernel<AT_DIST>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
 }
 
+// FQ3C_ATTN_PREFILL=0: no kernel of its own for a prompt's attention (flags bit 0), nor one launch with the norm in front: the op by itself, as any other
+bool prompt_kernels() {
+  static const bool on = [] { const char* e = getenv("FQ3C_ATTN_PREFILL"); return e == nullptr || atoi(e) != 0; }();
+  return on;
+}
+
 // ---- attention of few rows or a short window -----------------------------------------------------------------------------------
 // What fq3c_attn_rows_kernel's vector accesses and shared memory ask for; grid.y is the head.  By itself it pays from nine keys in sight on: fq3c_attn_kernel fetches up to
 // eight in two trips (16 heads of 64: 1 row 1.7 and 2.7 us, 8 rows 2.8 and 3.2, 9 rows 3.3 and 3.2; a window of 8, 33 rows 3.0 and 3.6, 600 rows 8.9 and 13.0), and from
@@ -2561,8 +2567,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
       case FQ3C_ROPE: launch_after(fq3c_rope_kernel, o.M, 256, 0, s, after, 1, o); break;
       case FQ3C_ATTN: {
         if (o.i2 > 128) return fail("attn: head_dim > 128");
-        static int use_apf = -1;
-        if (use_apf < 0) { const char* e5 = getenv("FQ3C_ATTN_PREFILL"); use_apf = (e5 == nullptr || atoi(e5) != 0) ? 1 : 0; }
+        const bool use_apf = prompt_kernels();
         if (use_apf && (o.flags & 1) && o.i2 == 128 && o.taps == 0 && !o.p0) {
           AttnArgs a{};
           a.q = o.A; a.k = reinterpret_cast<const bf16*>(o.A) + (size_t)o.i0 * 128; a.v = a.k + (size_t)o.i1 * 128;
@@ -2600,7 +2605,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
       }
       case FQ3C_QKNORM_ROPE_KV: {
         if (o.lda % 4 || !o.C || !o.C2 || !o.p0 || !o.p1 || !o.B || !o.bias) return fail("qknorm_rope_kv: missing operand");
-        if (i + 1 < n_ops && attn_rows_takes_prompt(o, ops[i + 1])) {      // with the attention behind it in one launch
+        if (i + 1 < n_ops && prompt_kernels() && attn_rows_takes_prompt(o, ops[i + 1])) {      // with the attention behind it in one launch
           const fq3c_op& at = ops[++i];
           const AttnRows r = attn_rows_plan(at, true);
           launch_after(fq3c_attn_rows_kernel<128, true>, dim3((unsigned)((at.M + r.rb - 1) / r.rb), (unsigned)at.i1), AR_WARPS * 32, r.smem, s, after, 1, at, o, r.rb, r.span, r.sp);

@@ -1,4 +1,8 @@
 """Attention of few rows or a short window (one CTA stages what its rows see), alone and together with the q / k norm, rotation and cache rows in front of it."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -141,3 +145,28 @@ def test_prompt_in_one_launch_has_the_bits_of_two(M, H, G):
         assert launch(n, attn_op(rows, out, M, H, G, 128, 4096, flags=1)) == 2 - scratch
         got.append((ck, cv, out))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def switched_off():
+    """In a process with FQ3C_ATTN_PREFILL=0: two launches, and the attention has the bits of one that is no prompt's."""
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    for M, H, G in ((39, 16, 8), (100, 16, 8), (150, 4, 4)):
+        g = torch.Generator(device="cuda").manual_seed(M)
+        rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g).bfloat16()  # noqa: E731
+        x, gq, gk, cos, sin = rand(M, (H + 2 * G) * 128), rand(128), rand(128), torch.ones(M, 128, device="cuda").bfloat16(), torch.zeros(M, 128, device="cuda").bfloat16()
+        ck, cv, out, want = *(torch.zeros(G, M, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2)), *(torch.zeros(M, H * 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        n = K.Op()
+        n.kind, n.M, n.N, n.A, n.lda, n.a_rows, n.i0, n.i1, n.f0, n.reserved = 8, M, x.shape[1], x.data_ptr(), x.shape[1], M, H, G, 1e-6, 1
+        n.p0, n.p1, n.B, n.bias, n.C, n.C2, n.ldc, n.col_mod = (*(t.data_ptr() for t in (gq, gk, cos, sin, ck, cv)), M, x.shape[1])
+        assert launch(n, attn_op(x, out, M, H, G, 128, 4096, flags=1)) == 2
+        launch(attn_op(x, want, M, H, G, 128, 4096))
+        assert torch.equal(out, want)
+    print("two launches each")
+
+
+def test_the_switch_covers_the_launch_with_the_norm():
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", "import sys; sys.path[:0] = [%r, %r]; import test_attention_rows_gpu as t; t.switched_off()" % (here, os.path.dirname(here))],
+                       env=dict(os.environ, FQ3C_ATTN_PREFILL="0"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "two launches each" in r.stdout, r.stderr[-2000:]
