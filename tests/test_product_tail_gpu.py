@@ -75,3 +75,38 @@ def test_same_bits_as_one_by_one(M, N, Kd, f32, pad, what):
     assert fused == (launches if apart else 2 if what == "mix over its slices" else 1)
     if what not in ("shifted", "mix over its slices"):
         assert all(torch.equal(after[k].float(), one[k].float()) for k in after)
+
+
+# overlaps that the ops define one by one: of entry with the same entry (one launch), and of entries with others', where the launches stay apart
+OVERLAPS = {"mix in a slice it reads": 1, "next norm over the residual": 1, "mix over the residual, one entry on": 2, "mix over the first norm's weights": 2, "weights in the product's row": 2, "mix weights in the first norm's copy": 2}
+
+
+@pytest.mark.parametrize("M,N,Kd,f32", [(1, 1024, 1024, False), (3, 1000, 2080, False), (4, 24, 40, False), (8, 130, 512, True), (1, 96, 100, True)])
+@pytest.mark.parametrize("what", list(OVERLAPS))
+def test_overlapping_buffers_have_the_values_of_one_by_one(M, N, Kd, f32, what):
+    ops, b = build(M, N, Kd, f32, "xielu" if what == "weights in the product's row" else "mix", 0)
+    _, dyt, mix = ops if len(ops) == 3 else (*ops, None)
+    b["res"] = torch.randn(M * N + 8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(N))      # with room behind the rows
+    if mix is not None:
+        dyt.res = b["res"].data_ptr()
+    if what == "mix in a slice it reads":
+        mix.C = b["hist"][1].data_ptr()
+    if what == "next norm over the residual":
+        mix.norm_out = b["res"].data_ptr()
+    if what == "mix over the residual, one entry on":
+        mix.C = b["res"].data_ptr() + 4
+    if what == "mix over the first norm's weights":      # (entries whose norm may still be to come)
+        b["big"] = torch.randn(M * N + 2 * N, device="cuda")
+        dyt.norm_w, mix.C = b["big"].data_ptr(), b["big"].data_ptr()
+    if what == "weights in the product's row":
+        dyt.p0 = b["y"].data_ptr() + 4 * (N - 2)
+    if what == "mix weights in the first norm's copy":      # two bf16 entries are a weight
+        mix.p0 = b["out16"].data_ptr()
+    keep = {k: t.clone() for k, t in b.items()}
+    apart = run(ops, False)
+    after = {k: t.clone() for k, t in b.items()}
+    for _ in range(5):
+        for k, t in keep.items():
+            b[k].copy_(t)
+        assert run(ops, True) == OVERLAPS[what] <= apart
+        assert all(torch.equal(after[k].nan_to_num(3.0), b[k].nan_to_num(3.0)) for k in after)
