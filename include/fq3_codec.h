@@ -291,6 +291,9 @@ int fq3c_abi_version(void);
 const char* fq3c_last_error(void);
 /* Launch every op in order on `stream` (no synchronisation). Returns 0 or a negative error code. */
 int fq3c_run(const fq3c_op* ops, int n_ops, void* stream);
+/* How a GEMM op would be launched on the persistent tcgen05 kernel (host arithmetic only): out[0] = 0 one CTA per SM with sixteen epilogue warps, 1 one with eight, 2 two with
+ * eight each; out[1..7] = columns of a tile, row tiles, column tiles, parts that a tile's sums come in, CTAs that share a tile, stages, CTAs.  Ops of other kernels: an error. */
+int fq3c_gemm_plan(const fq3c_op* op, int32_t* out);
 /* number of kernel launches issued so far by this process through fq3c_run / fq3c_graph_launch */
 int64_t fq3c_launch_count(void);
 /* ABI 11: nonzero when a kernel's bounded wait for its own copies or products ran out on the current device (its outputs are NaN); synchronises */

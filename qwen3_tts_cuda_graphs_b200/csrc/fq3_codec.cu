@@ -1567,6 +1567,22 @@ GemmLaunch gemm_plan(const fq3c_op& o) {
   return L;
 }
 
+// Which products go to the tensor pipe, and of those to the persistent kernel.  One k-block is enough: its vectorised epilogue beats the mma.sync kernel even at K = 96.
+bool gemm_on_tc(const fq3c_op& o) {
+  static const bool on = [] { const char* e = getenv("FQ3C_TCGEN05"); return e == nullptr || atoi(e) != 0; }();
+  static const int min_k = [] { const char* e = getenv("FQ3C_TC5_MINK"); return e ? atoi(e) : TK; }();
+  return on && o.N >= 16 && o.K >= min_k;
+}
+bool gemm_persists(const fq3c_op& o) { return gemm_on_tc(o) && (o.taps == 1 || o.cin % 16 == 0); }
+// Columns behind N that are scratch make a width of whole 16-column pieces (B's missing rows arrive as zeros): the epilogue of any other width stores every
+// entry by itself (1501 rows of 643 columns 31 us, of 656 9.3).
+fq3c_op gemm_whole_pieces(const fq3c_op& o) {
+  fq3c_op w = o;
+  if ((o.reserved & 8) && !(o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_RESID | FQ3C_SWIGLU | FQ3C_SNAKE2)) && o.ldc >= (o.N + 15) / 16 * 16 && !o.norm_out)
+    w.N = (o.N + 15) / 16 * 16;
+  return w;
+}
+
 // ---- attention of many queries on tcgen05 ---------------------------------------------------------------------------------------
 bool attn_attrs_ready() {
   static bool done[64] = {};
@@ -2386,6 +2402,14 @@ static SideStream* side_stream() {
   return &e;
 }
 static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, SideStream*& open);
+int fq3c_gemm_plan(const fq3c_op* op, int32_t* out) {
+  if (!op || !out || op->kind != FQ3C_GEMM || op->M <= 0 || op->m_begin < 0 || op->m_begin >= op->M || op->taps < 1 || op->taps > 8 || op->K % 8 || op->cin % 8 || !gemm_persists(*op))
+    return fail("gemm_plan: not a product of the persistent kernel");
+  const GemmLaunch L = gemm_plan(gemm_whole_pieces(*op));
+  const int32_t v[8] = {L.shape, L.g.bn, L.g.mt, L.g.nt, L.g.parts, L.g.splits, L.g.stages, (int32_t)L.grid};
+  std::copy(v, v + 8, out);
+  return 0;
+}
 int fq3c_run(const fq3c_op* ops, int n_ops, void* stream) {
   if (!wait_word_ready()) return fail("cannot make the error word of bounded waits");
   SideStream* open = nullptr;
@@ -2449,20 +2473,10 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         if (o.m_begin < 0 || o.m_begin >= o.M) return fail("gemm: m_begin outside [0, M)");
         if (o.norm_out && ((o.flags & (FQ3C_SWIGLU | FQ3C_OUT_F32)) || !o.norm_w || o.norm_ld < o.N))
           return fail("gemm: a fused RMSNorm needs a bf16 [M, N] output, weights and norm_ld >= N");
-        static int use_tc5 = -1;
-        if (use_tc5 < 0) {
-          const char* e = getenv("FQ3C_TCGEN05");
-          use_tc5 = (e == nullptr || atoi(e) != 0) ? 1 : 0;
-        }
+        const bool use_tc5 = gemm_on_tc(o);
         if (use_tc5 && !device_attrs_ready()) return fail("cannot reserve shared memory for the tcgen05 GEMM / prefill attention");
-        static int tc5_min_k = -1;
-        if (tc5_min_k < 0) { const char* e3 = getenv("FQ3C_TC5_MINK"); tc5_min_k = e3 ? atoi(e3) : TK; }  // one k-block is enough: the vectorised epilogue beats the mma.sync kernel even at K = 96
-        if (use_tc5 && o.N >= 16 && o.K >= tc5_min_k && (o.taps == 1 || o.cin % 16 == 0)) {
-          // Columns behind N that are scratch make a width of whole 16-column pieces (B's missing rows arrive as zeros): the epilogue of any other width stores every
-          // entry by itself (1501 rows of 643 columns 31 us, of 656 9.3).
-          fq3c_op w = o;
-          if ((o.reserved & 8) && !(o.flags & (FQ3C_BIAS | FQ3C_SCALE | FQ3C_RESID | FQ3C_SWIGLU | FQ3C_SNAKE2)) && o.ldc >= (o.N + 15) / 16 * 16 && !o.norm_out)
-            w.N = (o.N + 15) / 16 * 16;
+        if (gemm_persists(o)) {
+          const fq3c_op w = gemm_whole_pieces(o);
           const GemmLaunch L = gemm_plan(w);
           CUtensorMap tmA, tmB;
           if (make_map(&tmA, o.A, (uint64_t)o.cin, (uint64_t)o.a_rows, (uint64_t)o.lda, (uint32_t)L.g.a_rows) &&
@@ -2477,7 +2491,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
             break;
           }
         }
-        if (use_tc5 && o.N >= 16 && o.K >= tc5_min_k) {
+        if (use_tc5) {
           // Tile width: a multiple of 16 columns (a legal UMMA N at M = 128), chosen so that the grid covers the SMs.
           // Tall operands (M >= 128) keep BN >= 64 (every column tile re-reads the A rows); short ones (the transformer at
           // 8-33 frames) are weight-streaming problems: the width that minimises waves x tile cost, down to 16 columns.

@@ -6,15 +6,20 @@ from test_gemm_gpu import SEVEN, launch, make_op, product
 
 pytestmark = pytest.mark.gpu
 
-# rows, columns, inputs per tap, taps, split allowed
-CASES = [(64, 512, 256, (0,), False), (65, 512, 256, (0,), False),                       # eight and sixteen epilogue warps
-         (20000, 96, 96, (0,), False), (9600, 192, 256, (0,), False), (9600, 192, 320, (0,), False), (20000, 96, 40, (-1, 0), False),      # two CTAs per SM: up to four k-blocks
-         (700, 208, 192, (0,), False), (1900, 176, 64, (0,), False), (2500, 256, 128, (0,), False),      # column pieces that four groups of warps share unevenly
-         (64, 1024, 1536, (0,), True), (64, 1024, 2048, (0,), True), (100, 1024, 3072, (0,), True), (130, 1024, 3072, (0,), True), (40, 2048, 1024, (0,), True),
-         (17, 48, 2048, (0,), True), (200, 512, 512, SEVEN, True)]
+# rows, columns, inputs per tap, taps, split allowed | of the f32 launch: its shape, the columns of a tile, the parts of its sums (held to the plan in test_gemm_plan_cpu.py)
+WIDE, EIGHT, TWO = 0, 1, 2      # one CTA per SM with sixteen or eight epilogue warps, two with eight each
+CASES = [(64, 6144, 1024, (0,), False, EIGHT, 64, 1), (65, 6144, 1024, (0,), False, WIDE, 64, 1),      # eight and sixteen epilogue warps
+         (64, 512, 256, (0,), False, TWO, 16, 1), (65, 512, 256, (0,), False, TWO, 16, 1), (700, 208, 192, (0,), False, TWO, 16, 1), (1900, 176, 64, (0,), False, TWO, 16, 1),      # one piece a tile
+         (20000, 96, 96, (0,), False, TWO, 32, 1), (9600, 192, 256, (0,), False, TWO, 64, 1), (9600, 192, 320, (0,), False, WIDE, 64, 1), (20000, 96, 48, (-1, 0), False, TWO, 32, 1),      # up to four k-blocks
+         (20000, 96, 40, (-1, 0), False, None, None, None),      # c_in of 8 modulo 16: another kernel
+         # 3, 5, 7 and 13 column pieces, which four groups of warps share unevenly
+         (2500, 256, 128, (0,), False, WIDE, 48, 1), (6000, 208, 512, (0,), False, WIDE, 80, 1), (9600, 112, 512, (0,), False, WIDE, 112, 1), (3000, 1200, 512, (0,), False, WIDE, 208, 1),
+         (64, 1024, 1536, (0,), True, EIGHT, 32, 1), (64, 1024, 2048, (0,), True, EIGHT, 64, 8), (100, 1024, 3072, (0,), True, EIGHT, 64, 8), (130, 1024, 3072, (0,), True, EIGHT, 64, 4),
+         (40, 2048, 1024, (0,), True, EIGHT, 32, 1), (17, 48, 2048, (0,), True, EIGHT, 32, 8), (200, 512, 512, SEVEN, True, EIGHT, 64, 8), (130, 2048, 6144, (0,), True, EIGHT, 64, 2),
+         (200, 2048, 6144, (0,), True, EIGHT, 64, 2)]
 
 
-@pytest.mark.parametrize("M,N,cin,offs,split", CASES)
+@pytest.mark.parametrize("M,N,cin,offs,split", [c[:5] for c in CASES])
 def test_product_residual_snake_and_units(M, N, cin, offs, split):
     from qwen3_tts_cuda_graphs_b200 import codec as K
 
