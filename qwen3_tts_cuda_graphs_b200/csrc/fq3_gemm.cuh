@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
   // The two issuing warps run their loops whole, with one elected lane at the copies, products and commits: in code of a single lane every operand goes
   // through per-lane registers (700 - 800 cycles a k-block with `lane == 0`, 380 with the election around the loop).  What bounds a k-block of narrow tiles is
   // the chain of instructions from one issue to the next, so the inner loops hold no more than a pointer's step each: taps and their last, shorter k-blocks are
-  // outside of them.  347 -> 270 cycles a k-block (40 x 1024 x 8192: 25.9 -> 22.9 us); the tensor pipe needs 160 - 256 up to 128 columns.
+  // outside of them.  347 -> 300 cycles a k-block (40 x 1024 x 8192: 25.9 -> 22.9 us); the tensor pipe needs 160 - 256 up to 128 columns.
   const bool leader = elect_one();
   if (warp == TMA_WARP) {
     const uint32_t tx = (uint32_t)(g.a_rows * TK * 2 + g.bn * TK * 2), ring = 8u * g.stages;

@@ -8,7 +8,9 @@ each size:
   * decode: single-token steps at context T (tokens / s), replayed as CUDA graphs as the generation path does;
   * per op kind: device time of every op of the step's list launched alone (CUDA events, L2 flushed before each timed
     launch), its algorithmic FLOPs and bytes, and the fraction of the roofline max(FLOPs / measured bf16 peak, bytes /
-    measured copy bandwidth) it reaches.
+    measured copy bandwidth) it reaches.  A step runs some of them together - a product of few rows with the norm, depth mix
+    or activation behind it, a prompt's q / k norm with the attention - and a shared expert beside the routed ones: the
+    table's sum is more than the step.
 The closest existing model is the talker (a dense Qwen3 decoder): its dense prefill is an op list on the same library
 (prefill_dense.py), timed op by op the same way, and its decode step is the persistent decode kernel (bytes of weights / time).
 """

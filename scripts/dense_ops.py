@@ -1,4 +1,4 @@
-"""Per-op device time of the dense prefill plan for R rows."""
+"""Per-op device time of the dense prefill plan for R rows, each op launched alone (a plan of up to 64-112 rows runs qknorm and attn as one launch)."""
 import os, sys, torch, ctypes as C
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT); sys.path.insert(0, os.path.join(ROOT, "tests"))
