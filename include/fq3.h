@@ -2,7 +2,7 @@
  * fq3.h — C ABI of the B200-native Qwen3-TTS decode engine (libfq3.so).
  *
  * This is the drop-in boundary for the hot path of andimarafioti/qwen3-tts-cuda-graphs
- * (reference = /root/reference, Python, no native code).  Every entry point replaces one seam of the
+ * (the reference is Python, no native code).  Every entry point replaces one seam of the
  * reference's L2/L3 operators; the reference file:line each one stands in for is cited.
  * Plain pointers and sizes only — no torch types.  All device pointers are CUDA device addresses on the
  * current device; `stream` is a cudaStream_t passed as void*.  Every call returns 0 on success or a

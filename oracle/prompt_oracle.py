@@ -1,13 +1,13 @@
 """CPU restatement of the reference's prompt assembly — TEST INFRASTRUCTURE ONLY (see oracle/qwen3_tts_oracle.py).
 
 What is restated and where it comes from
-  * `_build_talker_inputs_local` ........ /root/reference/faster_qwen3_tts/model.py:331-553, statement by statement:
+  * `_build_talker_inputs_local` ........ faster_qwen3_tts/model.py:331-553, statement by statement:
       instruct rows (:349-354), speaker row (:361-375), language / dialect id (:377-393), tts bos/eos/pad rows
       (:395-403), codec prefix ids (:405-417), pad/bos codec rows and optional speaker row (:418-428), role rows
       (:434-436), text-side pad..bos + codec[:-1] (:437-443), ICL branch (:447-460), first-text-token row (:462-471),
       non_streaming_mode rewrite (:472-504), trailing text (:505-514), left-pad by flip/pad/flip + mask (:519-535),
       trailing hiddens right-padded with the tts_pad vector (:537-551).
-  * `generate_icl_prompt` ............... third-party `qwen-tts>=0.1.1` (pyproject.toml:29), NOT in /root/reference and not
+  * `generate_icl_prompt` ............... third-party `qwen-tts>=0.1.1` (pyproject.toml:29), NOT in the reference and not
       importable here.  Restated from its call site (model.py:452-459: arguments, return pair) and the layout recalled in
       SURVEY.md Appendix B.  PARITY UNPINNED for this function; everything else in this file follows in-tree reference
       lines.

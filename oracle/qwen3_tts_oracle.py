@@ -9,7 +9,7 @@ What is restated and where it comes from
   * sampling and repetition penalty ............................ faster_qwen3_tts/sampling.py:10-66
   * predictor 15-step order (small_to_mtp on every input) ...... faster_qwen3_tts/predictor_graph.py:115-167
   * decode position = cache_pos + rope_delta on all mrope axes . faster_qwen3_tts/talker_graph.py:198-214
-  * layer arithmetic (third-party, NOT in /root/reference): `qwen-tts>=0.1.1` (pyproject.toml:29, unpinned
+  * layer arithmetic (third-party, NOT in the reference): `qwen-tts>=0.1.1` (pyproject.toml:29, unpinned
     upper bound) whose talker/predictor are dense Qwen3 decoder stacks.  Restated from the in-container
     sibling transformers 5.5.0 `models/qwen3/modeling_qwen3.py` (RMSNorm, per-head q/k norm before RoPE,
     GQA eager attention, SwiGLU) — see SURVEY.md §8(c).

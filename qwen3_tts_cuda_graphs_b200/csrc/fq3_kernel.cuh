@@ -1,7 +1,7 @@
 // fq3_kernel.cuh — the persistent weight-streaming decode kernel (sm_100a), v9.
 //
 // Replaces the CUDA-graph replays of talker_graph.py:97-107,198-214 and predictor_graph.py:115-167 and
-// the eager per-frame glue of generate.py:149-199 (reference paths under /root/reference/faster_qwen3_tts).
+// the eager per-frame glue of generate.py:149-199 (paths within the reference package faster_qwen3_tts).
 //
 // Structure of one CTA (one per SM, all co-resident):
 //   warp 12      producer: walks the phase program and streams this CTA's row groups of every GEMV phase's weight

@@ -190,7 +190,7 @@ def tiny_eng():
 
 
 def test_repetition_penalty_known_answer(tiny_eng):
-    """/root/reference/tests/test_sampling.py:10-21, through fq3_apply_repetition_penalty."""
+    """The reference's tests/test_sampling.py:10-21, through fq3_apply_repetition_penalty."""
     from qwen3_tts_cuda_graphs_b200 import sampling
     sampling.set_default_engine(tiny_eng)
     logits = torch.zeros(1, 1, 10)
@@ -247,7 +247,7 @@ def test_sampler_matches_reference_fixtures(tiny_eng):
 # (e) the reference's duck-typed operator seam (tests/test_sampling.py:24-118), through the operator-at-a-time loop
 # ------------------------------------------------------------------------------------------------
 def test_min_new_tokens_with_dummy_operator_doubles(tiny_eng):
-    """Port of /root/reference/tests/test_sampling.py:24-118: DummyTalker / DummyPredictorGraph / DummyTalkerGraph drive
+    """Port of the reference's tests/test_sampling.py:24-118: DummyTalker / DummyPredictorGraph / DummyTalkerGraph drive
     fast_generate's operator path (`_generate_with_operators`); EOS is the greedy choice from the start, but may only be
     taken once min_new_tokens frames exist."""
     from qwen3_tts_cuda_graphs_b200 import sampling
