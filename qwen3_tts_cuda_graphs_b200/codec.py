@@ -150,6 +150,8 @@ def load_lib():
     lib.fq3c_launch_count.restype = C.c_int64
     lib.fq3c_wait_errors.restype = C.c_int
     lib.fq3c_wait_failed.restype = C.c_int
+    lib.fq3c_put_ints.restype = C.c_int
+    lib.fq3c_put_ints.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
     lib.fq3c_graph_create.restype = C.c_int
     lib.fq3c_graph_create.argtypes = [C.POINTER(Op), C.c_int, C.POINTER(C.c_void_p)]
     lib.fq3c_graph_launch.restype = C.c_int
@@ -290,6 +292,14 @@ def run_op_plan(lib, plan: _Plan, use_graphs: bool = True):
     else:
         rc = lib.fq3c_run(plan.arr, len(plan.ops), stream)
     if rc != 0:
+        raise CodecError(lib.fq3c_last_error().decode())
+
+
+def put_ints(lib, values, dst: torch.Tensor) -> None:
+    """dst (int32 on the device, contiguous) = values, in order on the current stream and without waiting for it; `values` may change at once."""
+    v = torch.as_tensor(list(values), dtype=torch.int32).cpu()
+    assert dst.dtype == torch.int32 and dst.is_contiguous() and dst.shape == v.shape
+    if lib.fq3c_put_ints(v.data_ptr(), v.numel(), dst.data_ptr(), torch.cuda.current_stream().cuda_stream) != 0:
         raise CodecError(lib.fq3c_last_error().decode())
 
 

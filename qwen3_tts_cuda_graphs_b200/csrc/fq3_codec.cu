@@ -1335,6 +1335,18 @@ __global__ void fq3c_copy_kernel(const fq3c_op o) {
   }
 }
 __global__ void fq3c_advance_kernel(int* counter, int by) { *counter += by; }
+
+// A step's token ids and wanted rows, as the launch's own arguments: a copy from pageable memory first waits until the stream has nothing left to do, so that every decoded
+// token's launches began some 40 us after the ones in front had ended (24 tokens behind a prompt of 203: 4920 us, this way 4130).
+struct PutInts {
+  static constexpr int MOST = 1000;      // with the two other fields within the 4 KB that a launch's arguments have everywhere
+  int32_t* dst;
+  int n;
+  int32_t v[MOST];
+};
+__global__ void fq3c_put_ints_kernel(const __grid_constant__ PutInts p) {
+  for (int i = threadIdx.x; i < p.n; i += blockDim.x) p.dst[i] = p.v[i];
+}
 // FQ3C_ROLL: blockIdx.x = history buffer, blockIdx.y = column slice (slices are independent).  dst row r <- src row r + new; when the
 // ranges overlap (new < hist) the rows go in batches of `new`: a batch's sources are the next batch's destinations, so a block
 // barrier separates them; within a batch sources and destinations are disjoint.
@@ -2663,6 +2675,18 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
   return 0;
 }
 
+
+int fq3c_put_ints(const int32_t* values, int n, int32_t* dst, void* stream) {
+  if (n < 0 || (n > 0 && (!values || !dst))) return fail("put_ints: bad arguments");
+  for (int at = 0; at < n; at += PutInts::MOST) {
+    PutInts p{dst + at, std::min(n - at, PutInts::MOST), {}};
+    std::copy(values + at, values + at + p.n, p.v);
+    fq3c_put_ints_kernel<<<1, p.n <= 32 ? 32 : 256, 0, (cudaStream_t)stream>>>(p);
+    count_launches(1);
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : fail(std::string("put_ints: ") + cudaGetErrorString(e));
+}
 
 /* A plan is static (same ops, same buffers for a given frame count): capture its launches once and replay them as one
  * CUDA graph (about a hundred short kernels per decode; the replay removes the per-launch CPU and scheduling gaps). */

@@ -122,14 +122,13 @@ class SequenceEngine:
             raise ValueError("wanted position outside the step")
         self.states.reserve(slot, M)
         e = self._step_plan(slot, M, layer_taps)
-        # from pageable memory: the copy is staged before the call returns, so the host list may change at once
-        e["ids"].copy_(torch.as_tensor(list(tokens), dtype=torch.int32))
+        _codec.put_ints(self.lib, tokens, e["ids"])
         _codec.run_op_plan(self.lib, e["plan"], self.use_graphs)
         self.last_taps = e["taps"]
         if not want:
             return None
         h = self._head_plan(slot, M, layer_taps, len(want), e["x"])
-        h["want"].copy_(torch.as_tensor(list(want), dtype=torch.int32))
+        _codec.put_ints(self.lib, want, h["want"])
         _codec.run_op_plan(self.lib, h["plan"], self.use_graphs)
         return h["logits"]
 
