@@ -1670,7 +1670,7 @@ constexpr int SEQ_GEMM_FLAGS = FQ3C_BIAS | FQ3C_GELU | FQ3C_GELU_TANH | FQ3C_SIG
 // a_f32 / b_f32: operand types.  exact: keep f32 A values as they are (CUDA cores) instead of rounding them onto the tensor cores.
 // tail: ops that go on with the product's entries, where it takes the few-row kernel (gemv_tail).
 bool takes_gemv(const SeqGemm& g) { return !g.seg && g.M <= 8 && (size_t)g.M * g.K * sizeof(float) <= 96 * 1024; }
-int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zcount, int row_tiles, cudaStream_t s, const SeqTail* tail = nullptr) {
+int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zcount, int row_tiles, cudaStream_t s, const bool after, const SeqTail* tail = nullptr) {
   if (g.flags & ~SEQ_GEMM_FLAGS) return fail("sequence product: unsupported epilogue flag");
   if (b_f32 && !a_f32) return fail("sequence product: f32 weights need f32 rows");
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || zcount <= 0) return 0;
@@ -1692,13 +1692,13 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     dim3 grid((g.N + 7) / 8, 1, zcount);
     static const SeqTail none{};
     if (tail && tail->n > 0 && a_f32 == b_f32) {
-      if (b_f32) fq3s_gemv_kernel<float, float, true><<<grid, 256, gemv_smem, s>>>(g, *tail);
-      else fq3s_gemv_kernel<bf16, bf16, true><<<grid, 256, gemv_smem, s>>>(g, *tail);
+      if (b_f32) launch_after(fq3s_gemv_kernel<float, float, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
+      else launch_after(fq3s_gemv_kernel<bf16, bf16, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
       return 0;
     }
-    if (b_f32) fq3s_gemv_kernel<float, float><<<grid, 256, gemv_smem, s>>>(g, none);
-    else if (a_f32) fq3s_gemv_kernel<float, bf16><<<grid, 256, gemv_smem, s>>>(g, none);
-    else fq3s_gemv_kernel<bf16, bf16><<<grid, 256, gemv_smem, s>>>(g, none);
+    if (b_f32) launch_after(fq3s_gemv_kernel<float, float>, grid, 256, gemv_smem, s, after, 1, g, none);
+    else if (a_f32) launch_after(fq3s_gemv_kernel<float, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
+    else launch_after(fq3s_gemv_kernel<bf16, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
     return 0;
   }
   if (g.seg && zcount == 1 && g.M <= 16 && (size_t)g.K * sizeof(float) <= 96 * 1024) {
@@ -1713,9 +1713,9 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     }
     dim3 grid((g.N + 7) / 8, g.M, 1);
     const size_t smem = (size_t)g.K * sizeof(float);
-    if (b_f32) fq3s_ggemv_kernel<float, float><<<grid, 256, smem, s>>>(g);
-    else if (a_f32) fq3s_ggemv_kernel<float, bf16><<<grid, 256, smem, s>>>(g);
-    else fq3s_ggemv_kernel<bf16, bf16><<<grid, 256, smem, s>>>(g);
+    if (b_f32) launch_after(fq3s_ggemv_kernel<float, float>, grid, 256, smem, s, after, 1, g);
+    else if (a_f32) launch_after(fq3s_ggemv_kernel<float, bf16>, grid, 256, smem, s, after, 1, g);
+    else launch_after(fq3s_ggemv_kernel<bf16, bf16>, grid, 256, smem, s, after, 1, g);
     return 0;
   }
   // bf16 rows of whole 16-byte pieces (what its copies ask for): the pipelined product, faster at every size (figures at the kernel)
@@ -1730,18 +1730,18 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       pattr[dev] = true;
     }
     const dim3 pgrid((g.N + GQ_BN - 1) / GQ_BN, (g.M + GQ_BM - 1) / GQ_BM + (g.seg ? g.E : 0), zcount);
-    if (g.flags & FQ3C_SWIGLU) fq3s_gemm_pipe_kernel<true><<<pgrid, 256, GQ_SMEM, s>>>(g);
-    else fq3s_gemm_pipe_kernel<false><<<pgrid, 256, GQ_SMEM, s>>>(g);
+    if (g.flags & FQ3C_SWIGLU) launch_after(fq3s_gemm_pipe_kernel<true>, pgrid, 256, GQ_SMEM, s, after, 1, g);
+    else launch_after(fq3s_gemm_pipe_kernel<false>, pgrid, 256, GQ_SMEM, s, after, 1, g);
     return 0;
   }
   // tall bf16 products (many rows per block / per expert, wide enough outputs): 128 x 128 tiles
   if (!b_f32 && !(a_f32 && exact) && g.N >= 128 && (g.seg ? g.M >= 96 * g.E : g.M >= 256)) {
     dim3 grid128((g.N + 127) / 128, (g.M + 127) / 128 + (g.seg ? g.E : 0), zcount);
     const bool glu = (g.flags & FQ3C_SWIGLU) != 0;
-    if (a_f32 && glu) fq3s_gemm_mma128_kernel<float, true><<<grid128, 256, 0, s>>>(g);
-    else if (a_f32) fq3s_gemm_mma128_kernel<float><<<grid128, 256, 0, s>>>(g);
-    else if (glu) fq3s_gemm_mma128_kernel<bf16, true><<<grid128, 256, 0, s>>>(g);
-    else fq3s_gemm_mma128_kernel<bf16><<<grid128, 256, 0, s>>>(g);
+    if (a_f32 && glu) launch_after(fq3s_gemm_mma128_kernel<float, true>, grid128, 256, 0, s, after, 1, g);
+    else if (a_f32) launch_after(fq3s_gemm_mma128_kernel<float>, grid128, 256, 0, s, after, 1, g);
+    else if (glu) launch_after(fq3s_gemm_mma128_kernel<bf16, true>, grid128, 256, 0, s, after, 1, g);
+    else launch_after(fq3s_gemm_mma128_kernel<bf16>, grid128, 256, 0, s, after, 1, g);
     return 0;
   }
   dim3 grid((g.N + 63) / 64, row_tiles, zcount);
@@ -1755,14 +1755,14 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       cudaFuncSetAttribute(fq3s_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
       attr[dev] = true;
     }
-    fq3s_gemm_f32_kernel<<<grid, 256, FG_SMEM, s>>>(g);
+    launch_after(fq3s_gemm_f32_kernel, grid, 256, FG_SMEM, s, after, 1, g);
   }
-  else if (b_f32) fq3s_gemm_kernel<float, float><<<grid, 256, 0, s>>>(g);
-  else if (a_f32 && exact) fq3s_gemm_kernel<float, bf16><<<grid, 256, 0, s>>>(g);
-  else if (a_f32 && (g.flags & FQ3C_SWIGLU)) fq3s_gemm_mma_kernel<float, true><<<grid, 128, 0, s>>>(g);
-  else if (a_f32) fq3s_gemm_mma_kernel<float><<<grid, 128, 0, s>>>(g);
-  else if (g.flags & FQ3C_SWIGLU) fq3s_gemm_mma_kernel<bf16, true><<<grid, 128, 0, s>>>(g);
-  else fq3s_gemm_mma_kernel<bf16><<<grid, 128, 0, s>>>(g);
+  else if (b_f32) launch_after(fq3s_gemm_kernel<float, float>, grid, 256, 0, s, after, 1, g);
+  else if (a_f32 && exact) launch_after(fq3s_gemm_kernel<float, bf16>, grid, 256, 0, s, after, 1, g);
+  else if (a_f32 && (g.flags & FQ3C_SWIGLU)) launch_after(fq3s_gemm_mma_kernel<float, true>, grid, 128, 0, s, after, 1, g);
+  else if (a_f32) launch_after(fq3s_gemm_mma_kernel<float>, grid, 128, 0, s, after, 1, g);
+  else if (g.flags & FQ3C_SWIGLU) launch_after(fq3s_gemm_mma_kernel<bf16, true>, grid, 128, 0, s, after, 1, g);
+  else launch_after(fq3s_gemm_mma_kernel<bf16>, grid, 128, 0, s, after, 1, g);
   return 0;
 }
 
@@ -1826,6 +1826,10 @@ void gemv_tail(const fq3c_op& o, const SeqGemm& g, const fq3c_op* next, const in
       param(q.scale, N);
       param(q.bias, N);
     }
+    // What it reads is asked for in front of the product's sums, so nothing in front of it in this launch may have written that; but a mix gets the norm's result by hand.
+    for (int a = 0; a < nw; ++a)
+      for (int b = nr; b < r; ++b)
+        if (!apart(writes[a], reads[b]) && !(mix && (next[0].flags & FQ3C_OUT_F32) && same(reads[b], rows(next[0].C, next[0].ldc, 4, N)) && same(writes[a], reads[b]))) return;
     const bool out32 = mix || (q.flags & FQ3C_OUT_F32);
     writes[w++] = rows(q.C, q.ldc, out32 ? 4 : 2, N);
     if (q.kind != FQ3C_XIELU && out32 && q.C2) writes[w++] = rows(q.C2, q.ldc, 2, N);
@@ -1842,24 +1846,24 @@ void gemv_tail(const fq3c_op& o, const SeqGemm& g, const fq3c_op* next, const in
     if (q.kind == FQ3C_XIELU) return;
   }
 }
-int seq_run(const fq3c_op& o, cudaStream_t s) {
+int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
   switch (o.kind) {
     case FQ3C_EMBED:
       if (!o.A || !o.B || !o.C) return fail("embed: missing operand");
       if (o.i0 > 1 && o.K < o.N) return fail("embed: copies need a stride of at least N elements");
       if (o.C2 && o.ldr < o.N * std::max(o.i1, 1)) return fail("embed: the operand copies do not fit their pitch");
-      if (o.flags & FQ3C_F32) fq3s_embed_kernel<float><<<o.M, row_threads(o.M, o.N, 128), 0, s>>>(o);
-      else fq3s_embed_kernel<bf16><<<o.M, row_threads(o.M, o.N, 128), 0, s>>>(o);
+      if (o.flags & FQ3C_F32) launch_after(fq3s_embed_kernel<float>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
+      else launch_after(fq3s_embed_kernel<bf16>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
       return 0;
     case FQ3C_TCONV:
       if (o.taps < 1 || !o.A || !o.B || !o.C || (o.taps > 1 && (!o.p0 || !o.p1))) return fail("tconv: missing operand");
       if (tconv_vec_ok(o)) {
         const dim3 grid((o.N / 4 + 127) / 128, (o.M + o.taps - 1 + TC_ROWS - 1) / TC_ROWS);
-        if (o.taps <= 4) fq3s_tconv_vec_kernel<4><<<grid, 128, 0, s>>>(o);
-        else fq3s_tconv_vec_kernel<8><<<grid, 128, 0, s>>>(o);
+        if (o.taps <= 4) launch_after(fq3s_tconv_vec_kernel<4>, grid, 128, 0, s, after, 1, o);
+        else launch_after(fq3s_tconv_vec_kernel<8>, grid, 128, 0, s, after, 1, o);
         return 0;
       }
-      fq3s_tconv_kernel<<<dim3((o.N + 255) / 256, o.M + o.taps - 1), 256, 0, s>>>(o);
+      launch_after(fq3s_tconv_kernel, dim3((o.N + 255) / 256, o.M + o.taps - 1), 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_GNORM:
       if (o.i0 < 1 || o.N % o.i0 || ((o.flags & FQ3C_RESID) && !o.res)) return fail("gnorm: groups must divide N");
@@ -1869,14 +1873,14 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
           (!(o.flags & (FQ3C_GATE_PRE | FQ3C_GATE_POST)) || o.i1 % 4 == 0) &&
           !((reinterpret_cast<uintptr_t>(o.A) | reinterpret_cast<uintptr_t>(o.C) | reinterpret_cast<uintptr_t>(o.C2) | reinterpret_cast<uintptr_t>(o.p1) |
              reinterpret_cast<uintptr_t>(o.res) | reinterpret_cast<uintptr_t>(o.scale)) & 15)) {
-        fq3s_gnorm_warp_kernel<<<(unsigned)(((int64_t)o.M * o.i0 + 3) / 4), 128, 0, s>>>(o);
+        launch_after(fq3s_gnorm_warp_kernel, (unsigned)(((int64_t)o.M * o.i0 + 3) / 4), 128, 0, s, after, 1, o);
         return 0;
       }
-      fq3s_gnorm_kernel<<<dim3(o.M, o.i0), row_threads(o.M, o.N / o.i0, 128), 0, s>>>(o);
+      launch_after(fq3s_gnorm_kernel, dim3(o.M, o.i0), row_threads(o.M, o.N / o.i0, 128), 0, s, after, 1, o);
       return 0;
     case FQ3C_POLYNORM:
       if (!o.p0) return fail("polynorm: coefficients required");
-      fq3s_polynorm_kernel<<<o.M, 256, 0, s>>>(o);
+      launch_after(fq3s_polynorm_kernel, o.M, 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_BDGEMM: {
       if (o.i0 < 1 || o.i1 < 1 || o.i2 < 1 || o.cin < 1) return fail("bdgemm: bad block shape");
@@ -1884,7 +1888,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       g.A = o.A; g.B = o.B; g.bias = reinterpret_cast<const float*>(o.bias); g.C = o.C;
       g.M = o.M; g.N = o.i2; g.K = o.cin; g.lda = o.lda; g.ldb = o.cin; g.ldc = o.ldc; g.flags = o.flags;
       g.a_mod = o.i1; g.a_zstride = o.cin; g.c_zstride = o.i2; g.b_zstride = (long long)o.i2 * o.cin;
-      return launch_seq_gemm(g, true, (o.flags & FQ3C_F32) != 0, (o.flags & FQ3C_NOROUND) != 0, o.i0, (o.M + 63) / 64, s);
+      return launch_seq_gemm(g, true, (o.flags & FQ3C_F32) != 0, (o.flags & FQ3C_NOROUND) != 0, o.i0, (o.M + 63) / 64, s, after);
     }
     case FQ3C_GGEMM: {
       if (o.i0 < 1 || !o.p0) return fail("ggemm: segment starts required");
@@ -1896,7 +1900,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       if (o.flags & FQ3C_SWIGLU) { g.rs_w = reinterpret_cast<const float*>(o.scale); g.rs_pos = reinterpret_cast<const int*>(o.ws); g.rs_top = o.i1; }
       if (g.rs_pos && (!g.rs_w || !g.rows || g.rs_top < 1)) return fail("ggemm: a router's weights need the choices' places, the row list and the choice count");
       const bool f32 = (o.flags & FQ3C_F32) != 0;
-      return launch_seq_gemm(g, f32 || (o.flags & FQ3C_A_F32), f32, false, 1, (o.M + 63) / 64 + o.i0, s);
+      return launch_seq_gemm(g, f32 || (o.flags & FQ3C_A_F32), f32, false, 1, (o.M + 63) / 64 + o.i0, s, after);
     }
     case FQ3C_LRU_SCAN: {
       if (!o.A || !o.B || !o.res || !o.scale || !o.p0 || !o.C || !o.C2) return fail("lru_scan: missing operand");
@@ -1906,10 +1910,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       const int per = (o.M + chunks - 1) / chunks;
       dim3 grid((o.N + 127) / 128, chunks);
       if (chunks > 1) {
-        fq3s_lru_fold_kernel<<<grid, 128, 0, s>>>(o, chunks, per, reinterpret_cast<float*>(o.ws));
+        launch_after(fq3s_lru_fold_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<float*>(o.ws));
         count_launches(1);
       }
-      fq3s_lru_scan_kernel<<<grid, 128, 0, s>>>(o, chunks, per, reinterpret_cast<const float*>(o.ws));
+      launch_after(fq3s_lru_scan_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<const float*>(o.ws));
       return 0;
     }
     case FQ3C_ROUTER: {
@@ -1918,22 +1922,22 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       if (tpb < 1) return fail("router: too many experts");
       if (tpb >= 32) tpb &= ~31;
       if (o.ws && (o.M != 1 || o.i0 > 16 || !o.p0 || !o.p1 || o.K < 0)) return fail("router: grouping in the same launch takes one token with at most 16 choices");
-      fq3s_router_kernel<<<(o.M + tpb - 1) / tpb, tpb, (size_t)o.N * tpb * 8, s>>>(o);
+      launch_after(fq3s_router_kernel, (o.M + tpb - 1) / tpb, tpb, (size_t)o.N * tpb * 8, s, after, 1, o);
       return 0;
     }
     case FQ3C_MOE_SORT: {
       if (o.i1 < 1 || !o.A || !o.C || !o.C2 || !o.ws) return fail("moe_sort: missing operand");
       const int warps = std::min(std::min(32, ((48 * 1024) / 4 - o.i1 - 1) / o.i1), std::max(1, (o.M * o.i0 + 31) / 32));
       if (warps < 1) return fail("moe_sort: too many experts");
-      fq3s_moe_sort_kernel<<<1, warps * 32, (size_t)(o.i1 + 1 + warps * o.i1) * 4, s>>>(o);
+      launch_after(fq3s_moe_sort_kernel, 1, warps * 32, (size_t)(o.i1 + 1 + warps * o.i1) * 4, s, after, 1, o);
       return 0;
     }
     case FQ3C_MOE_COMBINE:
       if (!o.A || !o.B || !o.p0 || !o.ws || !o.C) return fail("moe_combine: missing operand");
-      fq3s_moe_combine_kernel<<<o.M, 256, 0, s>>>(o);
+      launch_after(fq3s_moe_combine_kernel, o.M, 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_COMMIT:
-      fq3s_commit_kernel<<<dim3(o.M, 8), 256, 0, s>>>(reinterpret_cast<const long long*>(o.A), reinterpret_cast<int*>(o.C), o.i0);
+      launch_after(fq3s_commit_kernel, dim3(o.M, 8), 256, 0, s, after, 1, reinterpret_cast<const long long*>(o.A), reinterpret_cast<int*>(o.C), o.i0);
       return 0;
     case FQ3C_LATENT_ATTN: {
       if (o.i0 < 1 || o.i1 < 1 || !o.A || !o.B || !o.C) return fail("latent_attn: missing operand");
@@ -1969,11 +1973,11 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         }
         dim3 grid((o.M + QB - 1) / QB, (o.i0 + 15) / 16, splits);
         const int nth = 32 * QB * RSk;
-        if (nt_o <= 8) fq3s_latent_attn_mma_kernel<8><<<grid, nth, smem, s>>>(o, RSk, splits, TJ, QB);
-        else if (nt_o <= 16) fq3s_latent_attn_mma_kernel<16><<<grid, nth, smem, s>>>(o, RSk, splits, TJ, QB);
-        else fq3s_latent_attn_mma_kernel<32><<<grid, nth, smem, s>>>(o, RSk, splits, TJ, QB);
+        if (nt_o <= 8) launch_after(fq3s_latent_attn_mma_kernel<8>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        else if (nt_o <= 16) launch_after(fq3s_latent_attn_mma_kernel<16>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        else launch_after(fq3s_latent_attn_mma_kernel<32>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
         if (splits > 1) {
-          fq3s_latent_merge_kernel<<<dim3(o.M, o.i0), 128, 0, s>>>(o, splits);
+          launch_after(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
           count_launches(1);
         }
         return 0;
@@ -1991,10 +1995,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         attr[dev] = true;
       }
       dim3 grid(o.M, (o.i0 + HG - 1) / HG, splits);
-      if (o.flags & FQ3C_F32) fq3s_latent_attn_kernel<float><<<grid, 256, smem, s>>>(o, HG, splits);
-      else fq3s_latent_attn_kernel<bf16><<<grid, 256, smem, s>>>(o, HG, splits);
+      if (o.flags & FQ3C_F32) launch_after(fq3s_latent_attn_kernel<float>, grid, 256, smem, s, after, 1, o, HG, splits);
+      else launch_after(fq3s_latent_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, HG, splits);
       if (splits > 1) {
-        fq3s_latent_merge_kernel<<<dim3(o.M, o.i0), 128, 0, s>>>(o, splits);
+        launch_after(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
         count_launches(1);
       }
       return 0;
@@ -2004,9 +2008,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
     case FQ3C_XIELU: {
       if (const char* e = entry_op_error(o)) return fail(e);
       const dim3 grid((o.N + 255) / 256, o.M);
-      if (o.kind == FQ3C_DYT) fq3s_dyt_kernel<<<grid, 256, 0, s>>>(o);
-      else if (o.kind == FQ3C_DEPTH_MIX) fq3s_depth_mix_kernel<<<grid, 256, 0, s>>>(o);
-      else fq3s_xielu_kernel<<<grid, 256, 0, s>>>(o);
+      if (o.kind == FQ3C_DYT) launch_after(fq3s_dyt_kernel, grid, 256, 0, s, after, 1, o);
+      else if (o.kind == FQ3C_DEPTH_MIX) launch_after(fq3s_depth_mix_kernel, grid, 256, 0, s, after, 1, o);
+      else launch_after(fq3s_xielu_kernel, grid, 256, 0, s, after, 1, o);
       return 0;
     }
     case FQ3C_ROT_APPEND: {
@@ -2015,16 +2019,16 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         return fail("rot_append: bad configuration");
       if (o.m_begin > 0 && (o.i1 < 1 || o.cin < 1 || !o.norm_out || !o.ws || !o.p0)) return fail("rot_append: pooled blocks need both caches, their pooled rows and a position");
       const int rth = o.M <= 8 ? std::max(256, std::min(1024, 32 * (o.i0 + o.i1))) : 256;      // few rows: a warp per head
-      if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) fq3s_rot_append_kernel<float, true, 1024><<<1, rth, 0, s>>>(o);
-      else if (o.m_begin > 0 && o.M == 1) fq3s_rot_append_kernel<bf16, true, 1024><<<1, rth, 0, s>>>(o);
-      else if (rth > 256 && (o.flags & FQ3C_F32)) fq3s_rot_append_kernel<float, false, 1024><<<o.M, rth, 0, s>>>(o);
-      else if (rth > 256) fq3s_rot_append_kernel<bf16, false, 1024><<<o.M, rth, 0, s>>>(o);
-      else if (o.flags & FQ3C_F32) fq3s_rot_append_kernel<float><<<o.M, 256, 0, s>>>(o);
-      else fq3s_rot_append_kernel<bf16><<<o.M, 256, 0, s>>>(o);
+      if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, true, 1024>, 1, rth, 0, s, after, 1, o);
+      else if (o.m_begin > 0 && o.M == 1) launch_after(fq3s_rot_append_kernel<bf16, true, 1024>, 1, rth, 0, s, after, 1, o);
+      else if (rth > 256 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, false, 1024>, o.M, rth, 0, s, after, 1, o);
+      else if (rth > 256) launch_after(fq3s_rot_append_kernel<bf16, false, 1024>, o.M, rth, 0, s, after, 1, o);
+      else if (o.flags & FQ3C_F32) launch_after(fq3s_rot_append_kernel<float>, o.M, 256, 0, s, after, 1, o);
+      else launch_after(fq3s_rot_append_kernel<bf16>, o.M, 256, 0, s, after, 1, o);
       if (o.m_begin > 0 && o.M > 1) {
         const dim3 grid(o.M / o.m_begin + 1, (o.i1 * std::max(o.i2, o.cin) + 255) / 256, 2);
-        if (o.flags & FQ3C_F32) fq3s_pool_append_kernel<float><<<grid, 256, 0, s>>>(o);
-        else fq3s_pool_append_kernel<bf16><<<grid, 256, 0, s>>>(o);
+        if (o.flags & FQ3C_F32) launch_after(fq3s_pool_append_kernel<float>, grid, 256, 0, s, after, 1, o);
+        else launch_after(fq3s_pool_append_kernel<bf16>, grid, 256, 0, s, after, 1, o);
         count_launches(1);
       }
       return 0;
@@ -2052,7 +2056,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         a.gate_ld = o.col_mod; a.entry = o.res && (o.flags & FQ3C_GATE_ENTRY); a.out_f32 = (o.flags & FQ3C_OUT_F32) != 0; a.out = o.C; a.ldo = o.ldc;
         const int mode = o.bias ? AT_DIST : o.f1 > 0.f ? AT_CAP : AT_PLAIN;
         if (attn_tc_takes(a, mode)) {
-          launch_attn_tc(a, mode, s, false);
+          launch_attn_tc(a, mode, s, after);
           return 0;
         }
       }
@@ -2080,12 +2084,12 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         dim3 grid((o.M + QBLK - 1) / QBLK, o.i1);
         const size_t smem = cache_attn_mma_smem(ROWS, o.i2, o.cin);
         if (pool) {
-          if (o.cin <= 32) fq3s_cache_attn_mma_kernel<4, true><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
-          else if (o.cin <= 64) fq3s_cache_attn_mma_kernel<8, true><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
-          else fq3s_cache_attn_mma_kernel<16, true><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
-        } else if (o.cin <= 32) fq3s_cache_attn_mma_kernel<4><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
-        else if (o.cin <= 64) fq3s_cache_attn_mma_kernel<8><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
-        else fq3s_cache_attn_mma_kernel<16><<<grid, ROWS * 2, smem, s>>>(o, ROWS);
+          if (o.cin <= 32) launch_after(fq3s_cache_attn_mma_kernel<4, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+          else if (o.cin <= 64) launch_after(fq3s_cache_attn_mma_kernel<8, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+          else launch_after(fq3s_cache_attn_mma_kernel<16, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        } else if (o.cin <= 32) launch_after(fq3s_cache_attn_mma_kernel<4>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        else if (o.cin <= 64) launch_after(fq3s_cache_attn_mma_kernel<8>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        else launch_after(fq3s_cache_attn_mma_kernel<16>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
         return 0;
       }
       // an f32 cache and more than a few queries, heads of 128: 32-row blocks with pipelined tiles
@@ -2099,9 +2103,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
           fattr[dev] = true;
         }
         const int QB = FA_R / HG;
-        fq3s_attn_f32_kernel<<<dim3((o.M + QB - 1) / QB, o.i1, splits), 128, FA_SMEM, s>>>(o);
+        launch_after(fq3s_attn_f32_kernel, dim3((o.M + QB - 1) / QB, o.i1, splits), 128, FA_SMEM, s, after, 1, o);
         if (splits > 1) {
-          fq3s_cache_attn_merge_kernel<<<dim3(o.M, o.i0), 128, 0, s>>>(o, splits);
+          launch_after(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
           count_launches(1);
         }
         return 0;
@@ -2122,12 +2126,12 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         attr[dev] = true;
       }
       dim3 grid((o.M + QB - 1) / QB, o.i1, splits);
-      if (pool && (o.flags & FQ3C_F32)) fq3s_cache_attn_kernel<float, true><<<grid, 256, smem, s>>>(o, QB, TJ, splits);
-      else if (pool) fq3s_cache_attn_kernel<bf16, true><<<grid, 256, smem, s>>>(o, QB, TJ, splits);
-      else if (o.flags & FQ3C_F32) fq3s_cache_attn_kernel<float><<<grid, 256, smem, s>>>(o, QB, TJ, splits);
-      else fq3s_cache_attn_kernel<bf16><<<grid, 256, smem, s>>>(o, QB, TJ, splits);
+      if (pool && (o.flags & FQ3C_F32)) launch_after(fq3s_cache_attn_kernel<float, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else if (pool) launch_after(fq3s_cache_attn_kernel<bf16, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else if (o.flags & FQ3C_F32) launch_after(fq3s_cache_attn_kernel<float>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else launch_after(fq3s_cache_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
       if (splits > 1) {
-        fq3s_cache_attn_merge_kernel<<<dim3(o.M, o.i0), 128, 0, s>>>(o, splits);
+        launch_after(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
         count_launches(1);
       }
       return 0;
@@ -2144,13 +2148,13 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         cudaFuncSetAttribute(fq3s_hyper_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         hattr[dev] = true;
       }
-      if (o.i0 <= 8) fq3s_hyper_kernel<8><<<o.M, 256, (size_t)o.N * 4, s>>>(o);
-      else fq3s_hyper_kernel<16><<<o.M, 256, (size_t)o.N * 4, s>>>(o);
+      if (o.i0 <= 8) launch_after(fq3s_hyper_kernel<8>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
+      else launch_after(fq3s_hyper_kernel<16>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
       return 0;
     }
     case FQ3C_GLU:
       if (!o.A || !o.C || o.N < 1) return fail("glu: missing operand");
-      fq3s_glu_kernel<<<dim3((o.N + 255) / 256, o.M), 256, 0, s>>>(o);
+      launch_after(fq3s_glu_kernel, dim3((o.N + 255) / 256, o.M), 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_MSTATE_SCAN: {
       if (o.i0 < 1 || o.i1 < 1 || o.i0 % o.i1 || o.i2 < 1 || o.cin < 1 || !o.A || !o.p0 || !o.C || !o.C2) return fail("mstate_scan: bad configuration");
@@ -2182,20 +2186,20 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       const bool blocks = (o.taps == 0 || o.taps == 6) && o.M >= CD_MIN_ROWS && o.i2 <= CD_MAX_DK &&
                           o.ws_bytes / 4 >= cd_ws_floats(o.M, o.i0, o.i2, o.taps == 6) && !(reinterpret_cast<uintptr_t>(o.ws) & 15);
       if (o.taps == 4 && o.M > MS_CH) {
-        fq3s_mstate_gate_kernel<<<dim3(o.M, (o.i0 * o.i2 + 255) / 256), 256, 0, s>>>(o);
+        launch_after(fq3s_mstate_gate_kernel, dim3(o.M, (o.i0 * o.i2 + 255) / 256), 256, 0, s, after, 1, o);
         count_launches(1);
       } else if (o.taps == 5 && o.M > MS_CH) {
-        fq3s_mstate_max_kernel<<<o.i0, MM_THREADS, 0, s>>>(o);
+        launch_after(fq3s_mstate_max_kernel, o.i0, MM_THREADS, 0, s, after, 1, o);
         count_launches(1);
       } else if (o.taps == 6) {
         const int per = cdelta_prep_channels(o.M == 1 ? 1 : MS_PREP_ROWS);
         const dim3 grid((o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS, (o.i0 * o.i2 + per - 1) / per + (o.tap_off[2] > 0 ? (o.i0 * o.cin + per - 1) / per : 0) + (blocks ? 0 : 1));
         const size_t smem = sizeof(float) * MS_PREP_ROWS * (size_t)std::max(o.tap_off[0], o.tap_off[2]);
-        if (o.M == 1) fq3s_mstate_cdelta_prep_kernel<1><<<grid, 256, smem, s>>>(o, false);
-        else fq3s_mstate_cdelta_prep_kernel<MS_PREP_ROWS><<<grid, 256, smem, s>>>(o, blocks);
+        if (o.M == 1) launch_after(fq3s_mstate_cdelta_prep_kernel<1>, grid, 256, smem, s, after, 1, o, false);
+        else launch_after(fq3s_mstate_cdelta_prep_kernel<MS_PREP_ROWS>, grid, 256, smem, s, after, 1, o, blocks);
         count_launches(1);
       } else if (o.taps < 3 && !blocks) {
-        fq3s_mstate_prep_kernel<<<o.taps == 2 ? (o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS : o.M, 128, 0, s>>>(o);
+        launch_after(fq3s_mstate_prep_kernel, o.taps == 2 ? (o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS : o.M, 128, 0, s, after, 1, o);
         count_launches(1);
       }
       static bool sattr[64] = {};
@@ -2228,17 +2232,17 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
           cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<16>(CD_MAX_DK) * 4);
           battr[dev] = true;
         }
-        fq3s_cdelta_record_kernel<<<dim3((o.M + CD_C - 1) / CD_C, o.i0), CD_REC_THREADS, 4 * CD_C * cd_pitch(o.i2) * 4, s>>>(o);
+        launch_after(fq3s_cdelta_record_kernel, dim3((o.M + CD_C - 1) / CD_C, o.i0), CD_REC_THREADS, 4 * CD_C * cd_pitch(o.i2) * 4, s, after, 1, o);
         count_launches(1);
         // narrow state tiles while they do not outnumber the SMs, wide ones otherwise and for few state rows
         const bool narrow = o.i2 > 64 && o.i0 * ((o.cin + 7) / 8) <= 148;
         const dim3 grid((o.cin + (narrow ? 7 : 15)) / (narrow ? 8 : 16), o.i0);
         const size_t wsm = (narrow ? cd_walk_floats<8>(o.i2) : cd_walk_floats<16>(o.i2)) * 4;
-        if (narrow && o.i2 <= 128) fq3s_cdelta_walk_kernel<8, 1><<<grid, CD_WALK_THREADS, wsm, s>>>(o);
-        else if (narrow) fq3s_cdelta_walk_kernel<8, 2><<<grid, CD_WALK_THREADS, wsm, s>>>(o);
-        else if (o.i2 <= 64) fq3s_cdelta_walk_kernel<16, 1><<<grid, CD_WALK_THREADS, wsm, s>>>(o);
-        else if (o.i2 <= 128) fq3s_cdelta_walk_kernel<16, 2><<<grid, CD_WALK_THREADS, wsm, s>>>(o);
-        else fq3s_cdelta_walk_kernel<16, 4><<<grid, CD_WALK_THREADS, wsm, s>>>(o);
+        if (narrow && o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<8, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
+        else if (narrow) launch_after(fq3s_cdelta_walk_kernel<8, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
+        else if (o.i2 <= 64) launch_after(fq3s_cdelta_walk_kernel<16, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
+        else if (o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<16, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
+        else launch_after(fq3s_cdelta_walk_kernel<16, 4>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
         return 0;
       }
       // Long runs of a recurrence whose decays do not depend on the state: pieces walked twice (see the kernel), when the caller's
@@ -2266,16 +2270,16 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
         const dim3 grid((sv + cpt * MS_COLS - 1) / (cpt * MS_COLS), o.i0, nz);
         const size_t smem = sizeof(float) * 2 * mstate_buf_floats(bound, three ? 3 : 2, cpt);
 #define FQ3S_WALK(RPT, CPT) \
-    if (three && gated) fq3s_mstate_scan_kernel<RPT, 3, true, CPT><<<grid, 128, smem, s>>>(o, phase, piece, X, P); \
-    else if (three) fq3s_mstate_scan_kernel<RPT, 3, false, CPT><<<grid, 128, smem, s>>>(o, phase, piece, X, P); \
-    else if (gated) fq3s_mstate_scan_kernel<RPT, 2, true, CPT><<<grid, 128, smem, s>>>(o, phase, piece, X, P); \
-    else fq3s_mstate_scan_kernel<RPT, 2, false, CPT><<<grid, 128, smem, s>>>(o, phase, piece, X, P);
+    if (three && gated) launch_after(fq3s_mstate_scan_kernel<RPT, 3, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else if (three) launch_after(fq3s_mstate_scan_kernel<RPT, 3, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else if (gated) launch_after(fq3s_mstate_scan_kernel<RPT, 2, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else launch_after(fq3s_mstate_scan_kernel<RPT, 2, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P);
         if (cdelta) switch (bound) {
-          case 4: fq3s_mstate_scan_kernel<4, 3, false, 1, true><<<grid, 128, smem, s>>>(o, phase, piece, X, P); break;
-          case 8: fq3s_mstate_scan_kernel<8, 3, false, 1, true><<<grid, 128, smem, s>>>(o, phase, piece, X, P); break;
-          case 16: fq3s_mstate_scan_kernel<16, 3, false, 1, true><<<grid, 128, smem, s>>>(o, phase, piece, X, P); break;
-          case 32: fq3s_mstate_scan_kernel<32, 3, false, 1, true><<<grid, 128, smem, s>>>(o, phase, piece, X, P); break;
-          default: fq3s_mstate_scan_kernel<64, 3, false, 1, true><<<grid, 128, smem, s>>>(o, phase, piece, X, P); break;
+          case 4: launch_after(fq3s_mstate_scan_kernel<4, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 8: launch_after(fq3s_mstate_scan_kernel<8, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 16: launch_after(fq3s_mstate_scan_kernel<16, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 32: launch_after(fq3s_mstate_scan_kernel<32, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          default: launch_after(fq3s_mstate_scan_kernel<64, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
         }
         else if (cpt == 2) switch (bound) {
           case 4: FQ3S_WALK(4, 2) break;
@@ -2297,7 +2301,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       }
       walk(1, pieces - 1);
       const int64_t n = (int64_t)o.i0 * o.i2 * sv;
-      fq3s_mstate_carry_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(o, pieces, X, P, sv);
+      launch_after(fq3s_mstate_carry_kernel, (unsigned)((n + 255) / 256), 256, 0, s, after, 1, o, pieces, X, P, sv);
       walk(3, pieces);
       count_launches(2);
       return 0;
@@ -2316,10 +2320,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s) {
       if (o.N % 4 == 0 && o.N <= 1024 * SN_VECS && !((o.lda | o.ldc | o.norm_ld | o.K) & 3) && !o.C2 &&
           !((reinterpret_cast<uintptr_t>(o.A) | reinterpret_cast<uintptr_t>(o.C) | reinterpret_cast<uintptr_t>(o.norm_out) | reinterpret_cast<uintptr_t>(o.norm_w) |
             reinterpret_cast<uintptr_t>(o.bias)) & 15)) {
-        fq3s_sum_norm_vec_kernel<<<o.M, std::max(32, std::min(256, (o.N / 4 + 31) / 32 * 32)), 0, s>>>(o);
+        launch_after(fq3s_sum_norm_vec_kernel, o.M, std::max(32, std::min(256, (o.N / 4 + 31) / 32 * 32)), 0, s, after, 1, o);
         return 0;
       }
-      fq3s_sum_norm_kernel<<<o.M, row_threads(o.M, o.N, 256), (size_t)o.N * 4, s>>>(o);
+      launch_after(fq3s_sum_norm_kernel, o.M, row_threads(o.M, o.N, 256), (size_t)o.N * 4, s, after, 1, o);
       return 0;
     }
     default: return 1;
@@ -2434,8 +2438,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
   cudaStream_t s = main_stream;
   // The codec's kernels wait for the launches in front themselves and may begin early, as long as the launch in front on their stream belongs to this list
   // (what ran before the list is complete when its first launch begins): a prompt of 39 rows through 28 layers 1676 -> 1497 us, a codec window 1059 -> 972.
-  // The sequence models' own kernels are launched one behind the other (their GEMMs are not): early launches made their replays slower (a request of 24
-  // tokens 5.4 -> 6.4 ms).
+  // The sequence models' own kernels do so with few rows alone (seq_dep_begin); their GEMMs always.
   bool chained = false;
   for (int i = 0; i < n_ops; ++i) {
     const fq3c_op& o = ops[i];
@@ -2473,11 +2476,11 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           SeqGemm g{};
           g.A = o.A; g.B = o.B; g.bias = reinterpret_cast<const float*>(o.bias); g.C = o.C;
           g.M = o.M; g.N = o.N; g.K = o.K; g.lda = o.lda; g.ldb = o.K; g.ldc = o.ldc; g.flags = o.flags;
-          g.a_mod = 1;
+          g.a_mod = 1; g.early = o.reserved & 1;
           const bool f32 = (o.flags & FQ3C_F32) != 0;
           SeqTail tail{};
           gemv_tail(o, g, ops + i + 1, n_ops - i - 1, tail);
-          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s, &tail) != 0) return -1;
+          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s, after && o.M <= DEP_ROWS, &tail) != 0) return -1;
           i += tail.n;
           break;
         }
@@ -2663,7 +2666,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         break;
       }
       default: {
-        const int rc = seq_run(o, s);
+        const int rc = seq_run(o, s, after && (o.kind == FQ3C_COMMIT ? o.i0 : o.M) <= DEP_ROWS);
         if (rc == 1) return fail("unknown op kind");
         if (rc != 0) return rc;
       }

@@ -10,6 +10,7 @@ __device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinter
 // odd k) that are added at the end, so that both operands are read as they lie.  Three stages of 32 k.  Two products of 384 rows (1536 x 1024, 1024 x 1024): 166 -> 92 us.
 constexpr int FG_BM = 64, FG_BN = 64, FG_BK = 32, FG_P = FG_BK + 4, FG_ST = 3, FG_SMEM = FG_ST * (FG_BM + FG_BN) * FG_P * 4;
 __global__ void __launch_bounds__(256) fq3s_gemm_f32_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   extern __shared__ __align__(16) float fg[];
   float (*As)[FG_BM][FG_P] = reinterpret_cast<float (*)[FG_BM][FG_P]>(fg);
   float (*Bs)[FG_BN][FG_P] = reinterpret_cast<float (*)[FG_BN][FG_P]>(fg + FG_ST * FG_BM * FG_P);
@@ -141,6 +142,7 @@ __device__ __noinline__ void fa_row_again(const fq3c_op& o, const CacheAttnMask&
 constexpr int FA_R = 32, FA_T = 64, FA_P = 132, FA_PP = FA_T + 4;
 constexpr int FA_SMEM = (FA_R * FA_P + 2 * FA_T * FA_P + FA_R * FA_PP) * 4;
 __global__ void __launch_bounds__(128) fq3s_attn_f32_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) float fa[];
   float *qs = fa, *ks = qs + FA_R * FA_P, *vs = ks + FA_T * FA_P, *ps = vs + FA_T * FA_P;
   const int H = o.i0, HG = H / o.i1, QB = FA_R / HG, kvh = blockIdx.y, tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;

@@ -10,6 +10,15 @@ template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p) { return _
 __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// With few rows (decoding) a list is a chain of launches of some 3 us each, so the next one's blocks come up while this one works and wait here for its end.  One launch ahead, not more:
+// with the next launch let in before this wait, waiting blocks pile up (a token of 36 launches 163 us of the GPU's time without, 180 with many ahead, 149 with one).  With many rows
+// the blocks of the next launch would only take room: they then come up two on an SM beside others that stay empty (an attention layer of 384 rows in 32 bits 143 -> 159 us).
+constexpr int DEP_ROWS = 8;
+__device__ __forceinline__ void seq_dep_begin(const int rows) {
+  grid_dep_wait();
+  if (rows <= DEP_ROWS) grid_dep_launch();
+}
+
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -48,6 +57,7 @@ struct SeqGemm {
   // is C[r, n] = silu(w gate) * (w up) (FQ3C_GELU_TANH: gelu_tanh(w gate) * (w up)), N / 2 columns wide.  w = 1, or rs_w[r], or (rs_pos given: a router's choices) the weight
   // rs_w[m, j] of the choice j of token m = rows[r] whose sorted position rs_pos[m, j] is r.
   const float* rs_w; const int* rs_pos; int rs_top;
+  int early;   // few rows: no op of the list writes B, so its first entries are asked for before the launches in front have ended
 };
 __device__ __forceinline__ float sg_row_scale(const SeqGemm& g, const int r) {
   if (!g.rs_w) return 1.f;
@@ -68,6 +78,7 @@ constexpr int SG_BM = 64, SG_BN = 64, SG_BK = 16;
 
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(256) fq3s_gemm_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   __shared__ float As[SG_BK][SG_BM + 4];
   __shared__ float Bs[SG_BK][SG_BN + 4];
   const int tid = threadIdx.x, z = blockIdx.z;
@@ -249,6 +260,7 @@ __device__ __forceinline__ void sg_quad_epilogue(const SeqGemm& g, const float (
 }
 template <typename TA, bool GLU = false>      // GLU: the gated-unit epilogue (a variant of its own, so that the plain one compiles as it always did)
 __global__ void __launch_bounds__(128) fq3s_gemm_mma_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   constexpr int LD = 32 + 8;
   __shared__ __align__(16) bf16 As[64 * LD];
   __shared__ __align__(16) bf16 Bs[64 * LD];
@@ -337,6 +349,7 @@ __global__ void __launch_bounds__(128) fq3s_gemm_mma_kernel(const SeqGemm g) {
 constexpr int GQ_BM = 128, GQ_BN = 64, GQ_BK = 64, GQ_ST = 3, GQ_STAGE = (GQ_BM + GQ_BN) * GQ_BK * 2, GQ_SMEM = GQ_ST * GQ_STAGE;
 template <bool GLU>
 __global__ void __launch_bounds__(256, 3) fq3s_gemm_pipe_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   extern __shared__ __align__(128) unsigned char gq[];
   const int tid = threadIdx.x, z = blockIdx.z, warp = tid >> 5, lane = tid & 31;
   int row0, row_end;
@@ -423,6 +436,7 @@ __global__ void __launch_bounds__(256, 3) fq3s_gemm_pipe_kernel(const SeqGemm g)
 // by ldmatrix (f32 rows, or rows that are not whole 16-byte pieces).  Halves the operand traffic per output of the 64 x 64 kernel and runs 16 MMAs per warp between two barriers.
 template <typename TA, bool GLU = false>
 __global__ void __launch_bounds__(256) fq3s_gemm_mma128_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   constexpr int LD = 32 + 8, BM = 128, BN = 128;
   __shared__ __align__(16) bf16 As[BM * LD];
   __shared__ __align__(16) bf16 Bs[BN * LD];
@@ -553,35 +567,67 @@ __device__ __forceinline__ void stage_row_f32(float* dst, const TA* src, const i
 }
 
 // ---- ops on single entries of finished f32 rows: kernels of their own, or the tail of a product of few rows --------------------
+// Each is split in what it reads apart from its entry (a product's tail asks for that while the product runs) and the rest.
+struct NextNorm { float w, b; };
+__device__ __forceinline__ NextNorm next_norm(const fq3c_op& o, const int c) {
+  if (!o.norm_out) return NextNorm{0.f, 0.f};
+  const float* w = reinterpret_cast<const float*>(o.norm_w);
+  return NextNorm{w[c], w[o.N + c]};
+}
 // what follows a finished f32 value of the residual stream: the stream itself, its bf16 copy, and the next norm's output
-__device__ __forceinline__ void stream_out(const fq3c_op& o, const int m, const int c, const float v) {
+__device__ __forceinline__ void stream_out(const fq3c_op& o, const int m, const int c, const float v, const NextNorm& nn) {
   reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
   if (o.C2) reinterpret_cast<bf16*>(o.C2)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
   if (o.norm_out) {
-    const float* w = reinterpret_cast<const float*>(o.norm_w);
-    const float n = fmaf(tanhf(o.norm_eps * v), w[c], w[o.N + c]);
+    const float n = fmaf(tanhf(o.norm_eps * v), nn.w, nn.b);
     if (o.flags & FQ3C_F32) reinterpret_cast<float*>(o.norm_out)[(size_t)m * o.norm_ld + c] = n;
     else reinterpret_cast<bf16*>(o.norm_out)[(size_t)m * o.norm_ld + c] = __float2bfloat16_rn(n);
   }
 }
-__device__ __forceinline__ void dyt_at(const fq3c_op& o, const int m, const int c, const float x) {
-  float v = tanhf(o.f0 * x) * reinterpret_cast<const float*>(o.scale)[c];
-  if (o.bias) v += reinterpret_cast<const float*>(o.bias)[c];
-  if (o.flags & FQ3C_RESID) v += reinterpret_cast<const float*>(o.res)[(size_t)m * o.ldr + c];
-  if (o.flags & FQ3C_OUT_F32) stream_out(o, m, c, v);
-  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+struct DytEntry { float w, b, r; NextNorm nn; };
+__device__ __forceinline__ DytEntry dyt_entry(const fq3c_op& o, const int m, const int c) {
+  return DytEntry{reinterpret_cast<const float*>(o.scale)[c], o.bias ? reinterpret_cast<const float*>(o.bias)[c] : 0.f,
+                  o.flags & FQ3C_RESID ? reinterpret_cast<const float*>(o.res)[(size_t)m * o.ldr + c] : 0.f, next_norm(o, c)};
 }
-__device__ __forceinline__ void depth_mix_at(const fq3c_op& o, const int m, const int c) {
+__device__ __forceinline__ float dyt_at(const fq3c_op& o, const int m, const int c, const float x, const DytEntry& e) {
+  float v = tanhf(o.f0 * x) * e.w;
+  if (o.bias) v += e.b;
+  if (o.flags & FQ3C_RESID) v += e.r;
+  if (o.flags & FQ3C_OUT_F32) stream_out(o, m, c, v, e.nn);
+  else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
+  return v;
+}
+constexpr int MIX_AHEAD = 8;      // slices whose entries and weights are held ahead
+struct MixEntry { float a[MIX_AHEAD], w[MIX_AHEAD]; NextNorm nn; };
+__device__ __forceinline__ MixEntry mix_entry(const fq3c_op& o, const int m, const int c) {
+  MixEntry e;
+  const float* a = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + c;
+#pragma unroll
+  for (int j = 0; j < MIX_AHEAD; ++j) {
+    e.a[j] = j < o.i0 ? a[(size_t)j * (size_t)o.K] : 0.f;
+    e.w[j] = j < o.i0 ? reinterpret_cast<const float*>(o.p0)[j] : 0.f;
+  }
+  e.nn = next_norm(o, c);
+  return e;
+}
+// `fresh`: an entry that this thread wrote since mix_entry read it (or none)
+__device__ __forceinline__ void depth_mix_at(const fq3c_op& o, const int m, const int c, const MixEntry& e, const float* fresh, const float value) {
   const float* a = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + c;
   const float* w = reinterpret_cast<const float*>(o.p0);
   float v = 0.f;
-  for (int j = 0; j < o.i0; ++j) v = fmaf(w[j], a[(size_t)j * (size_t)o.K], v);
-  stream_out(o, m, c, v);
+#pragma unroll
+  for (int j = 0; j < MIX_AHEAD; ++j)
+    if (j < o.i0) v = fmaf(e.w[j], a + (size_t)j * (size_t)o.K == fresh ? value : e.a[j], v);
+  for (int j = MIX_AHEAD; j < o.i0; ++j) v = fmaf(w[j], a[(size_t)j * (size_t)o.K], v);
+  stream_out(o, m, c, v, e.nn);
 }
-__device__ __forceinline__ void xielu_at(const fq3c_op& o, const int m, const int c, const float z) {
+struct XieluEntry { float ap, aq; };
+__device__ __forceinline__ XieluEntry xielu_entry(const fq3c_op& o) {
   const float* p = reinterpret_cast<const float*>(o.p0);
-  const float ap = softplus_f(p[0]), aq = 0.5f + softplus_f(p[1]);
-  const float v = z > 0.f ? fmaf(ap * z, z, 0.5f * z) : fmaf(aq, expm1f(z) - z, 0.5f * z);
+  return XieluEntry{softplus_f(p[0]), 0.5f + softplus_f(p[1])};
+}
+__device__ __forceinline__ void xielu_at(const fq3c_op& o, const int m, const int c, const float z, const XieluEntry& e) {
+  const float v = z > 0.f ? fmaf(e.ap * z, z, 0.5f * z) : fmaf(e.aq, expm1f(z) - z, 0.5f * z);
   if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + c] = v;
   else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + c] = __float2bfloat16_rn(v);
 }
@@ -590,7 +636,8 @@ struct SeqTail { int n; fq3c_op op[2]; };
 
 // One output row with few rows in flight (decode: M <= 8): a warp per output column streams its weight row once, 16 bytes per
 // lane and load, and dots it with every A row (f32 or bf16 in shared memory as f32).  Bound by latency up to a few MB of weights: the launch, one trip to the weights
-// (the first loads leave before the rows are staged) and the reduction.
+// (the first loads leave before the launches in front have ended) and the reduction.  One row's entries go straight to the lanes that use them, and what the tail reads is asked for
+// in front of the sums: 17 products of a token 78 -> 60 us with the early launches, of which 12 are the latter two.
 // TAIL: lane m goes on with entry (m, n) of row m through the ops of `tail`, with their own arithmetic: each was a launch of its own of 2 us, of which a decoded token of
 // four layers had sixteen.
 template <typename TA, typename TB, bool TAIL = false>
@@ -607,20 +654,72 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
   const bool vec = ((reinterpret_cast<uintptr_t>(w) & 15) == 0) && (g.K % VEC == 0);
   // the first weight loads leave before the rows are staged: the two latencies overlap
   uint4 raw[U];
-  if (vec && n < g.N) {
+  auto first = [&] {
+    if (vec && n < g.N) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = (lane + 32 * u) * VEC;
-      raw[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+      for (int u = 0; u < U; ++u) {
+        const int k = (lane + 32 * u) * VEC;
+        raw[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+      }
     }
+  };
+  if (g.early) first();
+  seq_dep_begin(g.M);
+  if (!g.early) first();
+  // one row of whole 16-byte pieces: each lane's entries go straight to its registers
+  const bool direct = sizeof(TA) == sizeof(TB) && g.M == 1 && vec && (reinterpret_cast<uintptr_t>(Ap) & 15) == 0;
+  if (!direct) {
+    for (int m = 0; m < g.M; ++m) stage_row_f32<TA>(xs + (size_t)m * g.K, Ap + (size_t)m * g.lda, g.K, threadIdx.x, blockDim.x);
+    __syncthreads();
   }
-  for (int m = 0; m < g.M; ++m) stage_row_f32<TA>(xs + (size_t)m * g.K, Ap + (size_t)m * g.lda, g.K, threadIdx.x, blockDim.x);
-  __syncthreads();
   if (n >= g.N) return;
+  DytEntry dyt{};
+  MixEntry mix{};
+  XieluEntry xielu{};
+  if (TAIL && lane < g.M) {      // what the tail reads apart from its entry
+    if (tail.op[0].kind == FQ3C_XIELU) xielu = xielu_entry(tail.op[0]);
+    else dyt = dyt_entry(tail.op[0], lane, n);
+    if (tail.n > 1) mix = mix_entry(tail.op[1], lane, n);
+  }
   float acc[8];
 #pragma unroll
   for (int m = 0; m < 8; ++m) acc[m] = 0.f;
-  if (vec) {
+  auto entries = [](const uint4& r, float (&v)[VEC]) {
+    if (sizeof(TB) == 2) {
+      const uint32_t q4[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { v[(2 * q) % VEC] = __uint_as_float(q4[q] << 16); v[(2 * q + 1) % VEC] = __uint_as_float(q4[q] & 0xffff0000u); }
+    } else {
+      v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2 % VEC] = __uint_as_float(r.z); v[3 % VEC] = __uint_as_float(r.w);
+    }
+  };
+  if (direct) {
+    auto row = [&](const int k) { return k < g.K ? *reinterpret_cast<const uint4*>(Ap + k) : make_uint4(0u, 0u, 0u, 0u); };
+    uint4 a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) a[u] = row((lane + 32 * u) * VEC);
+    for (int k0 = lane * VEC; k0 < g.K; k0 += 32 * U * VEC) {
+      uint4 nxt[U], an[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + 32 * (U + u) * VEC;
+        nxt[u] = k < g.K ? __ldg(reinterpret_cast<const uint4*>(w + k)) : make_uint4(0u, 0u, 0u, 0u);
+        an[u] = row(k);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k0 + 32 * u * VEC < g.K) {
+          float wv[VEC], xv[VEC];
+          entries(raw[u], wv);
+          entries(a[u], xv);
+#pragma unroll
+          for (int q = 0; q < VEC; ++q) acc[0] = fmaf(wv[q], xv[q], acc[0]);
+        }
+        raw[u] = nxt[u];
+        a[u] = an[u];
+      }
+    }
+  } else if (vec) {
     for (int k0 = lane * VEC; k0 < g.K; k0 += 32 * U * VEC) {
       uint4 nxt[U];
 #pragma unroll
@@ -633,13 +732,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
         const int k = k0 + 32 * u * VEC;
         if (k < g.K) {
           float wv[VEC];
-          if (sizeof(TB) == 2) {
-            const uint32_t q4[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) { wv[(2 * q) % VEC] = __uint_as_float(q4[q] << 16); wv[(2 * q + 1) % VEC] = __uint_as_float(q4[q] & 0xffff0000u); }
-          } else {
-            wv[0] = __uint_as_float(raw[u].x); wv[1] = __uint_as_float(raw[u].y); wv[2 % VEC] = __uint_as_float(raw[u].z); wv[3 % VEC] = __uint_as_float(raw[u].w);
-          }
+          entries(raw[u], wv);
 #pragma unroll
           for (int m = 0; m < 8; ++m)
             if (m < g.M) {
@@ -669,9 +762,13 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
     }
     if (lane < g.M) {
       reinterpret_cast<float*>(g.C)[(size_t)lane * g.ldc + n] = v;
-      if (tail.op[0].kind == FQ3C_XIELU) xielu_at(tail.op[0], lane, n, v);
-      else dyt_at(tail.op[0], lane, n, v);
-      if (tail.n > 1) depth_mix_at(tail.op[1], lane, n);
+      float y = 0.f;
+      if (tail.op[0].kind == FQ3C_XIELU) xielu_at(tail.op[0], lane, n, v, xielu);
+      else y = dyt_at(tail.op[0], lane, n, v, dyt);
+      if (tail.n > 1) {
+        const bool f32 = tail.op[0].flags & FQ3C_OUT_F32;
+        depth_mix_at(tail.op[1], lane, n, mix, f32 ? reinterpret_cast<const float*>(tail.op[0].C) + (size_t)lane * tail.op[0].ldc + n : nullptr, y);
+      }
     }
     return;
   }
@@ -710,6 +807,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
 // expert comes from the segment starts, a warp per output column streams that expert's weight row once with 16-byte loads.
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(256) fq3s_ggemv_kernel(const SeqGemm g) {
+  seq_dep_begin(g.M);
   extern __shared__ float xs[];  // [K]
   const int p = blockIdx.y;
   int e = 0;
@@ -776,6 +874,7 @@ __global__ void __launch_bounds__(256) fq3s_ggemv_kernel(const SeqGemm g) {
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename TB>
 __global__ void fq3s_embed_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int m = blockIdx.x;
   const int id = reinterpret_cast<const int*>(o.A)[m];
   const TB* row = reinterpret_cast<const TB*>(o.B) + (size_t)id * o.N;
@@ -792,6 +891,7 @@ __global__ void fq3s_embed_kernel(const fq3c_op o) {
 
 // grid (ceil(N / 256), M + taps - 1): rows >= M write the next history
 __global__ void __launch_bounds__(256) fq3s_tconv_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= o.N) return;
   const int m = blockIdx.y, h = o.taps - 1;
@@ -821,6 +921,7 @@ __global__ void __launch_bounds__(256) fq3s_tconv_kernel(const fq3c_op o) {
 constexpr int TC_ROWS = 8;
 template <int TAPS>
 __global__ void __launch_bounds__(128) fq3s_tconv_vec_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= o.N) return;
   const int h = o.taps - 1, m0 = blockIdx.y * TC_ROWS;
@@ -877,6 +978,7 @@ __global__ void __launch_bounds__(128) fq3s_tconv_vec_kernel(const fq3c_op o) {
 // with period i2 when i2 > 0; divisors (bias, pitch cin) divide a group before anything else.
 __device__ __forceinline__ float gate_f(const float z, const bool plain) { return plain ? sigmoid_f(z) : z / (1.f + expf(-z)); }
 __global__ void __launch_bounds__(1024) fq3s_gnorm_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   __shared__ float red[32];
   const int m = blockIdx.x, gsz = o.N / o.i0, c0 = blockIdx.y * gsz;
   const float* x = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda + c0;
@@ -928,6 +1030,7 @@ __device__ __forceinline__ void st4(bf16* p, const float (&v)[4]) {
 // The same norm for many (row, group) pairs: a warp each, the group in registers, 16-byte loads.  grid (ceil(M * groups / 4)), 128 threads.
 constexpr int GN_VECS = 4;
 __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const long long pair = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (pair >= (long long)o.M * o.i0) return;
   const int lane = threadIdx.x & 31, m = (int)(pair / o.i0), gi = (int)(pair - (long long)m * o.i0), gsz = o.N / o.i0, c0 = gi * gsz;
@@ -987,6 +1090,7 @@ __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
 }
 
 __global__ void __launch_bounds__(256) fq3s_polynorm_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   __shared__ float red[32];
   const int m = blockIdx.x;
   const float* x = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda;
@@ -1021,6 +1125,7 @@ __device__ __forceinline__ void lru_coeffs(const fq3c_op& o, int t, int c, float
   b = sqrtf(fmaxf(-expm1f(2.f * la), 0.f)) * ig * u;
 }
 __global__ void __launch_bounds__(128) fq3s_lru_fold_kernel(const fq3c_op o, const int chunks, const int per, float* carry) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   if (c >= o.N) return;
   const float sp = softplus_f(reinterpret_cast<const float*>(o.scale)[c]);
@@ -1036,6 +1141,7 @@ __global__ void __launch_bounds__(128) fq3s_lru_fold_kernel(const fq3c_op o, con
   carry[((size_t)q * 2 + 1) * o.N + c] = s;
 }
 __global__ void __launch_bounds__(128) fq3s_lru_scan_kernel(const fq3c_op o, const int chunks, const int per, const float* carry) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   if (c >= o.N) return;
   const float sp = softplus_f(reinterpret_cast<const float*>(o.scale)[c]);
@@ -1116,6 +1222,7 @@ __device__ __forceinline__ void router_token(const fq3c_op& o, const int m, floa
 // With ws / p0 / p1 set (a single token, at most 16 choices, K = experts that have tensors) the launch also does the grouping
 // by expert that fq3s_moe_sort_kernel does for many tokens: segment starts -> p0, rows -> p1, each choice's place -> ws.
 __global__ void fq3s_router_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ float rsm[];
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < o.M) router_token(o, m, rsm, blockDim.x, threadIdx.x);
@@ -1146,6 +1253,7 @@ __global__ void fq3s_router_kernel(const fq3c_op o) {
 // same expert find each other with one match, so that only a count per (warp, expert) is walked serially - with one per (thread, expert) that walk over 1024 shares was
 // all the time there is.  1402 pairs of 16 experts 12.5 -> 4.6 us, 8192 of 32 25.6 -> 16.7; what is left are two passes over the pairs and four block barriers.
 __global__ void __launch_bounds__(1024) fq3s_moe_sort_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ int ssm[];   // [E + 1] starts, then [warps][E] counts
   const int E = o.i1, n = o.M * o.i0, nth = blockDim.x, warps = nth >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* ids = reinterpret_cast<const int*>(o.A);
@@ -1203,6 +1311,7 @@ __global__ void __launch_bounds__(1024) fq3s_moe_sort_kernel(const fq3c_op o) {
 }
 
 __global__ void __launch_bounds__(256) fq3s_moe_combine_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int m = blockIdx.x, top = o.i0;
   const int* ids = reinterpret_cast<const int*>(o.p0) + (size_t)m * top;
   const float* w = o.p1 ? reinterpret_cast<const float*>(o.p1) + (size_t)m * top : nullptr;
@@ -1225,6 +1334,7 @@ __global__ void __launch_bounds__(256) fq3s_moe_combine_kernel(const fq3c_op o) 
 
 // grid (copies, 8)
 __global__ void __launch_bounds__(256) fq3s_commit_kernel(const long long* desc, int* counter, int by) {
+  seq_dep_begin(by);
   const long long* d = desc + (size_t)blockIdx.x * 3;
   uint32_t* dst = reinterpret_cast<uint32_t*>(d[0]);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(d[1]);
@@ -1245,6 +1355,7 @@ __host__ __device__ inline size_t latent_attn_smem(int HG, int R, int E) {
 }
 template <typename TC>
 __global__ void __launch_bounds__(256) fq3s_latent_attn_kernel(const fq3c_op o, const int HG, const int splits) {
+  seq_dep_begin(o.M);
   extern __shared__ float lsm[];
   // E more columns behind the R latent ones (a rotated key part) enter the scores only; D = R + E is a cache row's width
   const int R = o.i1, E = o.cin, D = R + E, H = o.i0, m = blockIdx.x, h0 = blockIdx.y * HG, z = blockIdx.z;
@@ -1341,6 +1452,7 @@ __global__ void __launch_bounds__(256) fq3s_latent_attn_kernel(const fq3c_op o, 
 // grid (M, H).  The splits' maxima and sums are read once (a thread per split), their weights exp(max_s - max) live in shared
 // memory, and every thread then adds its columns with the loads of eight splits in flight.
 __global__ void __launch_bounds__(128) fq3s_latent_merge_kernel(const fq3c_op o, const int splits) {
+  seq_dep_begin(o.M);
   __shared__ float wsm[64];
   __shared__ float red[8];
   const int R = o.i1, H = o.i0, m = blockIdx.x, h = blockIdx.y;
@@ -1402,6 +1514,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 template <int NTM>
 __global__ void __launch_bounds__(256) fq3s_latent_attn_mma_kernel(const fq3c_op o, const int RS, const int splits, const int TJ, const int QB) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) unsigned char lm_raw[];
   const int R = o.i1, E = o.cin, D = R + E, H = o.i0, LDQ = D + 8;      // E score-only columns behind the R latent ones
   bf16* Qs = reinterpret_cast<bf16*>(lm_raw);          // [QB][16][LDQ]
@@ -1586,20 +1699,23 @@ __global__ void __launch_bounds__(256) fq3s_latent_attn_mma_kernel(const fq3c_op
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_dyt_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c < o.N) dyt_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c]);
+  if (c < o.N) dyt_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c], dyt_entry(o, m, c));
 }
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_depth_mix_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c < o.N) depth_mix_at(o, m, c);
+  if (c < o.N) depth_mix_at(o, m, c, mix_entry(o, m, c), nullptr, 0.f);
 }
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_xielu_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (c < o.N) xielu_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c]);
+  if (c < o.N) xielu_at(o, m, c, reinterpret_cast<const float*>(o.A)[(size_t)m * o.lda + c], xielu_entry(o));
 }
 
 // the mean of the P rows of block b of a cache -> row b of its pooled rows, for columns c0, c0 + step, .. below c1
@@ -1615,6 +1731,7 @@ __device__ __forceinline__ void pool_run(const TC* cache, const int ld, TC* pool
 // grid (M / P + 1, ceil(i1 * max(i2, cin) / 256), 2): z = 0 keys, 1 values
 template <typename TC>
 __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int pos0 = o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0, P = o.m_begin, b = pos0 / P + blockIdx.x;
   if ((b + 1) * P > pos0 + o.M) return;
   const int c = blockIdx.y * blockDim.x + threadIdx.x, n = o.i1 * (blockIdx.z ? o.cin : o.i2);
@@ -1631,6 +1748,7 @@ __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) 
 // fq3s_pool_append_kernel behind this launch.
 template <typename TC, bool POOL = false, int THREADS = 256>
 __global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int m = blockIdx.x, H = o.i0, G = o.i1, d = o.i2, dv = o.cin, half = o.taps >> 1;
   const int pos = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;
   float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda;
@@ -1755,6 +1873,7 @@ __device__ __forceinline__ void ca_stage_rows(float* dst, const int dld, const T
 }
 template <typename TC, bool POOL = false>
 __global__ void __launch_bounds__(256) fq3s_cache_attn_kernel(const fq3c_op o, const int QB, const int TJ, const int splits) {
+  seq_dep_begin(o.M);
   extern __shared__ float csm[];
   const int H = o.i0, G = o.i1, d = o.i2, dv = o.cin, HG = H / G, R = QB * HG;
   const int m0 = blockIdx.x * QB, g = blockIdx.y, z = blockIdx.z;
@@ -1874,6 +1993,7 @@ __global__ void __launch_bounds__(256) fq3s_cache_attn_kernel(const fq3c_op o, c
 
 // grid (M, H), 128 threads
 __global__ void __launch_bounds__(128) fq3s_cache_attn_merge_kernel(const fq3c_op o, const int splits) {
+  seq_dep_begin(o.M);
   __shared__ float wsm[64];
   __shared__ float red[32];
   const int m = blockIdx.x, h = blockIdx.y, H = o.i0, dv = o.cin;
@@ -1926,6 +2046,7 @@ __device__ __forceinline__ float fast_tanh(float x) {
 __host__ __device__ inline size_t cache_attn_mma_smem(int rows, int d, int dv) { return 2 * ((size_t)rows * (d + 8) + 2 * (size_t)CM_TJ * (d + 8) + 2 * (size_t)CM_TJ * (dv + 8)); }
 template <int NTM, bool POOL = false>      // POOL: tiles of pooled blocks in front of the tokens' (a variant of its own: the plain one compiles as it always did)
 __global__ void __launch_bounds__(256) fq3s_cache_attn_mma_kernel(const fq3c_op o, const int ROWS) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) unsigned char cm_raw[];
   const int H = o.i0, G = o.i1, d = o.i2, dv = o.cin, HG = H / G, QBLK = ROWS / HG, LDK = d + 8, LDV = dv + 8;
   bf16* Qs = reinterpret_cast<bf16*>(cm_raw);            // [ROWS][LDK]
@@ -2190,6 +2311,7 @@ constexpr int MS_MAX_RANK = 1024;     // inner size of the decay projection (mod
 constexpr int MS_PREP_ROWS = 8;       // rows per block of the first launch in mode 2
 // grid (M), or (ceil(M / MS_PREP_ROWS)) in mode 2; 128 threads
 __global__ void __launch_bounds__(128) fq3s_mstate_prep_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int m = blockIdx.x, H = o.i0, G = o.i1, dk = o.i2;
   if (o.taps == 2) {
     // z = U lat + b with the row's decay latent lat (m_begin entries of the raw rows, f32) and U = B [H * dk, m_begin] (bf16, F32: f32):
@@ -2309,6 +2431,7 @@ __device__ __forceinline__ void cdelta_up(const fq3c_op& o, const float* lat, co
 __host__ __device__ constexpr int cdelta_prep_channels(int rows) { return rows == 1 ? 128 : 512; }
 template <int ROWS>
 __global__ void __launch_bounds__(256) fq3s_mstate_cdelta_prep_kernel(const fq3c_op o, const bool logs) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) float cd_lat[];       // [inner size][8]
   const int H = o.i0, G = o.i1, dk = o.i2, m0 = blockIdx.x * MS_PREP_ROWS, nr = min(ROWS, o.M - m0), tid = threadIdx.x;
   constexpr int nth = 256, per = cdelta_prep_channels(ROWS);
@@ -2399,6 +2522,7 @@ __device__ __forceinline__ void forget_coeffs(const float q, const float z, cons
 }
 // grid (M, ceil(H * dk / 256)): ws row m of mode 4
 __global__ void __launch_bounds__(256) fq3s_mstate_gate_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int m = blockIdx.x, n = o.i0 * o.i2, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const float* raw = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda;
@@ -2416,6 +2540,7 @@ __device__ __forceinline__ void log_gates(const float zi, const float zf, const 
 // rounding, numerator, normaliser and e^(-m) refer to the same one.  Rows are fetched MM_BATCH at a time, ahead of the stores.
 constexpr int MM_THREADS = 512, MM_BATCH = 4;
 __global__ void __launch_bounds__(MM_THREADS) fq3s_mstate_max_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   __shared__ float sa[MM_THREADS], sb[MM_THREADS];
   const int h = blockIdx.x, H = o.i0, tid = threadIdx.x, per = (o.M + MM_THREADS - 1) / MM_THREADS, t0 = min(o.M, tid * per), t1 = min(o.M, t0 + per);
   const int cols = mstate_max_cols(H);
@@ -2519,6 +2644,7 @@ __host__ __device__ constexpr int mstate_buf_floats(int rpt, int nv = 2, int cpt
 // o = S'^T q + u (q . k), so both products run in the pass that decays the state, with one round of shuffles.
 template <int RPT, int NV = 2, bool GATED = false, int CPT = 1, bool CDELTA = false>
 __global__ void __launch_bounds__(128) fq3s_mstate_scan_kernel(const fq3c_op o, const int phase, const int piece, float* X, float* P) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) float msm[];
   constexpr int SL = RPT + 4, ROW = 8 * SL, CH = mstate_ch(CPT), COLS = MS_COLS * CPT;
   constexpr bool PK = NV == 2;      // with three staged vectors the walk is bound by shared memory, and pairs only cost registers
@@ -2836,6 +2962,7 @@ __global__ void __launch_bounds__(128) fq3s_mstate_scan_kernel(const fq3c_op o, 
 
 // grid (ceil(H * dk * sv / 256)), sv state columns: X[0] = the carried state; X[z + 1] = P[z] X[z] + X[z + 1] for the pieces in order.
 __global__ void __launch_bounds__(256) fq3s_mstate_carry_kernel(const fq3c_op o, const int pieces, float* X, const float* P, const int sv) {
+  seq_dep_begin(o.M);
   const size_t n = (size_t)o.i0 * o.i2 * sv, e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const size_t hi = e / sv;        // (head, state row)
@@ -2877,6 +3004,7 @@ constexpr float LOG2E_F = 1.4426950408889634f;
 __device__ __forceinline__ float pow2_f(const float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 // grid (blocks of tokens, H), CD_REC_THREADS threads; dynamic shared memory: sums (two floats), q and k, [CD_C][pitch] each
 __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(16) float cr[];
   __shared__ float beta[CD_C], N[CD_C][CD_C], fq[CD_C], fk[CD_C];
   const int H = o.i0, G = o.i1, dk = o.i2, h = blockIdx.y, g = h / (H / G), t0 = blockIdx.x * CD_C, tid = threadIdx.x;
@@ -3032,6 +3160,7 @@ __host__ __device__ constexpr int cd_walk_floats(int dk) {
 }
 template <int DVT, int RQ>
 __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ __align__(128) float cw[];
   __shared__ __align__(8) unsigned long long full[2];
   constexpr int NCP = DVT / 2, QS = 128 / NCP, CG = DVT / 4, KH = 4 / CG, PP = DVT + 1, JW = DVT / 4;
@@ -3229,6 +3358,7 @@ constexpr int HY_MAX = 16;      // streams; the kernel comes in an 8- and a 16-s
 // sublayer's output is given) and forms u; a second one norms it.  Everything f32.
 template <int MAXS>
 __global__ void __launch_bounds__(256) fq3s_hyper_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ float hsm[];
   __shared__ float red[32];
   const int m = blockIdx.x, S = o.i0;
@@ -3280,6 +3410,7 @@ __global__ void __launch_bounds__(256) fq3s_hyper_kernel(const fq3c_op o) {
 
 // grid (ceil(N / 256), M)
 __global__ void __launch_bounds__(256) fq3s_glu_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   const int c = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
   if (c >= o.N) return;
   const int r = o.ws ? reinterpret_cast<const int*>(o.ws)[q] : q;
@@ -3300,6 +3431,7 @@ __global__ void __launch_bounds__(256) fq3s_glu_kernel(const fq3c_op o) {
 // and keeps it; passes 2 and 3 take the mean and the mean squared deviation from the kept row; pass 4 writes the normed row.
 // A thread only ever reads back entries it wrote itself, and C may be slice 0 (every entry is read before it is written).
 __global__ void __launch_bounds__(1024) fq3s_sum_norm_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   extern __shared__ float snm[];
   __shared__ float red[32];
   const int m = blockIdx.x;
@@ -3351,6 +3483,7 @@ __global__ void __launch_bounds__(1024) fq3s_sum_norm_kernel(const fq3c_op o) {
 // The same for rows of whole 16-byte pieces: the row stays in registers.  grid (M), up to 256 threads.
 constexpr int SN_VECS = 4;
 __global__ void __launch_bounds__(256) fq3s_sum_norm_vec_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
   __shared__ float red[32];
   const int m = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
   const float* a = reinterpret_cast<const float*>(o.A) + (size_t)m * o.lda;
