@@ -1846,6 +1846,75 @@ void gemv_tail(const fq3c_op& o, const SeqGemm& g, const fq3c_op* next, const in
     if (q.kind == FQ3C_XIELU) return;
   }
 }
+// ---- attention over a cache, few rows ------------------------------------------------------------------------------------------
+bool rot_append_ok(const fq3c_op& o) {
+  return o.A && o.i0 >= 0 && o.i1 >= 0 && o.i2 >= 1 && o.taps >= 0 && !(o.taps & 1) && o.taps <= o.i2 && (o.taps == 0 || o.B) && (o.i1 == 0 || (o.C && (o.cin <= 0 || o.C2)));
+}
+const char* cache_attn_error(const fq3c_op& o) {
+  if (o.i0 < 1 || o.i1 < 1 || o.i0 % o.i1 || o.i2 < 1 || o.cin < 1 || !o.A || !o.B || !o.p1 || !o.C) return "cache_attn: bad configuration";
+  const int splits = std::max(1, o.m_begin);
+  if (o.tap_off[1] > 0 && (o.K < 1 || !o.C2 || !o.norm_out || o.bias || o.tap_off[0] > 0 || o.a_rows > 0))
+    return "cache_attn: pooled blocks go with a window and their pooled rows, not with kept first positions, a chunked mask or a distance penalty";
+  if (splits > 64) return "cache_attn: at most 64 key splits";
+  if (splits > 1 && (!o.ws || o.ws_bytes < (int64_t)o.M * o.i0 * splits * (o.cin + 2) * 4)) return "cache_attn: workspace too small for the splits";
+  return nullptr;
+}
+// Which calls of few rows go to fq3s_attn_few_kernel: what its accesses and variants ask for, and as many keys as the eight CTAs of a cluster walk faster than up to 64 do with a second
+// launch to merge them.  That is told by the keys that a row may see (the window, or what 32 per split say): one row behind 2000 positions, 4 heads a key head, 20.8 us by itself and 15.9
+// here, behind 8000 35.6 and 46.3; 8 heads a key head behind 1000 17.1 and 15.4, behind 2000 21.3 and 24.2; one head a key head behind 8000 30.8 and 28.7.
+bool attn_few_takes(const fq3c_op& o) {
+  const int splits = std::max(1, o.m_begin);
+  const long keys = o.K > 0 && o.a_rows <= 0 ? o.K : o.tap_off[0] > 0 ? o.tap_off[0] : splits < 64 ? 32L * splits : 1L << 30;
+  auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  const int V = o.flags & FQ3C_F32 ? 4 : 8, HG = o.i1 > 0 ? o.i0 / o.i1 : 0;
+  return o.M <= DEP_ROWS && (HG == 1 || keys <= (HG == 8 ? 1024 : 2048)) && (o.i2 == 64 || o.i2 == 128) && o.cin == o.i2 && o.i0 >= 1 && o.i1 >= 1 && o.i0 % o.i1 == 0 && (HG <= 4 || HG == 8) && o.i1 <= 65535 && o.tap_off[1] <= 0 &&
+         o.A && o.B && o.p1 && o.C && o.ldr % V == 0 && o.taps % V == 0 && !off(o.B) && !off(o.p1);
+}
+// `r` (rotation, cache rows) and the attention `o` of the same single row behind it
+bool attn_few_takes_rot(const fq3c_op& r, const fq3c_op& o) {
+  if (o.kind != FQ3C_CACHE_ATTN || r.M != 1 || o.M != 1 || r.m_begin > 0 || !attn_few_takes(o) || o.A != r.A || o.i0 != r.i0 || o.i2 != r.i2 || o.p0 != r.p0 || ((o.flags ^ r.flags) & FQ3C_F32)) return false;
+  if (r.i1 > 0 && (r.i1 != o.i1 || r.cin != o.cin || r.C != o.B || r.ldc != o.ldr || r.C2 != o.p1 || r.ldr != o.taps || r.C == r.C2)) return false;
+  // What one CTA writes early, others still read: the turned queries, the finished outputs
+  auto apart = [](const void* a, const long na, const void* b, const long nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return !a || !b || x + na <= y || y + nb <= x;
+  };
+  const long nq = 4L * o.i0 * o.i2, nk = 4L * r.i1 * r.i2, nout = (long)o.i0 * o.cin * (o.flags & FQ3C_OUT_F32 ? 4 : 2), ngate = 4L * (o.flags & FQ3C_GATE_ENTRY ? o.i0 * o.cin : o.i0);
+  const float* krow = reinterpret_cast<const float*>(r.res ? r.res : r.A);
+  const void* written[2] = {o.A, o.C};
+  const long bytes[2] = {nq, nout};
+  for (int w = 0; w < 2; ++w) {
+    if (r.i1 > 0 && (!apart(written[w], bytes[w], krow + r.K, nk) || !apart(written[w], bytes[w], krow + r.a_rows, nk))) return false;
+    if (!apart(written[w], bytes[w], o.res, ngate) || !apart(written[w], bytes[w], o.scale, 4L * o.i0) || !apart(written[w], bytes[w], o.bias, 8L * o.i0)) return false;
+    if (!apart(written[w], bytes[w], r.B, 2L * r.taps) || !apart(written[w], bytes[w], r.p1, 2L * r.taps) || !apart(written[w], bytes[w], r.scale, 4L * r.i2) || !apart(written[w], bytes[w], r.bias, 4L * r.i2) ||
+        !apart(written[w], bytes[w], o.p0, 4)) return false;
+  }
+  return apart(o.A, nq, o.C, nout);
+}
+template <typename TC, int D, bool ROT>
+void launch_attn_few(const fq3c_op& o, const fq3c_op& r, cudaStream_t s, const bool after) {
+  const int HG = o.i0 / o.i1;
+  const dim3 grid(AF_RANKS, (unsigned)o.i1, (unsigned)o.M);
+  const size_t smem = sizeof(float) * af_floats(HG, D);
+  if (HG == 1) launch_after(fq3s_attn_few_kernel<TC, D, 1, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 2) launch_after(fq3s_attn_few_kernel<TC, D, 2, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 3) launch_after(fq3s_attn_few_kernel<TC, D, 3, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 4) launch_after(fq3s_attn_few_kernel<TC, D, 4, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else launch_after(fq3s_attn_few_kernel<TC, D, 8, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+}
+// r: the ROT_APPEND in front that goes with it, or null
+void launch_attn_few(const fq3c_op& o, const fq3c_op* r, cudaStream_t s, const bool after) {
+  const bool f32 = (o.flags & FQ3C_F32) != 0;
+  const fq3c_op& q = r ? *r : o;
+  if (r) {
+    if (f32) { if (o.i2 == 64) launch_attn_few<float, 64, true>(o, q, s, after); else launch_attn_few<float, 128, true>(o, q, s, after); }
+    else { if (o.i2 == 64) launch_attn_few<bf16, 64, true>(o, q, s, after); else launch_attn_few<bf16, 128, true>(o, q, s, after); }
+  } else {
+    if (f32) { if (o.i2 == 64) launch_attn_few<float, 64, false>(o, q, s, after); else launch_attn_few<float, 128, false>(o, q, s, after); }
+    else { if (o.i2 == 64) launch_attn_few<bf16, 64, false>(o, q, s, after); else launch_attn_few<bf16, 128, false>(o, q, s, after); }
+  }
+}
+
 int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
   switch (o.kind) {
     case FQ3C_EMBED:
@@ -2014,9 +2083,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       return 0;
     }
     case FQ3C_ROT_APPEND: {
-      if (!o.A || o.i0 < 0 || o.i1 < 0 || o.i2 < 1 || o.taps < 0 || (o.taps & 1) || o.taps > o.i2 || (o.taps > 0 && !o.B) ||
-          (o.i1 > 0 && (!o.C || (o.cin > 0 && !o.C2))))
-        return fail("rot_append: bad configuration");
+      if (!rot_append_ok(o)) return fail("rot_append: bad configuration");
       if (o.m_begin > 0 && (o.i1 < 1 || o.cin < 1 || !o.norm_out || !o.ws || !o.p0)) return fail("rot_append: pooled blocks need both caches, their pooled rows and a position");
       const int rth = o.M <= 8 ? std::max(256, std::min(1024, 32 * (o.i0 + o.i1))) : 256;      // few rows: a warp per head
       if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, true, 1024>, 1, rth, 0, s, after, 1, o);
@@ -2034,13 +2101,13 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       return 0;
     }
     case FQ3C_CACHE_ATTN: {
-      if (o.i0 < 1 || o.i1 < 1 || o.i0 % o.i1 || o.i2 < 1 || o.cin < 1 || !o.A || !o.B || !o.p1 || !o.C) return fail("cache_attn: bad configuration");
+      if (const char* e = cache_attn_error(o)) return fail(e);
       const int splits = std::max(1, o.m_begin), HG = o.i0 / o.i1;
       const bool pool = o.tap_off[1] > 0;
-      if (pool && (o.K < 1 || !o.C2 || !o.norm_out || o.bias || o.tap_off[0] > 0 || o.a_rows > 0))
-        return fail("cache_attn: pooled blocks go with a window and their pooled rows, not with kept first positions, a chunked mask or a distance penalty");
-      if (splits > 64) return fail("cache_attn: at most 64 key splits");
-      if (splits > 1 && (!o.ws || o.ws_bytes < (int64_t)o.M * o.i0 * splits * (o.cin + 2) * 4)) return fail("cache_attn: workspace too small for the splits");
+      if (attn_few_takes(o)) {
+        launch_attn_few(o, nullptr, s, after);
+        return 0;
+      }
       // bf16 cache and a prompt portion: the tensor-core kernels (FQ3S_ATTN_MMA=0: CUDA cores everywhere).  Heads of 128 on tcgen05 from 9 rows on: against the
       // mma.sync kernel 9 rows of 16 heads over 4 behind 2000 positions 185 and 51 us, 1000 rows 303 and 76; only short portions at the very
       // beginning are slower (33-64 rows at position 0: 10.7-11.5 and 12.9), and the host does not know where a portion begins.
@@ -2665,6 +2732,13 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         fq3c_advance_kernel<<<1, 1, 0, s>>>(reinterpret_cast<int*>(o.C), o.i0);
         break;
       }
+      case FQ3C_ROT_APPEND:
+        if (i + 1 < n_ops && rot_append_ok(o) && attn_few_takes_rot(o, ops[i + 1]) && !cache_attn_error(ops[i + 1])) {      // with the attention behind it in one launch
+          ++i;
+          launch_attn_few(ops[i], &o, s, after);
+          break;
+        }
+        [[fallthrough]];
       default: {
         const int rc = seq_run(o, s, after && (o.kind == FQ3C_COMMIT ? o.i0 : o.M) <= DEP_ROWS);
         if (rc == 1) return fail("unknown op kind");

@@ -1746,59 +1746,66 @@ __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) 
 // m_begin = P > 0: every run of P positions bP .. bP + P - 1 that the step completes leaves the mean of its P cached keys and values as
 // row b of norm_out / ws.  A single row does it here (POOL; its block has just written the run's last row); more rows take
 // fq3s_pool_append_kernel behind this launch.
-template <typename TC, bool POOL = false, int THREADS = 256>
-__global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op o) {
-  seq_dep_begin(o.M);
-  const int m = blockIdx.x, H = o.i0, G = o.i1, d = o.i2, dv = o.cin, half = o.taps >> 1;
-  const int pos = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;
-  float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda;
-  const float* krow = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.norm_ld : row;
+// A warp turns (norms, tempers) one query or key head at position pos; put(i, v) takes entry i.  all: also the entries that stay as they are.
+template <typename Put>
+__device__ __forceinline__ void rot_head(const fq3c_op& o, const float* src, const bool isq, const int pos, const int lane, const bool all, Put put) {
+  const int d = o.i2, half = o.taps >> 1;
   const float* freq = reinterpret_cast<const float*>(o.B);
   const float* flo = reinterpret_cast<const float*>(o.p1);
   const float fp = (float)pos, amp = o.f1 != 0.f ? o.f1 : 1.f;
+  const float* nw = reinterpret_cast<const float*>(isq ? o.scale : o.bias);
+  const bool unit = nw || (o.flags & FQ3C_UNIT), normed = unit || (isq && o.f3 > 0.f);
+  float rs = 1.f;
+  if (unit) {
+    float ss = 0.f;
+    for (int c = lane; c < d; c += 32) ss = fmaf(src[c], src[c], ss);
+    rs = 1.f / sqrtf(warp_sum(ss) / (float)d + o.f0);
+  }
   // query temperature: grows with every f3 positions (the quotient of two integers below 2^24 never rounds up to the next integer)
-  const float temp = o.f3 > 0.f ? fmaf(o.f2, logf(floorf((fp + 1.f) / o.f3) + 1.f), 1.f) : 1.f;
+  if (isq) rs *= o.f3 > 0.f ? fmaf(o.f2, logf(floorf((fp + 1.f) / o.f3) + 1.f), 1.f) : 1.f;
+  const bool halves = (o.flags & FQ3C_ROT_HALF) != 0;      // pairs (i, i + half) instead of (2i, 2i + 1)
+  for (int i = lane; i < half; i += 32) {
+    float sn, cs;
+    const float ang = fp * freq[i];
+    sincosf(ang, &sn, &cs);
+    // what the product (and, with p1, the frequency) lost to rounding turns the pair a little further: at large angles it would show
+    float rest = fmaf(fp, freq[i], -ang);
+    if (flo) rest = fmaf(fp, flo[i], rest);
+    const float s1 = fmaf(cs, rest, sn), c1 = fmaf(-sn, rest, cs);
+    sn = s1 * amp; cs = c1 * amp;
+    const int ia = halves ? i : 2 * i, ib = halves ? i + half : 2 * i + 1;
+    float a = src[ia], b = src[ib];
+    if (normed) { a *= rs; b *= rs; }
+    if (nw) { a *= nw[ia]; b *= nw[ib]; }
+    const float x = a * cs - b * sn, y = b * cs + a * sn;
+    put(ia, x);
+    put(ib, y);
+  }
+  if (isq && !normed && !all) return;     // the rest of a query head stays as it is
+  for (int c = 2 * half + lane; c < d; c += 32) {
+    float v = normed ? src[c] * rs : src[c];
+    if (nw) v *= nw[c];
+    put(c, v);
+  }
+}
+template <typename TC, bool POOL = false, int THREADS = 256>
+__global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
+  const int m = blockIdx.x, H = o.i0, G = o.i1, d = o.i2, dv = o.cin;
+  const int pos = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;
+  float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda;
+  const float* krow = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.norm_ld : row;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
   TC* kc = G > 0 ? reinterpret_cast<TC*>(o.C) + (size_t)pos * o.ldc : nullptr;
   for (int hh = warp; hh < H + G; hh += nwarp) {
     const bool isq = hh < H;
     const float* src = isq ? row + (size_t)hh * d : krow + o.K + (size_t)(hh - H) * d;
-    const float* nw = reinterpret_cast<const float*>(isq ? o.scale : o.bias);
-    const bool unit = nw || (o.flags & FQ3C_UNIT), normed = unit || (isq && o.f3 > 0.f);
-    float rs = 1.f;
-    if (unit) {
-      float ss = 0.f;
-      for (int c = lane; c < d; c += 32) ss = fmaf(src[c], src[c], ss);
-      rs = 1.f / sqrtf(warp_sum(ss) / (float)d + o.f0);
-    }
-    if (isq) rs *= temp;
     float* qd = isq ? row + (size_t)hh * d : nullptr;
     TC* kd = isq ? nullptr : kc + (size_t)(hh - H) * d;
-    const bool halves = (o.flags & FQ3C_ROT_HALF) != 0;      // pairs (i, i + half) instead of (2i, 2i + 1)
-    for (int i = lane; i < half; i += 32) {
-      float sn, cs;
-      const float ang = fp * freq[i];
-      sincosf(ang, &sn, &cs);
-      // what the product (and, with p1, the frequency) lost to rounding turns the pair a little further: at large angles it would show
-      float rest = fmaf(fp, freq[i], -ang);
-      if (flo) rest = fmaf(fp, flo[i], rest);
-      const float s1 = fmaf(cs, rest, sn), c1 = fmaf(-sn, rest, cs);
-      sn = s1 * amp; cs = c1 * amp;
-      const int ia = halves ? i : 2 * i, ib = halves ? i + half : 2 * i + 1;
-      float a = src[ia], b = src[ib];
-      if (normed) { a *= rs; b *= rs; }
-      if (nw) { a *= nw[ia]; b *= nw[ib]; }
-      const float x = a * cs - b * sn, y = b * cs + a * sn;
-      if (isq) { qd[ia] = x; qd[ib] = y; }
-      else { stf(kd + ia, x); stf(kd + ib, y); }
-    }
-    if (isq && !normed) continue;     // the rest of a query head stays as it is
-    for (int c = 2 * half + lane; c < d; c += 32) {
-      float v = normed ? src[c] * rs : src[c];
-      if (nw) v *= nw[c];
-      if (isq) qd[c] = v;
-      else stf(kd + c, v);
-    }
+    rot_head(o, src, isq, pos, lane, false, [&](const int i, const float v) {
+      if (isq) qd[i] = v;
+      else stf(kd + i, v);
+    });
   }
   if (G <= 0 || dv <= 0) return;
   TC* vc = reinterpret_cast<TC*>(o.C2) + (size_t)pos * o.ldr;
@@ -2023,6 +2030,251 @@ __global__ void __launch_bounds__(128) fq3s_cache_attn_merge_kernel(const fq3c_o
     if (entry) v *= sigmoid_f(gr[(size_t)h * dv + c]);
     if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + (size_t)h * dv + c] = v;
     else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + (size_t)h * dv + c] = __float2bfloat16_rn(v);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------
+// The same attention for up to eight rows (decoding), heads of D = 64 or 128: a cluster of eight CTAs per (row, key head) shares the keys, eight at a time to each of its 64 warps, and
+// its partial results meet in shared memory, where every CTA finishes an eighth of the outputs: one launch instead of one per 32 keys and one to merge.  Four lanes score a key (a
+// quarter of its entries each, 16 bytes at a time, straight from the cache), a lane sums D / 32 value columns; the next eight keys and values are on their way meanwhile.  Latency
+// bounds it: one trip to the keys and values, three meetings.  (Two CTAs an SM where there are more than SMs: 8 rows of 16 heads over 4 behind 220 positions 19.0 and 12.0 us; a single row is
+// faster with the registers, 7.5 and 8.2.)
+// ROT (one row): also the ROT_APPEND `r` in front of it, another launch: every CTA turns its query heads for itself, the first one also writes them back and the new key and value to
+// the caches; the CTA whose eight keys the new one is among reads it from its own shared memory.
+// Rotation and attention of one row of 16 heads over 4 behind 220 positions: 15.5 us in three launches, 7.5; 8 rows 25.8 and 12.0; one row of 32-bit caches behind 1000 15.5 and 10.8.
+// ---------------------------------------------------------------------------------------------------------------------------
+constexpr int AF_RANKS = 8, AF_WARPS = 8;
+template <int BYTES> struct AfVec;
+template <> struct AfVec<4> { typedef uint32_t T; };
+template <> struct AfVec<8> { typedef uint2 T; };
+template <> struct AfVec<16> { typedef uint4 T; };
+__host__ __device__ constexpr int af_floats(int hg, int D) {      // queries | new key and value | the warps' outputs, maxima and sums | what arrives from the cluster
+  return hg * D + 2 * D + AF_WARPS * hg * (D + 2) + hg * D + AF_RANKS * hg * 2;
+}
+__device__ __forceinline__ void af_store(float* local, const int rank, const float v) {
+  uint32_t far;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(far), "f"(v) : "memory");
+}
+template <typename TC, int D, int HG, bool ROT>
+__global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <= 4 ? 2 : 1) fq3s_attn_few_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op r) {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (the other CTAs have begun when this completes)
+  seq_dep_begin(o.M);
+  extern __shared__ __align__(16) float af[];
+  constexpr int V = 16 / (int)sizeof(TC), NCH = D / V / 4, EL = D / 32;      // entries of 16 bytes, such pieces of a lane's key, value columns of a lane
+  typedef typename AfVec<EL * (int)sizeof(TC)>::T VT;
+  const int H = o.i0, g = blockIdx.y, m = blockIdx.z, rank = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, part = lane & 3;
+  float* qs = af;                                             // [HG][D]
+  TC* ks = reinterpret_cast<TC*>(qs + HG * D);                // [D] new key, [D] new value
+  TC* vs = reinterpret_cast<TC*>(qs + HG * D + D);
+  float* wo = qs + HG * D + 2 * D;                            // [warps][HG][D]
+  float* wm = wo + AF_WARPS * HG * D;                         // [warps][HG] maxima, sums
+  float* wl = wm + AF_WARPS * HG;
+  float* in = wl + AF_WARPS * HG;                             // [ranks][HG * D / ranks]
+  float* ml = in + HG * D;                                    // [ranks][HG][2]
+  const int i = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;      // the row's position
+  const CacheAttnMask mask{o.K, o.a_rows, o.tap_off[0], 0};
+  const TC* kc = reinterpret_cast<const TC*>(o.B) + (size_t)g * D;
+  const TC* vc = reinterpret_cast<const TC*>(o.p1) + (size_t)g * D;
+  float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda + (size_t)g * HG * D;
+  const bool fresh = ROT && r.i1 > 0;      // the key and value at position i are not in the caches yet
+  struct Tile { uint4 k[NCH]; VT v[8]; };
+  auto load = [&](const int u, Tile& t) {
+    const int j = u * 8 + (lane >> 2);
+    const bool see = mask.sees(i, j) && !(fresh && j == i);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) t.k[c] = see ? *reinterpret_cast<const uint4*>(kc + (size_t)j * o.ldr + (part + 4 * c) * V) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int jj = u * 8 + e;
+      t.v[e] = mask.sees(i, jj) && !(fresh && jj == i) ? *reinterpret_cast<const VT*>(vc + (size_t)jj * o.taps + lane * EL) : VT{};
+    }
+  };
+  const int last = i >> 3, step = AF_RANKS * AF_WARPS;
+  int u = (mask.lowest(i) >> 3) + warp * AF_RANKS + rank;
+  // eight keys that the row does not see (between the kept first ones and the window) are passed over
+  auto next = [&](int w) {
+    while (w <= last && mask.window > 0 && w * 8 + 7 <= i - mask.window && w * 8 >= mask.keep) w += step;
+    return w;
+  };
+  u = next(u);
+  Tile cur;
+  if (u <= last) load(u, cur);
+  if (ROT) {
+    const float* krow = r.res ? reinterpret_cast<const float*>(r.res) : reinterpret_cast<const float*>(r.A);
+    for (int hh = warp; hh < HG + (fresh ? 2 : 0); hh += AF_WARPS) {
+      if (hh < HG) rot_head(r, row + (size_t)hh * D, true, i, lane, true, [&](const int c, const float v) { qs[hh * D + c] = v; });
+      else if (hh == HG) {
+        TC* out = reinterpret_cast<TC*>(r.C) + (size_t)i * r.ldc + (size_t)g * D;
+        rot_head(r, krow + r.K + (size_t)g * D, false, i, lane, true, [&](const int c, const float v) {
+          stf(ks + c, v);
+          if (rank == 0) stf(out + c, v);
+        });
+      } else {
+        TC* out = reinterpret_cast<TC*>(r.C2) + (size_t)i * r.ldr + (size_t)g * D;
+        for (int c = lane; c < D; c += 32) {
+          const float v = krow[r.a_rows + (size_t)g * D + c];
+          stf(vs + c, v);
+          if (rank == 0) stf(out + c, v);
+        }
+      }
+    }
+  } else {
+    for (int c = tid; c < HG * D; c += AF_WARPS * 32) qs[c] = row[c];
+  }
+  __syncthreads();
+  const float* r12 = reinterpret_cast<const float*>(o.bias);
+  const float cap = o.f1, icap = o.f1 > 0.f ? 1.f / o.f1 : 0.f;
+  float mx[HG], ls[HG], oa[HG][EL];
+#pragma unroll
+  for (int h = 0; h < HG; ++h) {
+    mx[h] = -INFINITY; ls[h] = 0.f;
+#pragma unroll
+    for (int e = 0; e < EL; ++e) oa[h][e] = 0.f;
+  }
+  while (u <= last) {
+    const int un = next(u + step);
+    Tile nxt;
+    if (un <= last) load(un, nxt);
+    const int j = u * 8 + (lane >> 2);
+    if (fresh && u == last) {
+      if (j == i) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) cur.k[c] = *reinterpret_cast<const uint4*>(ks + (part + 4 * c) * V);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (u * 8 + e == i) cur.v[e] = *reinterpret_cast<const VT*>(vs + lane * EL);
+    }
+    float sc[HG];
+#pragma unroll
+    for (int h = 0; h < HG; ++h) sc[h] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      float kv[V];
+      ca_unpack(kv, cur.k[c], kc);
+#pragma unroll
+      for (int h = 0; h < HG; ++h)
+        {
+          const float4* q = reinterpret_cast<const float4*>(qs + h * D + (part + 4 * c) * V);
+#pragma unroll
+          for (int e = 0; e < V / 4; ++e) {
+            const float4 qv = q[e];
+            sc[h] = fmaf(qv.x, kv[4 * e], sc[h]); sc[h] = fmaf(qv.y, kv[4 * e + 1], sc[h]);
+            sc[h] = fmaf(qv.z, kv[4 * e + 2], sc[h]); sc[h] = fmaf(qv.w, kv[4 * e + 3], sc[h]);
+          }
+        }
+    }
+    const bool see = mask.sees(i, j);
+#pragma unroll
+    for (int h = 0; h < HG; ++h)
+      {
+        float x = sc[h];
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        x += __shfl_xor_sync(0xffffffffu, x, 2);
+        x *= o.f0;
+        if (cap > 0.f) x = cap * tanhf(x * icap);
+        if (r12) x -= r12[g * HG + h] * log1pf(r12[H + g * HG + h] * (float)(i - j));
+        if (!see) x = -INFINITY;
+        float tm = x;
+        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 4));
+        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 8));
+        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 16));
+        const float mn = fmaxf(mx[h], tm);
+        const float p = see ? expf(x - mn) : 0.f, a = mx[h] == -INFINITY ? 0.f : expf(mx[h] - mn);
+        mx[h] = mn;
+        ls[h] = ls[h] * a + p;
+        sc[h] = p;
+#pragma unroll
+        for (int e = 0; e < EL; ++e) oa[h][e] *= a;
+      }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float vv[EL];
+      if (sizeof(TC) == 2) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&cur.v[e]);
+#pragma unroll
+        for (int q = 0; q < EL / 2; ++q) { vv[2 * q] = __uint_as_float(w[q] << 16); vv[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u); }
+      } else {
+        const float* w = reinterpret_cast<const float*>(&cur.v[e]);
+#pragma unroll
+        for (int q = 0; q < EL; ++q) vv[q] = w[q];
+      }
+#pragma unroll
+      for (int h = 0; h < HG; ++h)
+        {
+          const float p = __shfl_sync(0xffffffffu, sc[h], 4 * e);
+#pragma unroll
+          for (int q = 0; q < EL; ++q) oa[h][q] = fmaf(p, vv[q], oa[h][q]);
+        }
+    }
+    cur = nxt;
+    u = un;
+  }
+#pragma unroll
+  for (int h = 0; h < HG; ++h)
+    {
+      float l = ls[h];      // of the lane's keys
+      l += __shfl_xor_sync(0xffffffffu, l, 4);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      if (lane == 0) { wm[warp * HG + h] = mx[h]; wl[warp * HG + h] = l; }
+#pragma unroll
+      for (int e = 0; e < EL; ++e) wo[(warp * HG + h) * D + lane * EL + e] = oa[h][e];
+    }
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // the CTA's result to where it is finished: an eighth of the entries to each CTA, maxima and sums to all
+  auto most = [&](const int h) {
+    float x = wm[h];
+#pragma unroll
+    for (int w = 1; w < AF_WARPS; ++w) x = fmaxf(x, wm[w * HG + h]);
+    return x;
+  };
+  auto weight = [&](const int w, const int h, const float mm) { return wm[w * HG + h] == -INFINITY ? 0.f : expf(wm[w * HG + h] - mm); };
+  const int share = HG * D / AF_RANKS;
+  for (int c = tid; c < HG * D; c += AF_WARPS * 32) {
+    const int h = c / D;
+    const float mm = most(h);
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < AF_WARPS; ++w) v = fmaf(weight(w, h, mm), wo[w * HG * D + c], v);
+    af_store(in + rank * share + c % share, c / share, v);
+  }
+  if (tid < HG * AF_RANKS) {
+    const int to = tid / HG, h = tid - to * HG;
+    const float mm = most(h);
+    float l = 0.f;
+#pragma unroll
+    for (int w = 0; w < AF_WARPS; ++w) l = fmaf(weight(w, h, mm), wl[w * HG + h], l);
+    af_store(ml + (rank * HG + h) * 2, to, mm);
+    af_store(ml + (rank * HG + h) * 2 + 1, to, l);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (ROT && rank == 0)      // everyone has read the row as it was
+    for (int c = tid; c < HG * D; c += AF_WARPS * 32) row[c] = qs[c];
+  const float* sink = reinterpret_cast<const float*>(o.scale);
+  const float* gate = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.col_mod : nullptr;
+  const bool entry = (o.flags & FQ3C_GATE_ENTRY) != 0;
+  for (int t = tid; t < share; t += AF_WARPS * 32) {
+    const int c = rank * share + t, h = c / D, hh = g * HG + h;
+    float mm = sink ? sink[hh] : -INFINITY;
+#pragma unroll
+    for (int s = 0; s < AF_RANKS; ++s) mm = fmaxf(mm, ml[(s * HG + h) * 2]);
+    float den = sink ? expf(sink[hh] - mm) : 0.f, v = 0.f;
+#pragma unroll
+    for (int s = 0; s < AF_RANKS; ++s) {
+      const float ms = ml[(s * HG + h) * 2], w = ms == -INFINITY ? 0.f : expf(ms - mm);
+      den = fmaf(w, ml[(s * HG + h) * 2 + 1], den);
+      v = fmaf(w, in[s * share + t], v);
+    }
+    const size_t at = (size_t)hh * D + (c - h * D);
+    v = v * (o.f2 != 0.f ? o.f2 : 1.f) / den;
+    if (gate) v *= sigmoid_f(gate[entry ? at : (size_t)hh]);
+    if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + at] = v;
+    else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + at] = __float2bfloat16_rn(v);
   }
 }
 
