@@ -1860,8 +1860,8 @@ const char* cache_attn_error(const fq3c_op& o) {
   return nullptr;
 }
 // Which calls of few rows go to fq3s_attn_few_kernel: what its accesses and variants ask for, and as many keys as the eight CTAs of a cluster walk faster than up to 64 do with a second
-// launch to merge them.  That is told by the keys that a row may see (the window, or what 32 per split say): one row behind 2000 positions, 4 heads a key head, 20.8 us by itself and 15.9
-// here, behind 8000 35.6 and 46.3; 8 heads a key head behind 1000 17.1 and 15.4, behind 2000 21.3 and 24.2; one head a key head behind 8000 30.8 and 28.7.
+// launch to merge them.  That is told by the keys that a row may see (the window, or what 32 per split say): one row behind 2000 positions, 4 heads a key head, 20.8 us by itself and 13.9
+// here, behind 8000 35.6 and 46; 8 heads a key head behind 1000 17.1 and 15.4, behind 2000 21.3 and 24.2; one head a key head behind 8000 30.8 and 28.7.
 bool attn_few_takes(const fq3c_op& o) {
   const int splits = std::max(1, o.m_begin);
   const long keys = o.K > 0 && o.a_rows <= 0 ? o.K : o.tap_off[0] > 0 ? o.tap_off[0] : splits < 64 ? 32L * splits : 1L << 30;
@@ -1913,6 +1913,45 @@ void launch_attn_few(const fq3c_op& o, const fq3c_op* r, cudaStream_t s, const b
     if (f32) { if (o.i2 == 64) launch_attn_few<float, 64, false>(o, q, s, after); else launch_attn_few<float, 128, false>(o, q, s, after); }
     else { if (o.i2 == 64) launch_attn_few<bf16, 64, false>(o, q, s, after); else launch_attn_few<bf16, 128, false>(o, q, s, after); }
   }
+}
+
+// ---- one decoded row of a delta-rule layer -------------------------------------------------------------------------------------
+// c, o, n: convolution, recurrence and norm of one row that one launch can do: the convolution's channels are the head's queries, keys and values as they stand, the norm is per head,
+// with a gate behind it or none.  In one launch a CTA reads what another one may have written already, so no op may write what it or an op in front of it reads, but for the entries it
+// hands on: the convolution's result, the read-out, and the state, which is read and written by the same lanes.
+bool delta_row_takes(const fq3c_op& c, const fq3c_op& o, const fq3c_op& n) {
+  if (c.kind != FQ3C_TCONV || o.kind != FQ3C_MSTATE_SCAN || n.kind != FQ3C_GNORM || c.M != 1 || o.M != 1 || n.M != 1 || o.taps != 0) return false;
+  const int H = o.i0, G = o.i1, dk = o.i2, dv = o.cin;
+  if (H < 1 || G < 1 || H % G || H > 65535 || (dk != 64 && dk != 128 && dk != 256) || dv < 8 || dv > 128 || dv % 8) return false;
+  if (!c.A || !c.B || !c.C || c.taps < 2 || c.taps > DS_TAPS || !c.p0 || !c.p1 || !(c.flags & FQ3C_OUT_F32) || ((c.flags & FQ3C_BIAS) && !c.bias)) return false;
+  if (!o.A || !o.p0 || !o.C || !o.C2 || !o.res || !o.scale || !o.ws || o.ws_bytes < (int64_t)mstate_ws_cols(H, G, dk, true) * 4) return false;
+  if (o.A != c.C || o.K != G * dk || o.a_rows != 2 * G * dk || c.N != 2 * G * dk + H * dv) return false;
+  if (n.i0 != H || n.N != H * dv || n.A != o.C || !n.C || (n.flags & ~(FQ3C_GATE_POST | FQ3C_SIGMOID | FQ3C_OUT_F32)) || ((n.flags & FQ3C_GATE_POST) && !n.p1) || n.bias || n.C2 || n.p0) return false;
+  struct Span { uintptr_t at, end; };
+  auto span = [](const void* p, const int64_t bytes) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    return p ? Span{a, a + (uintptr_t)bytes} : Span{0, 0};
+  };
+  auto apart = [](const Span& a, const Span& b) { return a.end <= b.at || b.end <= a.at; };
+  const int64_t conv = 4LL * c.N, hist = conv * (c.taps - 1), state = 4LL * H * dk * dv, out = 4LL * H * dv;
+  const Span cv = span(c.C, conv), next = span(c.p1, hist), y = span(o.C, out), st = span(o.p0, state), st2 = span(o.C2, state), yn = span(n.C, n.flags & FQ3C_OUT_F32 ? out : out / 2);
+  const Span reads[] = {span(c.A, conv), span(c.B, conv * c.taps), span(c.flags & FQ3C_BIAS ? c.bias : nullptr, conv), span(c.p0, hist), span(reinterpret_cast<const float*>(o.res) + o.col_mod, 4LL * H),
+                        span(reinterpret_cast<const float*>(o.res) + o.m_begin, 4LL * H), span(o.scale, 4LL * H), span(o.bias, 4LL * H), span(n.scale, 4LL * (n.i2 > 0 ? n.i2 : n.N)),
+                        span(n.flags & FQ3C_GATE_POST ? n.p1 : nullptr, out)};
+  const Span writes[] = {cv, next, y, st2, yn};
+  for (const Span& w : writes) {
+    for (const Span& r : reads) if (!apart(w, r)) return false;
+    if (!apart(w, st) && !(w.at == st2.at && w.end == st2.end && st.at == st2.at)) return false;
+  }
+  for (int a = 0; a < 5; ++a)
+    for (int b = 0; b < a; ++b) if (!apart(writes[a], writes[b])) return false;
+  return true;
+}
+void launch_delta_row(const fq3c_op& c, const fq3c_op& o, const fq3c_op& n, cudaStream_t s, const bool after) {
+  const dim3 grid(DS_RANKS, (unsigned)o.i0);
+  if (o.i2 == 64) launch_after(fq3s_delta_row_kernel<8>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
+  else if (o.i2 == 128) launch_after(fq3s_delta_row_kernel<16>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
+  else launch_after(fq3s_delta_row_kernel<32>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
 }
 
 int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
@@ -2732,8 +2771,15 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         fq3c_advance_kernel<<<1, 1, 0, s>>>(reinterpret_cast<int*>(o.C), o.i0);
         break;
       }
+      case FQ3C_TCONV:
+        if (i + 2 < n_ops && delta_row_takes(o, ops[i + 1], ops[i + 2])) {      // with the recurrence and the norm behind it in one launch
+          launch_delta_row(o, ops[i + 1], ops[i + 2], s, after);
+          i += 2;
+          break;
+        }
+        [[fallthrough]];
       case FQ3C_ROT_APPEND:
-        if (i + 1 < n_ops && rot_append_ok(o) && attn_few_takes_rot(o, ops[i + 1]) && !cache_attn_error(ops[i + 1])) {      // with the attention behind it in one launch
+        if (o.kind == FQ3C_ROT_APPEND && i + 1 < n_ops && rot_append_ok(o) && attn_few_takes_rot(o, ops[i + 1]) && !cache_attn_error(ops[i + 1])) {      // with the attention behind it in one launch
           ++i;
           launch_attn_few(ops[i], &o, s, after);
           break;

@@ -19,6 +19,15 @@ __device__ __forceinline__ void seq_dep_begin(const int rows) {
   if (rows <= DEP_ROWS) grid_dep_launch();
 }
 
+// The arguments of a launch come through a cache that does not have them yet.  A launch that is up early fetches them while it waits; one warp calls it.  (With that, and with all of
+// their inputs asked for at once, a decoded token's attention launch went from 16 100 to 11 900 cycles behind the wait, its delta-rule launch from 18 900 to 14 400.)
+template <typename T>
+__device__ __forceinline__ void args_ahead(const T& args) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(&args);
+#pragma unroll 1
+  for (int i = 0; i < (int)sizeof(T) / 4; i += 16) asm volatile("" ::"r"(w[i]));
+}
+
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -641,7 +650,7 @@ struct SeqTail { int n; fq3c_op op[2]; };
 // TAIL: lane m goes on with entry (m, n) of row m through the ops of `tail`, with their own arithmetic: each was a launch of its own of 2 us, of which a decoded token of
 // four layers had sixteen.
 template <typename TA, typename TB, bool TAIL = false>
-__global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const __grid_constant__ SeqTail tail) {
+__global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ SeqGemm g, const __grid_constant__ SeqTail tail) {
   extern __shared__ float xs[];  // [M][K]
   const int z = blockIdx.z;
   const TA* Ap = reinterpret_cast<const TA*>(g.A) + (size_t)(z % g.a_mod) * g.a_zstride;
@@ -664,6 +673,10 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const SeqGemm g, const _
     }
   };
   if (g.early) first();
+  if (warp == 0) {
+    args_ahead(g);
+    if (TAIL) args_ahead(tail);
+  }
   seq_dep_begin(g.M);
   if (!g.early) first();
   // one row of whole 16-byte pieces: each lane's entries go straight to its registers
@@ -1746,12 +1759,11 @@ __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) 
 // m_begin = P > 0: every run of P positions bP .. bP + P - 1 that the step completes leaves the mean of its P cached keys and values as
 // row b of norm_out / ws.  A single row does it here (POOL; its block has just written the run's last row); more rows take
 // fq3s_pool_append_kernel behind this launch.
-// A warp turns (norms, tempers) one query or key head at position pos; put(i, v) takes entry i.  all: also the entries that stay as they are.
+// A warp turns (norms, tempers) one query or key head at position pos; put(i, v) takes entry i.  freq, flo: the frequencies and what they lost to rounding (or null).
+// all: also the entries that stay as they are.
 template <typename Put>
-__device__ __forceinline__ void rot_head(const fq3c_op& o, const float* src, const bool isq, const int pos, const int lane, const bool all, Put put) {
+__device__ __forceinline__ void rot_head(const fq3c_op& o, const float* freq, const float* flo, const float* src, const bool isq, const int pos, const int lane, const bool all, Put put) {
   const int d = o.i2, half = o.taps >> 1;
-  const float* freq = reinterpret_cast<const float*>(o.B);
-  const float* flo = reinterpret_cast<const float*>(o.p1);
   const float fp = (float)pos, amp = o.f1 != 0.f ? o.f1 : 1.f;
   const float* nw = reinterpret_cast<const float*>(isq ? o.scale : o.bias);
   const bool unit = nw || (o.flags & FQ3C_UNIT), normed = unit || (isq && o.f3 > 0.f);
@@ -1802,7 +1814,7 @@ __global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op 
     const float* src = isq ? row + (size_t)hh * d : krow + o.K + (size_t)(hh - H) * d;
     float* qd = isq ? row + (size_t)hh * d : nullptr;
     TC* kd = isq ? nullptr : kc + (size_t)(hh - H) * d;
-    rot_head(o, src, isq, pos, lane, false, [&](const int i, const float v) {
+    rot_head(o, reinterpret_cast<const float*>(o.B), reinterpret_cast<const float*>(o.p1), src, isq, pos, lane, false, [&](const int i, const float v) {
       if (isq) qd[i] = v;
       else stf(kd + i, v);
     });
@@ -2041,16 +2053,15 @@ __global__ void __launch_bounds__(128) fq3s_cache_attn_merge_kernel(const fq3c_o
 // faster with the registers, 7.5 and 8.2.)
 // ROT (one row): also the ROT_APPEND `r` in front of it, another launch: every CTA turns its query heads for itself, the first one also writes them back and the new key and value to
 // the caches; the CTA whose eight keys the new one is among reads it from its own shared memory.
-// Rotation and attention of one row of 16 heads over 4 behind 220 positions: 15.5 us in three launches, 7.5; 8 rows 25.8 and 12.0; one row of 32-bit caches behind 1000 15.5 and 10.8.
+// Rotation and attention of one row of 16 heads over 4 behind 220 positions: 15.5 us in three launches, 6.2; 8 rows 25.8 and 11.1; one row of 32-bit caches behind 2000 21.8 and 14.5.
 // ---------------------------------------------------------------------------------------------------------------------------
 constexpr int AF_RANKS = 8, AF_WARPS = 8;
 template <int BYTES> struct AfVec;
 template <> struct AfVec<4> { typedef uint32_t T; };
 template <> struct AfVec<8> { typedef uint2 T; };
 template <> struct AfVec<16> { typedef uint4 T; };
-__host__ __device__ constexpr int af_floats(int hg, int D) {      // queries | new key and value | the warps' outputs, maxima and sums | what arrives from the cluster
-  return hg * D + 2 * D + AF_WARPS * hg * (D + 2) + hg * D + AF_RANKS * hg * 2;
-}
+// queries | new key and value | frequencies and their rests | the warps' outputs, maxima, sums and weights | what arrives from the cluster
+__host__ __device__ constexpr int af_floats(int hg, int D) { return hg * D + 4 * D + AF_WARPS * hg * (D + 3) + hg * D + AF_RANKS * hg * 2; }
 __device__ __forceinline__ void af_store(float* local, const int rank, const float v) {
   uint32_t far;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(smem_u32(local)), "r"(rank));
@@ -2059,6 +2070,10 @@ __device__ __forceinline__ void af_store(float* local, const int rank, const flo
 template <typename TC, int D, int HG, bool ROT>
 __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <= 4 ? 2 : 1) fq3s_attn_few_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op r) {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (the other CTAs have begun when this completes)
+  if (threadIdx.x < 32) {
+    args_ahead(o);
+    if (ROT) args_ahead(r);
+  }
   seq_dep_begin(o.M);
   extern __shared__ __align__(16) float af[];
   constexpr int V = 16 / (int)sizeof(TC), NCH = D / V / 4, EL = D / 32;      // entries of 16 bytes, such pieces of a lane's key, value columns of a lane
@@ -2066,12 +2081,15 @@ __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <
   const int H = o.i0, g = blockIdx.y, m = blockIdx.z, rank = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, part = lane & 3;
   float* qs = af;                                             // [HG][D]
-  TC* ks = reinterpret_cast<TC*>(qs + HG * D);                // [D] new key, [D] new value
-  TC* vs = reinterpret_cast<TC*>(qs + HG * D + D);
-  float* wo = qs + HG * D + 2 * D;                            // [warps][HG][D]
-  float* wm = wo + AF_WARPS * HG * D;                         // [warps][HG] maxima, sums
+  float* kn = qs + HG * D;                                    // [D] new key, [D] new value: as they are, then as the caches hold them
+  TC* ks = reinterpret_cast<TC*>(kn);
+  TC* vs = reinterpret_cast<TC*>(kn + D);
+  float* fr = kn + 2 * D;                                     // [D] frequencies, [D] rests
+  float* wo = fr + 2 * D;                                     // [warps][HG][D]
+  float* wm = wo + AF_WARPS * HG * D;                         // [warps][HG] maxima, sums, weights
   float* wl = wm + AF_WARPS * HG;
-  float* in = wl + AF_WARPS * HG;                             // [ranks][HG * D / ranks]
+  float* ww = wl + AF_WARPS * HG;
+  float* in = ww + AF_WARPS * HG;                             // [ranks][HG * D / ranks]
   float* ml = in + HG * D;                                    // [ranks][HG][2]
   const int i = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;      // the row's position
   const CacheAttnMask mask{o.K, o.a_rows, o.tap_off[0], 0};
@@ -2079,6 +2097,23 @@ __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <
   const TC* vc = reinterpret_cast<const TC*>(o.p1) + (size_t)g * D;
   float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda + (size_t)g * HG * D;
   const bool fresh = ROT && r.i1 > 0;      // the key and value at position i are not in the caches yet
+  {   // everything that the row's heads need on its way at once
+    constexpr int NQ = (HG * D + AF_WARPS * 32 - 1) / (AF_WARPS * 32);
+    float q[NQ], f = 0.f, x = 0.f;
+#pragma unroll
+    for (int e = 0; e < NQ; ++e) q[e] = tid + e * AF_WARPS * 32 < HG * D ? row[tid + e * AF_WARPS * 32] : 0.f;
+    if (ROT) {
+      const float* krow = r.res ? reinterpret_cast<const float*>(r.res) : reinterpret_cast<const float*>(r.A);
+      const int half = r.taps >> 1;
+      if (fresh && tid < 2 * D) x = krow[(tid < D ? r.K : r.a_rows - D) + (long)g * D + tid];
+      if (tid < half) f = reinterpret_cast<const float*>(r.B)[tid];
+      else if (r.p1 && tid >= D && tid < D + half) f = reinterpret_cast<const float*>(r.p1)[tid - D];
+    }
+#pragma unroll
+    for (int e = 0; e < NQ; ++e)
+      if (tid + e * AF_WARPS * 32 < HG * D) qs[tid + e * AF_WARPS * 32] = q[e];
+    if (ROT && tid < 2 * D) { kn[tid] = x; fr[tid] = f; }
+  }
   struct Tile { uint4 k[NCH]; VT v[8]; };
   auto load = [&](const int u, Tile& t) {
     const int j = u * 8 + (lane >> 2);
@@ -2102,26 +2137,36 @@ __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <
   Tile cur;
   if (u <= last) load(u, cur);
   if (ROT) {
-    const float* krow = r.res ? reinterpret_cast<const float*>(r.res) : reinterpret_cast<const float*>(r.A);
+    __syncthreads();
     for (int hh = warp; hh < HG + (fresh ? 2 : 0); hh += AF_WARPS) {
-      if (hh < HG) rot_head(r, row + (size_t)hh * D, true, i, lane, true, [&](const int c, const float v) { qs[hh * D + c] = v; });
+      const float* fl = r.p1 ? fr + D : nullptr;
+      if (hh < HG) rot_head(r, fr, fl, qs + hh * D, true, i, lane, true, [&](const int c, const float v) { qs[hh * D + c] = v; });
       else if (hh == HG) {
         TC* out = reinterpret_cast<TC*>(r.C) + (size_t)i * r.ldc + (size_t)g * D;
-        rot_head(r, krow + r.K + (size_t)g * D, false, i, lane, true, [&](const int c, const float v) {
-          stf(ks + c, v);
-          if (rank == 0) stf(out + c, v);
-        });
+        float v[EL];
+        rot_head(r, fr, fl, kn, false, i, lane, true, [&](const int c, const float x) { kn[c] = x; });
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < EL; ++e) v[e] = kn[lane + 32 * e];
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          stf(ks + lane + 32 * e, v[e]);
+          if (rank == 0) stf(out + lane + 32 * e, v[e]);
+        }
       } else {
         TC* out = reinterpret_cast<TC*>(r.C2) + (size_t)i * r.ldr + (size_t)g * D;
-        for (int c = lane; c < D; c += 32) {
-          const float v = krow[r.a_rows + (size_t)g * D + c];
-          stf(vs + c, v);
-          if (rank == 0) stf(out + c, v);
+        float v[EL];
+#pragma unroll
+        for (int e = 0; e < EL; ++e) v[e] = kn[D + lane + 32 * e];
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          stf(vs + lane + 32 * e, v[e]);
+          if (rank == 0) stf(out + lane + 32 * e, v[e]);
         }
       }
     }
-  } else {
-    for (int c = tid; c < HG * D; c += AF_WARPS * 32) qs[c] = row[c];
   }
   __syncthreads();
   const float* r12 = reinterpret_cast<const float*>(o.bias);
@@ -2226,53 +2271,54 @@ __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <
   __syncthreads();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   // the CTA's result to where it is finished: an eighth of the entries to each CTA, maxima and sums to all
-  auto most = [&](const int h) {
-    float x = wm[h];
-#pragma unroll
-    for (int w = 1; w < AF_WARPS; ++w) x = fmaxf(x, wm[w * HG + h]);
-    return x;
-  };
-  auto weight = [&](const int w, const int h, const float mm) { return wm[w * HG + h] == -INFINITY ? 0.f : expf(wm[w * HG + h] - mm); };
   const int share = HG * D / AF_RANKS;
+  if (tid < HG * AF_RANKS) {      // (eight warps, eight CTAs: thread (h, w) weighs warp w and tells CTA w)
+    const int w = tid / HG, h = tid - w * HG;
+    float mm = wm[h];
+#pragma unroll
+    for (int e = 1; e < AF_WARPS; ++e) mm = fmaxf(mm, wm[e * HG + h]);
+    ww[tid] = wm[tid] == -INFINITY ? 0.f : expf(wm[tid] - mm);
+    af_store(ml + (rank * HG + h) * 2, w, mm);
+  }
+  __syncthreads();
   for (int c = tid; c < HG * D; c += AF_WARPS * 32) {
     const int h = c / D;
-    const float mm = most(h);
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < AF_WARPS; ++w) v = fmaf(weight(w, h, mm), wo[w * HG * D + c], v);
+    for (int w = 0; w < AF_WARPS; ++w) v = fmaf(ww[w * HG + h], wo[w * HG * D + c], v);
     af_store(in + rank * share + c % share, c / share, v);
   }
   if (tid < HG * AF_RANKS) {
     const int to = tid / HG, h = tid - to * HG;
-    const float mm = most(h);
     float l = 0.f;
 #pragma unroll
-    for (int w = 0; w < AF_WARPS; ++w) l = fmaf(weight(w, h, mm), wl[w * HG + h], l);
-    af_store(ml + (rank * HG + h) * 2, to, mm);
+    for (int w = 0; w < AF_WARPS; ++w) l = fmaf(ww[w * HG + h], wl[w * HG + h], l);
     af_store(ml + (rank * HG + h) * 2 + 1, to, l);
   }
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // meanwhile: sinks and gates of this CTA's entries (share <= threads)
+  const float* sink = reinterpret_cast<const float*>(o.scale);
+  const float* gate = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.col_mod : nullptr;
+  const int c = rank * share + tid, h = c / D, hh = g * HG + h;
+  const size_t at = (size_t)hh * D + (c - h * D);
+  const float snk = sink && tid < share ? sink[hh] : -INFINITY;
+  const float open = gate && tid < share ? sigmoid_f(gate[o.flags & FQ3C_GATE_ENTRY ? at : (size_t)hh]) : 1.f;
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (ROT && rank == 0)      // everyone has read the row as it was
     for (int c = tid; c < HG * D; c += AF_WARPS * 32) row[c] = qs[c];
-  const float* sink = reinterpret_cast<const float*>(o.scale);
-  const float* gate = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.col_mod : nullptr;
-  const bool entry = (o.flags & FQ3C_GATE_ENTRY) != 0;
-  for (int t = tid; t < share; t += AF_WARPS * 32) {
-    const int c = rank * share + t, h = c / D, hh = g * HG + h;
-    float mm = sink ? sink[hh] : -INFINITY;
+  if (tid < share) {
+    float mm = snk;
 #pragma unroll
     for (int s = 0; s < AF_RANKS; ++s) mm = fmaxf(mm, ml[(s * HG + h) * 2]);
-    float den = sink ? expf(sink[hh] - mm) : 0.f, v = 0.f;
+    float den = sink ? expf(snk - mm) : 0.f, v = 0.f;
 #pragma unroll
     for (int s = 0; s < AF_RANKS; ++s) {
       const float ms = ml[(s * HG + h) * 2], w = ms == -INFINITY ? 0.f : expf(ms - mm);
       den = fmaf(w, ml[(s * HG + h) * 2 + 1], den);
-      v = fmaf(w, in[s * share + t], v);
+      v = fmaf(w, in[s * share + tid], v);
     }
-    const size_t at = (size_t)hh * D + (c - h * D);
     v = v * (o.f2 != 0.f ? o.f2 : 1.f) / den;
-    if (gate) v *= sigmoid_f(gate[entry ? at : (size_t)hh]);
+    if (gate) v *= open;
     if (o.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + at] = v;
     else reinterpret_cast<bf16*>(o.C)[(size_t)m * o.ldc + at] = __float2bfloat16_rn(v);
   }
@@ -3599,6 +3645,188 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
       for (int e = 0; e < 4; ++e)
         if (r + e < dk && c < dv) nst[(size_t)(r + e) * dv + c] = v[e];
     }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------
+// One decoded row of a delta-rule layer between its products: the convolution `c`, the step of the recurrence `o` and the gated norm per head `n`, one launch in place of four.
+// A cluster of eight CTAs per head, each with an eighth of the state columns; a state column is eight lanes', as in fq3s_mstate_scan_kernel, whose arithmetic and order this is (and the
+// other kernels' theirs).  Every CTA convolves and norms the head's query and key for itself; the read-out meets in the shared memory of all eight, where the norm's sum is formed.
+// Everything the ops write is written: by the CTA whose columns they are, or by the first one of the group.
+// Latency bounds it (one trip to the inputs, four meetings): in a decoded token the four launches of 8 heads of 128 x 128 took 12.7 us, this one 8.0 (launched over and over: 5.9).
+// grid (8, H) in clusters of 8, 128 threads; dk = 8 RPT, dv a multiple of 8 up to 128
+// ---------------------------------------------------------------------------------------------------------------------------
+constexpr int DS_RANKS = 8;
+constexpr int DS_TAPS = 8;      // of the convolution, at most
+struct ConvRow { float x, b, w[DS_TAPS], hist[DS_TAPS - 1]; };      // what channel c of a single row needs
+__device__ __forceinline__ ConvRow conv_row(const fq3c_op& o, const int c) {
+  ConvRow r;
+  const float* hist = reinterpret_cast<const float*>(o.p0);
+  r.x = reinterpret_cast<const float*>(o.A)[c];
+  r.b = (o.flags & FQ3C_BIAS) ? reinterpret_cast<const float*>(o.bias)[c] : 0.f;
+#pragma unroll
+  for (int j = 0; j < DS_TAPS; ++j) r.w[j] = j < o.taps ? reinterpret_cast<const float*>(o.B)[(size_t)c * o.taps + j] : 0.f;
+#pragma unroll
+  for (int j = 0; j < DS_TAPS - 1; ++j) r.hist[j] = j + 1 < o.taps ? hist[(size_t)j * o.N + c] : 0.f;
+  return r;
+}
+__device__ __forceinline__ float conv_value(const fq3c_op& o, const int c, const ConvRow& r) {
+  float a = r.b;
+#pragma unroll
+  for (int j = 0; j < DS_TAPS; ++j)
+    if (j < o.taps) a = fmaf(r.w[j], j + 1 < o.taps ? r.hist[j < DS_TAPS - 1 ? j : 0] : r.x, a);
+  if (o.flags & FQ3C_RESID) a += r.x;
+  if ((o.flags & FQ3C_SILU) && c >= o.i0) a = a / (1.f + expf(-a));
+  return a;
+}
+__device__ __forceinline__ void conv_out(const fq3c_op& o, const int c, const ConvRow& r, const float v) {      // and what it leaves behind
+  float* next = reinterpret_cast<float*>(const_cast<void*>(o.p1));
+#pragma unroll
+  for (int j = 0; j < DS_TAPS - 1; ++j)
+    if (j + 1 < o.taps) next[(size_t)j * o.N + c] = j + 2 < o.taps ? r.hist[j + 1 < DS_TAPS - 1 ? j + 1 : 0] : r.x;
+  reinterpret_cast<float*>(o.C)[c] = v;
+}
+template <int RPT>
+__global__ void __launch_bounds__(128) fq3s_delta_row_kernel(const __grid_constant__ fq3c_op c, const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op n) {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  if (threadIdx.x < 32) { args_ahead(c); args_ahead(o); args_ahead(n); }
+  seq_dep_begin(1);
+  constexpr int DK = 8 * RPT, SL = RPT + 4, TS = RPT * 16 + 4, NE = (2 * DK + 127) / 128;
+  // slices of RPT entries (rows), four floats apart: no bank conflicts
+  __shared__ __align__(16) float tile[8 * TS], qs[8 * SL], ks[8 * SL], vs[16], ys[128], red[32], two[2];
+  const int H = o.i0, G = o.i1, dv = o.cin, h = blockIdx.y, g = h / (H / G), rank = blockIdx.x, cols = dv / DS_RANKS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = tid & 7, cl = tid >> 3, col = rank * cols + cl;
+  const bool live = cl < cols, owner = rank == 0 && h == g * (H / G);      // (owner: of the group's query and key)
+  // the state's columns: whole 16-byte pieces of its rows where they are
+  const float* st = reinterpret_cast<const float*>(o.p0) + (size_t)h * DK * dv + rank * cols;
+  float* nst = reinterpret_cast<float*>(o.C2) + (size_t)h * DK * dv + rank * cols;
+  const bool pieces = cols % 4 == 0 && ((reinterpret_cast<uintptr_t>(st) | reinterpret_cast<uintptr_t>(nst)) & 15) == 0;
+  const int wide = pieces ? cols / 4 : cols;
+  auto tile_at = [&](const int i) { return (i / RPT) * TS + (i % RPT) * 16; };
+  for (int e = tid; e < DK * wide; e += 128) {
+    const int i = e / wide, j = e - i * wide;
+    if (pieces) cp_async16(tile + tile_at(i) + 4 * j, st + (size_t)i * dv + 4 * j, true);
+    else cp_async4(tile + tile_at(i) + j, st + (size_t)i * dv + j);
+  }
+  cp_async_commit();
+  // the channels of the query and the key, and this CTA's of the value: all inputs on their way, then the values
+  ConvRow in[NE], vin;
+  int ch[NE];
+  const int vch = o.a_rows + h * dv + rank * cols + tid;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    const int x = tid + 128 * e;
+    ch[e] = (x >= DK ? o.K + x - DK : x) + g * DK;
+    if (x < 2 * DK) in[e] = conv_row(c, ch[e]);
+  }
+  if (tid < cols) vin = conv_row(c, vch);
+  const float* raw = reinterpret_cast<const float*>(o.res);
+  const float c1 = expf(-expf(reinterpret_cast<const float*>(o.scale)[h]) * softplus_f(raw[o.col_mod + h] + (o.bias ? reinterpret_cast<const float*>(o.bias)[h] : 0.f)));
+  const float c2 = sigmoid_f(raw[o.m_begin + h]);
+  float cv[NE], vv = 0.f;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    const int x = tid + 128 * e, i = x >= DK ? x - DK : x;
+    if (x >= 2 * DK) continue;
+    cv[e] = conv_value(c, ch[e], in[e]);
+    (x >= DK ? ks : qs)[(i / RPT) * SL + i % RPT] = cv[e];
+  }
+  if (tid < cols) vs[tid] = vv = conv_value(c, vch, vin);
+  cp_async_wait<0>();
+  __syncthreads();
+  f32x2 S[RPT / 2];
+#pragma unroll
+  for (int r = 0; r < RPT / 2; ++r) {
+    const float* t = tile + tile_at(sub * RPT + 2 * r) + cl;
+    S[r] = live ? pack2(t[0], t[16]) : 0ull;
+  }
+  if (warp < 2) {
+    float* x = warp ? ks : qs;
+    float ss = 0.f, v[DK / 32];
+#pragma unroll
+    for (int e = 0; e < DK / 32; ++e) {
+      const int i = lane + 32 * e;
+      v[e] = x[(i / RPT) * SL + i % RPT];
+      ss = fmaf(v[e], v[e], ss);
+    }
+    ss = warp_sum(ss);
+    const float f = (1.f / sqrtf(ss + 1e-6f)) * (warp ? 1.f : 1.f / sqrtf((float)DK));
+#pragma unroll
+    for (int e = 0; e < DK / 32; ++e) {
+      const int i = lane + 32 * e;
+      x[(i / RPT) * SL + i % RPT] = v[e] * f;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {      // q . k
+    float dot = 0.f;
+#pragma unroll
+    for (int e = 0; e < DK / 32; ++e) {
+      const int i = lane + 32 * e, at = (i / RPT) * SL + i % RPT;
+      dot = fmaf(qs[at], ks[at], dot);
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) two[0] = dot;
+  }
+  const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(ks + sub * SL);
+  const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(qs + sub * SL);
+  f32x2 ka[2] = {0ull, 0ull}, qa[2] = {0ull, 0ull};
+#pragma unroll
+  for (int r = 0; r < RPT / 4; ++r) {
+    const ulonglong2 kv = k4[r], qv = q4[r];
+    ka[0] = fma2<true>(kv.x, S[2 * r], ka[0]);
+    ka[1] = fma2<true>(kv.y, S[2 * r + 1], ka[1]);
+    qa[0] = fma2<true>(qv.x, S[2 * r], qa[0]);
+    qa[1] = fma2<true>(qv.y, S[2 * r + 1], qa[1]);
+  }
+  float kt = (lo2(ka[0]) + hi2(ka[0])) + (lo2(ka[1]) + hi2(ka[1])), qt = (lo2(qa[0]) + hi2(qa[0])) + (lo2(qa[1]) + hi2(qa[1]));
+  kt += __shfl_xor_sync(0xffffffffu, kt, 1); qt += __shfl_xor_sync(0xffffffffu, qt, 1);
+  kt += __shfl_xor_sync(0xffffffffu, kt, 2); qt += __shfl_xor_sync(0xffffffffu, qt, 2);
+  kt += __shfl_xor_sync(0xffffffffu, kt, 4); qt += __shfl_xor_sync(0xffffffffu, qt, 4);
+  __syncthreads();
+  const float u = live ? c2 * (vs[cl] - c1 * kt) : 0.f, y = fmaf(u, two[0], c1 * qt);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // the others have begun
+  if (live) af_store(ys + col, sub, y);                                        // lane `sub` of a column to CTA `sub`
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  const f32x2 uu = pack2(u, u), cc = pack2(c1, c1);
+  if (live) {
+#pragma unroll
+    for (int r = 0; r < RPT / 4; ++r) {
+      const ulonglong2 kv = k4[r];
+      const f32x2 a = fma2<true>(kv.x, uu, mul2<true>(cc, S[2 * r])), b = fma2<true>(kv.y, uu, mul2<true>(cc, S[2 * r + 1]));
+      float* t = tile + tile_at(sub * RPT + 4 * r) + cl;
+      t[0] = lo2(a); t[16] = hi2(a); t[32] = lo2(b); t[48] = hi2(b);
+    }
+    if (sub == 0) reinterpret_cast<float*>(o.C)[(size_t)h * dv + col] = y;
+  }
+  // the norm's weights and gate, on their way while the CTAs meet
+  const int at = h * dv + rank * cols + tid;
+  const bool mine = tid < cols;
+  const float* w = reinterpret_cast<const float*>(n.scale);
+  const float wv = mine && w ? w[at % (n.i2 > 0 ? n.i2 : n.N)] : 1.f;
+  const bool post = (n.flags & FQ3C_GATE_POST) != 0;
+  const float gate = mine && post ? gate_f(reinterpret_cast<const float*>(n.p1)[at], (n.flags & FQ3C_SIGMOID) != 0) : 1.f;
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const float v = tid < dv ? ys[tid] : 0.f;
+  const float rs = 1.f / sqrtf(seq_block_sum(v * v, red) / (float)dv + n.f0);
+  if (mine) {
+    float z = ys[rank * cols + tid] * rs;
+    if (w) z *= wv;
+    if (post) z *= gate;
+    if (n.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(n.C)[at] = z;
+    else reinterpret_cast<bf16*>(n.C)[at] = __float2bfloat16_rn(z);
+  }
+  // what the next row reads (seq_block_sum's barriers stand behind the tile's new entries)
+  for (int e = tid; e < DK * wide; e += 128) {
+    const int i = e / wide, j = e - i * wide;
+    if (pieces) *reinterpret_cast<float4*>(nst + (size_t)i * dv + 4 * j) = *reinterpret_cast<const float4*>(tile + tile_at(i) + 4 * j);
+    else nst[(size_t)i * dv + j] = tile[tile_at(i) + j];
+  }
+  if (owner) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+      if (tid + 128 * e < 2 * DK) conv_out(c, ch[e], in[e], cv[e]);
+  }
+  if (tid < cols) conv_out(c, vch, vin, vv);
 }
 
 // ===========================================================================================================================
