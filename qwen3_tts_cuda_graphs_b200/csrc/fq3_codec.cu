@@ -35,7 +35,8 @@ inline void count_launches(int64_t n) { g_launches += n; t_launches += n; }
 // itself for the end of everything in front of it before it touches memory.  Without the launch attribute both return at once.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_begin() { grid_dep_launch(); grid_dep_wait(); }
+// One launch ahead: with the next one let in before this wait, launches pile up on the SMs (28 layers of a prompt of 39 rows 1128 us, this way 1118; a codec window 717 and 705).
+__device__ __forceinline__ void grid_dep_begin() { grid_dep_wait(); grid_dep_launch(); }
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -2330,25 +2331,29 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       if (blocks) {
         static bool battr[64] = {};
         if (dev >= 0 && dev < 64 && !battr[dev]) {
-          cudaFuncSetAttribute(fq3s_cdelta_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * CD_C * cd_pitch(CD_MAX_DK) * 4);
-          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<8>(CD_MAX_DK) * 4);
-          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<8>(CD_MAX_DK) * 4);
-          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<16>(CD_MAX_DK) * 4);
-          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<16>(CD_MAX_DK) * 4);
-          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_walk_floats<16>(CD_MAX_DK) * 4);
+          cudaFuncSetAttribute(fq3s_cdelta_record_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_record_smem(CD_MAX_DK, true));
+          cudaFuncSetAttribute(fq3s_cdelta_record_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cd_record_smem(CD_MAX_DK, false));
+          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_WALK_SMEM);
+          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_WALK_SMEM);
+          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_WALK_SMEM);
+          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_WALK_SMEM);
+          cudaFuncSetAttribute(fq3s_cdelta_walk_kernel<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_WALK_SMEM);
           battr[dev] = true;
         }
-        launch_after(fq3s_cdelta_record_kernel, dim3((o.M + CD_C - 1) / CD_C, o.i0), CD_REC_THREADS, 4 * CD_C * cd_pitch(o.i2) * 4, s, after, 1, o);
+        const dim3 rgrid((o.M + CD_C - 1) / CD_C, o.i0);
+        if (o.taps == 6) launch_after(fq3s_cdelta_record_kernel<true>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, true), s, after, 1, o);
+        else launch_after(fq3s_cdelta_record_kernel<false>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, false), s, after, 1, o);
         count_launches(1);
         // narrow state tiles while they do not outnumber the SMs, wide ones otherwise and for few state rows
         const bool narrow = o.i2 > 64 && o.i0 * ((o.cin + 7) / 8) <= 148;
         const dim3 grid((o.cin + (narrow ? 7 : 15)) / (narrow ? 8 : 16), o.i0);
-        const size_t wsm = (narrow ? cd_walk_floats<8>(o.i2) : cd_walk_floats<16>(o.i2)) * 4;
-        if (narrow && o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<8, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
-        else if (narrow) launch_after(fq3s_cdelta_walk_kernel<8, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
-        else if (o.i2 <= 64) launch_after(fq3s_cdelta_walk_kernel<16, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
-        else if (o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<16, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
-        else launch_after(fq3s_cdelta_walk_kernel<16, 4>, grid, CD_WALK_THREADS, wsm, s, after, 1, o);
+        const int dvt = narrow ? 8 : 16, ring = cd_walk_floats(dvt, o.i2, 4) * 4 <= CD_WALK_SMEM ? 4 : 3;
+        const size_t wsm = (size_t)cd_walk_floats(dvt, o.i2, ring) * 4;
+        if (narrow && o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<8, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (narrow) launch_after(fq3s_cdelta_walk_kernel<8, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (o.i2 <= 64) launch_after(fq3s_cdelta_walk_kernel<16, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<16, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else launch_after(fq3s_cdelta_walk_kernel<16, 4>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
         return 0;
       }
       // Long runs of a recurrence whose decays do not depend on the state: pieces walked twice (see the kernel), when the caller's

@@ -305,7 +305,6 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, words[0], 0);
-  grid_dep_launch();
 
   // The two issuing warps run their loops whole, with one elected lane at the copies, products and commits: in code of a single lane every operand goes
   // through per-lane registers (700 - 800 cycles a k-block with `lane == 0`, 380 with the election around the loop).  What bounds a k-block of narrow tiles is
@@ -328,6 +327,7 @@ __global__ void __launch_bounds__(gp_threads(EPI_WARPS), MINB) fq3c_gemm_persist
       }
     }
     grid_dep_wait();
+    grid_dep_launch();
     bool there = true, wrapped = false;
     uint32_t st8 = 0, dst = base, ph = 1;      // 8 x stage, its memory, the parity that the end of its last use has
     for (int t = t0; t < tiles && there; t += dt) {

@@ -3279,10 +3279,10 @@ __global__ void __launch_bounds__(256) fq3s_mstate_carry_kernel(const fq3c_op o,
 //   u_t = beta_t (v_t - S0^T (G_t k_t) - sum_(s < t) A_ts u_s),   A_ts = sum_c k_t k_s e^(b_t - b_s)
 //   o_t = S0^T (G_t q_t) + sum_(s <= t) B_ts u_s,                 B_ts = sum_c q_t k_s e^(b_t - b_s)
 // so with the unit lower triangle I + diag(beta) A and T = (I + diag(beta) A)^-1 diag(beta):
-//   U = T (V - Kt S0),   O = Qt S0 + B U,   S <- diag(G_last) S0 + Kb^T U,   Kt = G_t k_t, Qt = G_t q_t, Kb = k_s e^(b_last - b_s).
+//   U = T V - W S0,   O = Qt S0 + B U,   S <- diag(G_last) S0 + Kb^T U,   W = T Kt, Kt = G_t k_t, Qt = G_t q_t, Kb = k_s e^(b_last - b_s).
 // Every exponent is a sum of decays between two tokens, hence never positive; the sums are kept as two floats, so that a difference of two large
 // ones is as good as the sum it stands for.  Three launches: the decays' logarithms row by row (fq3s_mstate_cdelta_prep_kernel; mode 0: none), the
-// records [Kt | Qt | Kb | G_last | T | B] of all (block, head) pairs at once, and one walk over the blocks per (head, DVT state columns): three
+// records [W | Qt | Kb | G_last | T | B] of all (block, head) pairs at once, and one walk over the blocks per (head, DVT state columns): three
 // small dense products per block of tokens instead of a chain of dependent steps per token.  Tokens beyond the last row are empty (k = q = v = 0,
 // beta = 0, no decay).
 // ---------------------------------------------------------------------------------------------------------------------------
@@ -3300,41 +3300,59 @@ __host__ __device__ inline long long cd_ws_floats(int M, int H, int dk, bool cha
 }
 constexpr float LOG2E_F = 1.4426950408889634f;
 __device__ __forceinline__ float pow2_f(const float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-// grid (blocks of tokens, H), CD_REC_THREADS threads; dynamic shared memory: sums (two floats), q and k, [CD_C][pitch] each
+// grid (blocks of tokens, H), CD_REC_THREADS threads; dynamic shared memory: q and k, with a decay per channel its sums (two floats), [CD_C][pitch] each.
+// One decay per head (CHANNELS false): its differences are 16 x 16 numbers behind the products of keys and queries, not one per channel and pair inside of them (94 blocks x 8 heads of
+// 128: 42 us with an exponential per term, 18 without).
+__host__ __device__ constexpr int cd_record_smem(int dk, bool channels) { return (channels ? 4 : 2) * CD_C * cd_pitch(dk) * 4; }
+template <bool CHANNELS>
 __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(const fq3c_op o) {
   seq_dep_begin(o.M);
   extern __shared__ __align__(16) float cr[];
-  __shared__ float beta[CD_C], N[CD_C][CD_C], fq[CD_C], fk[CD_C];
+  __shared__ float beta[CD_C], N[CD_C][CD_C], fq[CD_C], fk[CD_C], sh[CD_C], sl[CD_C], Ts[CD_C][CD_C];
   const int H = o.i0, G = o.i1, dk = o.i2, h = blockIdx.y, g = h / (H / G), t0 = blockIdx.x * CD_C, tid = threadIdx.x;
   const int D = cd_rows(dk), P = cd_pitch(dk), nt = min(CD_C, o.M - t0);
-  const bool channels = o.taps == 6;
-  float* bh = cr;
-  float* bl = bh + CD_C * P;
-  float* qs = bl + CD_C * P;
+  float* qs = cr;
   float* ks = qs + CD_C * P;
+  float* bh = ks + CD_C * P;      // (CHANNELS)
+  float* bl = bh + CD_C * P;
   const float* raw = reinterpret_cast<const float*>(o.res) + (size_t)t0 * o.ldr;
   const float* rows = reinterpret_cast<const float*>(o.A) + (size_t)t0 * o.lda;
   const int lp = (H * dk + 3) & ~3;
   if (tid < CD_C) beta[tid] = tid < nt ? sigmoid_f(raw[(size_t)tid * o.ldr + o.m_begin + h]) : 0.f;
-  const float rate = channels ? 0.f : LOG2E_F * expf(reinterpret_cast<const float*>(o.scale)[h]);
-  const float dtb = (!channels && o.bias) ? reinterpret_cast<const float*>(o.bias)[h] : 0.f;
   for (int c = tid; c < D; c += CD_REC_THREADS) {
-    float hi = 0.f, lo = 0.f, l[CD_C];
 #pragma unroll
     for (int t = 0; t < CD_C; ++t) {
       const bool ok = t < nt && c < dk;
-      l[t] = !ok ? 0.f : channels ? reinterpret_cast<const float*>(o.ws)[(size_t)(t0 + t) * lp + h * dk + c]
-                                  : -rate * softplus_f(raw[(size_t)t * o.ldr + o.col_mod + h] + dtb);
       qs[t * P + c] = ok ? rows[(size_t)t * o.lda + g * dk + c] : 0.f;
       ks[t * P + c] = ok ? rows[(size_t)t * o.lda + o.K + g * dk + c] : 0.f;
     }
+  }
+  // the sums of the decays' logarithms: the exact sum of two floats is again two floats; the small part collects
+  auto add = [](float& hi, float& lo, const float l) {
+    const float x = fmaxf(l, -1000.f), t = hi + x, bb = t - hi;
+    lo += (hi - (t - bb)) + (x - bb);
+    hi = t;
+  };
+  if (CHANNELS) {
+    for (int c = tid; c < D; c += CD_REC_THREADS) {
+      float hi = 0.f, lo = 0.f, l[CD_C];
 #pragma unroll
-    for (int t = 0; t < CD_C; ++t) {       // the exact sum of two floats is again two floats; the small part collects
-      const float x = fmaxf(l[t], -1000.f), s = hi + x, bb = s - hi;
-      lo += (hi - (s - bb)) + (x - bb);
-      hi = s;
-      bh[t * P + c] = hi;
-      bl[t * P + c] = lo;
+      for (int t = 0; t < CD_C; ++t) l[t] = t < nt && c < dk ? reinterpret_cast<const float*>(o.ws)[(size_t)(t0 + t) * lp + h * dk + c] : 0.f;
+#pragma unroll
+      for (int t = 0; t < CD_C; ++t) {
+        add(hi, lo, l[t]);
+        bh[t * P + c] = hi;
+        bl[t * P + c] = lo;
+      }
+    }
+  } else if (tid >= CD_REC_THREADS - 32) {      // (a warp with fewer columns to load)
+    const int lane = tid & 31;
+    const float rate = LOG2E_F * expf(reinterpret_cast<const float*>(o.scale)[h]), dtb = o.bias ? reinterpret_cast<const float*>(o.bias)[h] : 0.f;
+    const float mine = lane < nt ? -rate * softplus_f(raw[(size_t)lane * o.ldr + o.col_mod + h] + dtb) : 0.f;
+    float hi = 0.f, lo = 0.f;
+    for (int t = 0; t < CD_C; ++t) {
+      add(hi, lo, __shfl_sync(0xffffffffu, mine, t));
+      if (lane == t) { sh[t] = hi; sl[t] = lo; }
     }
   }
   __syncthreads();
@@ -3347,21 +3365,26 @@ __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(cons
     if (lane == 0) (v < CD_C ? fq : fk)[v & (CD_C - 1)] = (v < CD_C ? 1.f / sqrtf((float)dk) : 1.f) / sqrtf(ss + 1e-6f);
   }
   __syncthreads();
-  float* rec = reinterpret_cast<float*>(o.ws) + cd_log_floats(o.M, H, dk, channels) + ((size_t)blockIdx.x * H + h) * cd_record(dk);
+  float* rec = reinterpret_cast<float*>(o.ws) + cd_log_floats(o.M, H, dk, CHANNELS) + ((size_t)blockIdx.x * H + h) * cd_record(dk);
+  auto pow4 = [](const float4& x) { return make_float4(pow2_f(x.x), pow2_f(x.y), pow2_f(x.z), pow2_f(x.w)); };
+  auto mul4 = [](const float4& a, const float4& b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); };
   for (int i = tid; i < CD_C * (D >> 2); i += CD_REC_THREADS) {
     const int t = i / (D >> 2), c = (i - t * (D >> 2)) * 4, at = t * P + c;
-    const float4 hi = ld4(bh + at), lo = ld4(bl + at), eh = ld4(bh + (CD_C - 1) * P + c), el = ld4(bl + (CD_C - 1) * P + c);
-    float4 q = ld4(qs + at), k = ld4(ks + at);
-    q.x *= fq[t]; q.y *= fq[t]; q.z *= fq[t]; q.w *= fq[t];
-    k.x *= fk[t]; k.y *= fk[t]; k.z *= fk[t]; k.w *= fk[t];
+    const float4 q = mul4(ld4(qs + at), make_float4(fq[t], fq[t], fq[t], fq[t])), k = mul4(ld4(ks + at), make_float4(fk[t], fk[t], fk[t], fk[t]));
     *reinterpret_cast<float4*>(qs + at) = q;
     *reinterpret_cast<float4*>(ks + at) = k;
-    const float4 d = make_float4(pow2_f(hi.x), pow2_f(hi.y), pow2_f(hi.z), pow2_f(hi.w));
-    *reinterpret_cast<float4*>(rec + at) = make_float4(k.x * d.x, k.y * d.y, k.z * d.z, k.w * d.w);
-    *reinterpret_cast<float4*>(rec + CD_C * P + at) = make_float4(q.x * d.x, q.y * d.y, q.z * d.z, q.w * d.w);
-    *reinterpret_cast<float4*>(rec + 2 * CD_C * P + at) =
-        make_float4(k.x * pow2_f((eh.x - hi.x) + (el.x - lo.x)), k.y * pow2_f((eh.y - hi.y) + (el.y - lo.y)),
-                    k.z * pow2_f((eh.z - hi.z) + (el.z - lo.z)), k.w * pow2_f((eh.w - hi.w) + (el.w - lo.w)));
+    float4 d, e;
+    if (CHANNELS) {
+      const float4 hi = ld4(bh + at), lo = ld4(bl + at), eh = ld4(bh + (CD_C - 1) * P + c), el = ld4(bl + (CD_C - 1) * P + c);
+      d = pow4(hi);
+      e = pow4(make_float4((eh.x - hi.x) + (el.x - lo.x), (eh.y - hi.y) + (el.y - lo.y), (eh.z - hi.z) + (el.z - lo.z), (eh.w - hi.w) + (el.w - lo.w)));
+    } else {
+      const float x = pow2_f(sh[t]), y = pow2_f((sh[CD_C - 1] - sh[t]) + (sl[CD_C - 1] - sl[t]));
+      d = make_float4(x, x, x, x);
+      e = make_float4(y, y, y, y);
+    }
+    *reinterpret_cast<float4*>(rec + CD_C * P + at) = mul4(q, d);
+    *reinterpret_cast<float4*>(rec + 2 * CD_C * P + at) = mul4(k, e);
     if (t == CD_C - 1) *reinterpret_cast<float4*>(rec + 3 * CD_C * P + c) = d;
   }
   __syncthreads();
@@ -3380,20 +3403,24 @@ __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(cons
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         const int at = (2 * ti + x) * P + c;
-        ht[x] = ld4(bh + at); lt[x] = ld4(bl + at); kt[x] = ld4(ks + at); qt[x] = ld4(qs + at);
+        if (CHANNELS) { ht[x] = ld4(bh + at); lt[x] = ld4(bl + at); }
+        kt[x] = ld4(ks + at); qt[x] = ld4(qs + at);
       }
 #pragma unroll
       for (int y = 0; y < 2; ++y) {
         const int at = (2 * si + y) * P + c;
-        const float4 hs = ld4(bh + at), ls = ld4(bl + at), k = ld4(ks + at);
+        const float4 k = ld4(ks + at);
+        float4 hs, ls;
+        if (CHANNELS) { hs = ld4(bh + at); ls = ld4(bl + at); }
 #pragma unroll
         for (int x = 0; x < 2; ++x) {      // (above the diagonal the exponent is positive and may overflow: not stored)
-          const float e0 = k.x * pow2_f((ht[x].x - hs.x) + (lt[x].x - ls.x)), e1 = k.y * pow2_f((ht[x].y - hs.y) + (lt[x].y - ls.y));
-          const float e2 = k.z * pow2_f((ht[x].z - hs.z) + (lt[x].z - ls.z)), e3 = k.w * pow2_f((ht[x].w - hs.w) + (lt[x].w - ls.w));
-          a[x][y] = fmaf(kt[x].x, e0, a[x][y]); b[x][y] = fmaf(qt[x].x, e0, b[x][y]);
-          a[x][y] = fmaf(kt[x].y, e1, a[x][y]); b[x][y] = fmaf(qt[x].y, e1, b[x][y]);
-          a[x][y] = fmaf(kt[x].z, e2, a[x][y]); b[x][y] = fmaf(qt[x].z, e2, b[x][y]);
-          a[x][y] = fmaf(kt[x].w, e3, a[x][y]); b[x][y] = fmaf(qt[x].w, e3, b[x][y]);
+          float4 e = k;
+          if (CHANNELS)
+            e = mul4(k, pow4(make_float4((ht[x].x - hs.x) + (lt[x].x - ls.x), (ht[x].y - hs.y) + (lt[x].y - ls.y), (ht[x].z - hs.z) + (lt[x].z - ls.z), (ht[x].w - hs.w) + (lt[x].w - ls.w))));
+          a[x][y] = fmaf(kt[x].x, e.x, a[x][y]); b[x][y] = fmaf(qt[x].x, e.x, b[x][y]);
+          a[x][y] = fmaf(kt[x].y, e.y, a[x][y]); b[x][y] = fmaf(qt[x].y, e.y, b[x][y]);
+          a[x][y] = fmaf(kt[x].z, e.z, a[x][y]); b[x][y] = fmaf(qt[x].z, e.z, b[x][y]);
+          a[x][y] = fmaf(kt[x].w, e.w, a[x][y]); b[x][y] = fmaf(qt[x].w, e.w, b[x][y]);
         }
       }
     }
@@ -3406,10 +3433,11 @@ __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(cons
         const int t = 2 * ti + x, s = 2 * si + y;
         if ((tid & 3) == 2 * x + y) {        // one of the tile's four threads keeps it
           if (s <= t) {
-            N[t][s] = beta[t] * a[x][y];
-            Bm[t * CD_TP + s] = b[x][y];
+            const float e = CHANNELS ? 1.f : pow2_f((sh[t] - sh[s]) + (sl[t] - sl[s]));
+            N[t][s] = beta[t] * (a[x][y] * e);
+            Bm[t * CD_TP + s] = b[x][y] * e;
           }
-          if (s != t) Tm[(s < t ? s : t) * CD_TP + (s < t ? t : s)] = 0.f, Bm[(s < t ? s : t) * CD_TP + (s < t ? t : s)] = 0.f;
+          if (s != t) Ts[s < t ? s : t][s < t ? t : s] = 0.f, Bm[(s < t ? s : t) * CD_TP + (s < t ? t : s)] = 0.f;
         }
       }
   }
@@ -3422,8 +3450,33 @@ __global__ void __launch_bounds__(CD_REC_THREADS) fq3s_cdelta_record_kernel(cons
 #pragma unroll
       for (int s = 0; s < t; ++s) v = fmaf(-N[t][s], x[s], v);
       x[t] = v;
-      if (t >= tid) Tm[t * CD_TP + tid] = v;
+      if (t >= tid) Ts[t][tid] = v;
     }
+  }
+  if (warp > 0)      // meanwhile the keys become Kt
+    for (int i = tid - 32; i < CD_C * (D >> 2); i += CD_REC_THREADS - 32) {
+      const int t = i / (D >> 2), at = t * P + (i - t * (D >> 2)) * 4;
+      const float x = CHANNELS ? 0.f : pow2_f(sh[t]);
+      *reinterpret_cast<float4*>(ks + at) = mul4(ld4(ks + at), CHANNELS ? pow4(ld4(bh + at)) : make_float4(x, x, x, x));
+    }
+  __syncthreads();
+  for (int i = tid; i < CD_C * CD_C; i += CD_REC_THREADS) Tm[(i / CD_C) * CD_TP + i % CD_C] = Ts[i / CD_C][i % CD_C];
+  for (int i = tid; i < (D >> 2) * (CD_C / 4); i += CD_REC_THREADS) {      // W: four channels of tokens t4, t4 + 4, ..
+    const int c = (i % (D >> 2)) * 4, t4 = i / (D >> 2);
+    float4 w[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) w[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int s = 0; s < CD_C; ++s) {
+      const float4 k = ld4(ks + s * P + c);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float t = Ts[t4 + 4 * x][s];
+        w[x].x = fmaf(t, k.x, w[x].x); w[x].y = fmaf(t, k.y, w[x].y); w[x].z = fmaf(t, k.z, w[x].z); w[x].w = fmaf(t, k.w, w[x].w);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) *reinterpret_cast<float4*>(rec + (t4 + 4 * x) * P + c) = w[x];
   }
 }
 
@@ -3446,159 +3499,181 @@ __device__ __forceinline__ bool mbar_wait_bounded(const uint32_t bar, const uint
   }
   return false;
 }
-// grid (ceil(dv / DVT), H), 160 threads: four warps compute, the fifth asks for the records, one bulk copy per block of tokens, one block ahead.
-// The state tile [D rows, DVT columns] lives in registers (four rows x two columns x RQ per thread) and, as the operand of the next block's
-// products, transposed in shared memory.  [Kt; Qt] S0: a warp takes a quarter of the state rows for all 2 CD_C x DVT sums (a lane: rows r, r + 8,
-// r + 16, r + 24 and four columns; with eight columns the half-warps split the quarter once more and exchange halves of their sums), the quarters
-// are added where the sums are used.  U and O: a lane per (token, column).
-constexpr int CD_WALK_THREADS = 160;
-template <int DVT>
-__host__ __device__ constexpr int cd_walk_floats(int dk) {
-  return 2 * cd_record(dk) + DVT * cd_pitch(dk) + 4 * 2 * CD_C * (DVT + 1) + DVT * CD_TP + 4;
+// grid (ceil(dv / DVT), H), nine warps.  What one block of tokens hands to the next is the state alone, so four warps do nothing but that: W S0, U = T V - W S0, S <- diag(G_last) S0 +
+// Kb^T U.  The other four do what hangs on it: O = Qt S0 + B U of the block before, T V of the next one, for which its record has to be there, and then, while the state moves on, Qt S0.
+// The last warp asks for the records, one bulk copy per block of tokens, `ring` - 2 blocks ahead.
+// The state tile [D rows, DVT columns] lives in registers of the first four warps (four rows x two columns x RQ per thread) and, as the operand of the products, transposed in shared
+// memory, twice.  A product [16 tokens] x [DVT columns]: a warp takes a quarter of the state rows (a lane: rows r, r + 8 and four columns; with eight columns the half-warps split the
+// quarter once more and exchange halves of their sums), the quarters are added where the sums are used.  T V, U and O: a lane per (token, column).
+// Shared memory bounds it (a float for each of a warp's lanes is a cycle: the two products 384 each, the state's move 384, the rest 500, the copies 220 of a block's 2040): 94 blocks,
+// 8 heads of 128 x 128, with all of it one behind the other in four warps 108 us, so 100.
+constexpr int CD_WALK_THREADS = 288, CD_WALK_SMEM = 226 * 1024;
+__host__ __device__ constexpr int cd_walk_floats(int dvt, int dk, int ring) {
+  return ring * cd_record(dk) + 2 * dvt * cd_pitch(dk) + 2 * 4 * CD_C * (dvt + 1) + 5 * dvt * CD_TP + 8;
 }
+template <int ID, int COUNT> __device__ __forceinline__ void bar_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
+template <int ID, int COUNT> __device__ __forceinline__ void bar_arrive() { asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(COUNT) : "memory"); }
 template <int DVT, int RQ>
-__global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(const fq3c_op o) {
+__global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(const fq3c_op o, const int ring) {
   seq_dep_begin(o.M);
   extern __shared__ __align__(128) float cw[];
-  __shared__ __align__(8) unsigned long long full[2];
-  constexpr int NCP = DVT / 2, QS = 128 / NCP, CG = DVT / 4, KH = 4 / CG, PP = DVT + 1, JW = DVT / 4;
-  const int H = o.i0, dk = o.i2, dv = o.cin, h = blockIdx.y, j0 = blockIdx.x * DVT, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ __align__(8) unsigned long long full[4];
+  __shared__ int gone;                               // a wait ran out
+  constexpr int NCP = DVT / 2, QS = 128 / NCP, CG = DVT / 4, KH = 4 / CG, PP = DVT + 1, JW = DVT / 4, NJ = JW / 2;
+  const int H = o.i0, dk = o.i2, dv = o.cin, h = blockIdx.y, j0 = blockIdx.x * DVT, tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
+  const int role = threadIdx.x >> 7;                 // 0: the warps that carry the state, 1: the others, 2: the one that asks for the records
+  const bool chain = role == 0;
   const int D = cd_rows(dk), P = cd_pitch(dk), REC = cd_record(dk), nblk = (o.M + CD_C - 1) / CD_C;
-  float* St = cw + 2 * REC;                          // [DVT][P]
-  float* Xs = St + DVT * P;                          // [DVT][CD_TP]: V - Kt S0, then U
-  float* Pp = Xs + DVT * CD_TP;                      // [4][2 CD_C][PP]
+  float* St = cw + ring * REC;                       // [2][DVT][P]
+  float* Pp = St + 2 * DVT * P;                      // [4][CD_C][PP] of W S0, then of Qt S0
+  float* Pq = Pp + 4 * CD_C * PP;
+  float* Us = Pq + 4 * CD_C * PP;                    // [2][DVT][CD_TP]
+  float* Vs = Us + 2 * DVT * CD_TP;                  // [DVT][CD_TP] V of the next block
+  float* TV = Vs + DVT * CD_TP;                      // [2][DVT][CD_TP]
   const float* recs = reinterpret_cast<const float*>(o.ws) + cd_log_floats(o.M, H, dk, o.taps == 6) + (size_t)h * REC;
-  auto fetch = [&](const int n) {       // one thread
-    const uint32_t bar = smem_u32(&full[n & 1]);
+  auto fetch = [&](const int n, const int at) {       // one thread; record n into slot n % ring
+    const uint32_t bar = smem_u32(&full[at]);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)REC * 4u) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(cw + (n & 1) * REC)),
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(cw + at * REC)),
                  "l"(recs + (size_t)n * H * REC), "r"((uint32_t)REC * 4u), "r"(bar)
                  : "memory");
   };
-  if (tid == 128) {
-    mbar_init(smem_u32(&full[0]), 1);
-    mbar_init(smem_u32(&full[1]), 1);
+  if (threadIdx.x == 256) {
+    gone = 0;
+    for (int i = 0; i < ring; ++i) mbar_init(smem_u32(&full[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fetch(0);
+    for (int n = 0; n < min(ring, nblk); ++n) fetch(n, n);
   }
   __syncthreads();             // the barriers are initialised
-  if (warp == 4) {
-    for (int n = 0; n < nblk; ++n) {
-      if (__syncthreads_or(0)) return;       // the four warps gave up
-      if (lane == 0 && n + 1 < nblk) fetch(n + 1);
-      __syncthreads();
-      __syncthreads();
-    }
-    return;
-  }
   // this thread's part of the state: rows rq + q QS (quads), columns 2 cp, 2 cp + 1
   const int cp = tid % NCP, rq = tid / NCP;
   f32x2 S[RQ][2][2];          // [quad][column][row pair]
-  const float* st = reinterpret_cast<const float*>(o.p0) + (size_t)h * dk * dv;
+  if (chain) {
+    const float* st = reinterpret_cast<const float*>(o.p0) + (size_t)h * dk * dv;
 #pragma unroll
-  for (int q = 0; q < RQ; ++q)
+    for (int q = 0; q < RQ; ++q)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int r = (rq + q * QS) * 4, c = j0 + 2 * cp + j;
-      float v[4];
+      for (int j = 0; j < 2; ++j) {
+        const int r = (rq + q * QS) * 4, c = j0 + 2 * cp + j;
+        float v[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = (r + e < dk && c < dv) ? st[(size_t)(r + e) * dv + c] : 0.f;
-      S[q][j][0] = pack2(v[0], v[1]);
-      S[q][j][1] = pack2(v[2], v[3]);
-      if (r < D) *reinterpret_cast<float4*>(St + (2 * cp + j) * P + r) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-  // this thread's (token, column) pairs of U and O: token lane % 16, columns warp JW + lane / 16 (+ 2)
+        for (int e = 0; e < 4; ++e) v[e] = (r + e < dk && c < dv) ? st[(size_t)(r + e) * dv + c] : 0.f;
+        S[q][j][0] = pack2(v[0], v[1]);
+        S[q][j][1] = pack2(v[2], v[3]);
+        if (r < D) *reinterpret_cast<float4*>(St + (2 * cp + j) * P + r) = make_float4(v[0], v[1], v[2], v[3]);
+      }
+  }
+  // this thread's (token, column) pairs of T V, U and O: token lane % 16, columns warp JW + lane / 16 (+ 2)
   const int t = lane & (CD_C - 1), jb = warp * JW + (lane >> 4);
   const float* vrow = reinterpret_cast<const float*>(o.A) + o.a_rows + (size_t)h * dv + j0;
-  float vn[JW / 2];
+  float vn[NJ];
   auto load_v = [&](const int n) {
 #pragma unroll
-    for (int e = 0; e < JW / 2; ++e) {
+    for (int e = 0; e < NJ; ++e) {
       const int m = n * CD_C + t, j = jb + 2 * e;
       vn[e] = (m < o.M && j0 + j < dv) ? __ldg(vrow + (size_t)m * o.lda + j) : 0.f;
     }
   };
-  load_v(0);
-  const int rl = lane & 7, cl = (lane >> 3) % CG, kh = (lane >> 3) / CG, KW = (D >> 2) / KH;      // products: rows rl + 8 i of [Kt; Qt], columns cl + CG i
-  for (int n = 0; n < nblk; ++n) {
-    const bool there = mbar_wait_bounded(smem_u32(&full[n & 1]), (uint32_t)((n >> 1) & 1));
-    // the record is there, the transposed state too; everyone is done with the other buffer
-    if (__syncthreads_or(!there)) {
-      if (tid == 0) { wait_ran_out(); mbar_wait_bounded(smem_u32(&full[n & 1]), (uint32_t)((n >> 1) & 1)); }
-      for (int i = tid; i < o.M * DVT; i += 128)
+  auto row_times = [&](const float* m, const float* x) {       // sum_s m[t][s] x[s]
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int s = 0; s < CD_C; s += 4) {
+      const float4 mv = ld4(m + t * CD_TP + s), xv = ld4(x + s);
+      a = fmaf(mv.x, xv.x, a); b = fmaf(mv.y, xv.y, b);
+      a = fmaf(mv.z, xv.z, a); b = fmaf(mv.w, xv.w, b);
+    }
+    return a + b;
+  };
+  auto next_tv = [&](const int n, const float* rec) {      // T V of block n, whose record is there (the columns of a warp are its own); V of the one behind it is asked for
+#pragma unroll
+    for (int e = 0; e < NJ; ++e) Vs[(jb + 2 * e) * CD_TP + t] = vn[e];
+    load_v(n + 1);
+    __syncwarp();
+    const float* Tm = rec + 3 * CD_C * P + D;
+#pragma unroll
+    for (int e = 0; e < NJ; ++e) TV[((n & 1) * DVT + jb + 2 * e) * CD_TP + t] = row_times(Tm, Vs + (jb + 2 * e) * CD_TP);
+    __syncwarp();
+  };
+  const int rl = lane & 7, cl = (lane >> 3) % CG, kh = (lane >> 3) / CG, KW = (D >> 2) / KH;      // products: rows rl + 8 i, columns cl + CG j
+  auto product = [&](const float* rows, const float* state, float* out) {
+    f32x2 acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    const float* kr = rows + rl * P + (warp * KH + kh) * KW;
+    const float* sr = state + cl * P + (warp * KH + kh) * KW;
+#pragma unroll 4
+    for (int k = 0; k < KW; k += 4) {
+      ulonglong2 a[2], b[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(kr + 8 * i * P + k);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(sr + CG * j * P + k);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j] = fma2<true>(a[i].x, b[j].x, acc[i][j]);
+          acc[i][j] = fma2<true>(a[i].y, b[j].y, acc[i][j]);
+        }
+    }
+    float* pw = out + warp * CD_C * PP;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float v = lo2(acc[0][j]) + hi2(acc[0][j]), w = lo2(acc[1][j]) + hi2(acc[1][j]);
+      if (KH == 2) {       // a half-warp keeps one of the two rows
+        pw[(rl + 8 * kh) * PP + cl + CG * j] = (kh ? w : v) + __shfl_xor_sync(0xffffffffu, kh ? v : w, 16);
+      } else {
+        pw[rl * PP + cl + CG * j] = v;
+        pw[(rl + 8) * PP + cl + CG * j] = w;
+      }
+    }
+  };
+  auto quarters = [&](const float* part, const int j) {
+    const float* p = part + t * PP + j;
+    return (p[0] + p[CD_C * PP]) + (p[2 * CD_C * PP] + p[3 * CD_C * PP]);
+  };
+  if (role == 1) {
+    load_v(0);
+    if (mbar_wait_bounded(smem_u32(&full[0]), 0u)) next_tv(0, cw);
+    else gone = 1;
+  }
+  // slots of records n - 1, n and n + 1 (no division in the chain: the one thread that asked for the next record held it up by 500 cycles when it was one of these)
+  int sp = ring - 1, sn = 0, sx = 1;
+  uint32_t px = 0;      // parity of record n + 1
+  for (int n = 0;; ++n) {
+    __syncthreads();
+    // the state of block n, its T V and its record are there, U and Qt S0 of block n - 1 too; everyone is done with the rest of block n - 1
+    if (gone) {
+      __syncthreads();
+      if (threadIdx.x == 256) {      // the copies on their way end before the memory is given back
+        wait_ran_out();
+        for (int i = max(0, n - 2); i < min(max(n - 2, 0) + ring, nblk); ++i) mbar_wait_bounded(smem_u32(&full[i % ring]), (uint32_t)((i / ring) & 1), 1 << 14);
+      }
+      for (int i = threadIdx.x; i < o.M * DVT; i += CD_WALK_THREADS)
         if (j0 + i % DVT < dv) reinterpret_cast<float*>(o.C)[(size_t)(i / DVT) * o.ldc + (size_t)h * dv + j0 + i % DVT] = __int_as_float(0x7fc00000);
       return;
     }
-    const float* rec = cw + (n & 1) * REC;
-    {
-      f32x2 acc[4][4];
+    if (role != 1 && n == nblk) break;
+    const float* rec = cw + sn * REC;
+    const float* S0 = St + (n & 1) * DVT * P;
+    if (chain) {
+      product(rec, S0, Pp);
+      bar_sync<1, 128>();
+      bar_arrive<3, 256>();
+      float* U = Us + (n & 1) * DVT * CD_TP;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-      const float* kr = rec + rl * P + (warp * KH + kh) * KW;
-      const float* sr = St + cl * P + (warp * KH + kh) * KW;
-#pragma unroll 2
-      for (int k = 0; k < KW; k += 4) {
-        ulonglong2 a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(kr + 8 * i * P + k);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(sr + CG * j * P + k);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[i][j] = fma2<true>(a[i].x, b[j].x, acc[i][j]);
-            acc[i][j] = fma2<true>(a[i].y, b[j].y, acc[i][j]);
-          }
+      for (int e = 0; e < NJ; ++e) {
+        const int j = jb + 2 * e;
+        U[j * CD_TP + t] = TV[((n & 1) * DVT + j) * CD_TP + t] - quarters(Pp, j);
       }
-      float* pw = Pp + warp * 2 * CD_C * PP;
-#pragma unroll
-      for (int i = 0; i < 4; i += KH)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float v = lo2(acc[i][j]) + hi2(acc[i][j]);
-          if (KH == 2) {       // a half-warp keeps every other row of its four
-            const float w = lo2(acc[i + KH - 1][j]) + hi2(acc[i + KH - 1][j]);
-            v = (kh ? w : v) + __shfl_xor_sync(0xffffffffu, kh ? v : w, 16);
-          }
-          pw[(rl + 8 * (i + (KH == 2 ? kh : 0))) * PP + cl + CG * j] = v;
-        }
-    }
-    __syncthreads();
-    const float* Tm = rec + 3 * CD_C * P + D;
-    const float* Bm = Tm + CD_C * CD_TP;
-    auto quarters = [&](const int r, const int j) {
-      const float* p = Pp + r * PP + j;
-      return (p[0] + p[2 * CD_C * PP]) + (p[4 * CD_C * PP] + p[6 * CD_C * PP]);
-    };
-    auto row_times = [&](const float* m, const int j) {       // sum_s m[t][s] Xs[j][s]
-      const float* x = Xs + j * CD_TP;
-      float a = 0.f, b = 0.f;
-#pragma unroll
-      for (int s = 0; s < CD_C; s += 4) {
-        const float4 mv = ld4(m + t * CD_TP + s), xv = ld4(x + s);
-        a = fmaf(mv.x, xv.x, a); b = fmaf(mv.y, xv.y, b);
-        a = fmaf(mv.z, xv.z, a); b = fmaf(mv.w, xv.w, b);
-      }
-      return a + b;
-    };
-    float u[JW / 2];
-#pragma unroll
-    for (int e = 0; e < JW / 2; ++e) Xs[(jb + 2 * e) * CD_TP + t] = vn[e] - quarters(t, jb + 2 * e);
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < JW / 2; ++e) u[e] = row_times(Tm, jb + 2 * e);
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < JW / 2; ++e) Xs[(jb + 2 * e) * CD_TP + t] = u[e];
-    if (n + 1 < nblk) load_v(n + 1);
-    __syncthreads();
-    {   // S <- diag(G_last) S + Kb^T U
+      bar_sync<1, 128>();
+      // S <- diag(G_last) S + Kb^T U
       const float* Kb = rec + 2 * CD_C * P;
       const float* Gl = rec + 3 * CD_C * P;
-      const float* u0 = Xs + 2 * cp * CD_TP;
+      const float* u0 = U + 2 * cp * CD_TP;
+      float* S1 = St + ((n + 1) & 1) * DVT * P;
 #pragma unroll
       for (int q = 0; q < RQ; ++q) {
         const int r = (rq + q * QS) * 4;
@@ -3624,16 +3699,34 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-          *reinterpret_cast<ulonglong2*>(St + (2 * cp + j) * P + r) = make_ulonglong2(S[q][j][0], S[q][j][1]);
+          *reinterpret_cast<ulonglong2*>(S1 + (2 * cp + j) * P + r) = make_ulonglong2(S[q][j][0], S[q][j][1]);
       }
-    }
+    } else if (role == 2) {
+      if (lane == 0 && n > 1 && n - 2 + ring < nblk) fetch(n - 2 + ring, sp == 0 ? ring - 1 : sp - 1);
+    } else {
+      if (n > 0) {      // O = Qt S0 + B U
+        const float* Bm = cw + sp * REC + 3 * CD_C * P + D + CD_C * CD_TP;
+        const float* U = Us + ((n - 1) & 1) * DVT * CD_TP;
 #pragma unroll
-    for (int e = 0; e < JW / 2; ++e) {       // O = Qt S0 + B U
-      const int j = jb + 2 * e, m = n * CD_C + t;
-      const float ov = quarters(CD_C + t, j) + row_times(Bm, j);
-      if (m < o.M && j0 + j < dv) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + (size_t)h * dv + j0 + j] = ov;
+        for (int e = 0; e < NJ; ++e) {
+          const int j = jb + 2 * e, m = (n - 1) * CD_C + t;
+          const float ov = quarters(Pq, j) + row_times(Bm, U + j * CD_TP);
+          if (m < o.M && j0 + j < dv) reinterpret_cast<float*>(o.C)[(size_t)m * o.ldc + (size_t)h * dv + j0 + j] = ov;
+        }
+      }
+      if (n == nblk) break;
+      if (n + 1 < nblk) {
+        if (mbar_wait_bounded(smem_u32(&full[sx]), px)) next_tv(n + 1, cw + sx * REC);
+        else gone = 1;
+      }
+      bar_sync<3, 256>();      // the other product has ended, and everyone here has read Pq
+      product(rec + CD_C * P, S0, Pq);
     }
+    sp = sn;
+    sn = sx;
+    if (++sx == ring) { sx = 0; px ^= 1u; }
   }
+  if (!chain) return;
   float* nst = reinterpret_cast<float*>(o.C2) + (size_t)h * dk * dv;
 #pragma unroll
   for (int q = 0; q < RQ; ++q)
