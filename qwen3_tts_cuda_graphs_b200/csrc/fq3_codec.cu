@@ -1982,7 +1982,11 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
           (!(o.flags & (FQ3C_GATE_PRE | FQ3C_GATE_POST)) || o.i1 % 4 == 0) &&
           !((reinterpret_cast<uintptr_t>(o.A) | reinterpret_cast<uintptr_t>(o.C) | reinterpret_cast<uintptr_t>(o.C2) | reinterpret_cast<uintptr_t>(o.p1) |
              reinterpret_cast<uintptr_t>(o.res) | reinterpret_cast<uintptr_t>(o.scale)) & 15)) {
-        launch_after(fq3s_gnorm_warp_kernel, (unsigned)(((int64_t)o.M * o.i0 + 3) / 4), 128, 0, s, after, 1, o);
+        const unsigned blocks = (unsigned)(((int64_t)o.M * o.i0 + 3) / 4);
+        const int vecs = (o.N / o.i0 + 127) / 128;
+        if (vecs == 1) launch_after(fq3s_gnorm_warp_kernel<1>, blocks, 128, 0, s, after, 1, o);
+        else if (vecs == 2) launch_after(fq3s_gnorm_warp_kernel<2>, blocks, 128, 0, s, after, 1, o);
+        else launch_after(fq3s_gnorm_warp_kernel<GN_VECS>, blocks, 128, 0, s, after, 1, o);
         return 0;
       }
       launch_after(fq3s_gnorm_kernel, dim3(o.M, o.i0), row_threads(o.M, o.N / o.i0, 128), 0, s, after, 1, o);
@@ -2125,6 +2129,13 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
     case FQ3C_ROT_APPEND: {
       if (!rot_append_ok(o)) return fail("rot_append: bad configuration");
       if (o.m_begin > 0 && (o.i1 < 1 || o.cin < 1 || !o.norm_out || !o.ws || !o.p0)) return fail("rot_append: pooled blocks need both caches, their pooled rows and a position");
+      // what the flat kernel holds: no norm, no temperature, no pooled rows; the value heads not among the queries that it turns in place
+      if (o.M > DEP_ROWS && o.m_begin <= 0 && !o.scale && !o.bias && !(o.flags & FQ3C_UNIT) && !(o.f3 > 0.f) && o.taps <= 4096) {
+        const size_t smem = sizeof(float2) * (o.taps / 2);
+        if (o.flags & FQ3C_F32) launch_after(fq3s_rot_append_flat_kernel<float>, o.M, 256, smem, s, after, 1, o);
+        else launch_after(fq3s_rot_append_flat_kernel<bf16>, o.M, 256, smem, s, after, 1, o);
+        return 0;
+      }
       const int rth = o.M <= 8 ? std::max(256, std::min(1024, 32 * (o.i0 + o.i1))) : 256;      // few rows: a warp per head
       if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, true, 1024>, 1, rth, 0, s, after, 1, o);
       else if (o.m_begin > 0 && o.M == 1) launch_after(fq3s_rot_append_kernel<bf16, true, 1024>, 1, rth, 0, s, after, 1, o);

@@ -1041,7 +1041,10 @@ __device__ __forceinline__ void st4(bf16* p, const float (&v)[4]) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 // The same norm for many (row, group) pairs: a warp each, the group in registers, 16-byte loads.  grid (ceil(M * groups / 4)), 128 threads.
+// VECS: 16-byte pieces of a lane, as many as the group needs (gates cost an exponential and a division each, also of pieces that are not there: 1501 rows of 8 groups of 128 with four
+// 18.1 us, with one 7.0).
 constexpr int GN_VECS = 4;
+template <int VECS>
 __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
   seq_dep_begin(o.M);
   const long long pair = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -1051,9 +1054,9 @@ __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
   const bool pre = (o.flags & FQ3C_GATE_PRE) != 0, post = (o.flags & FQ3C_GATE_POST) != 0, plain = (o.flags & FQ3C_SIGMOID) != 0;
   const float* gate = (pre || post) ? reinterpret_cast<const float*>(o.p1) + (size_t)m * o.i1 + c0 : nullptr;
   const float inv = o.bias ? 1.f / reinterpret_cast<const float*>(o.bias)[(size_t)m * o.cin + gi] : 1.f;
-  float v[GN_VECS][4], g[GN_VECS][4];
+  float v[VECS][4], g[VECS][4];
 #pragma unroll
-  for (int q = 0; q < GN_VECS; ++q) {
+  for (int q = 0; q < VECS; ++q) {
     const int i = (q * 32 + lane) * 4;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (i < gsz) { a = ld4(x + i); if (gate) b = ld4(gate + i); }
@@ -1062,7 +1065,7 @@ __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
   }
   float sm = 0.f, ss = 0.f;
 #pragma unroll
-  for (int q = 0; q < GN_VECS; ++q)
+  for (int q = 0; q < VECS; ++q)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (gate) g[q][e] = gate_f(g[q][e], plain);
@@ -1071,7 +1074,7 @@ __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
     }
   const float mean = (o.flags & FQ3C_CENTER) ? warp_sum(sm) / (float)gsz : 0.f;
 #pragma unroll
-  for (int q = 0; q < GN_VECS; ++q)
+  for (int q = 0; q < VECS; ++q)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       v[q][e] -= mean;
@@ -1082,7 +1085,7 @@ __global__ void __launch_bounds__(128) fq3s_gnorm_warp_kernel(const fq3c_op o) {
   const int wmod = o.i2 > 0 ? o.i2 : o.N;
   const size_t orow = (size_t)m + (o.p0 ? (size_t)*reinterpret_cast<const int*>(o.p0) : 0);
 #pragma unroll
-  for (int q = 0; q < GN_VECS; ++q) {
+  for (int q = 0; q < VECS; ++q) {
     const int i = (q * 32 + lane) * 4;
     if (i >= gsz) continue;
     float4 wv = make_float4(1.f, 1.f, 1.f, 1.f), r = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1759,12 +1762,21 @@ __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) 
 // m_begin = P > 0: every run of P positions bP .. bP + P - 1 that the step completes leaves the mean of its P cached keys and values as
 // row b of norm_out / ws.  A single row does it here (POOL; its block has just written the run's last row); more rows take
 // fq3s_pool_append_kernel behind this launch.
-// A warp turns (norms, tempers) one query or key head at position pos; put(i, v) takes entry i.  freq, flo: the frequencies and what they lost to rounding (or null).
-// all: also the entries that stay as they are.
+// Sine and cosine by which pair i turns at position pos, times the amplitude.  freq, flo: the frequencies and what they lost to rounding (or null).
+__device__ __forceinline__ float2 rot_angle(const fq3c_op& o, const float* freq, const float* flo, const int i, const float fp) {
+  float sn, cs;
+  const float ang = fp * freq[i], amp = o.f1 != 0.f ? o.f1 : 1.f;
+  sincosf(ang, &sn, &cs);
+  // what the product (and, with flo, the frequency) lost to rounding turns the pair a little further: at large angles it would show
+  float rest = fmaf(fp, freq[i], -ang);
+  if (flo) rest = fmaf(fp, flo[i], rest);
+  return make_float2(fmaf(cs, rest, sn) * amp, fmaf(-sn, rest, cs) * amp);
+}
+// A warp turns (norms, tempers) one query or key head at position pos; put(i, v) takes entry i.  all: also the entries that stay as they are.
 template <typename Put>
 __device__ __forceinline__ void rot_head(const fq3c_op& o, const float* freq, const float* flo, const float* src, const bool isq, const int pos, const int lane, const bool all, Put put) {
   const int d = o.i2, half = o.taps >> 1;
-  const float fp = (float)pos, amp = o.f1 != 0.f ? o.f1 : 1.f;
+  const float fp = (float)pos;
   const float* nw = reinterpret_cast<const float*>(isq ? o.scale : o.bias);
   const bool unit = nw || (o.flags & FQ3C_UNIT), normed = unit || (isq && o.f3 > 0.f);
   float rs = 1.f;
@@ -1777,14 +1789,8 @@ __device__ __forceinline__ void rot_head(const fq3c_op& o, const float* freq, co
   if (isq) rs *= o.f3 > 0.f ? fmaf(o.f2, logf(floorf((fp + 1.f) / o.f3) + 1.f), 1.f) : 1.f;
   const bool halves = (o.flags & FQ3C_ROT_HALF) != 0;      // pairs (i, i + half) instead of (2i, 2i + 1)
   for (int i = lane; i < half; i += 32) {
-    float sn, cs;
-    const float ang = fp * freq[i];
-    sincosf(ang, &sn, &cs);
-    // what the product (and, with p1, the frequency) lost to rounding turns the pair a little further: at large angles it would show
-    float rest = fmaf(fp, freq[i], -ang);
-    if (flo) rest = fmaf(fp, flo[i], rest);
-    const float s1 = fmaf(cs, rest, sn), c1 = fmaf(-sn, rest, cs);
-    sn = s1 * amp; cs = c1 * amp;
+    const float2 sc = rot_angle(o, freq, flo, i, fp);
+    const float sn = sc.x, cs = sc.y;
     const int ia = halves ? i : 2 * i, ib = halves ? i + half : 2 * i + 1;
     float a = src[ia], b = src[ib];
     if (normed) { a *= rs; b *= rs; }
@@ -1827,6 +1833,49 @@ __global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op 
     __syncthreads();
     pool_run<TC>(reinterpret_cast<const TC*>(o.C), o.ldc, reinterpret_cast<TC*>(o.norm_out), pos / o.m_begin, o.m_begin, threadIdx.x, G * d, blockDim.x);
     pool_run<TC>(reinterpret_cast<const TC*>(o.C2), o.ldr, reinterpret_cast<TC*>(o.ws), pos / o.m_begin, o.m_begin, threadIdx.x, G * dv, blockDim.x);
+  }
+}
+
+// The same for many rows whose heads are neither normed nor tempered: a block per row forms each pair's sine and cosine once, for all heads, and its threads take the entries as they
+// come (a warp per head had three heads one behind the other, each with its own sine: 2048 rows of 16 + 4 heads, 32 of 128 entries turned, 15.2 us; this way 9.0).
+// grid (M), 256 threads, dynamic shared memory: a float2 per pair
+template <typename TC>
+__global__ void __launch_bounds__(256) fq3s_rot_append_flat_kernel(const fq3c_op o) {
+  seq_dep_begin(o.M);
+  extern __shared__ float2 turn[];
+  const int m = blockIdx.x, H = o.i0, G = o.i1, d = o.i2, dv = o.cin, half = o.taps >> 1;
+  const int pos = (o.p0 ? *reinterpret_cast<const int*>(o.p0) : 0) + m;
+  float* row = const_cast<float*>(reinterpret_cast<const float*>(o.A)) + (size_t)m * o.lda;
+  const float* krow = o.res ? reinterpret_cast<const float*>(o.res) + (size_t)m * o.norm_ld : row;
+  const bool halves = (o.flags & FQ3C_ROT_HALF) != 0;      // pairs (i, i + half) instead of (2i, 2i + 1)
+  for (int i = threadIdx.x; i < half; i += blockDim.x) turn[i] = rot_angle(o, reinterpret_cast<const float*>(o.B), reinterpret_cast<const float*>(o.p1), i, (float)pos);
+  TC* kc = G > 0 ? reinterpret_cast<TC*>(o.C) + (size_t)pos * o.ldc : nullptr;
+  if (G > 0 && dv > 0) {      // (nothing here waits for the sines)
+    TC* vc = reinterpret_cast<TC*>(o.C2) + (size_t)pos * o.ldr;
+    const float* v = krow + o.a_rows;
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < G * dv; idx += blockDim.x) stf(vc + idx, v[idx]);
+  }
+  const int rest = d - 2 * half;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < G * rest; idx += blockDim.x) {
+    const int g = idx / rest, at = g * d + 2 * half + idx - g * rest;
+    stf(kc + at, krow[o.K + at]);
+  }
+  __syncthreads();
+#pragma unroll 2
+  for (int idx = threadIdx.x; idx < (H + G) * half; idx += blockDim.x) {
+    const int hh = idx / half, i = idx - hh * half, ia = halves ? i : 2 * i, ib = halves ? i + half : 2 * i + 1;
+    const bool isq = hh < H;
+    const float* src = isq ? row + (size_t)hh * d : krow + o.K + (size_t)(hh - H) * d;
+    const float a = src[ia], b = src[ib], sn = turn[i].x, cs = turn[i].y, x = a * cs - b * sn, y = b * cs + a * sn;
+    if (isq) {
+      float* q = row + (size_t)hh * d;
+      q[ia] = x; q[ib] = y;
+    } else {
+      TC* k = kc + (size_t)(hh - H) * d;
+      stf(k + ia, x); stf(k + ib, y);
+    }
   }
 }
 
