@@ -1426,6 +1426,7 @@ __global__ void __launch_bounds__(C1_ROWS) fq3c_conv1_kernel(const fq3c_op o, co
 #include "fq3_seq.cuh"
 #include "fq3_f32.cuh"
 #include "fq3_gemm.cuh"
+#include "fq3_ggemm.cuh"
 #include "fq3_attn.cuh"
 
 int fail(const std::string& m) { g_err = m; return -1; }
@@ -1718,6 +1719,21 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     else if (a_f32) launch_after(fq3s_ggemv_kernel<float, bf16>, grid, 256, smem, s, after, 1, g);
     else launch_after(fq3s_ggemv_kernel<bf16, bf16>, grid, 256, smem, s, after, 1, g);
     return 0;
+  }
+  // Experts on tcgen05: whole 16-byte pieces, each expert's weights behind the last one's.  A tile's 128 rows and 128 columns pay from some two hundred chosen rows on; below, the 64-column
+  // tiles of the other kernel have more CTAs in flight (layers without a shared expert: 33 rows x 2 of 16 experts 50.8 and 54.4 us, 17 x 4 of 8 50.6 and 55.6, 200 x 1 of 16 54.7 and 45.9,
+  // 64 x 4 of 32 104 and 80, 701 x 2 of 16 81 and 51, 2048 x 4 of 32, 2048 wide, 527 and 245).
+  if (g.seg && zcount == 1 && !a_f32 && !b_f32 && g.M >= 192 && g.K >= TK && g.K % 8 == 0 && g.lda % 8 == 0 && g.ldb == g.K && g.b_estride == (long long)g.N * g.K && (long long)g.E * g.N < (1LL << 31) &&
+      !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) && device_attrs_ready()) {
+    CUtensorMap tmB;
+    if (make_map(&tmB, g.B, (uint64_t)g.K, (uint64_t)g.E * g.N, (uint64_t)g.K, GT_BN)) {
+      const dim3 grid((g.N + GT_BN - 1) / GT_BN, (g.M + TM - 1) / TM + g.E);
+      const bool glu = g.flags & FQ3C_SWIGLU;      // whole 32 bytes of a row (16 columns: of gated units 16 bytes)
+      const int whole = !(reinterpret_cast<uintptr_t>(g.C) & (glu ? 15 : 31)) && g.ldc % (glu || (g.flags & FQ3C_OUT_F32) ? 8 : 16) == 0;
+      if (glu) launch_after(fq3s_ggemm_tc_kernel<true>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
+      else launch_after(fq3s_ggemm_tc_kernel<false>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
+      return 0;
+    }
   }
   // bf16 rows of whole 16-byte pieces (what its copies ask for): the pipelined product, faster at every size (figures at the kernel)
   if (!a_f32 && !b_f32 && !((g.K | g.lda | g.ldb | g.a_zstride) & 7) && !((g.b_zstride | g.b_estride) & 7) &&
@@ -2513,6 +2529,8 @@ static bool device_attrs_ready() {
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_gemm_persist_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_HALF) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3s_ggemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(fq3s_ggemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_rows_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_rows_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(fq3c_attn_rows_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AR_SMEM_MAX) != cudaSuccess ||
