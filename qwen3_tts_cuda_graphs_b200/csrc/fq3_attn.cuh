@@ -10,6 +10,7 @@ struct AttnArgs {
   long ldq, ldk, ldv;
   int H, G, M;
   int groups;               // row groups per CTA: 1 or 2
+  int ends;                 // 1: a CTA's two groups are one from the end of the rows and one from their beginning, else they are neighbours
   int two_from;             // > 0: launched with one, but behind more positions than these a CTA takes two and every other one leaves
   const int* p0;            // position of query 0 (device), or null: 0
   float scale, cap, mult;   // mult != 0 multiplies the output
@@ -67,6 +68,19 @@ __device__ __forceinline__ float ex2f(const float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// cap * tanh(x), cap * tanh(y) for |x|, |y| up to AT_NEAR: x (1 - t/3 + 2 t^2/15 - 17 t^3/315 + 62 t^4/2835), t = x^2, the first terms of the series, which leave 2.4e-7 of the result.  Seven
+// packed multiply-adds for two scores, where the exponential and the reciprocal of fast_tanh (1e-6) are two more turns each on the special-function unit beside the weight's own.
+constexpr float AT_NEAR = 0.35f;
+__device__ __forceinline__ void cap_near(float& x, float& y, const float cap) {
+  const f32x2 v = pack2(x, y), t = mul2<true>(v, v);
+  f32x2 p = fma2<true>(t, pack2(62.f / 2835.f, 62.f / 2835.f), pack2(-17.f / 315.f, -17.f / 315.f));
+  p = fma2<true>(t, p, pack2(2.f / 15.f, 2.f / 15.f));
+  p = fma2<true>(t, p, pack2(-1.f / 3.f, -1.f / 3.f));
+  const f32x2 c = mul2<true>(v, pack2(cap, cap));
+  p = fma2<true>(mul2<true>(t, p), c, c);
+  x = lo2(p); y = hi2(p);
 }
 
 // 16 finished entries of an output row, f32 or rounded
@@ -176,13 +190,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
 
   const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
   const bool one = groups == 1;      // its tiles take the score columns of both groups in turn
-  const int m0 = (gx - 1 - (int)blockIdx.x) * groups * QB;   // the last queries (most keys) start first
+  // the last queries (most keys) start first
+  const int all = (a.M + QB - 1) / QB, late = all - 1 - (int)blockIdx.x, m0 = (gx - 1 - (int)blockIdx.x) * groups * QB;
+  const bool ends = a.ends && !one;
+  const int mg[2] = {ends ? late * QB : m0, ends ? ((int)blockIdx.x < late ? (int)blockIdx.x * QB : a.M) : m0 + QB};      // each group's first query
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
-    nq[g] = g < groups ? max(0, min(QB, a.M - m0 - g * QB)) : 0;
-    first[g] = P + m0 + g * QB;
+    nq[g] = g < groups ? max(0, min(QB, a.M - mg[g])) : 0;
+    first[g] = P + mg[g];
     last[g] = first[g] + nq[g] - 1;
     tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
     int lo = a.window > 0 ? max(0, first[g] - a.window + 1) : 0;
@@ -190,7 +207,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     tlo[g] = lo / AT_KEYS;
   }
   const int tkeep = a.window > 0 && a.chunk <= 0 ? (a.keep + AT_KEYS - 1) / AT_KEYS : 0;
-  const int ntiles = max(tiles[0], tiles[1]), jend = P + min(a.M, m0 + groups * QB) - 1;
+  const int ntiles = max(tiles[0], tiles[1]), jend = nq[1] > 0 ? max(last[0], last[1]) : last[0];
   auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
 
   if (warp == 19) {
@@ -349,7 +366,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           for (int i = 0; i < 8; ++i) {
             const int r = (half * 4 + wq) * 16 + b + i, qi = min(r / HG, nqg - 1), hh = min(r - qi * HG, HG - 1);
             x[i] = *reinterpret_cast<const Quad*>(reinterpret_cast<const typename std::conditional<MODE == AT_PROMPT, bf16, float>::type*>(a.q) +
-                                                  (size_t)(m0 + g * QB + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
+                                                  (size_t)((g ? mg[1] : mg[0]) + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -385,14 +402,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         return other[turn * 512];
       };
       // the score of entry i of the tile in front of the mask, from the raw product
-      auto score2 = [&](float& x, float& y, const int key) {
+      auto score2 = [&](float& x, float& y, const int key, const bool near) {
         if (MODE == AT_PROMPT) {
           round2(x, y);
           x *= a.scale; y *= a.scale;
           round2(x, y);
         } else {
           x *= a.scale; y *= a.scale;
-          if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) { x = a.cap * fast_tanh(x * icap); y = a.cap * fast_tanh(y * icap); }
+          if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) {
+            x *= icap; y *= icap;
+            if (near) cap_near(x, y, a.cap);
+            else { x = a.cap * fast_tanh(x); y = a.cap * fast_tanh(y); }
+          }
           if (MODE == AT_DIST && a.r12) {
             x -= r1 * __logf(fmaf(r2, fmaxf((float)(pos - key), 0.f), 1.f));
             y -= r1 * __logf(fmaf(r2, fmaxf((float)(pos - key - 1), 0.f), 1.f));
@@ -419,8 +440,20 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
         for (int h = 0; h < 2; ++h) {
           if (h == 0) tmem_ld32(s_t + 32, s[1]);      // on its way while the first half is worked on
           if (k0 + h * 32 <= wlast) {      // (keys behind every row of the warp: masked below, whatever they are)
+            bool near = false;
+            if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) {      // of a whole warp: no score of its rows is far up the cap (a NaN is)
+              float far = fabsf(s[h][0]);
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i);
+              for (int i = 1; i < 32; ++i) far = fmaxf(far, fabsf(s[h][i]));
+              near = __all_sync(0xffffffffu, far * a.scale * icap <= AT_NEAR);
+            }
+            if (near) {
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i, true);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) score2(s[h][i], s[h][i + 1], k0 + h * 32 + i, false);
+            }
           }
           if (!whole) {
             // which of the 32 keys the row sees, as bits: conditions per score became divergent branches (8 400 cycles a tile)
@@ -542,7 +575,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     }
     const int n = (nq[0] + nq[1]) * HG * 128;
     for (int i = tid; i < n; i += AT_THREADS) {
-      const size_t at = (size_t)(m0 + i / (HG * 128)) * a.ldo + (size_t)kvh * HG * 128 + i % (HG * 128);
+      const int q = i / (HG * 128), m = q < nq[0] ? mg[0] + q : mg[1] + q - nq[0];
+      const size_t at = (size_t)m * a.ldo + (size_t)kvh * HG * 128 + i % (HG * 128);
       if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = __int_as_float(0x7fffffff);
       else reinterpret_cast<uint16_t*>(a.out)[at] = 0x7fff;
     }

@@ -1619,14 +1619,19 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
   const int group = 128 / (a.H / a.G);
   const long ctas = (long)((a.M + group - 1) / group) * a.G;      // of one group each
   a.groups = ctas <= GP_SMS ? 1 : 2;
-  a.two_from = 0;
-  // With a cap the special-function unit sets the pace, which a second group fills little: two groups take 1.55 times one's time.  So one pays for some more CTAs than SMs, where
-  // the first rows' short ones make room for the others: without a window, few positions in front of the rows, and the more so the fewer key heads the rows are spread over.  Two
-  // groups against one, 16 heads over 4: 1300 rows (164 CTAs) 67 and 44 us, behind 1500 positions 132 and 112, behind 4000 238 and 246; 2048 (256) 101 and 91, behind 500 122 and
-  // 118, behind 1500 166 and 172; of 32 heads over 8 1100 rows (280) 61 and 66, of 16 over 16 1900 (240) 85 and 94; under a window of 256 1800 rows (228) 31 and 36.
-  if (mode == AT_CAP && a.groups == 2 && a.window <= 0 && a.chunk <= 0 && ctas <= (a.G <= 4 ? 256 : 168)) {
-    a.groups = 1;
-    if (a.p0) a.two_from = a.G <= 4 && ctas <= 200 ? a.M / 4 * 3 : a.M / 4;
+  a.two_from = a.ends = 0;
+  // Up to twice as many row groups as SMs, and no window: a CTA's two groups are one from the end of the rows and one from their beginning, whose few tiles are among the other's, so
+  // that no CTA has two of the longest (and the last one alone in the end).  Neighbours, ends (us of a layer, 16 heads over 4): 2048 rows with a cap 112 and 102, without 101 and 92,
+  // 1700 behind 300 98 and 90; two layers of the talker (16 over 8), 1900 rows 366 and 354, 1500 318 and 307.  Under a window the neighbours share their tiles: 2048 rows of 256 63 and 69.
+  // Of few more groups than SMs one to a CTA is faster still, the short ones go in behind the others: one, ends: 1300 rows (164 groups) 66 and 71, with a cap 69 and 79, 1500 (188) 75
+  // and 75, with a cap 80 and 83, 1700 (213) 90 and 83, 96 and 94; the talker's 1200 rows (152) 261 and 274, 1350 (169) 297 and 293.  Behind many positions all groups are long: with
+  // two_from the kernel then takes two (1500 behind 500, cap: 102 and 98; 1300 behind 700 86 and 88).
+  if (a.groups == 2 && a.window <= 0 && a.chunk <= 0 && mode != AT_DIST && (ctas + 1) / 2 <= GP_SMS) {
+    a.ends = 1;
+    if (ctas <= (mode == AT_PROMPT ? 160 : mode == AT_CAP ? 200 : 188)) {
+      a.groups = 1;
+      if (a.p0) a.two_from = ctas <= 176 ? a.M / 4 * 3 : a.M / 4;
+    }
   }
   const int per = a.groups * group;
   const dim3 grid((a.M + per - 1) / per, a.G);
