@@ -191,15 +191,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   const int HG = a.H / a.G, QB = 128 / HG, kvh = blockIdx.y;
   const bool one = groups == 1;      // its tiles take the score columns of both groups in turn
   // the last queries (most keys) start first
-  const int all = (a.M + QB - 1) / QB, late = all - 1 - (int)blockIdx.x, m0 = (gx - 1 - (int)blockIdx.x) * groups * QB;
-  const bool ends = a.ends && !one;
-  const int mg[2] = {ends ? late * QB : m0, ends ? ((int)blockIdx.x < late ? (int)blockIdx.x * QB : a.M) : m0 + QB};      // each group's first query
+  int m0 = (gx - 1 - (int)blockIdx.x) * groups * QB, m1 = m0 + QB;      // each group's first query
+  if (a.ends && !one) {
+    const int late = (a.M + QB - 1) / QB - 1 - (int)blockIdx.x;
+    m0 = late * QB;
+    m1 = (int)blockIdx.x < late ? (int)blockIdx.x * QB : a.M;
+  }
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
-    nq[g] = g < groups ? max(0, min(QB, a.M - mg[g])) : 0;
-    first[g] = P + mg[g];
+    nq[g] = g < groups ? max(0, min(QB, a.M - (g ? m1 : m0))) : 0;
+    first[g] = P + (g ? m1 : m0);
     last[g] = first[g] + nq[g] - 1;
     tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
     int lo = a.window > 0 ? max(0, first[g] - a.window + 1) : 0;
@@ -366,7 +369,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           for (int i = 0; i < 8; ++i) {
             const int r = (half * 4 + wq) * 16 + b + i, qi = min(r / HG, nqg - 1), hh = min(r - qi * HG, HG - 1);
             x[i] = *reinterpret_cast<const Quad*>(reinterpret_cast<const typename std::conditional<MODE == AT_PROMPT, bf16, float>::type*>(a.q) +
-                                                  (size_t)((g ? mg[1] : mg[0]) + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
+                                                  (size_t)(firstg - P + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -575,7 +578,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     }
     const int n = (nq[0] + nq[1]) * HG * 128;
     for (int i = tid; i < n; i += AT_THREADS) {
-      const int q = i / (HG * 128), m = q < nq[0] ? mg[0] + q : mg[1] + q - nq[0];
+      const int q = i / (HG * 128), m = q < nq[0] ? m0 + q : m1 + q - nq[0];
       const size_t at = (size_t)m * a.ldo + (size_t)kvh * HG * 128 + i % (HG * 128);
       if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = __int_as_float(0x7fffffff);
       else reinterpret_cast<uint16_t*>(a.out)[at] = 0x7fff;

@@ -36,7 +36,12 @@ inline void count_launches(int64_t n) { g_launches += n; t_launches += n; }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // One launch ahead: with the next one let in before this wait, launches pile up on the SMs (28 layers of a prompt of 39 rows 1128 us, this way 1118; a codec window 717 and 705).
-__device__ __forceinline__ void grid_dep_begin() { grid_dep_wait(); grid_dep_launch(); }
+// Not behind many rows, whose launches take longer than those behind them need to come up (four layers of 1000 rows 413 and 416).
+__device__ __forceinline__ void grid_dep_begin(const int rows = 0) {
+  if (rows > 512) grid_dep_launch();
+  grid_dep_wait();
+  if (rows <= 512) grid_dep_launch();
+}
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -674,7 +679,7 @@ bool norm_vec_ok(const void* x, const void* y, const void* w, const int N, const
 constexpr int RN_WARPS = 4;
 __global__ void __launch_bounds__(RN_WARPS * 32) fq3c_rownorm_vec_kernel(const bf16* x, const int ldx, bf16* y, const int ldy, const float* w, const float eps, const int row0, const int rows,
                                                                          const int N) {
-  grid_dep_begin();
+  grid_dep_begin(rows);
   const int row = blockIdx.x * RN_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(row0 + row) * ldx);
@@ -1015,7 +1020,7 @@ __global__ void __launch_bounds__(APF_WARPS * 32) fq3c_attn_prefill_kernel(const
 //   k / v heads: the finished row is also written to the static KV cache C (K) / C2 (V), laid out [kv_head][ldc][128].
 // Same arithmetic as head_norm_rope / the KV append of the decode kernel (fq3_kernel.cuh), so decode steps can attend to it.
 __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
-  grid_dep_begin();
+  grid_dep_begin(o.M);
   const int nq = o.i0, nkv = o.i1, pos0 = o.i2, nheads = nq + 2 * nkv;
   const int wpb = blockDim.x >> 5;
   const int gw = blockIdx.x * wpb + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1698,6 +1703,16 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     }
     dim3 grid((g.N + 7) / 8, 1, zcount);
     static const SeqTail none{};
+    const int piece = b_f32 ? 4 : 8;
+    const bool one = g.M == 1 && zcount == 1 && a_f32 == b_f32 && g.K % piece == 0 && g.ldb % piece == 0 && !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15);
+    if (one) {
+      const bool more = tail && tail->n > 0;
+      if (more && b_f32) launch_after(fq3s_gemv_kernel<float, float, true, true>, grid, 256, 0, s, after, 1, g, *tail);
+      else if (more) launch_after(fq3s_gemv_kernel<bf16, bf16, true, true>, grid, 256, 0, s, after, 1, g, *tail);
+      else if (b_f32) launch_after(fq3s_gemv_kernel<float, float, false, true>, grid, 256, 0, s, after, 1, g, none);
+      else launch_after(fq3s_gemv_kernel<bf16, bf16, false, true>, grid, 256, 0, s, after, 1, g, none);
+      return 0;
+    }
     if (tail && tail->n > 0 && a_f32 == b_f32) {
       if (b_f32) launch_after(fq3s_gemv_kernel<float, float, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
       else launch_after(fq3s_gemv_kernel<bf16, bf16, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
@@ -1889,7 +1904,7 @@ bool attn_few_takes(const fq3c_op& o) {
   const long keys = o.K > 0 && o.a_rows <= 0 ? o.K : o.tap_off[0] > 0 ? o.tap_off[0] : splits < 64 ? 32L * splits : 1L << 30;
   auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
   const int V = o.flags & FQ3C_F32 ? 4 : 8, HG = o.i1 > 0 ? o.i0 / o.i1 : 0;
-  return o.M <= DEP_ROWS && (HG == 1 || keys <= (HG == 8 ? 1024 : 2048)) && (o.i2 == 64 || o.i2 == 128) && o.cin == o.i2 && o.i0 >= 1 && o.i1 >= 1 && o.i0 % o.i1 == 0 && (HG <= 4 || HG == 8) && o.i1 <= 65535 && o.tap_off[1] <= 0 &&
+  return o.M <= AF_ROWS && (HG == 1 || keys <= (HG == 8 ? 1024 : 2048)) && (o.i2 == 64 || o.i2 == 128) && o.cin == o.i2 && o.i0 >= 1 && o.i1 >= 1 && o.i0 % o.i1 == 0 && (HG <= 4 || HG == 8) && o.i1 <= 65535 && o.tap_off[1] <= 0 &&
          o.A && o.B && o.p1 && o.C && o.ldr % V == 0 && o.taps % V == 0 && !off(o.B) && !off(o.p1);
 }
 // `r` (rotation, cache rows) and the attention `o` of the same single row behind it
@@ -2151,7 +2166,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       if (!rot_append_ok(o)) return fail("rot_append: bad configuration");
       if (o.m_begin > 0 && (o.i1 < 1 || o.cin < 1 || !o.norm_out || !o.ws || !o.p0)) return fail("rot_append: pooled blocks need both caches, their pooled rows and a position");
       // what the flat kernel holds: no norm, no temperature, no pooled rows; the value heads not among the queries that it turns in place
-      if (o.M > DEP_ROWS && o.m_begin <= 0 && !o.scale && !o.bias && !(o.flags & FQ3C_UNIT) && !(o.f3 > 0.f) && o.taps <= 4096) {
+      if (o.M > 8 && o.m_begin <= 0 && !o.scale && !o.bias && !(o.flags & FQ3C_UNIT) && !(o.f3 > 0.f) && o.taps <= 4096) {
         const size_t smem = sizeof(float2) * (o.taps / 2);
         if (o.flags & FQ3C_F32) launch_after(fq3s_rot_append_flat_kernel<float>, o.M, 256, smem, s, after, 1, o);
         else launch_after(fq3s_rot_append_flat_kernel<bf16>, o.M, 256, smem, s, after, 1, o);

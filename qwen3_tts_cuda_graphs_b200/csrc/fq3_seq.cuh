@@ -11,9 +11,10 @@ __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 // With few rows (decoding) a list is a chain of launches of some 3 us each, so the next one's blocks come up while this one works and wait here for its end.  One launch ahead, not more:
-// with the next launch let in before this wait, waiting blocks pile up (a token of 36 launches 163 us of the GPU's time without, 180 with many ahead, 149 with one).  With many rows
-// the blocks of the next launch would only take room: they then come up two on an SM beside others that stay empty (an attention layer of 384 rows in 32 bits 143 -> 159 us).
-constexpr int DEP_ROWS = 8;
+// with the next launch let in before this wait, waiting blocks pile up (a token of 36 launches 163 us of the GPU's time without, 180 with many ahead, 149 with one).  With more
+// rows blocks that come up early come up several on one SM, beside others that stay empty, which a launch that has work for all of them pays for (an attention layer of 4 rows
+// behind 300 positions 39 us without, 59 with; of 384 rows in 32 bits 143 and 159).
+constexpr int DEP_ROWS = 2;
 __device__ __forceinline__ void seq_dep_begin(const int rows) {
   grid_dep_wait();
   if (rows <= DEP_ROWS) grid_dep_launch();
@@ -649,7 +650,9 @@ struct SeqTail { int n; fq3c_op op[2]; };
 // in front of the sums: 17 products of a token 78 -> 60 us with the early launches, of which 12 are the latter two.
 // TAIL: lane m goes on with entry (m, n) of row m through the ops of `tail`, with their own arithmetic: each was a launch of its own of 2 us, of which a decoded token of
 // four layers had sixteen.
-template <typename TA, typename TB, bool TAIL = false>
+// ONE: a single row, rows and columns of whole 16-byte pieces of one type (a variant of its own: the registers that it takes cost the others two of four blocks an SM, four rows of
+// 16 heads' projections 5 us).
+template <typename TA, typename TB, bool TAIL = false, bool ONE = false>
 __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ SeqGemm g, const __grid_constant__ SeqTail tail) {
   extern __shared__ float xs[];  // [M][K]
   const int z = blockIdx.z;
@@ -673,15 +676,13 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ 
     }
   };
   if (g.early) first();
-  if (warp == 0) {
+  if (warp == 0 && g.M <= DEP_ROWS) {
     args_ahead(g);
     if (TAIL) args_ahead(tail);
   }
   seq_dep_begin(g.M);
   if (!g.early) first();
-  // one row of whole 16-byte pieces: each lane's entries go straight to its registers
-  const bool direct = sizeof(TA) == sizeof(TB) && g.M == 1 && vec && (reinterpret_cast<uintptr_t>(Ap) & 15) == 0;
-  if (!direct) {
+  if (!ONE) {
     for (int m = 0; m < g.M; ++m) stage_row_f32<TA>(xs + (size_t)m * g.K, Ap + (size_t)m * g.lda, g.K, threadIdx.x, blockDim.x);
     __syncthreads();
   }
@@ -689,11 +690,14 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ 
   DytEntry dyt{};
   MixEntry mix{};
   XieluEntry xielu{};
-  if (TAIL && lane < g.M) {      // what the tail reads apart from its entry
-    if (tail.op[0].kind == FQ3C_XIELU) xielu = xielu_entry(tail.op[0]);
-    else dyt = dyt_entry(tail.op[0], lane, n);
-    if (tail.n > 1) mix = mix_entry(tail.op[1], lane, n);
-  }
+  auto apart = [&] {      // what the tail reads apart from its entry
+    if (TAIL && lane < g.M) {
+      if (tail.op[0].kind == FQ3C_XIELU) xielu = xielu_entry(tail.op[0]);
+      else dyt = dyt_entry(tail.op[0], lane, n);
+      if (tail.n > 1) mix = mix_entry(tail.op[1], lane, n);
+    }
+  };
+  if (ONE) apart();
   float acc[8];
 #pragma unroll
   for (int m = 0; m < 8; ++m) acc[m] = 0.f;
@@ -706,7 +710,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ 
       v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2 % VEC] = __uint_as_float(r.z); v[3 % VEC] = __uint_as_float(r.w);
     }
   };
-  if (direct) {
+  if (ONE) {      // each lane's entries go straight to its registers
     auto row = [&](const int k) { return k < g.K ? *reinterpret_cast<const uint4*>(Ap + k) : make_uint4(0u, 0u, 0u, 0u); };
     uint4 a[U];
 #pragma unroll
@@ -766,6 +770,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ 
     }
   }
   if (TAIL) {
+    if (!ONE) apart();
     float v = 0.f;
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -2104,7 +2109,7 @@ __global__ void __launch_bounds__(128) fq3s_cache_attn_merge_kernel(const fq3c_o
 // the caches; the CTA whose eight keys the new one is among reads it from its own shared memory.
 // Rotation and attention of one row of 16 heads over 4 behind 220 positions: 15.5 us in three launches, 6.2; 8 rows 25.8 and 11.1; one row of 32-bit caches behind 2000 21.8 and 14.5.
 // ---------------------------------------------------------------------------------------------------------------------------
-constexpr int AF_RANKS = 8, AF_WARPS = 8;
+constexpr int AF_RANKS = 8, AF_WARPS = 8, AF_ROWS = 8;
 template <int BYTES> struct AfVec;
 template <> struct AfVec<4> { typedef uint32_t T; };
 template <> struct AfVec<8> { typedef uint2 T; };
@@ -2119,7 +2124,7 @@ __device__ __forceinline__ void af_store(float* local, const int rank, const flo
 template <typename TC, int D, int HG, bool ROT>
 __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <= 4 ? 2 : 1) fq3s_attn_few_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op r) {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (the other CTAs have begun when this completes)
-  if (threadIdx.x < 32) {
+  if (threadIdx.x < 32 && o.M <= DEP_ROWS) {
     args_ahead(o);
     if (ROT) args_ahead(r);
   }
