@@ -1740,10 +1740,10 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     else launch_after(fq3s_ggemv_kernel<bf16, bf16>, grid, 256, smem, s, after, 1, g);
     return 0;
   }
-  // Experts on tcgen05: whole 16-byte pieces, each expert's weights behind the last one's.  A tile's 128 rows and 128 columns pay from some two hundred chosen rows on; below, the 64-column
-  // tiles of the other kernel have more CTAs in flight (layers without a shared expert: 33 rows x 2 of 16 experts 50.8 and 54.4 us, 17 x 4 of 8 50.6 and 55.6, 200 x 1 of 16 54.7 and 45.9,
-  // 64 x 4 of 32 104 and 80, 701 x 2 of 16 81 and 51, 2048 x 4 of 32, 2048 wide, 527 and 245).
-  if (g.seg && zcount == 1 && !a_f32 && !b_f32 && g.M >= 192 && g.K >= TK && g.K % 8 == 0 && g.lda % 8 == 0 && g.ldb == g.K && g.b_estride == (long long)g.N * g.K && (long long)g.E * g.N < (1LL << 31) &&
+  // Experts on tcgen05: whole 16-byte pieces, each expert's weights behind the last one's, a k-block or more; at every number of rows that comes here faster than the mma.sync kernel
+  // behind it, which keeps shorter sums (layers without a shared expert: 9 rows x 2 of 16 experts 48.5 and 41.3 us, 17 x 4 of 8 52.5 and 48.6, 100 x 1 of 16 54.6 and 46.4, 701 x 2 of 16
+  // 81 and 51, 2048 x 4 of 32, 2048 wide, 527 and 245).
+  if (g.seg && zcount == 1 && !a_f32 && !b_f32 && g.K >= TK && g.K % 8 == 0 && g.lda % 8 == 0 && g.ldb == g.K && g.b_estride == (long long)g.N * g.K && (long long)g.E * g.N < (1LL << 31) &&
       !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) && device_attrs_ready()) {
     CUtensorMap tmB;
     if (make_map(&tmB, g.B, (uint64_t)g.K, (uint64_t)g.E * g.N, (uint64_t)g.K, GT_BN)) {

@@ -351,11 +351,9 @@ __global__ void __launch_bounds__(128) fq3s_gemm_mma_kernel(const SeqGemm g) {
   sg_quad_epilogue<GLU>(g, acc, row0 + wm, row_end, col0 + wn, z * g.c_zstride, lane);
 }
 
-// Rows of whole 16-byte pieces, bf16 on both sides (the grouped products of the experts): 128 x 64 tiles, eight warps, each a 32 x 32 quadrant (a quadrant
-// behind the expert's last row does nothing), three stages of 64 k by cp.async, 16-byte pieces exclusive-ored with the row against bank conflicts.  The sums run
-// over k in the other kernels' order.  Bound by the L2 latency of the stages in flight (three blocks per SM, 48 KB each).  A whole layer of 16 experts, two a row (1024 x 768 gated,
-// shared expert and router beside them), against the 64 x 64 and 128 x 128 tiles staged through registers: 33 rows 101 -> 70 us, 701 171 -> 115, 1500 250 -> 165,
-// 3000 360 -> 235, 6000 562 -> 397: at every size, so there is no line between the two.
+// Rows of whole 16-byte pieces, bf16 on both sides, where the tcgen05 kernel of the experts' products does not take them (sums of less than 64): 128 x 64 tiles, eight warps, each a
+// 32 x 32 quadrant (a quadrant behind the expert's last row does nothing), three stages of 64 k by cp.async, 16-byte pieces exclusive-ored with the row against bank conflicts.  The
+// sums run over k in the other kernels' order.  Bound by the L2 latency of the stages in flight (three blocks per SM, 48 KB each).
 constexpr int GQ_BM = 128, GQ_BN = 64, GQ_BK = 64, GQ_ST = 3, GQ_STAGE = (GQ_BM + GQ_BN) * GQ_BK * 2, GQ_SMEM = GQ_ST * GQ_STAGE;
 template <bool GLU>
 __global__ void __launch_bounds__(256, 3) fq3s_gemm_pipe_kernel(const SeqGemm g) {
