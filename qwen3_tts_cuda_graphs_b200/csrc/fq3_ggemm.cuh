@@ -7,8 +7,8 @@
 // Warps 0-7 gather the rows by 16-byte copies into the swizzled stages (a row list for the first product, the rows themselves for the second), the last warp asks for the weights by TMA,
 // one box a stage, the one before it issues the MMAs; warps 0-7 then take the accumulator through the epilogue, a row per lane, 16 columns at a time.  Two CTAs share an SM, so that one's
 // epilogue runs beside the other's products; 96 KB of stages each.
-// What bounds it: the operand bytes of L2 and the chain of a tile's 12 - 32 k-blocks; rows behind an expert's last one are zeros.  1402 rows of 16 experts: 1536 x 1024 with gated units
-// 34.8 us on mma.sync, 17.7 here; 1024 x 768 24.5 and 9.9.  (Activations by a flag per tile: with one per entry the second product fetched their code sixteen times over, 17.6 us.)
+// What bounds it: the latency of the three stages along a tile's 12 - 32 k-blocks (four stages of 64 columns: 21.0 and 12.2 us); rows behind an expert's last one are zeros.  1402 rows of 16 experts: 1536 x 1024 with gated units
+// 34.8 us on mma.sync, 16.9 here; 1024 x 768 24.5 and 9.2.  (Activations by a flag per tile: with one per entry the second product fetched their code sixteen times over, 17.6 us.)
 constexpr int GT_BN = 128, GT_ST = 3, GT_LOADERS = 256, GT_THREADS = GT_LOADERS + 64;
 constexpr int GT_A_BYTES = TM * TK * 2, GT_STAGE_BYTES = GT_A_BYTES + GT_BN * TK * 2, GT_SMEM = GT_ST * GT_STAGE_BYTES + 1024 + 128;
 
@@ -155,9 +155,8 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
     }
     unsigned char* dst = gbase + lr * 128 + ((piece ^ (lr & 7)) << 4);      // (rows 32 apart share the swizzle)
     for (int kt = 0, st = 0; kt < KT; ++kt) {
-      if (kt >= GT_ST) {      // one lane a warp polls
-        if (lane == 0) there = gp_wait(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, GP_TRIES);
-        there = __shfl_sync(0xffffffffu, there, 0);
+      if (kt >= GT_ST) {      // (all lanes: with one that polls for the others 17.8 and 9.8 us)
+        there = gp_wait_all(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, GP_TRIES);
         if (!there) break;
       }
       const bool in = kt * TK + piece * 8 < g.K;
