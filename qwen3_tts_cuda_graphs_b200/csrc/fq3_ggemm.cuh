@@ -82,7 +82,7 @@ __device__ __forceinline__ void gt_epilogue(const SeqGemm& g, const int r, const
 template <bool GLU>
 __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __grid_constant__ SeqGemm g, const __grid_constant__ CUtensorMap tmB, const int whole) {
   constexpr int MMA_WARP = GT_LOADERS / 32, TMA_WARP = MMA_WARP + 1;
-  grid_dep_wait();
+  seq_dep_begin(g.M);
   int row0 = -1, row_end = 0, e = 0;
   for (int t = blockIdx.y; e < g.E; ++e) {
     const int s0 = g.seg[e], s1 = g.seg[e + 1], nt = (s1 - s0 + TM - 1) / TM;

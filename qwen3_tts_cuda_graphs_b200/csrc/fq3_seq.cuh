@@ -15,9 +15,11 @@ __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn
 // rows blocks that come up early come up several on one SM, beside others that stay empty, which a launch that has work for all of them pays for (an attention layer of 4 rows
 // behind 300 positions 39 us without, 59 with; of 384 rows in 32 bits 143 and 159).
 constexpr int DEP_ROWS = 2;
+// (run_ops launches them early under the same condition; the wait itself costs a launch that is not early some 0.15 us.)
 __device__ __forceinline__ void seq_dep_begin(const int rows) {
+  if (rows > DEP_ROWS) return;
   grid_dep_wait();
-  if (rows <= DEP_ROWS) grid_dep_launch();
+  grid_dep_launch();
 }
 
 // The arguments of a launch come through a cache that does not have them yet.  A launch that is up early fetches them while it waits; one warp calls it.  (With that, and with all of
