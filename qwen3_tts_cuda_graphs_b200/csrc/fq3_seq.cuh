@@ -3688,9 +3688,10 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
     const float* p = part + t * PP + j;
     return (p[0] + p[CD_C * PP]) + (p[2 * CD_C * PP] + p[3 * CD_C * PP]);
   };
+  auto there = [&](const int at, const uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[at]), parity)); };      // (one answer for a warp: it meets behind it)
   if (role == 1) {
     load_v(0);
-    if (mbar_wait_bounded(smem_u32(&full[0]), 0u)) next_tv(0, cw);
+    if (there(0, 0u)) next_tv(0, cw);
     else gone = 1;
   }
   // slots of records n - 1, n and n + 1 (no division in the chain: the one thread that asked for the next record held it up by 500 cycles when it was one of these)
@@ -3770,7 +3771,7 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
       }
       if (n == nblk) break;
       if (n + 1 < nblk) {
-        if (mbar_wait_bounded(smem_u32(&full[sx]), px)) next_tv(n + 1, cw + sx * REC);
+        if (there(sx, px)) next_tv(n + 1, cw + sx * REC);
         else gone = 1;
       }
       bar_sync<3, 256>();      // the other product has ended, and everyone here has read Pq
