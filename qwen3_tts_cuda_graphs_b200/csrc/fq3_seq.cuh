@@ -2281,7 +2281,8 @@ __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <
         tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 8));
         tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 16));
         const float mn = fmaxf(mx[h], tm);
-        const float p = see ? expf(x - mn) : 0.f, a = mx[h] == -INFINITY ? 0.f : expf(mx[h] - mn);
+        // (also a key that the row sees may score -infinity, alone among these eight or with all of them: mn is -infinity then)
+        const float p = x == -INFINITY ? 0.f : expf(x - mn), a = mx[h] == -INFINITY ? 0.f : expf(mx[h] - mn);
         mx[h] = mn;
         ls[h] = ls[h] * a + p;
         sc[h] = p;

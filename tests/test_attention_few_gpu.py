@@ -126,3 +126,36 @@ def test_against_float64(D, f32, H, G, option):
             assert (out.double() - want[0]).abs().max() <= (5e-5 if f32 else 2e-2) * max(1.0, float(want[0].abs().max()))
             assert (out.double() - want[0]).norm() <= (1e-5 if f32 else 4e-3) * want[0].norm()
         assert all(torch.allclose(a, b, rtol=1e-4, atol=1e-5, equal_nan=True) for a, b in zip(results[0][:2], results[1][:2])) and torch.equal(results[0][2].float().nan_to_num(7.0), results[1][2].float().nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("H,G", [(2, 2), (4, 2), (6, 2), (8, 2), (8, 1)])
+@pytest.mark.parametrize("pos,low", [(64, [64]), (8, [8]), (200, list(range(96, 104))), (70, list(range(64, 71))), (15, list(range(8, 15))), (9, list(range(9)))])
+@pytest.mark.parametrize("turned", [True, False])      # with the rotation in front in the same launch, and the attention by itself
+def test_visible_keys_that_score_minus_infinity(f32, H, G, pos, low, turned):
+    """Keys of weight zero: alone among the eight of their warp (the newest one too), all of the eight, all but the newest key."""
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    lib, D, dt = K.load_lib(), 128, torch.float32 if f32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(pos + H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    o = dict(rot=32, dt=dt, freq=10000.0 ** (-torch.arange(16, device="cuda", dtype=torch.float32) / 16), borrowed=not turned)
+    cols = (H + 2 * G) * D
+    rows, kc, vc = rnd(1, cols), rnd(pos + 1, G * D).to(dt), rnd(pos + 1, G * D).to(dt)
+    rows[0, D - 1:H * D:D] = 0.5      # (an entry behind those that turn)
+    kc[low, D - 1::D] = -torch.inf
+    if pos in low:
+        rows[0, (H + 1) * D - 1:(H + G) * D:D] = -torch.inf
+    want = reference(rows.double(), kc.double(), vc.double(), pos, H, G, D, o)[0]
+    out, where = torch.zeros(1, H * D, device="cuda"), torch.tensor([pos], device="cuda", dtype=torch.int32)
+    r, a = K.Op(), K.Op()
+    r.kind, r.M, r.i0, r.i1, r.i2, r.cin, r.taps, r.K, r.a_rows, r.lda, r.flags = K.K_ROT_APPEND, 1, H, G if turned else 0, D, D, 32, H * D, (H + G) * D, cols, K.F_F32 if f32 else 0
+    r.A, r.B, r.p0 = rows.data_ptr(), o["freq"].data_ptr(), where.data_ptr()
+    if turned:
+        r.C, r.ldc, r.C2, r.ldr = kc.data_ptr(), G * D, vc.data_ptr(), G * D
+    a.kind, a.M, a.N, a.i0, a.i1, a.i2, a.cin, a.f0, a.lda, a.ldr, a.taps, a.ldc, a.flags = K.K_CACHE_ATTN, 1, H * D, H, G, D, D, D ** -0.5, cols, G * D, G * D, H * D, (K.F_F32 if f32 else 0) | K.F_OUT_F32
+    a.A, a.B, a.p1, a.p0, a.C = rows.data_ptr(), kc.data_ptr(), vc.data_ptr(), where.data_ptr(), out.data_ptr()
+    for part in ([[r, a]] if turned else [[r], [a]]):
+        assert lib.fq3c_run((K.Op * len(part))(*part), len(part), torch.cuda.current_stream().cuda_stream) == 0, lib.fq3c_last_error()
+    # as in the test above; a new key that rounds the other way moves its score by 2^-8 of a term
+    assert want.isfinite().all() and (out.double() - want).norm() <= (1e-5 if f32 else 4e-3) * want.norm()
