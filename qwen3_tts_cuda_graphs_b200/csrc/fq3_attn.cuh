@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
               float far = fabsf(s[h][0]);
 #pragma unroll
               for (int i = 1; i < 32; ++i) far = fmaxf(far, fabsf(s[h][i]));
-              near = __all_sync(0xffffffffu, far * a.scale * icap <= AT_NEAR);
+              near = __all_sync(0xffffffffu, far * fabsf(a.scale) * icap <= AT_NEAR);
             }
             if (near) {
 #pragma unroll

@@ -31,3 +31,25 @@ def test_against_float64(M, pos, H, G, cap, spread):
         # weights of 16 bits (2^-17 of each) and scores off by some 1e-6 of the cap or of their sum of 128 products
         bound = (2.0 ** -16 + 4e-6 * max(cap, 8.0 * spread)) * (w @ vv.abs()) + 1e-6
         assert ((out[:, h * D:(h + 1) * D].double() - w @ vv).abs() <= bound).all()
+
+
+def capped(q, k, v, H, G, cap, scale, pos=0):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    lib, M, D = K.load_lib(), q.shape[0], 128
+    out, where = torch.zeros(M, H * D, device="cuda"), torch.tensor([pos], device="cuda", dtype=torch.int32)
+    a = K.Op()
+    a.kind, a.M, a.N, a.i0, a.i1, a.i2, a.cin, a.f0, a.f1, a.lda, a.ldr, a.taps, a.ldc, a.flags = K.K_CACHE_ATTN, M, H * D, H, G, D, D, scale, cap, H * D, G * D, G * D, H * D, K.F_OUT_F32
+    a.A, a.B, a.p1, a.p0, a.C = q.data_ptr(), k.data_ptr(), v.data_ptr(), where.data_ptr(), out.data_ptr()
+    assert lib.fq3c_run((K.Op * 1)(a), 1, torch.cuda.current_stream().cuda_stream) == 0, lib.fq3c_last_error()
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("M,H,G", [(9, 4, 2), (200, 16, 4), (1500, 4, 4)])
+def test_a_cap_under_a_negative_scale(M, H, G):
+    """The products of q and k under -s are those of -q and k under s: same bits, wherever the scores lie under the cap."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    q, k, v = torch.randn(M, H * 128, device="cuda", generator=g) * 4, *(torch.randn(M, G * 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    for cap in (4.0, 200.0):
+        assert torch.equal(capped(q, k, v, H, G, cap, -(128 ** -0.5)), capped(-q, k, v, H, G, cap, 128 ** -0.5))
