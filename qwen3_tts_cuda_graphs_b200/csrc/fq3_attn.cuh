@@ -73,6 +73,11 @@ __device__ __forceinline__ float ex2f(const float x) {
 // cap * tanh(x), cap * tanh(y) for |x|, |y| up to AT_NEAR: x (1 - t/3 + 2 t^2/15 - 17 t^3/315 + 62 t^4/2835), t = x^2, the first terms of the series, which leave 2.4e-7 of the result.  Seven
 // packed multiply-adds for two scores, where the exponential and the reciprocal of fast_tanh (1e-6) are two more turns each on the special-function unit beside the weight's own.
 constexpr float AT_NEAR = 0.35f;
+__device__ __forceinline__ float max_nan(const float x, const float y) {      // a NaN stays one
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(x), "f"(y));
+  return m;
+}
 __device__ __forceinline__ void cap_near(float& x, float& y, const float cap) {
   const f32x2 v = pack2(x, y), t = mul2<true>(v, v);
   f32x2 p = fma2<true>(t, pack2(62.f / 2835.f, 62.f / 2835.f), pack2(-17.f / 315.f, -17.f / 315.f));
@@ -82,7 +87,6 @@ __device__ __forceinline__ void cap_near(float& x, float& y, const float cap) {
   p = fma2<true>(mul2<true>(t, p), c, c);
   x = lo2(p); y = hi2(p);
 }
-
 // 16 finished entries of an output row, f32 or rounded
 __device__ __forceinline__ void at_store(const AttnArgs& a, const size_t at, const float (&v)[16]) {
   if (a.out_f32) {
@@ -444,10 +448,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           if (h == 0) tmem_ld32(s_t + 32, s[1]);      // on its way while the first half is worked on
           if (k0 + h * 32 <= wlast) {      // (keys behind every row of the warp: masked below, whatever they are)
             bool near = false;
-            if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) {      // of a whole warp: no score of its rows is far up the cap (a NaN is)
+            if (MODE == AT_CAP || (MODE == AT_DIST && a.cap > 0.f)) {      // of a whole warp: no score of its rows is far up the cap.  A NaN counts as far, where it becomes -cap, whatever the others are
               float far = fabsf(s[h][0]);
 #pragma unroll
-              for (int i = 1; i < 32; ++i) far = fmaxf(far, fabsf(s[h][i]));
+              for (int i = 1; i < 32; ++i) far = max_nan(far, fabsf(s[h][i]));
               near = __all_sync(0xffffffffu, far * fabsf(a.scale) * icap <= AT_NEAR);
             }
             if (near) {

@@ -53,3 +53,24 @@ def test_a_cap_under_a_negative_scale(M, H, G):
     q, k, v = torch.randn(M, H * 128, device="cuda", generator=g) * 4, *(torch.randn(M, G * 128, device="cuda", generator=g).bfloat16() for _ in range(2))
     for cap in (4.0, 200.0):
         assert torch.equal(capped(q, k, v, H, G, cap, -(128 ** -0.5)), capped(-q, k, v, H, G, cap, 128 ** -0.5))
+
+
+@pytest.mark.parametrize("pos", [0, 70])
+@pytest.mark.parametrize("spread", [1.0, 8.0])      # all scores near, some of most warps far up the cap
+def test_a_capped_score_that_is_nan(pos, spread):
+    """It counts as -cap, whatever the scores beside it are."""
+    M, H, G, cap = 300, 8, 2, 20.0
+    g = torch.Generator(device="cuda").manual_seed(pos)
+    q, k, v = (torch.randn(M, H * 128, device="cuda", generator=g) * spread).bfloat16().float(), *(torch.randn(pos + M, G * 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    hide = torch.arange(pos + M, device="cuda")[None] > torch.arange(pos, pos + M, device="cuda")[:, None]
+    for at in (pos + 1, pos + 40, pos + 201, pos + M - 1):
+        bad = k.clone()
+        bad[at, 5] = torch.nan
+        out = capped(q, bad, v, H, G, cap, 128 ** -0.5, pos)
+        for h in range(H):
+            n = h // (H // G)
+            s = cap * torch.tanh((q[:, h * 128:(h + 1) * 128].double() @ bad[:, n * 128:(n + 1) * 128].double().T * 128 ** -0.5) / cap)
+            w = s.nan_to_num(-cap).masked_fill(hide, -torch.inf).softmax(-1)
+            vv = v[:, n * 128:(n + 1) * 128].double()
+            bound = (2.0 ** -16 + 4e-6 * cap) * (w @ vv.abs()) + 1e-6      # as above
+            assert ((out[:, h * 128:(h + 1) * 128].double() - w @ vv).abs() <= bound).all()
