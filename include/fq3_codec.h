@@ -273,7 +273,7 @@ typedef struct fq3c_op {
   int32_t reserved;      /* GEMM, bit 0: no op of the list writes B, so a launch may read it before the launches in front of it have ended; bit 2: see ws;
                             bit 3: the columns of C's rows from N up to the next multiple of 16 (ldc has to hold them) are scratch.
                             QKNORM_ROPE_KV, bit 0: A's rows are scratch that the ATTN behind it alone reads (one launch may do both, and the
-                            rows then stay as they are).  GEMM,
+                            rows then stay as they are).  GEMM, GGEMM,
                             ATTN and CACHE_ATTN on tcgen05, bit 1: the first operand tile is never asked for and the waits are short, so
                             that one runs out (tests of the error path: NaN outputs, fq3c_wait_errors) */
   /* GEMM, optional (ABI 5): the RMSNorm that reads the finished output rows, fused behind the epilogue — a decoder layer's norm

@@ -2045,7 +2045,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       g.A = o.A; g.B = o.B; g.bias = nullptr; g.C = o.C;
       g.M = o.M; g.N = o.N; g.K = o.K; g.lda = o.lda; g.ldb = o.K; g.ldc = o.ldc; g.flags = o.flags & ~FQ3C_BIAS;
       g.a_mod = 1; g.seg = reinterpret_cast<const int*>(o.p0); g.rows = reinterpret_cast<const int*>(o.p1); g.E = o.i0;
-      g.b_estride = (long long)o.N * o.K;
+      g.b_estride = (long long)o.N * o.K; g.lost = (o.reserved >> 1) & 1;
       if (o.flags & FQ3C_SWIGLU) { g.rs_w = reinterpret_cast<const float*>(o.scale); g.rs_pos = reinterpret_cast<const int*>(o.ws); g.rs_top = o.i1; }
       if (g.rs_pos && (!g.rs_w || !g.rows || g.rs_top < 1)) return fail("ggemm: a router's weights need the choices' places, the row list and the choice count");
       const bool f32 = (o.flags & FQ3C_F32) != 0;

@@ -93,12 +93,13 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
   extern __shared__ unsigned char gt_raw[];
   const uint32_t raw = smem_u32(gt_raw), base = (raw + 1023u) & ~1023u;
   unsigned char* gbase = gt_raw + (base - raw);
-  const uint32_t full = base + GT_ST * GT_STAGE_BYTES, empty = full + 8u * GT_ST, done = empty + 8u * GT_ST;
-  uint32_t* words = reinterpret_cast<uint32_t*>(gbase + GT_ST * GT_STAGE_BYTES + 16 * GT_ST + 16);      // tensor-memory address | a wait ran out | weight boxes asked for
+  // rows of a stage are there, its weights are there (a barrier of their own: the copy engine alone completes it, also when the loaders gave up; the second wait a k-block costs up to 1 %), the stage is free, all products are done
+  const uint32_t full = base + GT_ST * GT_STAGE_BYTES, boxes = full + 8u * GT_ST, empty = boxes + 8u * GT_ST, done = empty + 8u * GT_ST;
+  uint32_t* words = reinterpret_cast<uint32_t*>(gbase + GT_ST * GT_STAGE_BYTES + 24 * GT_ST + 8);      // tensor-memory address | a wait ran out | weight boxes asked for
   volatile int* dead = reinterpret_cast<volatile int*>(words + 1);
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, n0 = blockIdx.x * GT_BN, KT = (g.K + TK - 1) / TK;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, n0 = blockIdx.x * GT_BN, KT = (g.K + TK - 1) / TK, tries = g.lost ? GP_TRIES_TEST : GP_TRIES;
   if (tid == 0) {
-    for (int s = 0; s < GT_ST; ++s) { mbar_init(full + 8u * s, GT_LOADERS + 1); mbar_init(empty + 8u * s, 1); }
+    for (int s = 0; s < GT_ST; ++s) { mbar_init(full + 8u * s, GT_LOADERS); mbar_init(boxes + 8u * s, 1); mbar_init(empty + 8u * s, 1); }
     mbar_init(done, 1);
     words[1] = 0;
     words[2] = 0;
@@ -117,10 +118,10 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
   if (warp == TMA_WARP) {
     int n = 0;
     for (int kt = 0, st = 0; kt < KT && there; ++kt) {
-      if (kt >= GT_ST && !gp_wait_all(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, GP_TRIES)) { there = false; break; }
+      if (kt >= GT_ST && !gp_wait_all(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, tries)) { there = false; break; }
       if (leader) {
-        mbar_expect(full + 8u * st, GT_BN * TK * 2);
-        tma_2d(base + st * GT_STAGE_BYTES + GT_A_BYTES, &tmB, kt * TK, e * g.N + n0, full + 8u * st);
+        mbar_expect(boxes + 8u * st, GT_BN * TK * 2);
+        if (kt > 0 || !g.lost) tma_2d(base + st * GT_STAGE_BYTES + GT_A_BYTES, &tmB, kt * TK, e * g.N + n0, boxes + 8u * st);
       }
       ++n;
       if (++st == GT_ST) st = 0;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GT_BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
     const uint64_t d0 = umma_desc_sw128(base);
     for (int kt = 0, st = 0; kt < KT; ++kt) {
-      if (!gp_wait_all(full + 8u * st, (uint32_t)((kt / GT_ST) & 1), dead, GP_TRIES)) { there = false; break; }
+      if (!gp_wait_all(boxes + 8u * st, (uint32_t)((kt / GT_ST) & 1), dead, tries) || !gp_wait_all(full + 8u * st, (uint32_t)((kt / GT_ST) & 1), dead, tries)) { there = false; break; }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the rows came through the generic proxy
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t da = d0 + st * (GT_STAGE_BYTES >> 4), db = da + (GT_A_BYTES >> 4);
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
     unsigned char* dst = gbase + lr * 128 + ((piece ^ (lr & 7)) << 4);      // (rows 32 apart share the swizzle)
     for (int kt = 0, st = 0; kt < KT; ++kt) {
       if (kt >= GT_ST) {      // (all lanes: with one that polls for the others 17.8 and 9.8 us)
-        there = gp_wait_all(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, GP_TRIES);
+        there = gp_wait_all(empty + 8u * st, (uint32_t)((kt / GT_ST - 1) & 1), dead, tries);
         if (!there) break;
       }
       const bool in = kt * TK + piece * 8 < g.K;
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
       if (++st == GT_ST) st = 0;
     }
     // warp w reads tensor-memory lanes 32 (w & 3) .. +31; the first four warps take the lower columns
-    if (there) there = gp_wait_warp(done, 0u, dead, GP_TRIES);
+    if (there) there = gp_wait_warp(done, 0u, dead, tries);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int r = row0 + (warp & 3) * 32 + lane, c0 = (warp >> 2) * (GT_BN / 2);
     const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(GT_THREADS, 2) fq3s_ggemm_tc_kernel(const __gr
     }
     if (tid < GT_ST && tid < (int)words[2]) {
       const int i = (int)words[2] - 1 - tid;
-      mbar_wait_bounded(full + 8u * (i % GT_ST), (uint32_t)((i / GT_ST) & 1), 1 << 14);
+      mbar_wait_bounded(boxes + 8u * (i % GT_ST), (uint32_t)((i / GT_ST) & 1), 1 << 14);
     }
     const int cols = GLU ? GT_BN / 2 : GT_BN, width = GLU ? g.N / 2 : g.N, c0 = GLU ? n0 / 2 : n0;
     for (int i = tid; i < (row_end - row0) * cols; i += GT_THREADS) {

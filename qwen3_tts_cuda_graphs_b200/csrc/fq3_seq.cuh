@@ -70,6 +70,7 @@ struct SeqGemm {
   // rs_w[m, j] of the choice j of token m = rows[r] whose sorted position rs_pos[m, j] is r.
   const float* rs_w; const int* rs_pos; int rs_top;
   int early;   // few rows: no op of the list writes B, so its first entries are asked for before the launches in front have ended
+  int lost;    // tests, grouped products on tcgen05: 1 = the first weight box is never asked for and the waits are short, so that one runs out
 };
 __device__ __forceinline__ float sg_row_scale(const SeqGemm& g, const int r) {
   if (!g.rs_w) return 1.f;

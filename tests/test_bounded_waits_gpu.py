@@ -33,6 +33,15 @@ elif what == "prompt attention":
     o.kind, o.flags, o.M, o.N, o.A, o.lda, o.a_rows = K.K_ATTN, 1, M, H * 128, a.data_ptr(), a.shape[1], M
     o.C, o.ldc, o.col_mod, o.i0, o.i1, o.i2, o.K, o.reserved = out.data_ptr(), H * 128, H * 128, H, G, 128, 2048, 2
     outs = [out]
+elif what.startswith("experts"):
+    E, rows, N, kk = 3, 300, 272, {"experts": 512, "experts, one k-block": 64, "experts, units": 512}[what]
+    glu = what == "experts, units"
+    a, w, seg = torch.randn(rows, kk, device=dev).bfloat16(), torch.randn(E, N, kk, device=dev).bfloat16(), torch.tensor([0, 130, 130, rows], device=dev, dtype=torch.int32)
+    out = torch.zeros(rows, N // 2 if glu else N, device=dev, dtype=torch.bfloat16 if glu else torch.float32)
+    o = K.Op()
+    o.kind, o.M, o.N, o.K, o.i0, o.lda, o.ldc, o.flags, o.reserved = K.K_GGEMM, rows, N, kk, E, kk, out.shape[1], K.F_SWIGLU if glu else K.F_OUT_F32, 2
+    o.A, o.B, o.p0, o.C = a.data_ptr(), w.data_ptr(), seg.data_ptr(), out.data_ptr()
+    outs = [out]
 else:
     M, H, G = 200, 6, 2
     q, kv, pos = torch.randn(M, H * 128, device=dev), torch.randn(M, G * 128, device=dev).bfloat16(), torch.zeros(1, dtype=torch.int32, device=dev)
@@ -55,7 +64,7 @@ assert torch.allclose((x @ x).double(), x.double() @ x.double(), atol=1e-1)
 """
 
 
-@pytest.mark.parametrize("what", ["gemm", "gemm split", "gemm gated", "gemm snake", "prompt attention", "cache attention"])
+@pytest.mark.parametrize("what", ["gemm", "gemm split", "gemm gated", "gemm snake", "prompt attention", "cache attention", "experts", "experts, one k-block", "experts, units"])
 def test_a_wait_that_runs_out(what):
     here = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", PROGRAM, what, here], cwd=os.path.dirname(here), capture_output=True, text=True, timeout=300)
