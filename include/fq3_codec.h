@@ -274,8 +274,8 @@ typedef struct fq3c_op {
                             bit 3: the columns of C's rows from N up to the next multiple of 16 (ldc has to hold them) are scratch.
                             QKNORM_ROPE_KV, bit 0: A's rows are scratch that the ATTN behind it alone reads (one launch may do both, and the
                             rows then stay as they are).  GEMM, GGEMM,
-                            ATTN and CACHE_ATTN on tcgen05, bit 1: the first operand tile is never asked for and the waits are short, so
-                            that one runs out (tests of the error path: NaN outputs, fq3c_wait_errors) */
+                            ATTN and CACHE_ATTN on tcgen05, bit 1: the first operand tile (MSTATE_SCAN in blocks of tokens: the
+                            last block's record) is never asked for and the waits are short, so that one runs out (tests of the error path: NaN outputs, fq3c_wait_errors) */
   /* GEMM, optional (ABI 5): the RMSNorm that reads the finished output rows, fused behind the epilogue — a decoder layer's norm
    * reads exactly the residual stream its o / down projection just wrote.  norm_out bf16 [M, norm_ld] = FQ3C_RMSNORM(C rows)
    * with weights norm_w (f32 [N]) and eps norm_eps, same arithmetic and summation order as the stand-alone op.  It is one

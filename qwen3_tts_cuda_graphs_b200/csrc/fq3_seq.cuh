@@ -3574,12 +3574,13 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
   seq_dep_begin(o.M);
   extern __shared__ __align__(128) float cw[];
   __shared__ __align__(8) unsigned long long full[4];
-  __shared__ int gone;                               // a wait ran out
+  __shared__ int gone[2];                            // a wait ran out, told in round n through word n & 1 (what is written meanwhile is for the next round, and the other word)
   constexpr int NCP = DVT / 2, QS = 128 / NCP, CG = DVT / 4, KH = 4 / CG, PP = DVT + 1, JW = DVT / 4, NJ = JW / 2;
   const int H = o.i0, dk = o.i2, dv = o.cin, h = blockIdx.y, j0 = blockIdx.x * DVT, tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
   const int role = threadIdx.x >> 7;                 // 0: the warps that carry the state, 1: the others, 2: the one that asks for the records
   const bool chain = role == 0;
   const int D = cd_rows(dk), P = cd_pitch(dk), REC = cd_record(dk), nblk = (o.M + CD_C - 1) / CD_C;
+  const int lost = o.reserved & 2 ? nblk - 1 : -1, tries = o.reserved & 2 ? 4096 : 1 << 20;      // (tests: the last record is never asked for)
   float* St = cw + ring * REC;                       // [2][DVT][P]
   float* Pp = St + 2 * DVT * P;                      // [4][CD_C][PP] of W S0, then of Qt S0
   float* Pq = Pp + 4 * CD_C * PP;
@@ -3590,12 +3591,13 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
   auto fetch = [&](const int n, const int at) {       // one thread; record n into slot n % ring
     const uint32_t bar = smem_u32(&full[at]);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)REC * 4u) : "memory");
+    if (n == lost) return;
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(cw + at * REC)),
                  "l"(recs + (size_t)n * H * REC), "r"((uint32_t)REC * 4u), "r"(bar)
                  : "memory");
   };
   if (threadIdx.x == 256) {
-    gone = 0;
+    gone[0] = gone[1] = 0;
     for (int i = 0; i < ring; ++i) mbar_init(smem_u32(&full[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int n = 0; n < min(ring, nblk); ++n) fetch(n, n);
@@ -3690,11 +3692,11 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
     const float* p = part + t * PP + j;
     return (p[0] + p[CD_C * PP]) + (p[2 * CD_C * PP] + p[3 * CD_C * PP]);
   };
-  auto there = [&](const int at, const uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[at]), parity)); };      // (one answer for a warp: it meets behind it)
+  auto there = [&](const int at, const uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[at]), parity, tries)); };      // (one answer for a warp: it meets behind it)
   if (role == 1) {
     load_v(0);
     if (there(0, 0u)) next_tv(0, cw);
-    else gone = 1;
+    else gone[0] = 1;
   }
   // slots of records n - 1, n and n + 1 (no division in the chain: the one thread that asked for the next record held it up by 500 cycles when it was one of these)
   int sp = ring - 1, sn = 0, sx = 1;
@@ -3702,7 +3704,7 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
   for (int n = 0;; ++n) {
     __syncthreads();
     // the state of block n, its T V and its record are there, U and Qt S0 of block n - 1 too; everyone is done with the rest of block n - 1
-    if (gone) {
+    if (gone[n & 1]) {
       __syncthreads();
       if (threadIdx.x == 256) {      // the copies on their way end before the memory is given back
         wait_ran_out();
@@ -3774,7 +3776,7 @@ __global__ void __launch_bounds__(CD_WALK_THREADS, 1) fq3s_cdelta_walk_kernel(co
       if (n == nblk) break;
       if (n + 1 < nblk) {
         if (there(sx, px)) next_tv(n + 1, cw + sx * REC);
-        else gone = 1;
+        else gone[(n + 1) & 1] = 1;
       }
       bar_sync<3, 256>();      // the other product has ended, and everyone here has read Pq
       product(rec + CD_C * P, S0, Pq);

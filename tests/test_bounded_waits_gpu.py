@@ -33,6 +33,16 @@ elif what == "prompt attention":
     o.kind, o.flags, o.M, o.N, o.A, o.lda, o.a_rows = K.K_ATTN, 1, M, H * 128, a.data_ptr(), a.shape[1], M
     o.C, o.ldc, o.col_mod, o.i0, o.i1, o.i2, o.K, o.reserved = out.data_ptr(), H * 128, H * 128, H, G, 128, 2048, 2
     outs = [out]
+elif what.startswith("delta rule"):
+    M, H, G, dk, dv = {"delta rule, two blocks": (32, 2, 1, 64, 40), "delta rule": (333, 8, 4, 128, 128)}[what]
+    nc = 2 * G * dk + H * dv
+    rows, raw, one, st = torch.randn(M, nc, device=dev), torch.randn(M, 2 * H, device=dev), torch.zeros(H, device=dev), torch.randn(H * dk, dv, device=dev)
+    out, ws = torch.zeros(M, H * dv, device=dev), torch.zeros(-(-M // 16) * H * (48 * (dk + 4) + dk + 640), device=dev)
+    o = K.Op()
+    o.kind, o.M, o.N, o.i0, o.i1, o.i2, o.cin, o.K, o.a_rows, o.A, o.lda = K.K_MSTATE_SCAN, M, H * dv, H, G, dk, dv, G * dk, 2 * G * dk, rows.data_ptr(), nc
+    o.res, o.ldr, o.col_mod, o.m_begin, o.scale, o.flags, o.reserved = raw.data_ptr(), 2 * H, 0, H, one.data_ptr(), K.F_OUT_F32, 2
+    o.p0, o.C2, o.C, o.ldc, o.ws, o.ws_bytes = st.data_ptr(), st.data_ptr(), out.data_ptr(), H * dv, ws.data_ptr(), ws.numel() * 4
+    outs = [out]
 elif what.startswith("experts"):
     E, rows, N, kk = 3, 300, 272, {"experts": 512, "experts, one k-block": 64, "experts, units": 512}[what]
     glu = what == "experts, units"
@@ -64,7 +74,7 @@ assert torch.allclose((x @ x).double(), x.double() @ x.double(), atol=1e-1)
 """
 
 
-@pytest.mark.parametrize("what", ["gemm", "gemm split", "gemm gated", "gemm snake", "prompt attention", "cache attention", "experts", "experts, one k-block", "experts, units"])
+@pytest.mark.parametrize("what", ["gemm", "gemm split", "gemm gated", "gemm snake", "prompt attention", "cache attention", "experts", "experts, one k-block", "experts, units", "delta rule", "delta rule, two blocks"])
 def test_a_wait_that_runs_out(what):
     here = os.path.dirname(os.path.abspath(__file__))
     r = subprocess.run([sys.executable, "-c", PROGRAM, what, here], cwd=os.path.dirname(here), capture_output=True, text=True, timeout=300)
