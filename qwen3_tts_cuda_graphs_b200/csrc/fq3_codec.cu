@@ -1478,6 +1478,14 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
   cfg.attrs = at; cfg.numAttrs = n;
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+// The sequence models' kernels wait (seq_dep_begin) only with few rows, so they are launched early by the same number that they test: the rows that their own arguments hold.
+template <typename... A> int dep_rows(const fq3c_op& o, const A&...) { return o.M; }
+template <typename... A> int dep_rows(const SeqGemm& g, const A&...) { return g.M; }
+inline int dep_rows(const long long*, const int*, const int by) { return by; }      // fq3s_commit_kernel
+template <typename... P, typename... A>
+void launch_seq(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool after, int cluster, const A&... args) {
+  launch_after(kernel, grid, block, smem, s, after && seq_early(dep_rows(args...)), cluster, args...);
+}
 
 // the norm of a finished product's rows
 void launch_rownorm(const fq3c_op& o, cudaStream_t s, const bool after) {
@@ -1707,20 +1715,20 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     const bool one = g.M == 1 && zcount == 1 && a_f32 == b_f32 && g.K % piece == 0 && g.ldb % piece == 0 && !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15);
     if (one) {
       const bool more = tail && tail->n > 0;
-      if (more && b_f32) launch_after(fq3s_gemv_kernel<float, float, true, true>, grid, 256, 0, s, after, 1, g, *tail);
-      else if (more) launch_after(fq3s_gemv_kernel<bf16, bf16, true, true>, grid, 256, 0, s, after, 1, g, *tail);
-      else if (b_f32) launch_after(fq3s_gemv_kernel<float, float, false, true>, grid, 256, 0, s, after, 1, g, none);
-      else launch_after(fq3s_gemv_kernel<bf16, bf16, false, true>, grid, 256, 0, s, after, 1, g, none);
+      if (more && b_f32) launch_seq(fq3s_gemv_kernel<float, float, true, true>, grid, 256, 0, s, after, 1, g, *tail);
+      else if (more) launch_seq(fq3s_gemv_kernel<bf16, bf16, true, true>, grid, 256, 0, s, after, 1, g, *tail);
+      else if (b_f32) launch_seq(fq3s_gemv_kernel<float, float, false, true>, grid, 256, 0, s, after, 1, g, none);
+      else launch_seq(fq3s_gemv_kernel<bf16, bf16, false, true>, grid, 256, 0, s, after, 1, g, none);
       return 0;
     }
     if (tail && tail->n > 0 && a_f32 == b_f32) {
-      if (b_f32) launch_after(fq3s_gemv_kernel<float, float, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
-      else launch_after(fq3s_gemv_kernel<bf16, bf16, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
+      if (b_f32) launch_seq(fq3s_gemv_kernel<float, float, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
+      else launch_seq(fq3s_gemv_kernel<bf16, bf16, true>, grid, 256, gemv_smem, s, after, 1, g, *tail);
       return 0;
     }
-    if (b_f32) launch_after(fq3s_gemv_kernel<float, float>, grid, 256, gemv_smem, s, after, 1, g, none);
-    else if (a_f32) launch_after(fq3s_gemv_kernel<float, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
-    else launch_after(fq3s_gemv_kernel<bf16, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
+    if (b_f32) launch_seq(fq3s_gemv_kernel<float, float>, grid, 256, gemv_smem, s, after, 1, g, none);
+    else if (a_f32) launch_seq(fq3s_gemv_kernel<float, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
+    else launch_seq(fq3s_gemv_kernel<bf16, bf16>, grid, 256, gemv_smem, s, after, 1, g, none);
     return 0;
   }
   if (g.seg && zcount == 1 && g.M <= 16 && (size_t)g.K * sizeof(float) <= 96 * 1024) {
@@ -1735,9 +1743,9 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     }
     dim3 grid((g.N + 7) / 8, g.M, 1);
     const size_t smem = (size_t)g.K * sizeof(float);
-    if (b_f32) launch_after(fq3s_ggemv_kernel<float, float>, grid, 256, smem, s, after, 1, g);
-    else if (a_f32) launch_after(fq3s_ggemv_kernel<float, bf16>, grid, 256, smem, s, after, 1, g);
-    else launch_after(fq3s_ggemv_kernel<bf16, bf16>, grid, 256, smem, s, after, 1, g);
+    if (b_f32) launch_seq(fq3s_ggemv_kernel<float, float>, grid, 256, smem, s, after, 1, g);
+    else if (a_f32) launch_seq(fq3s_ggemv_kernel<float, bf16>, grid, 256, smem, s, after, 1, g);
+    else launch_seq(fq3s_ggemv_kernel<bf16, bf16>, grid, 256, smem, s, after, 1, g);
     return 0;
   }
   // Experts on tcgen05: whole 16-byte pieces, each expert's weights behind the last one's, a k-block or more; at every number of rows that comes here faster than the mma.sync kernel
@@ -1750,8 +1758,8 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       const dim3 grid((g.N + GT_BN - 1) / GT_BN, (g.M + TM - 1) / TM + g.E);
       const bool glu = g.flags & FQ3C_SWIGLU;      // whole 32 bytes of a row (16 columns: of gated units 16 bytes)
       const int whole = !(reinterpret_cast<uintptr_t>(g.C) & (glu ? 15 : 31)) && g.ldc % (glu || (g.flags & FQ3C_OUT_F32) ? 8 : 16) == 0;
-      if (glu) launch_after(fq3s_ggemm_tc_kernel<true>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
-      else launch_after(fq3s_ggemm_tc_kernel<false>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
+      if (glu) launch_seq(fq3s_ggemm_tc_kernel<true>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
+      else launch_seq(fq3s_ggemm_tc_kernel<false>, grid, GT_THREADS, GT_SMEM, s, after, 1, g, tmB, whole);
       return 0;
     }
   }
@@ -1767,18 +1775,18 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       pattr[dev] = true;
     }
     const dim3 pgrid((g.N + GQ_BN - 1) / GQ_BN, (g.M + GQ_BM - 1) / GQ_BM + (g.seg ? g.E : 0), zcount);
-    if (g.flags & FQ3C_SWIGLU) launch_after(fq3s_gemm_pipe_kernel<true>, pgrid, 256, GQ_SMEM, s, after, 1, g);
-    else launch_after(fq3s_gemm_pipe_kernel<false>, pgrid, 256, GQ_SMEM, s, after, 1, g);
+    if (g.flags & FQ3C_SWIGLU) launch_seq(fq3s_gemm_pipe_kernel<true>, pgrid, 256, GQ_SMEM, s, after, 1, g);
+    else launch_seq(fq3s_gemm_pipe_kernel<false>, pgrid, 256, GQ_SMEM, s, after, 1, g);
     return 0;
   }
   // tall bf16 products (many rows per block / per expert, wide enough outputs): 128 x 128 tiles
   if (!b_f32 && !(a_f32 && exact) && g.N >= 128 && (g.seg ? g.M >= 96 * g.E : g.M >= 256)) {
     dim3 grid128((g.N + 127) / 128, (g.M + 127) / 128 + (g.seg ? g.E : 0), zcount);
     const bool glu = (g.flags & FQ3C_SWIGLU) != 0;
-    if (a_f32 && glu) launch_after(fq3s_gemm_mma128_kernel<float, true>, grid128, 256, 0, s, after, 1, g);
-    else if (a_f32) launch_after(fq3s_gemm_mma128_kernel<float>, grid128, 256, 0, s, after, 1, g);
-    else if (glu) launch_after(fq3s_gemm_mma128_kernel<bf16, true>, grid128, 256, 0, s, after, 1, g);
-    else launch_after(fq3s_gemm_mma128_kernel<bf16>, grid128, 256, 0, s, after, 1, g);
+    if (a_f32 && glu) launch_seq(fq3s_gemm_mma128_kernel<float, true>, grid128, 256, 0, s, after, 1, g);
+    else if (a_f32) launch_seq(fq3s_gemm_mma128_kernel<float>, grid128, 256, 0, s, after, 1, g);
+    else if (glu) launch_seq(fq3s_gemm_mma128_kernel<bf16, true>, grid128, 256, 0, s, after, 1, g);
+    else launch_seq(fq3s_gemm_mma128_kernel<bf16>, grid128, 256, 0, s, after, 1, g);
     return 0;
   }
   dim3 grid((g.N + 63) / 64, row_tiles, zcount);
@@ -1792,14 +1800,14 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       cudaFuncSetAttribute(fq3s_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
       attr[dev] = true;
     }
-    launch_after(fq3s_gemm_f32_kernel, grid, 256, FG_SMEM, s, after, 1, g);
+    launch_seq(fq3s_gemm_f32_kernel, grid, 256, FG_SMEM, s, after, 1, g);
   }
-  else if (b_f32) launch_after(fq3s_gemm_kernel<float, float>, grid, 256, 0, s, after, 1, g);
-  else if (a_f32 && exact) launch_after(fq3s_gemm_kernel<float, bf16>, grid, 256, 0, s, after, 1, g);
-  else if (a_f32 && (g.flags & FQ3C_SWIGLU)) launch_after(fq3s_gemm_mma_kernel<float, true>, grid, 128, 0, s, after, 1, g);
-  else if (a_f32) launch_after(fq3s_gemm_mma_kernel<float>, grid, 128, 0, s, after, 1, g);
-  else if (g.flags & FQ3C_SWIGLU) launch_after(fq3s_gemm_mma_kernel<bf16, true>, grid, 128, 0, s, after, 1, g);
-  else launch_after(fq3s_gemm_mma_kernel<bf16>, grid, 128, 0, s, after, 1, g);
+  else if (b_f32) launch_seq(fq3s_gemm_kernel<float, float>, grid, 256, 0, s, after, 1, g);
+  else if (a_f32 && exact) launch_seq(fq3s_gemm_kernel<float, bf16>, grid, 256, 0, s, after, 1, g);
+  else if (a_f32 && (g.flags & FQ3C_SWIGLU)) launch_seq(fq3s_gemm_mma_kernel<float, true>, grid, 128, 0, s, after, 1, g);
+  else if (a_f32) launch_seq(fq3s_gemm_mma_kernel<float>, grid, 128, 0, s, after, 1, g);
+  else if (g.flags & FQ3C_SWIGLU) launch_seq(fq3s_gemm_mma_kernel<bf16, true>, grid, 128, 0, s, after, 1, g);
+  else launch_seq(fq3s_gemm_mma_kernel<bf16>, grid, 128, 0, s, after, 1, g);
   return 0;
 }
 
@@ -1933,11 +1941,11 @@ void launch_attn_few(const fq3c_op& o, const fq3c_op& r, cudaStream_t s, const b
   const int HG = o.i0 / o.i1;
   const dim3 grid(AF_RANKS, (unsigned)o.i1, (unsigned)o.M);
   const size_t smem = sizeof(float) * af_floats(HG, D);
-  if (HG == 1) launch_after(fq3s_attn_few_kernel<TC, D, 1, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
-  else if (HG == 2) launch_after(fq3s_attn_few_kernel<TC, D, 2, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
-  else if (HG == 3) launch_after(fq3s_attn_few_kernel<TC, D, 3, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
-  else if (HG == 4) launch_after(fq3s_attn_few_kernel<TC, D, 4, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
-  else launch_after(fq3s_attn_few_kernel<TC, D, 8, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  if (HG == 1) launch_seq(fq3s_attn_few_kernel<TC, D, 1, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 2) launch_seq(fq3s_attn_few_kernel<TC, D, 2, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 3) launch_seq(fq3s_attn_few_kernel<TC, D, 3, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else if (HG == 4) launch_seq(fq3s_attn_few_kernel<TC, D, 4, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
+  else launch_seq(fq3s_attn_few_kernel<TC, D, 8, ROT>, grid, AF_WARPS * 32, smem, s, after, AF_RANKS, o, r);
 }
 // r: the ROT_APPEND in front that goes with it, or null
 void launch_attn_few(const fq3c_op& o, const fq3c_op* r, cudaStream_t s, const bool after) {
@@ -1986,9 +1994,9 @@ bool delta_row_takes(const fq3c_op& c, const fq3c_op& o, const fq3c_op& n) {
 }
 void launch_delta_row(const fq3c_op& c, const fq3c_op& o, const fq3c_op& n, cudaStream_t s, const bool after) {
   const dim3 grid(DS_RANKS, (unsigned)o.i0);
-  if (o.i2 == 64) launch_after(fq3s_delta_row_kernel<8>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
-  else if (o.i2 == 128) launch_after(fq3s_delta_row_kernel<16>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
-  else launch_after(fq3s_delta_row_kernel<32>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
+  if (o.i2 == 64) launch_seq(fq3s_delta_row_kernel<8>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
+  else if (o.i2 == 128) launch_seq(fq3s_delta_row_kernel<16>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
+  else launch_seq(fq3s_delta_row_kernel<32>, grid, 128, 0, s, after, DS_RANKS, c, o, n);
 }
 
 int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
@@ -1997,18 +2005,18 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       if (!o.A || !o.B || !o.C) return fail("embed: missing operand");
       if (o.i0 > 1 && o.K < o.N) return fail("embed: copies need a stride of at least N elements");
       if (o.C2 && o.ldr < o.N * std::max(o.i1, 1)) return fail("embed: the operand copies do not fit their pitch");
-      if (o.flags & FQ3C_F32) launch_after(fq3s_embed_kernel<float>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
-      else launch_after(fq3s_embed_kernel<bf16>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
+      if (o.flags & FQ3C_F32) launch_seq(fq3s_embed_kernel<float>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
+      else launch_seq(fq3s_embed_kernel<bf16>, o.M, row_threads(o.M, o.N, 128), 0, s, after, 1, o);
       return 0;
     case FQ3C_TCONV:
       if (o.taps < 1 || !o.A || !o.B || !o.C || (o.taps > 1 && (!o.p0 || !o.p1))) return fail("tconv: missing operand");
       if (tconv_vec_ok(o)) {
         const dim3 grid((o.N / 4 + 127) / 128, (o.M + o.taps - 1 + TC_ROWS - 1) / TC_ROWS);
-        if (o.taps <= 4) launch_after(fq3s_tconv_vec_kernel<4>, grid, 128, 0, s, after, 1, o);
-        else launch_after(fq3s_tconv_vec_kernel<8>, grid, 128, 0, s, after, 1, o);
+        if (o.taps <= 4) launch_seq(fq3s_tconv_vec_kernel<4>, grid, 128, 0, s, after, 1, o);
+        else launch_seq(fq3s_tconv_vec_kernel<8>, grid, 128, 0, s, after, 1, o);
         return 0;
       }
-      launch_after(fq3s_tconv_kernel, dim3((o.N + 255) / 256, o.M + o.taps - 1), 256, 0, s, after, 1, o);
+      launch_seq(fq3s_tconv_kernel, dim3((o.N + 255) / 256, o.M + o.taps - 1), 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_GNORM:
       if (o.i0 < 1 || o.N % o.i0 || ((o.flags & FQ3C_RESID) && !o.res)) return fail("gnorm: groups must divide N");
@@ -2020,16 +2028,16 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
              reinterpret_cast<uintptr_t>(o.res) | reinterpret_cast<uintptr_t>(o.scale)) & 15)) {
         const unsigned blocks = (unsigned)(((int64_t)o.M * o.i0 + 3) / 4);
         const int vecs = (o.N / o.i0 + 127) / 128;
-        if (vecs == 1) launch_after(fq3s_gnorm_warp_kernel<1>, blocks, 128, 0, s, after, 1, o);
-        else if (vecs == 2) launch_after(fq3s_gnorm_warp_kernel<2>, blocks, 128, 0, s, after, 1, o);
-        else launch_after(fq3s_gnorm_warp_kernel<GN_VECS>, blocks, 128, 0, s, after, 1, o);
+        if (vecs == 1) launch_seq(fq3s_gnorm_warp_kernel<1>, blocks, 128, 0, s, after, 1, o);
+        else if (vecs == 2) launch_seq(fq3s_gnorm_warp_kernel<2>, blocks, 128, 0, s, after, 1, o);
+        else launch_seq(fq3s_gnorm_warp_kernel<GN_VECS>, blocks, 128, 0, s, after, 1, o);
         return 0;
       }
-      launch_after(fq3s_gnorm_kernel, dim3(o.M, o.i0), row_threads(o.M, o.N / o.i0, 128), 0, s, after, 1, o);
+      launch_seq(fq3s_gnorm_kernel, dim3(o.M, o.i0), row_threads(o.M, o.N / o.i0, 128), 0, s, after, 1, o);
       return 0;
     case FQ3C_POLYNORM:
       if (!o.p0) return fail("polynorm: coefficients required");
-      launch_after(fq3s_polynorm_kernel, o.M, 256, 0, s, after, 1, o);
+      launch_seq(fq3s_polynorm_kernel, o.M, 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_BDGEMM: {
       if (o.i0 < 1 || o.i1 < 1 || o.i2 < 1 || o.cin < 1) return fail("bdgemm: bad block shape");
@@ -2059,10 +2067,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       const int per = (o.M + chunks - 1) / chunks;
       dim3 grid((o.N + 127) / 128, chunks);
       if (chunks > 1) {
-        launch_after(fq3s_lru_fold_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<float*>(o.ws));
+        launch_seq(fq3s_lru_fold_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<float*>(o.ws));
         count_launches(1);
       }
-      launch_after(fq3s_lru_scan_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<const float*>(o.ws));
+      launch_seq(fq3s_lru_scan_kernel, grid, 128, 0, s, after, 1, o, chunks, per, reinterpret_cast<const float*>(o.ws));
       return 0;
     }
     case FQ3C_ROUTER: {
@@ -2071,22 +2079,22 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       if (tpb < 1) return fail("router: too many experts");
       if (tpb >= 32) tpb &= ~31;
       if (o.ws && (o.M != 1 || o.i0 > 16 || !o.p0 || !o.p1 || o.K < 0)) return fail("router: grouping in the same launch takes one token with at most 16 choices");
-      launch_after(fq3s_router_kernel, (o.M + tpb - 1) / tpb, tpb, (size_t)o.N * tpb * 8, s, after, 1, o);
+      launch_seq(fq3s_router_kernel, (o.M + tpb - 1) / tpb, tpb, (size_t)o.N * tpb * 8, s, after, 1, o);
       return 0;
     }
     case FQ3C_MOE_SORT: {
       if (o.i1 < 1 || !o.A || !o.C || !o.C2 || !o.ws) return fail("moe_sort: missing operand");
       const int warps = std::min(std::min(32, ((48 * 1024) / 4 - o.i1 - 1) / o.i1), std::max(1, (o.M * o.i0 + 31) / 32));
       if (warps < 1) return fail("moe_sort: too many experts");
-      launch_after(fq3s_moe_sort_kernel, 1, warps * 32, (size_t)(o.i1 + 1 + warps * o.i1) * 4, s, after, 1, o);
+      launch_seq(fq3s_moe_sort_kernel, 1, warps * 32, (size_t)(o.i1 + 1 + warps * o.i1) * 4, s, after, 1, o);
       return 0;
     }
     case FQ3C_MOE_COMBINE:
       if (!o.A || !o.B || !o.p0 || !o.ws || !o.C) return fail("moe_combine: missing operand");
-      launch_after(fq3s_moe_combine_kernel, o.M, 256, 0, s, after, 1, o);
+      launch_seq(fq3s_moe_combine_kernel, o.M, 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_COMMIT:
-      launch_after(fq3s_commit_kernel, dim3(o.M, 8), 256, 0, s, after, 1, reinterpret_cast<const long long*>(o.A), reinterpret_cast<int*>(o.C), o.i0);
+      launch_seq(fq3s_commit_kernel, dim3(o.M, 8), 256, 0, s, after, 1, reinterpret_cast<const long long*>(o.A), reinterpret_cast<int*>(o.C), o.i0);
       return 0;
     case FQ3C_LATENT_ATTN: {
       if (o.i0 < 1 || o.i1 < 1 || !o.A || !o.B || !o.C) return fail("latent_attn: missing operand");
@@ -2122,11 +2130,11 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         }
         dim3 grid((o.M + QB - 1) / QB, (o.i0 + 15) / 16, splits);
         const int nth = 32 * QB * RSk;
-        if (nt_o <= 8) launch_after(fq3s_latent_attn_mma_kernel<8>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
-        else if (nt_o <= 16) launch_after(fq3s_latent_attn_mma_kernel<16>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
-        else launch_after(fq3s_latent_attn_mma_kernel<32>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        if (nt_o <= 8) launch_seq(fq3s_latent_attn_mma_kernel<8>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        else if (nt_o <= 16) launch_seq(fq3s_latent_attn_mma_kernel<16>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        else launch_seq(fq3s_latent_attn_mma_kernel<32>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
         if (splits > 1) {
-          launch_after(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
+          launch_seq(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
           count_launches(1);
         }
         return 0;
@@ -2144,10 +2152,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         attr[dev] = true;
       }
       dim3 grid(o.M, (o.i0 + HG - 1) / HG, splits);
-      if (o.flags & FQ3C_F32) launch_after(fq3s_latent_attn_kernel<float>, grid, 256, smem, s, after, 1, o, HG, splits);
-      else launch_after(fq3s_latent_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, HG, splits);
+      if (o.flags & FQ3C_F32) launch_seq(fq3s_latent_attn_kernel<float>, grid, 256, smem, s, after, 1, o, HG, splits);
+      else launch_seq(fq3s_latent_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, HG, splits);
       if (splits > 1) {
-        launch_after(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
+        launch_seq(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
         count_launches(1);
       }
       return 0;
@@ -2157,9 +2165,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
     case FQ3C_XIELU: {
       if (const char* e = entry_op_error(o)) return fail(e);
       const dim3 grid((o.N + 255) / 256, o.M);
-      if (o.kind == FQ3C_DYT) launch_after(fq3s_dyt_kernel, grid, 256, 0, s, after, 1, o);
-      else if (o.kind == FQ3C_DEPTH_MIX) launch_after(fq3s_depth_mix_kernel, grid, 256, 0, s, after, 1, o);
-      else launch_after(fq3s_xielu_kernel, grid, 256, 0, s, after, 1, o);
+      if (o.kind == FQ3C_DYT) launch_seq(fq3s_dyt_kernel, grid, 256, 0, s, after, 1, o);
+      else if (o.kind == FQ3C_DEPTH_MIX) launch_seq(fq3s_depth_mix_kernel, grid, 256, 0, s, after, 1, o);
+      else launch_seq(fq3s_xielu_kernel, grid, 256, 0, s, after, 1, o);
       return 0;
     }
     case FQ3C_ROT_APPEND: {
@@ -2168,21 +2176,21 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       // what the flat kernel holds: no norm, no temperature, no pooled rows; the value heads not among the queries that it turns in place
       if (o.M > 8 && o.m_begin <= 0 && !o.scale && !o.bias && !(o.flags & FQ3C_UNIT) && !(o.f3 > 0.f) && o.taps <= 4096) {
         const size_t smem = sizeof(float2) * (o.taps / 2);
-        if (o.flags & FQ3C_F32) launch_after(fq3s_rot_append_flat_kernel<float>, o.M, 256, smem, s, after, 1, o);
-        else launch_after(fq3s_rot_append_flat_kernel<bf16>, o.M, 256, smem, s, after, 1, o);
+        if (o.flags & FQ3C_F32) launch_seq(fq3s_rot_append_flat_kernel<float>, o.M, 256, smem, s, after, 1, o);
+        else launch_seq(fq3s_rot_append_flat_kernel<bf16>, o.M, 256, smem, s, after, 1, o);
         return 0;
       }
       const int rth = o.M <= 8 ? std::max(256, std::min(1024, 32 * (o.i0 + o.i1))) : 256;      // few rows: a warp per head
-      if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, true, 1024>, 1, rth, 0, s, after, 1, o);
-      else if (o.m_begin > 0 && o.M == 1) launch_after(fq3s_rot_append_kernel<bf16, true, 1024>, 1, rth, 0, s, after, 1, o);
-      else if (rth > 256 && (o.flags & FQ3C_F32)) launch_after(fq3s_rot_append_kernel<float, false, 1024>, o.M, rth, 0, s, after, 1, o);
-      else if (rth > 256) launch_after(fq3s_rot_append_kernel<bf16, false, 1024>, o.M, rth, 0, s, after, 1, o);
-      else if (o.flags & FQ3C_F32) launch_after(fq3s_rot_append_kernel<float>, o.M, 256, 0, s, after, 1, o);
-      else launch_after(fq3s_rot_append_kernel<bf16>, o.M, 256, 0, s, after, 1, o);
+      if (o.m_begin > 0 && o.M == 1 && (o.flags & FQ3C_F32)) launch_seq(fq3s_rot_append_kernel<float, true, 1024>, 1, rth, 0, s, after, 1, o);
+      else if (o.m_begin > 0 && o.M == 1) launch_seq(fq3s_rot_append_kernel<bf16, true, 1024>, 1, rth, 0, s, after, 1, o);
+      else if (rth > 256 && (o.flags & FQ3C_F32)) launch_seq(fq3s_rot_append_kernel<float, false, 1024>, o.M, rth, 0, s, after, 1, o);
+      else if (rth > 256) launch_seq(fq3s_rot_append_kernel<bf16, false, 1024>, o.M, rth, 0, s, after, 1, o);
+      else if (o.flags & FQ3C_F32) launch_seq(fq3s_rot_append_kernel<float>, o.M, 256, 0, s, after, 1, o);
+      else launch_seq(fq3s_rot_append_kernel<bf16>, o.M, 256, 0, s, after, 1, o);
       if (o.m_begin > 0 && o.M > 1) {
         const dim3 grid(o.M / o.m_begin + 1, (o.i1 * std::max(o.i2, o.cin) + 255) / 256, 2);
-        if (o.flags & FQ3C_F32) launch_after(fq3s_pool_append_kernel<float>, grid, 256, 0, s, after, 1, o);
-        else launch_after(fq3s_pool_append_kernel<bf16>, grid, 256, 0, s, after, 1, o);
+        if (o.flags & FQ3C_F32) launch_seq(fq3s_pool_append_kernel<float>, grid, 256, 0, s, after, 1, o);
+        else launch_seq(fq3s_pool_append_kernel<bf16>, grid, 256, 0, s, after, 1, o);
         count_launches(1);
       }
       return 0;
@@ -2210,7 +2218,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         a.gate_ld = o.col_mod; a.entry = o.res && (o.flags & FQ3C_GATE_ENTRY); a.out_f32 = (o.flags & FQ3C_OUT_F32) != 0; a.out = o.C; a.ldo = o.ldc;
         const int mode = o.bias ? AT_DIST : o.f1 > 0.f ? AT_CAP : AT_PLAIN;
         if (attn_tc_takes(a, mode)) {
-          launch_attn_tc(a, mode, s, after);
+          launch_attn_tc(a, mode, s, false);      // (many rows)
           return 0;
         }
       }
@@ -2238,12 +2246,12 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         dim3 grid((o.M + QBLK - 1) / QBLK, o.i1);
         const size_t smem = cache_attn_mma_smem(ROWS, o.i2, o.cin);
         if (pool) {
-          if (o.cin <= 32) launch_after(fq3s_cache_attn_mma_kernel<4, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
-          else if (o.cin <= 64) launch_after(fq3s_cache_attn_mma_kernel<8, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
-          else launch_after(fq3s_cache_attn_mma_kernel<16, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
-        } else if (o.cin <= 32) launch_after(fq3s_cache_attn_mma_kernel<4>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
-        else if (o.cin <= 64) launch_after(fq3s_cache_attn_mma_kernel<8>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
-        else launch_after(fq3s_cache_attn_mma_kernel<16>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+          if (o.cin <= 32) launch_seq(fq3s_cache_attn_mma_kernel<4, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+          else if (o.cin <= 64) launch_seq(fq3s_cache_attn_mma_kernel<8, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+          else launch_seq(fq3s_cache_attn_mma_kernel<16, true>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        } else if (o.cin <= 32) launch_seq(fq3s_cache_attn_mma_kernel<4>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        else if (o.cin <= 64) launch_seq(fq3s_cache_attn_mma_kernel<8>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
+        else launch_seq(fq3s_cache_attn_mma_kernel<16>, grid, ROWS * 2, smem, s, after, 1, o, ROWS);
         return 0;
       }
       // an f32 cache and more than a few queries, heads of 128: 32-row blocks with pipelined tiles
@@ -2257,9 +2265,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
           fattr[dev] = true;
         }
         const int QB = FA_R / HG;
-        launch_after(fq3s_attn_f32_kernel, dim3((o.M + QB - 1) / QB, o.i1, splits), 128, FA_SMEM, s, after, 1, o);
+        launch_seq(fq3s_attn_f32_kernel, dim3((o.M + QB - 1) / QB, o.i1, splits), 128, FA_SMEM, s, after, 1, o);
         if (splits > 1) {
-          launch_after(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
+          launch_seq(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
           count_launches(1);
         }
         return 0;
@@ -2280,12 +2288,12 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         attr[dev] = true;
       }
       dim3 grid((o.M + QB - 1) / QB, o.i1, splits);
-      if (pool && (o.flags & FQ3C_F32)) launch_after(fq3s_cache_attn_kernel<float, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
-      else if (pool) launch_after(fq3s_cache_attn_kernel<bf16, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
-      else if (o.flags & FQ3C_F32) launch_after(fq3s_cache_attn_kernel<float>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
-      else launch_after(fq3s_cache_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      if (pool && (o.flags & FQ3C_F32)) launch_seq(fq3s_cache_attn_kernel<float, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else if (pool) launch_seq(fq3s_cache_attn_kernel<bf16, true>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else if (o.flags & FQ3C_F32) launch_seq(fq3s_cache_attn_kernel<float>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
+      else launch_seq(fq3s_cache_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, QB, TJ, splits);
       if (splits > 1) {
-        launch_after(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
+        launch_seq(fq3s_cache_attn_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
         count_launches(1);
       }
       return 0;
@@ -2302,13 +2310,13 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         cudaFuncSetAttribute(fq3s_hyper_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         hattr[dev] = true;
       }
-      if (o.i0 <= 8) launch_after(fq3s_hyper_kernel<8>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
-      else launch_after(fq3s_hyper_kernel<16>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
+      if (o.i0 <= 8) launch_seq(fq3s_hyper_kernel<8>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
+      else launch_seq(fq3s_hyper_kernel<16>, o.M, 256, (size_t)o.N * 4, s, after, 1, o);
       return 0;
     }
     case FQ3C_GLU:
       if (!o.A || !o.C || o.N < 1) return fail("glu: missing operand");
-      launch_after(fq3s_glu_kernel, dim3((o.N + 255) / 256, o.M), 256, 0, s, after, 1, o);
+      launch_seq(fq3s_glu_kernel, dim3((o.N + 255) / 256, o.M), 256, 0, s, after, 1, o);
       return 0;
     case FQ3C_MSTATE_SCAN: {
       if (o.i0 < 1 || o.i1 < 1 || o.i0 % o.i1 || o.i2 < 1 || o.cin < 1 || !o.A || !o.p0 || !o.C || !o.C2) return fail("mstate_scan: bad configuration");
@@ -2340,20 +2348,20 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       const bool blocks = (o.taps == 0 || o.taps == 6) && o.M >= CD_MIN_ROWS && o.i2 <= CD_MAX_DK &&
                           o.ws_bytes / 4 >= cd_ws_floats(o.M, o.i0, o.i2, o.taps == 6) && !(reinterpret_cast<uintptr_t>(o.ws) & 15);
       if (o.taps == 4 && o.M > MS_CH) {
-        launch_after(fq3s_mstate_gate_kernel, dim3(o.M, (o.i0 * o.i2 + 255) / 256), 256, 0, s, after, 1, o);
+        launch_seq(fq3s_mstate_gate_kernel, dim3(o.M, (o.i0 * o.i2 + 255) / 256), 256, 0, s, after, 1, o);
         count_launches(1);
       } else if (o.taps == 5 && o.M > MS_CH) {
-        launch_after(fq3s_mstate_max_kernel, o.i0, MM_THREADS, 0, s, after, 1, o);
+        launch_seq(fq3s_mstate_max_kernel, o.i0, MM_THREADS, 0, s, after, 1, o);
         count_launches(1);
       } else if (o.taps == 6) {
         const int per = cdelta_prep_channels(o.M == 1 ? 1 : MS_PREP_ROWS);
         const dim3 grid((o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS, (o.i0 * o.i2 + per - 1) / per + (o.tap_off[2] > 0 ? (o.i0 * o.cin + per - 1) / per : 0) + (blocks ? 0 : 1));
         const size_t smem = sizeof(float) * MS_PREP_ROWS * (size_t)std::max(o.tap_off[0], o.tap_off[2]);
-        if (o.M == 1) launch_after(fq3s_mstate_cdelta_prep_kernel<1>, grid, 256, smem, s, after, 1, o, false);
-        else launch_after(fq3s_mstate_cdelta_prep_kernel<MS_PREP_ROWS>, grid, 256, smem, s, after, 1, o, blocks);
+        if (o.M == 1) launch_seq(fq3s_mstate_cdelta_prep_kernel<1>, grid, 256, smem, s, after, 1, o, false);
+        else launch_seq(fq3s_mstate_cdelta_prep_kernel<MS_PREP_ROWS>, grid, 256, smem, s, after, 1, o, blocks);
         count_launches(1);
       } else if (o.taps < 3 && !blocks) {
-        launch_after(fq3s_mstate_prep_kernel, o.taps == 2 ? (o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS : o.M, 128, 0, s, after, 1, o);
+        launch_seq(fq3s_mstate_prep_kernel, o.taps == 2 ? (o.M + MS_PREP_ROWS - 1) / MS_PREP_ROWS : o.M, 128, 0, s, after, 1, o);
         count_launches(1);
       }
       static bool sattr[64] = {};
@@ -2388,19 +2396,19 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
           battr[dev] = true;
         }
         const dim3 rgrid((o.M + CD_C - 1) / CD_C, o.i0);
-        if (o.taps == 6) launch_after(fq3s_cdelta_record_kernel<true>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, true), s, after, 1, o);
-        else launch_after(fq3s_cdelta_record_kernel<false>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, false), s, after, 1, o);
+        if (o.taps == 6) launch_seq(fq3s_cdelta_record_kernel<true>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, true), s, after, 1, o);
+        else launch_seq(fq3s_cdelta_record_kernel<false>, rgrid, CD_REC_THREADS, cd_record_smem(o.i2, false), s, after, 1, o);
         count_launches(1);
         // narrow state tiles while they do not outnumber the SMs, wide ones otherwise and for few state rows
         const bool narrow = o.i2 > 64 && o.i0 * ((o.cin + 7) / 8) <= 148;
         const dim3 grid((o.cin + (narrow ? 7 : 15)) / (narrow ? 8 : 16), o.i0);
         const int dvt = narrow ? 8 : 16, ring = cd_walk_floats(dvt, o.i2, 4) * 4 <= CD_WALK_SMEM ? 4 : 3;
         const size_t wsm = (size_t)cd_walk_floats(dvt, o.i2, ring) * 4;
-        if (narrow && o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<8, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
-        else if (narrow) launch_after(fq3s_cdelta_walk_kernel<8, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
-        else if (o.i2 <= 64) launch_after(fq3s_cdelta_walk_kernel<16, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
-        else if (o.i2 <= 128) launch_after(fq3s_cdelta_walk_kernel<16, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
-        else launch_after(fq3s_cdelta_walk_kernel<16, 4>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        if (narrow && o.i2 <= 128) launch_seq(fq3s_cdelta_walk_kernel<8, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (narrow) launch_seq(fq3s_cdelta_walk_kernel<8, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (o.i2 <= 64) launch_seq(fq3s_cdelta_walk_kernel<16, 1>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else if (o.i2 <= 128) launch_seq(fq3s_cdelta_walk_kernel<16, 2>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
+        else launch_seq(fq3s_cdelta_walk_kernel<16, 4>, grid, CD_WALK_THREADS, wsm, s, after, 1, o, ring);
         return 0;
       }
       // Long runs of a recurrence whose decays do not depend on the state: pieces walked twice (see the kernel), when the caller's
@@ -2428,16 +2436,16 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         const dim3 grid((sv + cpt * MS_COLS - 1) / (cpt * MS_COLS), o.i0, nz);
         const size_t smem = sizeof(float) * 2 * mstate_buf_floats(bound, three ? 3 : 2, cpt);
 #define FQ3S_WALK(RPT, CPT) \
-    if (three && gated) launch_after(fq3s_mstate_scan_kernel<RPT, 3, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
-    else if (three) launch_after(fq3s_mstate_scan_kernel<RPT, 3, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
-    else if (gated) launch_after(fq3s_mstate_scan_kernel<RPT, 2, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
-    else launch_after(fq3s_mstate_scan_kernel<RPT, 2, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P);
+    if (three && gated) launch_seq(fq3s_mstate_scan_kernel<RPT, 3, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else if (three) launch_seq(fq3s_mstate_scan_kernel<RPT, 3, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else if (gated) launch_seq(fq3s_mstate_scan_kernel<RPT, 2, true, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); \
+    else launch_seq(fq3s_mstate_scan_kernel<RPT, 2, false, CPT>, grid, 128, smem, s, after, 1, o, phase, piece, X, P);
         if (cdelta) switch (bound) {
-          case 4: launch_after(fq3s_mstate_scan_kernel<4, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
-          case 8: launch_after(fq3s_mstate_scan_kernel<8, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
-          case 16: launch_after(fq3s_mstate_scan_kernel<16, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
-          case 32: launch_after(fq3s_mstate_scan_kernel<32, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
-          default: launch_after(fq3s_mstate_scan_kernel<64, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 4: launch_seq(fq3s_mstate_scan_kernel<4, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 8: launch_seq(fq3s_mstate_scan_kernel<8, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 16: launch_seq(fq3s_mstate_scan_kernel<16, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          case 32: launch_seq(fq3s_mstate_scan_kernel<32, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
+          default: launch_seq(fq3s_mstate_scan_kernel<64, 3, false, 1, true>, grid, 128, smem, s, after, 1, o, phase, piece, X, P); break;
         }
         else if (cpt == 2) switch (bound) {
           case 4: FQ3S_WALK(4, 2) break;
@@ -2459,7 +2467,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       }
       walk(1, pieces - 1);
       const int64_t n = (int64_t)o.i0 * o.i2 * sv;
-      launch_after(fq3s_mstate_carry_kernel, (unsigned)((n + 255) / 256), 256, 0, s, after, 1, o, pieces, X, P, sv);
+      launch_seq(fq3s_mstate_carry_kernel, (unsigned)((n + 255) / 256), 256, 0, s, after, 1, o, pieces, X, P, sv);
       walk(3, pieces);
       count_launches(2);
       return 0;
@@ -2478,10 +2486,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
       if (o.N % 4 == 0 && o.N <= 1024 * SN_VECS && !((o.lda | o.ldc | o.norm_ld | o.K) & 3) && !o.C2 &&
           !((reinterpret_cast<uintptr_t>(o.A) | reinterpret_cast<uintptr_t>(o.C) | reinterpret_cast<uintptr_t>(o.norm_out) | reinterpret_cast<uintptr_t>(o.norm_w) |
             reinterpret_cast<uintptr_t>(o.bias)) & 15)) {
-        launch_after(fq3s_sum_norm_vec_kernel, o.M, std::max(32, std::min(256, (o.N / 4 + 31) / 32 * 32)), 0, s, after, 1, o);
+        launch_seq(fq3s_sum_norm_vec_kernel, o.M, std::max(32, std::min(256, (o.N / 4 + 31) / 32 * 32)), 0, s, after, 1, o);
         return 0;
       }
-      launch_after(fq3s_sum_norm_kernel, o.M, row_threads(o.M, o.N, 256), (size_t)o.N * 4, s, after, 1, o);
+      launch_seq(fq3s_sum_norm_kernel, o.M, row_threads(o.M, o.N, 256), (size_t)o.N * 4, s, after, 1, o);
       return 0;
     }
     default: return 1;
@@ -2640,7 +2648,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
           const bool f32 = (o.flags & FQ3C_F32) != 0;
           SeqTail tail{};
           gemv_tail(o, g, ops + i + 1, n_ops - i - 1, tail);
-          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s, after && o.M <= DEP_ROWS, &tail) != 0) return -1;
+          if (launch_seq_gemm(g, f32, f32, true, 1, (o.M + 63) / 64, s, after, &tail) != 0) return -1;
           i += tail.n;
           break;
         }
@@ -2840,7 +2848,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
         }
         [[fallthrough]];
       default: {
-        const int rc = seq_run(o, s, after && (o.kind == FQ3C_COMMIT ? o.i0 : o.M) <= DEP_ROWS);
+        const int rc = seq_run(o, s, after);
         if (rc == 1) return fail("unknown op kind");
         if (rc != 0) return rc;
       }

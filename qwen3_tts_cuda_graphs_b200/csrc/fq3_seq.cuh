@@ -15,9 +15,10 @@ __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn
 // rows blocks that come up early come up several on one SM, beside others that stay empty, which a launch that has work for all of them pays for (an attention layer of 4 rows
 // behind 300 positions 39 us without, 59 with; of 384 rows in 32 bits 143 and 159).
 constexpr int DEP_ROWS = 2;
-// (run_ops launches them early under the same condition; the wait itself costs a launch that is not early some 0.15 us.)
+// (launch_seq launches them early under the same condition on the same argument; the wait itself costs a launch that is not early some 0.15 us.)
+__host__ __device__ constexpr bool seq_early(const int rows) { return rows <= DEP_ROWS; }
 __device__ __forceinline__ void seq_dep_begin(const int rows) {
-  if (rows > DEP_ROWS) return;
+  if (!seq_early(rows)) return;
   grid_dep_wait();
   grid_dep_launch();
 }
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(256) fq3s_gemv_kernel(const __grid_constant__ 
     }
   };
   if (g.early) first();
-  if (warp == 0 && g.M <= DEP_ROWS) {
+  if (warp == 0 && seq_early(g.M)) {
     args_ahead(g);
     if (TAIL) args_ahead(tail);
   }
@@ -2125,7 +2126,7 @@ __device__ __forceinline__ void af_store(float* local, const int rank, const flo
 template <typename TC, int D, int HG, bool ROT>
 __global__ void __launch_bounds__(AF_WARPS * 32, !ROT && sizeof(TC) == 2 && HG <= 4 ? 2 : 1) fq3s_attn_few_kernel(const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op r) {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (the other CTAs have begun when this completes)
-  if (threadIdx.x < 32 && o.M <= DEP_ROWS) {
+  if (threadIdx.x < 32 && seq_early(o.M)) {
     args_ahead(o);
     if (ROT) args_ahead(r);
   }
@@ -3841,7 +3842,7 @@ template <int RPT>
 __global__ void __launch_bounds__(128) fq3s_delta_row_kernel(const __grid_constant__ fq3c_op c, const __grid_constant__ fq3c_op o, const __grid_constant__ fq3c_op n) {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   if (threadIdx.x < 32) { args_ahead(c); args_ahead(o); args_ahead(n); }
-  seq_dep_begin(1);
+  seq_dep_begin(c.M);      // (1)
   constexpr int DK = 8 * RPT, SL = RPT + 4, TS = RPT * 16 + 4, NE = (2 * DK + 127) / 128;
   // slices of RPT entries (rows), four floats apart: no bank conflicts
   __shared__ __align__(16) float tile[8 * TS], qs[8 * SL], ks[8 * SL], vs[16], ys[128], red[32], two[2];
