@@ -10,11 +10,12 @@ template <> __device__ __forceinline__ float ldf<bf16>(const bf16* p) { return _
 __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-// With few rows (decoding) a list is a chain of launches of some 3 us each, so the next one's blocks come up while this one works and wait here for its end.  One launch ahead, not more:
+// With one row (decoding) a list is a chain of launches of some 3 us each, so the next one's blocks come up while this one works and wait here for its end.  One launch ahead, not more:
 // with the next launch let in before this wait, waiting blocks pile up (a token of 36 launches 163 us of the GPU's time without, 180 with many ahead, 149 with one).  With more
-// rows blocks that come up early come up several on one SM, beside others that stay empty, which a launch that has work for all of them pays for (an attention layer of 4 rows
-// behind 300 positions 39 us without, 59 with; of 384 rows in 32 bits 143 and 159).
-constexpr int DEP_ROWS = 2;
+// rows blocks that come up early come up several on one SM, beside others that stay empty, which a launch that has work for all of them pays for: of twelve models, 1024 and 2048 wide,
+// a step of two rows was up to 0.81 times as fast with early launches as before them (one of three layers run twice 304 us and 378) and is 0.98 - 1.04 times as fast without; an attention
+// layer of 4 rows behind 300 positions 39 us without, 59 with; of 384 rows in 32 bits 143 and 159.
+constexpr int DEP_ROWS = 1;
 // (launch_seq launches them early under the same condition on the same argument; the wait itself costs a launch that is not early some 0.15 us.)
 __host__ __device__ constexpr bool seq_early(const int rows) { return rows <= DEP_ROWS; }
 __device__ __forceinline__ void seq_dep_begin(const int rows) {
