@@ -1797,10 +1797,14 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-      cudaFuncSetAttribute(fq3s_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
+      cudaFuncSetAttribute(fq3s_gemm_f32_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem(1));
+      cudaFuncSetAttribute(fq3s_gemm_f32_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, fg_smem(4));
       attr[dev] = true;
     }
-    launch_seq(fq3s_gemm_f32_kernel, grid, 256, FG_SMEM, s, after, 1, g);
+    // Four groups of threads where the tiles are a single wave of blocks, one group from there on (us, one and four; tiles x k): 64 rows of 1536 x 1024 (24 x 1024) 41.0 and 37.5, 384 (144)
+    // 42.0 and 38.1, 500 (192) 70.3 and 73.9, 2048 (768) 198 and 218; 700 rows of 1024 x 64 (176 x 64) 10.2 and 12.1, 100 (32) 7.7 and 7.0.
+    if ((long)grid.x * grid.y * grid.z <= GP_SMS) launch_seq(fq3s_gemm_f32_kernel<4>, grid, 256, fg_smem(4), s, after, 1, g);
+    else launch_seq(fq3s_gemm_f32_kernel<1>, grid, 256, fg_smem(1), s, after, 1, g);
   }
   else if (b_f32) launch_seq(fq3s_gemm_kernel<float, float>, grid, 256, 0, s, after, 1, g);
   else if (a_f32 && exact) launch_seq(fq3s_gemm_kernel<float, bf16>, grid, 256, 0, s, after, 1, g);

@@ -6,13 +6,35 @@
 
 __device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }   // four consecutive floats as two pairs
 
-// C = A B^T like fq3s_gemm_kernel<float, float>, for rows of whole 16-byte pieces.  64 x 64 tiles, three stages of 32 k; four groups of 64 threads take eight k of a stage each, a thread
-// 8 x 8 outputs of its group's partial tile; a sum is kept as two (even and odd k), so that both operands are read as they lie, and the groups' four are added at the end.
-// Shared memory and the f32 pipe bound it together (32 768 cycles of a tile of 1024 k each, little of which overlaps: a thread loads 16 floats for 64 multiply-adds; with 4 x 4 outputs
-// shared memory took twice that).  Two products of 384 rows (1536 x 1024, 1024 x 1024): 86 us with 4 x 4 outputs, 79 so, and 6.1e-7 off float64 where they were 8.4e-7.
+// C = A B^T like fq3s_gemm_kernel<float, float>, for rows of whole 16-byte pieces.  64 x 64 tiles, three stages of 32 k; a sum is kept as two (even and odd k) that are added at the end,
+// so that both operands are read as they lie.  Shared memory and the f32 pipe bound it together.
+// GROUPS = 1: a thread has 4 x 4 outputs, two or more blocks an SM.  GROUPS = 4: four groups of 64 threads take eight k of a stage each, a thread 8 x 8 outputs of its group's partial tile
+// (16 floats loaded for 64 multiply-adds, half as many as with 4 x 4), the groups' four are added at the end; its registers make it one block an SM, so it is for tiles that are a single
+// wave (figures where it is chosen).
 constexpr int FG_BM = 64, FG_BN = 64, FG_BK = 32, FG_P = FG_BK + 4, FG_ST = 3, FG_CP = FG_BN + 8;
-constexpr int FG_SMEM = FG_ST * (FG_BM + FG_BN) * FG_P * 4 > 4 * FG_BM * FG_CP * 4 ? FG_ST * (FG_BM + FG_BN) * FG_P * 4 : 4 * FG_BM * FG_CP * 4;
-__global__ void __launch_bounds__(256, 1) fq3s_gemm_f32_kernel(const SeqGemm g) {
+constexpr int fg_smem(const int groups) {
+  const int stages = FG_ST * (FG_BM + FG_BN) * FG_P * 4, parts = groups > 1 ? groups * FG_BM * FG_CP * 4 : 0;
+  return stages > parts ? stages : parts;
+}
+// a finished entry v of row r, column n (z's columns begin at ccol)
+__device__ __forceinline__ void fg_store(const SeqGemm& g, const int r, const int row_end, const int ccol, const int n, float v) {
+  if (g.flags & FQ3C_SWIGLU) {      // the unit's other column is the neighbouring lane's
+    const float up = __shfl_down_sync(0xffffffffu, v, 1);
+    if (r < row_end && n + 1 < g.N && !(n & 1)) sg_store_glu(g, r, ccol, n, v, up, sg_row_scale(g, r));
+    return;
+  }
+  if (r >= row_end || n >= g.N) return;
+  if (g.flags & FQ3C_BIAS) v += g.bias[ccol + n];
+  if (g.flags & FQ3C_GELU) v = gelu_f(v);
+  if (g.flags & FQ3C_GELU_TANH) v = gelu_tanh_f(v);
+  if (g.flags & FQ3C_SIGMOID) v = sigmoid_f(v);
+  if (g.flags & FQ3C_RELU2) { v = fmaxf(v, 0.f); v *= v; }
+  const size_t ci = (size_t)r * g.ldc + ccol + n;
+  if (g.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(g.C)[ci] = v;
+  else reinterpret_cast<bf16*>(g.C)[ci] = __float2bfloat16_rn(v);
+}
+template <int GROUPS>
+__global__ void __launch_bounds__(256) fq3s_gemm_f32_kernel(const SeqGemm g) {
   seq_dep_begin(g.M);
   extern __shared__ __align__(16) float fg[];
   float (*As)[FG_BM][FG_P] = reinterpret_cast<float (*)[FG_BM][FG_P]>(fg);
@@ -60,12 +82,13 @@ __global__ void __launch_bounds__(256, 1) fq3s_gemm_f32_kernel(const SeqGemm g) 
     }
     cp_async_commit();
   };
-  const int kg = tid >> 6, ty = (tid >> 3) & 7, tx = tid & 7;
-  f32x2 acc[8][8];
+  constexpr int E = GROUPS > 1 ? 8 : 4, L = 64 / E;      // outputs of a thread: E x E, rows and columns L apart
+  const int kg = GROUPS > 1 ? tid >> 6 : 0, ty = tid / L % L, tx = tid % L;
+  f32x2 acc[E][E];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < E; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < E; ++j) acc[i][j] = 0ull;
   stage(0);
   stage(1);
   for (int kt = 0; kt < KT; ++kt) {
@@ -74,49 +97,41 @@ __global__ void __launch_bounds__(256, 1) fq3s_gemm_f32_kernel(const SeqGemm g) 
     stage(kt + 2);
     const int st = kt % FG_ST;
 #pragma unroll
-    for (int k = 0; k < FG_BK / 4; k += 4) {
-      ulonglong2 a[8], b[8];
+    for (int k = 0; k < FG_BK / GROUPS; k += 4) {
+      ulonglong2 a[E], b[E];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = ld_pairs(&Bs[st][tx + 8 * j][kg * (FG_BK / 4) + k]);
+      for (int j = 0; j < E; ++j) b[j] = ld_pairs(&Bs[st][tx + L * j][kg * (FG_BK / GROUPS) + k]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = ld_pairs(&As[st][ty + 8 * i][kg * (FG_BK / 4) + k]);
+      for (int i = 0; i < E; ++i) a[i] = ld_pairs(&As[st][ty + L * i][kg * (FG_BK / GROUPS) + k]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < E; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma2<true>(a[i].x, b[j].x, acc[i][j]);
+        for (int j = 0; j < E; ++j) acc[i][j] = fma2<true>(a[i].x, b[j].x, acc[i][j]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < E; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma2<true>(a[i].y, b[j].y, acc[i][j]);
+        for (int j = 0; j < E; ++j) acc[i][j] = fma2<true>(a[i].y, b[j].y, acc[i][j]);
     }
+  }
+  const int ccol = z * g.c_zstride;
+  if (GROUPS == 1) {
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+#pragma unroll
+      for (int j = 0; j < E; ++j) fg_store(g, row0 + ty + L * i, row_end, ccol, col0 + tx + L * j, lo2(acc[i][j]) + hi2(acc[i][j]));
+    return;
   }
   cp_async_wait<0>();
   __syncthreads();      // the stages become the groups' partial tiles
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < E; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) fg[(kg * FG_BM + ty + 8 * i) * FG_CP + tx + 8 * j] = lo2(acc[i][j]) + hi2(acc[i][j]);
+    for (int j = 0; j < E; ++j) fg[(kg * FG_BM + ty + L * i) * FG_CP + tx + L * j] = lo2(acc[i][j]) + hi2(acc[i][j]);
   __syncthreads();
-  const int ccol = z * g.c_zstride, n = col0 + (tid & 63);
 #pragma unroll 4
   for (int i = tid >> 6; i < FG_BM; i += 4) {
-    const int r = row0 + i;
     const float* p = fg + i * FG_CP + (tid & 63);
-    float v = (p[0] + p[FG_BM * FG_CP]) + (p[2 * FG_BM * FG_CP] + p[3 * FG_BM * FG_CP]);
-    if (g.flags & FQ3C_SWIGLU) {      // the unit's other column is the neighbouring lane's
-      const float up = __shfl_down_sync(0xffffffffu, v, 1);
-      if (r < row_end && n + 1 < g.N && !(n & 1)) sg_store_glu(g, r, ccol, n, v, up, sg_row_scale(g, r));
-      continue;
-    }
-    if (r >= row_end || n >= g.N) continue;
-    if (g.flags & FQ3C_BIAS) v += g.bias[ccol + n];
-    if (g.flags & FQ3C_GELU) v = gelu_f(v);
-    if (g.flags & FQ3C_GELU_TANH) v = gelu_tanh_f(v);
-    if (g.flags & FQ3C_SIGMOID) v = sigmoid_f(v);
-    if (g.flags & FQ3C_RELU2) { v = fmaxf(v, 0.f); v *= v; }
-    const size_t ci = (size_t)r * g.ldc + ccol + n;
-    if (g.flags & FQ3C_OUT_F32) reinterpret_cast<float*>(g.C)[ci] = v;
-    else reinterpret_cast<bf16*>(g.C)[ci] = __float2bfloat16_rn(v);
+    fg_store(g, row0 + i, row_end, ccol, col0 + (tid & 63), (p[0] + p[FG_BM * FG_CP]) + (p[2 * FG_BM * FG_CP] + p[3 * FG_BM * FG_CP]));
   }
 }
 

@@ -31,6 +31,11 @@ def test_product(M, N, K):
         assert (out[M] == 5).all()
 
 
+@pytest.mark.parametrize("M, N, K", [(768, 768, 20), (769, 736, 100), (2100, 320, 64), (640, 960, 1024)])      # 144, 156, 165, 150 tiles
+def test_product_of_a_wave_and_more(M, N, K):
+    test_product(M, N, K)
+
+
 # rows, positions in front, heads, key heads, key splits, options
 @pytest.mark.parametrize("rows, first, heads, kv, splits, opt", [(9, 0, 4, 2, 1, {}), (33, 31, 8, 2, 1, {}), (64, 64, 6, 2, 3, {}), (100, 300, 8, 2, 4, dict(window=64)), (90, 200, 4, 4, 1, dict(window=40, keep=3)),
                                                                   (200, 100, 2, 1, 2, dict(chunk=70)), (40, 500, 12, 4, 16, dict(cap=30.0)), (384, 300, 8, 2, 3, dict(window=512)), (12, 0, 32, 1, 5, {})])
