@@ -1482,6 +1482,9 @@ void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 template <typename... A> int dep_rows(const fq3c_op& o, const A&...) { return o.M; }
 template <typename... A> int dep_rows(const SeqGemm& g, const A&...) { return g.M; }
 inline int dep_rows(const long long*, const int*, const int by) { return by; }      // fq3s_commit_kernel
+// Walks over a cache in splits, whose blocks are large: not early with more of them than SMs, where they come up unevenly (one row of 32 heads over 4 behind 2000 positions 23.4 us, early
+// 25.7).
+inline bool blocks_fit(const dim3& grid) { return (long)grid.x * grid.y * grid.z <= GP_SMS; }
 template <typename... P, typename... A>
 void launch_seq(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool after, int cluster, const A&... args) {
   launch_after(kernel, grid, block, smem, s, after && seq_early(dep_rows(args...)), cluster, args...);
@@ -2139,9 +2142,10 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         }
         dim3 grid((o.M + QB - 1) / QB, (o.i0 + 15) / 16, splits);
         const int nth = 32 * QB * RSk;
-        if (nt_o <= 8) launch_seq(fq3s_latent_attn_mma_kernel<8>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
-        else if (nt_o <= 16) launch_seq(fq3s_latent_attn_mma_kernel<16>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
-        else launch_seq(fq3s_latent_attn_mma_kernel<32>, grid, nth, smem, s, after, 1, o, RSk, splits, TJ, QB);
+        const bool early = after && blocks_fit(grid);
+        if (nt_o <= 8) launch_seq(fq3s_latent_attn_mma_kernel<8>, grid, nth, smem, s, early, 1, o, RSk, splits, TJ, QB);
+        else if (nt_o <= 16) launch_seq(fq3s_latent_attn_mma_kernel<16>, grid, nth, smem, s, early, 1, o, RSk, splits, TJ, QB);
+        else launch_seq(fq3s_latent_attn_mma_kernel<32>, grid, nth, smem, s, early, 1, o, RSk, splits, TJ, QB);
         if (splits > 1) {
           launch_seq(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
           count_launches(1);
@@ -2161,8 +2165,9 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         attr[dev] = true;
       }
       dim3 grid(o.M, (o.i0 + HG - 1) / HG, splits);
-      if (o.flags & FQ3C_F32) launch_seq(fq3s_latent_attn_kernel<float>, grid, 256, smem, s, after, 1, o, HG, splits);
-      else launch_seq(fq3s_latent_attn_kernel<bf16>, grid, 256, smem, s, after, 1, o, HG, splits);
+      // (never early: a token of four such layers in 32 bits behind 1000 positions 595 us, early 692)
+      if (o.flags & FQ3C_F32) launch_seq(fq3s_latent_attn_kernel<float>, grid, 256, smem, s, false, 1, o, HG, splits);
+      else launch_seq(fq3s_latent_attn_kernel<bf16>, grid, 256, smem, s, false, 1, o, HG, splits);
       if (splits > 1) {
         launch_seq(fq3s_latent_merge_kernel, dim3(o.M, o.i0), 128, 0, s, after, 1, o, splits);
         count_launches(1);
@@ -2297,8 +2302,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
         attr[dev] = true;
       }
       dim3 grid((o.M + QB - 1) / QB, o.i1, splits);
-      // (not early with more blocks than SMs, which come up unevenly: one row of 32 heads over 4 behind 2000 positions 23.4 us, early 25.7)
-      const bool early = after && (long)grid.x * grid.y * grid.z <= GP_SMS;
+      const bool early = after && blocks_fit(grid);
       if (pool && (o.flags & FQ3C_F32)) launch_seq(fq3s_cache_attn_kernel<float, true>, grid, 256, smem, s, early, 1, o, QB, TJ, splits);
       else if (pool) launch_seq(fq3s_cache_attn_kernel<bf16, true>, grid, 256, smem, s, early, 1, o, QB, TJ, splits);
       else if (o.flags & FQ3C_F32) launch_seq(fq3s_cache_attn_kernel<float>, grid, 256, smem, s, early, 1, o, QB, TJ, splits);
