@@ -1916,14 +1916,15 @@ const char* cache_attn_error(const fq3c_op& o) {
 // 4 heads a key head, 17.6 us by itself and 17.9 here; 8 heads a key head behind 1000 15.0 and 10.8, behind 2000 20.6 and 24; one head a key head behind 8000 63 and 24 (16 heads), 27 and 19 (one).
 // And as many clusters (rows x key heads) as are on the GPU at a time, or nearly: 15 of the variants with one CTA an SM, 30 of those with two, which win with two rounds of them as well
 // (8 rows of 32 heads over 8 behind 200 23.1 and 15.9; of 64 over 16, four rounds, 27.0 and 29.0; heads of 64, 32 over 32, behind 30 10.4 and 26.7).  Of the others two rounds are worth
-// it where the keys are few and the kernels beside take two launches (32-bit caches, four rows of 8 heads over 8: behind 30, one launch, 14.2 and 14.8 with 8 rows; behind 1000 14.2 and 15.1; behind 4000 29 and 39).
+// it where the kernels beside take two launches and the keys are few, or heads of 128 share them (32-bit caches: four rows of 8 heads over 8 behind 500 12.4 and 10.9, behind 1000 14.2 and
+// 15.1, behind 4000 29 and 39; four of 32 over 8 behind 1980 45.2 and 39.0; two of 64 over 16 behind 30, one launch, 11.7 and 13.5).
 bool attn_few_takes(const fq3c_op& o) {
   const int splits = std::max(1, o.m_begin);
   const long keys = o.K > 0 && o.a_rows <= 0 ? o.K : o.tap_off[0] > 0 ? o.tap_off[0] : splits < 64 ? 32L * splits : 1L << 30;
   auto off = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
   const int V = o.flags & FQ3C_F32 ? 4 : 8, HG = o.i1 > 0 ? o.i0 / o.i1 : 0;
   const long clusters = (long)o.M * o.i1;
-  const bool fits = V == 8 && HG <= 4 ? clusters <= (o.i2 == 128 ? 64 : 32) : clusters <= 15 || (clusters <= 32 && splits > 1 && keys <= 512);
+  const bool fits = V == 8 && HG <= 4 ? clusters <= (o.i2 == 128 ? 64 : 32) : clusters <= 15 || (clusters <= 32 && splits > 1 && (keys <= 512 || (HG > 1 && o.i2 == 128)));
   return fits && o.M <= AF_ROWS && (HG == 1 || keys <= (HG == 8 ? 1024 : 2048)) && (o.i2 == 64 || o.i2 == 128) && o.cin == o.i2 && o.i0 >= 1 && o.i1 >= 1 && o.i0 % o.i1 == 0 && (HG <= 4 || HG == 8) && o.i1 <= 65535 && o.tap_off[1] <= 0 &&
          o.A && o.B && o.p1 && o.C && o.ldr % V == 0 && o.taps % V == 0 && !off(o.B) && !off(o.p1);
 }

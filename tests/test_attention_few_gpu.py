@@ -159,3 +159,31 @@ def test_visible_keys_that_score_minus_infinity(f32, H, G, pos, low, turned):
         assert lib.fq3c_run((K.Op * len(part))(*part), len(part), torch.cuda.current_stream().cuda_stream) == 0, lib.fq3c_last_error()
     # as in the test above; a new key that rounds the other way moves its score by 2^-8 of a term
     assert want.isfinite().all() and (out.double() - want).norm() <= (1e-5 if f32 else 4e-3) * want.norm()
+
+
+@pytest.mark.parametrize("M,pos,H,G,D,f32,splits,launches", [
+    (1, 5000, 4, 4, 128, False, 64, 1), (2, 2047, 2, 2, 64, True, 64, 1), (1, 9000, 1, 1, 128, True, 64, 1),      # one head a key head: any number of keys
+    (1, 2015, 8, 2, 128, False, 63, 1), (1, 2016, 8, 2, 128, False, 64, 2),      # 63 splits say that there are at most 2016 keys, 64 say nothing
+    (8, 100, 16, 8, 128, False, 4, 1), (8, 100, 9, 9, 128, False, 4, 2), (4, 70, 8, 8, 64, False, 3, 1), (3, 70, 11, 11, 64, False, 3, 2),      # clusters of the variants with two CTAs an SM
+    (3, 33, 10, 5, 128, True, 1, 1), (4, 28, 8, 4, 128, True, 1, 1), (8, 500, 16, 4, 128, True, 63, 1), (4, 500, 8, 8, 128, True, 16, 1), (4, 530, 8, 8, 128, True, 17, 2), (3, 60, 11, 11, 128, True, 2, 2)])      # and of the others
+def test_which_calls_take_a_cluster(M, pos, H, G, D, f32, splits, launches):
+    from qwen3_tts_cuda_graphs_b200 import codec as K
+
+    lib, dt = K.load_lib(), torch.float32 if f32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(pos + H)
+    rows, kc, vc = torch.randn(M, H * D, device="cuda", generator=g), *(torch.randn(pos + M, G * D, device="cuda", generator=g).to(dt) for _ in range(2))
+    out, ws, where = torch.zeros(M, H * D, device="cuda"), torch.zeros(M * H * splits * (D + 2), device="cuda"), torch.tensor([pos], device="cuda", dtype=torch.int32)
+    a = K.Op()
+    a.kind, a.M, a.N, a.i0, a.i1, a.i2, a.cin, a.f0, a.lda, a.ldr, a.taps, a.ldc, a.flags = K.K_CACHE_ATTN, M, H * D, H, G, D, D, D ** -0.5, H * D, G * D, G * D, H * D, (K.F_F32 if f32 else 0) | K.F_OUT_F32
+    a.A, a.B, a.p1, a.p0, a.C, a.ws, a.ws_bytes, a.m_begin = rows.data_ptr(), kc.data_ptr(), vc.data_ptr(), where.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel() * 4, splits
+    before = lib.fq3c_launch_count()
+    assert lib.fq3c_run((K.Op * 1)(a), 1, torch.cuda.current_stream().cuda_stream) == 0, lib.fq3c_last_error()
+    assert lib.fq3c_launch_count() - before == launches
+    see = torch.arange(pos + M, device="cuda")[None] <= torch.arange(pos, pos + M, device="cuda")[:, None]
+    for h in range(H):
+        n = h // (H // G)
+        s = (rows[:, h * D:(h + 1) * D].double() @ kc[:, n * D:(n + 1) * D].double().T * D ** -0.5).masked_fill(~see, -torch.inf)
+        p, v = s.softmax(-1), vc[:, n * D:(n + 1) * D].double()
+        # every entry: scores of about 1 from D products in 32 bits (some 1e-6 of them), so each weight is off by that, an exponential and a rounding or two, and their sum as well
+        assert ((out[:, h * D:(h + 1) * D].double() - p @ v).abs() <= 1e-5 * (p @ v.abs())).all()
+        assert (out[:, h * D:(h + 1) * D].double() - p @ v).norm() <= 2e-6 * (p @ v).norm()
