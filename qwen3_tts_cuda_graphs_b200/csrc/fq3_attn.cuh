@@ -10,7 +10,7 @@ struct AttnArgs {
   long ldq, ldk, ldv;
   int H, G, M;
   int groups;               // row groups per CTA: 1 or 2
-  int ends;                 // 1: a CTA's two groups are one from the end of the rows and one from their beginning, else they are neighbours
+  int ends;                 // 1: a CTA's two groups are one from the end of the rows and one from their beginning (the ENDS variant), else they are neighbours
   int two_from;             // > 0: launched with one, but behind more positions than these a CTA takes two and every other one leaves
   const int* p0;            // position of query 0 (device), or null: 0
   float scale, cap, mult;   // mult != 0 multiplies the output
@@ -149,7 +149,9 @@ __device__ __noinline__ void at_row_again(const AttnArgs& a, const int m, const 
 // rest) and, with a cap, by the special-function unit (three a score).
 // Without a wave's worth of row groups a CTA has one, so that no group waits for the other's issue slots; one group's next scores are issued in front of its values.
 // A tile takes one group some 3.7 us with a cap, two 6.0.  Norm and attention of 85 prompt rows of 16 heads over 8 10.9 us, 144 13.3, 262 17.0.
-template <int MODE>
+// ENDS: two groups may be from either end of the rows (a variant of its own: a second group that is not behind the first costs the tiles' loop registers, 0.8 us of 12.6 for 200 prompt rows
+// of 16 heads over 8).
+template <int MODE, bool ENDS>
 __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __grid_constant__ AttnArgs a) {
   extern __shared__ unsigned char at_raw[];
   const uint32_t raw = smem_u32(at_raw), base = (raw + 1023u) & ~1023u;
@@ -196,17 +198,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
   const bool one = groups == 1;      // its tiles take the score columns of both groups in turn
   // the last queries (most keys) start first
   int m0 = (gx - 1 - (int)blockIdx.x) * groups * QB, m1 = m0 + QB;      // each group's first query
-  if (a.ends && !one) {
+  if (ENDS && !one) {
     const int late = (a.M + QB - 1) / QB - 1 - (int)blockIdx.x;
     m0 = late * QB;
     m1 = (int)blockIdx.x < late ? (int)blockIdx.x * QB : a.M;
   }
+  auto row0 = [&](const int g) { return ENDS ? (g ? m1 : m0) : m0 + g * QB; };
   const int P = a.p0 ? *a.p0 : 0;
   int nq[2], first[2], last[2], tiles[2], tlo[2];                 // per group: live queries, their positions, tiles up to the last, first tile of window or chunk
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
-    nq[g] = g < groups ? max(0, min(QB, a.M - (g ? m1 : m0))) : 0;
-    first[g] = P + (g ? m1 : m0);
+    nq[g] = g < groups ? max(0, min(QB, a.M - row0(g))) : 0;
+    first[g] = P + row0(g);
     last[g] = first[g] + nq[g] - 1;
     tiles[g] = nq[g] > 0 ? last[g] / AT_KEYS + 1 : 0;
     int lo = a.window > 0 ? max(0, first[g] - a.window + 1) : 0;
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     tlo[g] = lo / AT_KEYS;
   }
   const int tkeep = a.window > 0 && a.chunk <= 0 ? (a.keep + AT_KEYS - 1) / AT_KEYS : 0;
-  const int ntiles = max(tiles[0], tiles[1]), jend = nq[1] > 0 ? max(last[0], last[1]) : last[0];
+  const int ntiles = max(tiles[0], tiles[1]), jend = ENDS ? (nq[1] > 0 ? max(last[0], last[1]) : last[0]) : P + min(a.M, m0 + groups * QB) - 1;
   auto need = [&](const int g, const int t) { return t < tiles[g] && (t >= tlo[g] || t < tkeep); };
 
   if (warp == 19) {
@@ -373,7 +376,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
           for (int i = 0; i < 8; ++i) {
             const int r = (half * 4 + wq) * 16 + b + i, qi = min(r / HG, nqg - 1), hh = min(r - qi * HG, HG - 1);
             x[i] = *reinterpret_cast<const Quad*>(reinterpret_cast<const typename std::conditional<MODE == AT_PROMPT, bf16, float>::type*>(a.q) +
-                                                  (size_t)(firstg - P + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
+                                                  (size_t)(row0(g) + qi) * a.ldq + (size_t)(kvh * HG + hh) * 128 + lane * 4);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -582,7 +585,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) fq3c_attn_tc_kernel(const __gri
     }
     const int n = (nq[0] + nq[1]) * HG * 128;
     for (int i = tid; i < n; i += AT_THREADS) {
-      const int q = i / (HG * 128), m = q < nq[0] ? m0 + q : m1 + q - nq[0];
+      const int q = i / (HG * 128), m = ENDS && q >= nq[0] ? m1 + q - nq[0] : m0 + q;
       const size_t at = (size_t)m * a.ldo + (size_t)kvh * HG * 128 + i % (HG * 128);
       if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = __int_as_float(0x7fffffff);
       else reinterpret_cast<uint16_t*>(a.out)[at] = 0x7fff;

@@ -1618,11 +1618,10 @@ bool attn_attrs_ready() {
   static bool done[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  auto room = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess; };
   if (!done[dev])
-    done[dev] = cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_PROMPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
-                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
-                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess &&
-                cudaFuncSetAttribute(fq3c_attn_tc_kernel<AT_DIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) == cudaSuccess;
+    done[dev] = room(fq3c_attn_tc_kernel<AT_PROMPT, false>) && room(fq3c_attn_tc_kernel<AT_PROMPT, true>) && room(fq3c_attn_tc_kernel<AT_PLAIN, false>) &&
+                room(fq3c_attn_tc_kernel<AT_PLAIN, true>) && room(fq3c_attn_tc_kernel<AT_CAP, false>) && room(fq3c_attn_tc_kernel<AT_CAP, true>) && room(fq3c_attn_tc_kernel<AT_DIST, false>);
   return done[dev];
 }
 // What the kernel's 8- and 16-byte accesses ask for.
@@ -1651,10 +1650,14 @@ void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after
   }
   const int per = a.groups * group;
   const dim3 grid((a.M + per - 1) / per, a.G);
-  if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
-  else if (mode == AT_PLAIN) launch_after(fq3c_attn_tc_kernel<AT_PLAIN>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
-  else if (mode == AT_CAP) launch_after(fq3c_attn_tc_kernel<AT_CAP>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
-  else launch_after(fq3c_attn_tc_kernel<AT_DIST>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  const bool ends = a.ends && (a.groups == 2 || a.two_from > 0);
+  if (mode == AT_PROMPT && ends) launch_after(fq3c_attn_tc_kernel<AT_PROMPT, true>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_PROMPT) launch_after(fq3c_attn_tc_kernel<AT_PROMPT, false>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_PLAIN && ends) launch_after(fq3c_attn_tc_kernel<AT_PLAIN, true>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_PLAIN) launch_after(fq3c_attn_tc_kernel<AT_PLAIN, false>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_CAP && ends) launch_after(fq3c_attn_tc_kernel<AT_CAP, true>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else if (mode == AT_CAP) launch_after(fq3c_attn_tc_kernel<AT_CAP, false>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
+  else launch_after(fq3c_attn_tc_kernel<AT_DIST, false>, grid, AT_THREADS, AT_SMEM, s, after, 1, a);
 }
 
 // FQ3C_ATTN_PREFILL=0: no kernel of its own for a prompt's attention (flags bit 0), nor one launch with the norm in front: the op by itself, as any other
