@@ -31,16 +31,17 @@ std::atomic<int64_t> g_launches{0};
 thread_local int64_t t_launches = 0;
 inline void count_launches(int64_t n) { g_launches += n; t_launches += n; }
 
-// Programmatic dependent launch: a kernel that the host launches with launch_after lets the next launch begin as soon as all its blocks run, and waits
-// itself for the end of everything in front of it before it touches memory.  Without the launch attribute both return at once.
+// Programmatic dependent launch: a kernel that the host launches with launch_after may begin before the ones in front of it have ended.  It waits for their end itself before it touches
+// memory (but for weights that no op of the list writes, and its own arguments), and says when the next launch may come up.  Without the launch attribute both return at once.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // One launch ahead: with the next one let in before this wait, launches pile up on the SMs (28 layers of a prompt of 39 rows 1128 us, this way 1118; a codec window 717 and 705).
-// Not behind many rows, whose launches take longer than those behind them need to come up (four layers of 1000 rows 413 and 416).
-__device__ __forceinline__ void grid_dep_begin(const int rows = 0) {
-  if (rows > 512) grid_dep_launch();
+// ahead: the next one at once.  For many rows, whose launches take longer than those behind them need to come up (four layers of 1000 rows 413 and 416), and for the norm of wide rows, in
+// front of a product whose weights are worth asking for early (six layers of 17 rows, 2048 wide, 373 us at once, 391 behind the wait; 1024 wide 24 - 80 rows are 0.5 - 3 % faster behind it).
+__device__ __forceinline__ void grid_dep_begin(const bool ahead = false) {
+  if (ahead) grid_dep_launch();
   grid_dep_wait();
-  if (rows <= 512) grid_dep_launch();
+  if (!ahead) grid_dep_launch();
 }
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -679,7 +680,7 @@ bool norm_vec_ok(const void* x, const void* y, const void* w, const int N, const
 constexpr int RN_WARPS = 4;
 __global__ void __launch_bounds__(RN_WARPS * 32) fq3c_rownorm_vec_kernel(const bf16* x, const int ldx, bf16* y, const int ldy, const float* w, const float eps, const int row0, const int rows,
                                                                          const int N) {
-  grid_dep_begin(rows);
+  grid_dep_begin(rows > 512 || N > 1024);
   const int row = blockIdx.x * RN_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(row0 + row) * ldx);
@@ -1020,7 +1021,7 @@ __global__ void __launch_bounds__(APF_WARPS * 32) fq3c_attn_prefill_kernel(const
 //   k / v heads: the finished row is also written to the static KV cache C (K) / C2 (V), laid out [kv_head][ldc][128].
 // Same arithmetic as head_norm_rope / the KV append of the decode kernel (fq3_kernel.cuh), so decode steps can attend to it.
 __global__ void fq3c_qknorm_rope_kv_kernel(const fq3c_op o) {
-  grid_dep_begin(o.M);
+  grid_dep_begin(o.M > 512);
   const int nq = o.i0, nkv = o.i1, pos0 = o.i2, nheads = nq + 2 * nkv;
   const int wpb = blockDim.x >> 5;
   const int gw = blockIdx.x * wpb + (threadIdx.x >> 5), lane = threadIdx.x & 31;
