@@ -1633,20 +1633,24 @@ bool attn_tc_takes(const AttnArgs& a, const int mode) {
 }
 void launch_attn_tc(AttnArgs a, const int mode, cudaStream_t s, const bool after) {
   const int group = 128 / (a.H / a.G);
-  const long ctas = (long)((a.M + group - 1) / group) * a.G;      // of one group each
+  const int rows_of = (a.M + group - 1) / group;      // row groups of a key head
+  const long ctas = (long)rows_of * a.G;      // of one group each
   a.groups = ctas <= GP_SMS ? 1 : 2;
   a.two_from = a.ends = 0;
   // Up to twice as many row groups as SMs, and no window: a CTA's two groups are one from the end of the rows and one from their beginning, whose few tiles are among the other's, so
   // that no CTA has two of the longest (and the last one alone in the end).  Neighbours, ends (us of a layer, 16 heads over 4): 2048 rows with a cap 112 and 102, without 101 and 92,
   // 1700 behind 300 98 and 90; two layers of the talker (16 over 8), 1900 rows 366 and 354, 1500 318 and 307.  Under a window the neighbours share their tiles: 2048 rows of 256 63 and 69.
-  // Of few more groups than SMs one to a CTA is faster still, the short ones go in behind the others: one, ends: 1300 rows (164 groups) 66 and 71, with a cap 69 and 79, 1500 (188) 75
-  // and 75, with a cap 80 and 83, 1700 (213) 90 and 83, 96 and 94; the talker's 1200 rows (152) 261 and 274, 1350 (169) 297 and 293.  Behind many positions all groups are long: with
-  // two_from the kernel then takes two (1500 behind 500, cap: 102 and 98; 1300 behind 700 86 and 88).
+  // Of few more groups than SMs one to a CTA is faster still, as long as those that come last are short: blocks come up a key head behind the other, the longest group of each first, so
+  // the last ones are the last key head's shortest, up to nine tenths of its groups (attention alone, one and ends, us: 1300 rows of 16 heads over 4, 16 groups over of a key head's 41, 36
+  // and 42, with a cap 39 and 46; 1500, 40 of 47, 45 and 48; 1300 of 16 over 8, 20 of 21, 45 and 45; 1300 of 16 over 16, 28 of 11, 48 and 40).  Behind many positions all groups are long,
+  // and the more so the more are over: with two_from the kernel then takes two (1300 of 16 over 4 behind 650 55 and 59, with a cap 61 and 69; of 16 over 8 73 and 62).  Over 170 sizes of
+  // 15 head layouts at five positions each that is within 1 % of the better of the two on the average.
   if (a.groups == 2 && a.window <= 0 && a.chunk <= 0 && mode != AT_DIST && (ctas + 1) / 2 <= GP_SMS) {
+    const long over = 10 * (ctas - GP_SMS);
     a.ends = 1;
-    if (ctas <= (mode == AT_PROMPT ? 160 : mode == AT_CAP ? 200 : 188)) {
+    if (over <= 9L * rows_of) {
       a.groups = 1;
-      if (a.p0) a.two_from = ctas <= 176 ? a.M / 4 * 3 : a.M / 4;
+      if (a.p0) a.two_from = over <= 3L * rows_of ? a.M / 4 * 3 : mode == AT_CAP && over <= 7L * rows_of ? a.M / 2 : a.M / 4;
     }
   }
   const int per = a.groups * group;
