@@ -294,7 +294,7 @@ int fq3c_run(const fq3c_op* ops, int n_ops, void* stream);
 /* How a GEMM op would be launched on the persistent tcgen05 kernel (host arithmetic only): out[0] = 0 one CTA per SM with sixteen epilogue warps, 1 one with eight, 2 two with
  * eight each; out[1..7] = columns of a tile, row tiles, column tiles, parts that a tile's sums come in, CTAs that share a tile, stages, CTAs.  Ops of other kernels: an error. */
 int fq3c_gemm_plan(const fq3c_op* op, int32_t* out);
-/* dst[0 .. n) on the device = values[0 .. n), in order on `stream` and without waiting for it; the values are read before the call returns (a launch per 1000 of them) */
+/* ABI 12: dst[0 .. n) on the device = values[0 .. n), in order on `stream` and without waiting for it; the values are read before the call returns (a launch per 1000 of them) */
 int fq3c_put_ints(const int32_t* values, int n, int32_t* dst, void* stream);
 /* number of kernel launches issued so far by this process through fq3c_run / fq3c_graph_launch */
 int64_t fq3c_launch_count(void);

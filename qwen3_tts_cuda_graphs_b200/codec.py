@@ -144,6 +144,8 @@ def load_lib():
         raise CodecError(f"{path} is missing: run `python -m qwen3_tts_cuda_graphs_b200.build` (there is no CPU fallback)")
     lib = C.CDLL(path)
     lib.fq3c_abi_version.restype = C.c_int
+    if lib.fq3c_abi_version() != 12:      # (in front of everything that another version may not have)
+        raise CodecError("libfq3codec.so ABI version mismatch")
     lib.fq3c_last_error.restype = C.c_char_p
     lib.fq3c_run.restype = C.c_int
     lib.fq3c_run.argtypes = [C.POINTER(Op), C.c_int, C.c_void_p]
@@ -158,8 +160,6 @@ def load_lib():
     lib.fq3c_graph_launch.argtypes = [C.c_void_p, C.c_void_p]
     lib.fq3c_graph_destroy.restype = C.c_int
     lib.fq3c_graph_destroy.argtypes = [C.c_void_p]
-    if lib.fq3c_abi_version() != 11:
-        raise CodecError("libfq3codec.so ABI version mismatch")
     _lib = lib
     return lib
 
@@ -298,7 +298,8 @@ def run_op_plan(lib, plan: _Plan, use_graphs: bool = True):
 def put_ints(lib, values, dst: torch.Tensor) -> None:
     """dst (int32 on the device, contiguous) = values, in order on the current stream and without waiting for it; `values` may change at once."""
     v = torch.as_tensor(list(values), dtype=torch.int32).cpu()
-    assert dst.dtype == torch.int32 and dst.is_contiguous() and dst.shape == v.shape
+    if dst.dtype != torch.int32 or not dst.is_contiguous() or dst.shape != v.shape:
+        raise ValueError("put_ints: a contiguous int32 tensor of as many entries as values")
     if lib.fq3c_put_ints(v.data_ptr(), v.numel(), dst.data_ptr(), torch.cuda.current_stream().cuda_stream) != 0:
         raise CodecError(lib.fq3c_last_error().decode())
 

@@ -2524,7 +2524,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
 
 extern "C" {
 
-int fq3c_abi_version(void) { return 11; }
+int fq3c_abi_version(void) { return 12; }
 const char* fq3c_last_error(void) { return g_err.c_str(); }
 int64_t fq3c_launch_count(void) { return g_launches.load(); }
 int fq3c_wait_errors(void) {

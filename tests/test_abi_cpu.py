@@ -100,3 +100,34 @@ def test_ctypes_struct_layouts_match_the_headers(tmp_path):
         assert ctypes.sizeof(ctype) == got[cname].pop("size"), cname
         mirror = {n: getattr(ctype, n).offset for n, *_ in ctype._fields_}
         assert list(mirror.values()) == list(got[cname].values()), (cname, mirror, got[cname])
+
+
+def test_another_version_of_the_codec_library_is_refused(monkeypatch):
+    """With the message meant for it, also where it lacks functions of this version."""
+    from qwen3_tts_cuda_graphs_b200 import codec
+
+    class Version:
+        restype = None
+
+        def __call__(self):
+            return 11
+
+    class Older:
+        fq3c_abi_version = Version()
+
+    monkeypatch.setattr(codec, "_lib", None)
+    monkeypatch.setattr(codec._build, "lib_path", lambda name: __file__)
+    monkeypatch.setattr(codec._build, "is_stale", lambda name: False)
+    monkeypatch.setattr(codec.C, "CDLL", lambda path: Older())
+    with pytest.raises(codec.CodecError, match="ABI version"):
+        codec.load_lib()
+
+
+def test_put_ints_refuses_other_destinations():
+    import torch
+
+    from qwen3_tts_cuda_graphs_b200 import codec
+
+    for dst in (torch.zeros(3, dtype=torch.int64), torch.zeros(2, dtype=torch.int32), torch.zeros(6, dtype=torch.int32)[::2]):
+        with pytest.raises(ValueError):
+            codec.put_ints(None, [1, 2, 3], dst)
