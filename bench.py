@@ -234,8 +234,7 @@ def kernel_source_hash() -> str:
 
 
 def ncu_traffic(frames_per_launch):
-    """DRAM bytes per launch of the decode kernel from the committed `ncu --set full` capture (profiles/ncu_traffic.json,
-    written by scripts/evidence.sh).  Returned only if the capture was taken from THIS kernel source (kernel_hash) and launch
+    """DRAM bytes per launch of the decode kernel from the committed `ncu --set full` capture (profiles/ncu_traffic.json).  Returned only if the capture was taken from THIS kernel source (kernel_hash) and launch
     shape; otherwise (None, why) — a stale number is worse than none."""
     try:
         d = json.load(open(os.path.join(ROOT, "profiles", "ncu_traffic.json")))

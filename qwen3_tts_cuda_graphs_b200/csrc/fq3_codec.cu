@@ -1774,7 +1774,7 @@ int launch_seq_gemm(const SeqGemm& g, bool a_f32, bool b_f32, bool exact, int zc
       return 0;
     }
   }
-  // bf16 rows of whole 16-byte pieces (what its copies ask for): the pipelined product, faster at every size (figures at the kernel)
+  // bf16 rows of whole 16-byte pieces (what its copies ask for), where the tcgen05 kernel has not taken them: experts with sums of 8 - 56, or weights that are not one behind the other
   if (!a_f32 && !b_f32 && !((g.K | g.lda | g.ldb | g.a_zstride) & 7) && !((g.b_zstride | g.b_estride) & 7) &&
       !((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15)) {
     static bool pattr[64] = {};
@@ -2196,7 +2196,7 @@ int seq_run(const fq3c_op& o, cudaStream_t s, bool after) {
     case FQ3C_ROT_APPEND: {
       if (!rot_append_ok(o)) return fail("rot_append: bad configuration");
       if (o.m_begin > 0 && (o.i1 < 1 || o.cin < 1 || !o.norm_out || !o.ws || !o.p0)) return fail("rot_append: pooled blocks need both caches, their pooled rows and a position");
-      // what the flat kernel holds: no norm, no temperature, no pooled rows; the value heads not among the queries that it turns in place
+      // what the flat kernel holds: no norm, no temperature, no pooled rows.  (Like the other one it turns queries in place while it reads keys and values: those lie in columns of their own.)
       if (o.M > 8 && o.m_begin <= 0 && !o.scale && !o.bias && !(o.flags & FQ3C_UNIT) && !(o.f3 > 0.f) && o.taps <= 4096) {
         const size_t smem = sizeof(float2) * (o.taps / 2);
         if (o.flags & FQ3C_F32) launch_seq(fq3s_rot_append_flat_kernel<float>, o.M, 256, smem, s, after, 1, o);
@@ -2630,7 +2630,7 @@ static int run_ops(const fq3c_op* ops, int n_ops, cudaStream_t main_stream, Side
   cudaStream_t s = main_stream;
   // The codec's kernels wait for the launches in front themselves and may begin early, as long as the launch in front on their stream belongs to this list
   // (what ran before the list is complete when its first launch begins): a prompt of 39 rows through 28 layers 1676 -> 1497 us, a codec window 1059 -> 972.
-  // The sequence models' own kernels do so with few rows alone (seq_dep_begin); their GEMMs always.
+  // The sequence models' own kernels, products of few rows among them, do so with one row alone (seq_early); their tcgen05 GEMMs always.
   bool chained = false;
   for (int i = 0; i < n_ops; ++i) {
     const fq3c_op& o = ops[i];

@@ -1763,13 +1763,6 @@ __global__ void __launch_bounds__(256) fq3s_pool_append_kernel(const fq3c_op o) 
   else pool_run<TC>(reinterpret_cast<const TC*>(o.C2), o.ldr, reinterpret_cast<TC*>(o.ws), b, P, c, min(n, c + 1), 1);
 }
 
-// grid (M), up to THREADS threads (256, or 1024 for a few rows), a warp per query / key head.  Angles in f32: position (exact as a float below 2^24) times the frequency,
-// full-range sincosf; cos and sin times the amplitude f1 when that is set.  With norm weights a head is first divided by its root
-// mean square (eps f0) and multiplied by them; with FQ3C_UNIT it is divided only (a rotation keeps the root mean square, so it does
-// not matter which comes first).  Queries in place, keys (read from `res` rows when given) into the cache.
-// m_begin = P > 0: every run of P positions bP .. bP + P - 1 that the step completes leaves the mean of its P cached keys and values as
-// row b of norm_out / ws.  A single row does it here (POOL; its block has just written the run's last row); more rows take
-// fq3s_pool_append_kernel behind this launch.
 // Sine and cosine by which pair i turns at position pos, times the amplitude.  freq, flo: the frequencies and what they lost to rounding (or null).
 __device__ __forceinline__ float2 rot_angle(const fq3c_op& o, const float* freq, const float* flo, const int i, const float fp) {
   float sn, cs;
@@ -1814,6 +1807,13 @@ __device__ __forceinline__ void rot_head(const fq3c_op& o, const float* freq, co
     put(c, v);
   }
 }
+// grid (M), up to THREADS threads (256, or 1024 for a few rows), a warp per query / key head.  Angles in f32: position (exact as a float below 2^24) times the frequency,
+// full-range sincosf; cos and sin times the amplitude f1 when that is set.  With norm weights a head is first divided by its root
+// mean square (eps f0) and multiplied by them; with FQ3C_UNIT it is divided only (a rotation keeps the root mean square, so it does
+// not matter which comes first).  Queries in place, keys (read from `res` rows when given) into the cache.
+// m_begin = P > 0: every run of P positions bP .. bP + P - 1 that the step completes leaves the mean of its P cached keys and values as
+// row b of norm_out / ws.  A single row does it here (POOL; its block has just written the run's last row); more rows take
+// fq3s_pool_append_kernel behind this launch.
 template <typename TC, bool POOL = false, int THREADS = 256>
 __global__ void __launch_bounds__(THREADS) fq3s_rot_append_kernel(const fq3c_op o) {
   seq_dep_begin(o.M);
