@@ -34,7 +34,7 @@ __device__ __forceinline__ void fg_store(const SeqGemm& g, const int r, const in
   else reinterpret_cast<bf16*>(g.C)[ci] = __float2bfloat16_rn(v);
 }
 template <int GROUPS>
-__global__ void __launch_bounds__(256) fq3s_gemm_f32_kernel(const SeqGemm g) {
+__global__ void __launch_bounds__(256, GROUPS > 1 ? 1 : 2) fq3s_gemm_f32_kernel(const SeqGemm g) {
   seq_dep_begin(g.M);
   extern __shared__ __align__(16) float fg[];
   float (*As)[FG_BM][FG_P] = reinterpret_cast<float (*)[FG_BM][FG_P]>(fg);
